@@ -1289,6 +1289,50 @@ def attention_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     return out
 
 
+def attention_f32_takes(dtype, n_heads: int, n_kv_heads: int, head_dim: int) -> bool:
+    """Whether `attention_f32` exists for these sizes (otherwise float32 goes to `attention_generic`)."""
+    return dtype == torch.float32 and bool(lib().rlis_attention_f32_takes(n_heads, n_kv_heads, head_dim))
+
+
+def attention_f32_pieces(max_ctx: int, window: int = 0) -> int:
+    """For how many pieces of a context `attention_f32` launches CTAs for single tokens: the most that a context of up to
+    `max_ctx` keys has, rounded up to a power of two, so that a recorded decode step serves while contexts double
+    (a CTA without a piece returns at once)."""
+    piece = lib().rlis_attention_f32_piece()
+    most = -(-max_ctx // piece)
+    if window:          # a window's first and last key lie in pieces of their own
+        most = min(most, -(-window // piece) + 1)
+    return 1 << (max(1, most) - 1).bit_length()
+
+
+def attention_f32(q, k_cache, v_cache, out, step, group: int, n_heads: int, n_kv_heads: int, head_dim: int, page_size: int,
+                  scale: float, window: int = 0) -> torch.Tensor:
+    """`attention` of the float32 path where `attention_f32_takes`: single tokens with their context cut into pieces, the
+    other tokens of the step a tile at a time; the same bits for a token either way."""
+    T = q.shape[0]
+    _req(q, "q", torch.float32, (T, n_heads * head_dim))
+    _req(out, "out", torch.float32, (T, n_heads * head_dim))
+    _req(k_cache, "k_cache", torch.float32, (None, n_kv_heads, page_size, head_dim))
+    _req(v_cache, "v_cache", torch.float32, (None, n_kv_heads, page_size, head_dim))
+    tables = step.block_tables[group]
+
+    def launch(rows, n_rows, partial, pieces):
+        check(lib().rlis_attention_f32(
+            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), partial.data_ptr() if partial is not None else None,
+            step.seq_of_token.data_ptr(), step.positions.data_ptr(), tables.data_ptr(), rows.data_ptr() if rows is not None else None,
+            tables.shape[1], n_rows, pieces, n_heads, n_kv_heads, head_dim, page_size, float(scale), int(window), _stream()),
+            "attention_f32")
+        _count("attention_f32.pieces" if partial is not None else "attention_f32")
+
+    if step.n_decode:
+        pieces = attention_f32_pieces(step.max_decode_ctx, window)
+        partial = step.buffer("attn_partial", (step.n_decode * n_heads * pieces * (head_dim + 2),), torch.float32)
+        launch(step.dec_rows, step.n_decode, partial, pieces)
+    if step.n_prefill_tokens:
+        launch(step.prefill_rows if step.n_decode else None, step.n_prefill_tokens, None, 1)
+    return out
+
+
 DECODE_MIN_KEYS_PER_SPLIT = 128
 
 
@@ -1480,8 +1524,10 @@ def attention(q, k_cache, v_cache, out, step, group: int, n_heads: int, n_kv_hea
               head_dim: int, page_size: int, scale: float, window: int = 0) -> torch.Tensor:
     """Attention of every token of the step over its request's cached keys, by the kernels that
     fit the step.  bfloat16: single decoded tokens go to the split decode kernel, portions of
-    prompts to the flash kernel (head sizes 64 and 128); everything else, and all of float32, to
-    the kernel for any query length.  The choice never changes the result beyond rounding."""
+    prompts to the flash kernel (head sizes 64 and 128).  float32: `attention_f32` for the sizes it takes.  Everything else
+    goes to the kernel for any query length.  The choice never changes the result beyond rounding."""
+    if attention_f32_takes(q.dtype, n_heads, n_kv_heads, head_dim):
+        return attention_f32(q, k_cache, v_cache, out, step, group, n_heads, n_kv_heads, head_dim, page_size, scale, window)
     tables = step.block_tables[group]
     bf = q.dtype == torch.bfloat16
     dec_fast = bf and step.n_decode > 0 and n_heads // n_kv_heads <= 8 and head_dim % 8 == 0

@@ -59,7 +59,11 @@ class GQAAttention(Mixer):
     def launch_variant(self, step):
         # decode attention cuts the context into pieces by the longest context of the step
         s = self.spec
-        return ops.decode_splits(step.n_decode, s.n_kv_heads, step.max_decode_ctx) if step.n_decode else None
+        if not step.n_decode:
+            return None
+        if ops.attention_f32_takes(self.dtype, s.n_heads, s.n_kv_heads, s.head_dim):
+            return ops.attention_f32_pieces(step.max_decode_ctx, self.window)
+        return ops.decode_splits(step.n_decode, s.n_kv_heads, step.max_decode_ctx)
 
     def fuses_norms(self, step) -> bool:
         s = self.spec

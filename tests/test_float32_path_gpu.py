@@ -51,3 +51,66 @@ def test_products_of_a_batch_read_and_write_slices_of_wider_rows(M, B, K, N, pad
     for b in range(B):
         assert torch.equal(out[:, b, :N], ops.gemm_f32(a[:, b, pad:].contiguous(), w[b].contiguous()))
     assert pad == 0 or bool((out[:, :, N:] == 7.0).all())
+
+
+class Step:
+    """The arrays of a step in which requests with `lens` cached tokens run their last `q_lens` tokens."""
+
+    def __init__(self, lens, q_lens, tables, single):
+        dev = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+        self.positions = torch.cat([torch.arange(n - m, n, dtype=torch.int32) for n, m in zip(lens, q_lens)]).cuda()
+        self.seq_of_token = torch.cat([torch.full((m,), b, dtype=torch.int32) for b, m in enumerate(q_lens)]).cuda()
+        self.block_tables = [tables.cuda()]
+        rows, dec, pf = 0, [], []
+        for m in q_lens:
+            (dec if single or m == 1 else pf).extend(range(rows, rows + m))
+            rows += m
+        self.n_decode, self.n_prefill_tokens = len(dec), len(pf)
+        self.dec_rows, self.prefill_rows = dev(dec), dev(pf) if dec else None
+        self.max_decode_ctx = max(lens)
+
+    def buffer(self, name, shape, dtype):
+        return torch.full(tuple(shape), float("nan"), dtype=dtype, device="cuda")
+
+
+@pytest.mark.parametrize("nh,nkv,d,page,window", [(32, 8, 64, 16, 0), (6, 2, 128, 16, 0), (8, 1, 16, 8, 0), (5, 5, 48, 4, 0), (10, 2, 80, 32, 0),
+                                                  (8, 2, 64, 16, 1), (8, 2, 64, 16, 33), (4, 2, 32, 16, 256), (3, 1, 64, 16, 400)])
+def test_float32_attention_gives_a_token_the_same_bits_however_the_step_is_cut(nh, nkv, d, page, window):
+    """Contexts around the edges of blocks (32) and pieces (256): against the kernel with a warp a head (the same up to the
+    order of the sums), and every token as one of a prompt against itself as a single token."""
+    from rust_llm_inference_server_b200 import ops
+    lens, q_lens = [1, 32, 33, 255, 256, 257, 513, 800], [1, 32, 1, 255, 70, 257, 1, 800]
+    g = torch.Generator().manual_seed(nh + window)
+    pages = -(-max(lens) // page)
+    tables = torch.randperm(len(lens) * pages, generator=g).to(torch.int32).view(len(lens), pages)
+    kc, vc = (torch.randn(len(lens) * pages, nkv, page, d, generator=g).cuda() for _ in range(2))
+    q = torch.randn(sum(q_lens), nh * d, generator=g).cuda()
+    assert ops.attention_f32_takes(q.dtype, nh, nkv, d)
+    args = (0, nh, nkv, d, page, 1 / math.sqrt(d), window)
+    mixed, single = (ops.attention(q, kc, vc, torch.full_like(q, 7.0), Step(lens, q_lens, tables, s), *args) for s in (False, True))
+    assert torch.equal(mixed, single)
+    st = Step(lens, q_lens, tables, False)
+    want = ops.attention_generic(q, kc, vc, torch.empty_like(q), st.seq_of_token, st.positions, st.block_tables[0], *args[1:])
+    # sums of at most 800 terms of weights that add up to one and values around one
+    assert (mixed - want).abs().max() <= 2e-5
+
+
+def test_float32_attention_shows_a_page_that_is_not_there():
+    from rust_llm_inference_server_b200 import ops
+    tables = torch.arange(20, dtype=torch.int32).view(1, 20)
+    tables[0, 17] = -1                      # keys 272 .. 287, in the second piece
+    kc, vc, q = torch.randn(20, 1, 16, 64).cuda(), torch.randn(20, 1, 16, 64).cuda(), torch.randn(300, 64).cuda()
+    for single in (False, True):
+        out = ops.attention(q, kc, vc, torch.zeros_like(q), Step([300], [300], tables, single), 0, 1, 1, 64, 16, 0.125, 0)
+        assert bool(torch.isfinite(out[:272]).all()) and bool(torch.isnan(out[272:]).all())
+
+
+def test_pieces_cover_every_context():
+    """Without a GPU's help: as many pieces as the longest context (or window) can touch, and a power of two."""
+    from rust_llm_inference_server_b200 import ops
+    piece = 256
+    for ctx in (1, 255, 256, 257, 512, 513, 4095, 4097):
+        for window in (0, 1, 255, 256, 257, 1000):
+            touched = max(p // piece - (max(0, p - window + 1) if window else 0) // piece + 1 for p in range(ctx))
+            n = ops.attention_f32_pieces(ctx, window)
+            assert n >= touched and n & (n - 1) == 0 and n < 2 * touched + 2
