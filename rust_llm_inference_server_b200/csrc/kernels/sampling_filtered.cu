@@ -23,9 +23,12 @@ namespace {
 constexpr int FT = 1024;
 typedef unsigned long long u64;
 
+// Every bit flipped below zero, the sign alone otherwise.  A NaN without a sign stands beside zero, so that it does not push a
+// token out of a top-k set (`u | 0x80000000` came to that by itself: the compiler takes it for -|f|, a canonical NaN).
 __device__ __forceinline__ uint32_t order_key(float f) {
     const uint32_t u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+    if (u - 0x7f800001u < 0x007fffffu) return 0x7fffffffu;
+    return u ^ ((uint32_t)((int)u >> 31) | 0x80000000u);
 }
 __device__ __forceinline__ u64 fixed_weight(float logit, float mx, float inv_t) {
     const float w = expf((logit - mx) * inv_t);           // in (0, 1]
@@ -248,12 +251,23 @@ __global__ __launch_bounds__(FT) void sample_filtered_kernel(const float* __rest
 int g_filtered_cluster = 1;      // 0: the one-CTA kernel for every vocabulary (tests of that kernel)
 
 // ------------------------------------------------------------------------------------------------
-// The same rule with a thread-block cluster per row.  One CTA reading a row of 128 k logits a dozen
-// times took 1.9 ms; here the row is read once: a cluster of CC CTAs of 512 threads holds it in
-// registers (thread t of CTA c: E consecutive token ids, so that CTA order and thread order are
-// vocabulary order), every pass works on registers, histograms and sums of the CTAs meet through
-// distributed shared memory, and every CTA draws the same conclusions from the same totals.  Same
-// integers, same token as the one-CTA kernel above, which stays for vocabularies too large for it.
+// The same rule with a thread-block cluster per row: CC CTAs of 512 threads hold the row's order keys in registers (thread
+// t of CTA c: E consecutive token ids, so that CTA order and thread order are vocabulary order), every pass
+// works on registers, histograms and sums of the CTAs meet through distributed shared memory, and every CTA draws the same
+// conclusions from the same totals.  Same integers, same token as the one-CTA kernel above, which stays for
+// vocabularies too large for it.
+//
+// A threshold is found by narrowing an interval of keys in histograms of 1,024 bins, counted from the top.  The first one
+// takes bins of 2^17 keys down from the row's highest key: 64 bins an octave of the logits' values over sixteen octaves,
+// so logits that crowd into a few octaves still spread over hundreds of bins (with 8 bits of the key a pass they met in half a dozen, and
+// the adds in shared memory queued up).  What lies further down is left out and only looked at if the threshold is
+// not above it.  The tokens of the bin that holds the threshold, a hundred or two, are then put in one list and
+// compared each with each; only where there are more than 256 (ties, above all) the bins narrow further, to 2^7 keys and to
+// one.  A top-k set of up to 256 goes to the list at once when top-p narrows it.  Masses are added as
+// three 32-bit numbers of 14, 14 and 13 bits of the weight: a CTA's 16,384 tokens cannot overflow them, and shared memory adds
+// 32 bits natively.  The first histogram of masses is filled in the pass that adds up the whole mass, and
+// weights are made again from the keys where they are needed, so that a thread stays within 64 registers and two CTAs
+// share an SM.  64 rows of 128,256 logits with top-p, top-k or both: 410 us with 8-bit passes, 103 us.
 constexpr int CT = 512;
 
 __device__ __forceinline__ u64 ld_dsmem_u64(const u64* local, uint32_t rank) {
@@ -276,81 +290,61 @@ __device__ __forceinline__ u64 cluster_total_u64(const u64* local, uint32_t cc) 
     for (uint32_t c = 0; c < cc; ++c) t += ld_dsmem_u64(local, c);
     return t;
 }
-__device__ __forceinline__ u64 cluster_total_u32(const uint32_t* local, uint32_t cc) {
-    u64 t = 0ull;
-    for (uint32_t c = 0; c < cc; ++c) t += ld_dsmem_u32(local, c);
-    return t;
-}
-
-// Three sums over the CTA at once.  `scratch`: 3 x (CT / 32 + 1) values.
-__device__ __forceinline__ void cta_sum3_u64(u64& a, u64& b, u64& c, u64 (*scratch)[CT / 32 + 1]) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
-        c += __shfl_xor_sync(0xffffffffu, c, o);
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) { scratch[0][warp] = a; scratch[1][warp] = b; scratch[2][warp] = c; }
-    __syncthreads();
-    if (warp < 3) {
-        u64 s = lane < CT / 32 ? scratch[warp][lane] : 0ull;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) scratch[warp][CT / 32] = s;
-    }
-    __syncthreads();
-    a = scratch[0][CT / 32]; b = scratch[1][CT / 32]; c = scratch[2][CT / 32];
-    __syncthreads();
-}
-
-// The radix step on 256 totals held one a thread (threads 0..255; `mine` is 0 elsewhere): the highest
-// bin b whose totals from the top reach `need` (`base` + sum of bins above b + bin b >= need; with
-// `nonempty`, bin b itself must hold something), and the sum of the bins above it.  Bin 0 if none.
-// A scan by one thread took 4 us a pass.
-__device__ __forceinline__ void pick_bin(u64 mine, u64 base, u64 need, bool nonempty, u64* warp_tot, int* best,
-                                         u64* above_out, uint32_t* bin_out) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    u64 incl = mine;                                   // sum of this warp's bins at or above this one
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const u64 n = __shfl_down_sync(0xffffffffu, incl, o);
-        if (lane + o < 32) incl += n;
-    }
-    if (tid < 256 && lane == 0) warp_tot[warp] = incl;
-    if (tid == 0) *best = 0;
-    __syncthreads();
-    u64 above = incl - mine;
-    if (tid < 256)
-        for (int w = warp + 1; w < 8; ++w) above += warp_tot[w];
-    if (tid < 256 && base + above + mine >= need && (!nonempty || mine > 0ull)) atomicMax(best, tid);
-    __syncthreads();
-    if (tid == *best) {
-        *above_out = base + above;
-        *bin_out = (uint32_t)tid;
-    }
-    __syncthreads();
-}
+constexpr int BINS = 1024, TOP_SHIFT = 17;
+constexpr uint32_t LIST = 256;       // tokens that are compared one with the other, a thread each (all pairs: 4 us; a level of bins takes 5)
 
 struct ClusterShared {
-    uint32_t hist_c[2][256];     // counts of a radix pass (two buffers: a pass is read by the others while the next is filled)
-    u64 hist_w[2][256];          // masses of a radix pass
-    u64 xch[16][3];              // a CTA's sums of a phase, read by the whole cluster
+    uint32_t hist[3][3][BINS];   // a level's counts, or its masses in three parts; three levels in turn: one is filled, the one before it
+                                 // may still be read by other CTAs, the one after it is emptied
+    u64 xch[8];                  // a CTA's sum of a phase, read by the whole cluster
     float xmax;
-    u64 scratch3[3][CT / 32 + 1];
+    uint32_t xkey, xnan;
+    float fmax_of[CT / 32];
+    uint32_t kmax_of[CT / 32];
     u64 scan[CT / 32];
-    uint32_t prefix;
-    u64 above;
-    u64 warp_tot[8];
     int best;
-    uint32_t bin;
+    u64 above, inside;
+    uint32_t n_list, best_key;
+    uint32_t list[LIST], all_keys[LIST];
+    u64 all_values[LIST];
 };
 
+__device__ __forceinline__ uint2 ld_dsmem_2u32(const uint32_t* local, uint32_t rank) {
+    uint32_t remote;
+    uint2 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(remote) : "memory");
+    return v;
+}
+
+// This thread's share of a sum over the CTA, inclusive of the threads before it in order, and the CTA's sum.
+__device__ __forceinline__ u64 cta_prefix_u64(u64 mine, u64* scan, u64& total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    u64 incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u64 n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += n;
+    }
+    if (lane == 31) scan[warp] = incl;
+    __syncthreads();
+    u64 before = 0ull;
+    total = 0ull;
+#pragma unroll
+    for (int i = 0; i < CT / 32; ++i) {
+        const u64 w = scan[i];
+        if (i < warp) before += w;
+        total += w;
+    }
+    __syncthreads();
+    return before + incl;
+}
+
 template <int E>
-__global__ __launch_bounds__(CT) void sample_filtered_cluster_kernel(const float* __restrict__ logits,
-                                                                     const uint32_t* __restrict__ params,
-                                                                     int* __restrict__ out, int vocab,
-                                                                     long long row_stride) {
+__global__ __launch_bounds__(CT, 2) void sample_filtered_cluster_kernel(const float* __restrict__ logits,
+                                                                        const uint32_t* __restrict__ params,
+                                                                        int* __restrict__ out, int vocab,
+                                                                        long long row_stride) {
     pdl_wait();
     __shared__ ClusterShared sh;
     const uint32_t rank = blockIdx.x, cc = gridDim.x;
@@ -363,184 +357,223 @@ __global__ __launch_bounds__(CT) void sample_filtered_cluster_kernel(const float
     const u64 u53 = (u64)params[5 * r + 3] | ((u64)params[5 * r + 4] << 32);
     const bool use_k = top_k > 0 && top_k < vocab;
     const bool use_p = top_p < 1.0f;
-    int phase = 0;                                   // which xch slot the next cluster-wide sum uses
 
-    // this thread's E consecutive tokens
+    // this thread's E consecutive tokens; those past the vocabulary take part in nothing
     const int v0 = ((int)rank * CT + tid) * E;
-    float lg[E];
+    const int n_mine = max(0, min(E, vocab - v0));
     uint32_t key[E];
-    bool rows16 = ((reinterpret_cast<uintptr_t>(row) & 15) == 0) && v0 + E <= vocab;
-    if (rows16) {
+    float mx = -INFINITY;
+    uint32_t top_key = 0u;
+    uint32_t nans = 0u;                              // which of them are NaN: their weight is what a NaN becomes as an integer
+    if (((reinterpret_cast<uintptr_t>(row) & 15) == 0) && n_mine == E) {
 #pragma unroll
         for (int i = 0; i < E; i += 4) {
             const float4 x = *reinterpret_cast<const float4*>(row + v0 + i);
-            lg[i] = x.x; lg[i + 1] = x.y; lg[i + 2] = x.z; lg[i + 3] = x.w;
+            mx = fmaxf(fmaxf(mx, fmaxf(x.x, x.y)), fmaxf(x.z, x.w));
+            key[i] = order_key(x.x); key[i + 1] = order_key(x.y); key[i + 2] = order_key(x.z); key[i + 3] = order_key(x.w);
+            nans |= ((x.x != x.x ? 1u : 0u) | (x.y != x.y ? 2u : 0u) | (x.z != x.z ? 4u : 0u) | (x.w != x.w ? 8u : 0u)) << i;
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < E; ++i) lg[i] = v0 + i < vocab ? row[v0 + i] : -INFINITY;
+        for (int i = 0; i < E; ++i) {
+            const float l = i < n_mine ? row[v0 + i] : -INFINITY;
+            mx = fmaxf(mx, l);
+            key[i] = i < n_mine ? order_key(l) : 0u;
+            nans |= l != l ? 1u << i : 0u;
+        }
     }
-    const int n_mine = max(0, min(E, vocab - v0));   // tokens past the vocabulary take part in nothing
-
-    // the row's maximum
-    float mx = -INFINITY;
 #pragma unroll
-    for (int i = 0; i < E; ++i) {
-        if (i < n_mine) mx = fmaxf(mx, lg[i]);
-        key[i] = order_key(lg[i]);
-    }
+    for (int i = 0; i < E; ++i) top_key = max(top_key, key[i]);
+
+    // the row's maximum, and its highest key (a NaN's, where there is one)
     mx = warp_max(mx);
-    float* fscr = reinterpret_cast<float*>(sh.scratch3[0]);
-    if (lane == 0) fscr[warp] = mx;
-    __syncthreads();
+    top_key = __reduce_max_sync(0xffffffffu, top_key);
+    if (lane == 0) { sh.fmax_of[warp] = mx; sh.kmax_of[warp] = top_key; }
+    for (int i = tid; i < 3 * BINS; i += CT) sh.hist[0][0][i] = 0u;
+    const bool cta_nan = __syncthreads_or(nans != 0u);
     if (tid == 0) {
-        float m = fscr[0];
-        for (int i = 1; i < CT / 32; ++i) m = fmaxf(m, fscr[i]);
-        sh.xmax = m;
+        sh.xnan = cta_nan ? 1u : 0u;
+        for (int i = 1; i < CT / 32; ++i) { mx = fmaxf(mx, sh.fmax_of[i]); top_key = max(top_key, sh.kmax_of[i]); }
+        sh.xmax = mx;
+        sh.xkey = top_key;
     }
     cluster_sync_all();
-    mx = -INFINITY;
-    for (uint32_t c = 0; c < cc; ++c) mx = fmaxf(mx, ld_dsmem(&sh.xmax, c));
-    // weights in float32, once; the fixed-point integer is made from them where needed
-    float wf[E];
-#pragma unroll
-    for (int i = 0; i < E; ++i) wf[i] = expf((lg[i] - mx) * inv_t);
-    auto fixed = [&](int i) -> u64 { return (u64)(wf[i] * 1099511627776.0f); };
+    uint32_t any_nan = 0u;
+    for (uint32_t c = 0; c < cc; ++c) {
+        mx = fmaxf(mx, ld_dsmem(&sh.xmax, c));
+        top_key = max(top_key, ld_dsmem_u32(&sh.xkey, c));
+        any_nan |= ld_dsmem_u32(&sh.xnan, c);
+    }
+    auto weight = [&](int i) -> u64 { return (nans >> i) & 1u ? 1ull << 63 : fixed_weight(key_value(key[i]), mx, inv_t); };
 
-    // sums of three numbers over the whole cluster, the same in every CTA
-    auto cluster_sums = [&](u64& a, u64& b, u64& c3) {
-        cta_sum3_u64(a, b, c3, sh.scratch3);
-        u64* slot = sh.xch[phase & 15];
-        ++phase;
-        if (tid == 0) { slot[0] = a; slot[1] = b; slot[2] = c3; }
-        cluster_sync_all();
-        a = cluster_total_u64(slot, cc);
-        b = cluster_total_u64(slot + 1, cc);
-        c3 = cluster_total_u64(slot + 2, cc);
-    };
-    // over the row: keys above `key0`, keys equal to it, mass of those above
-    auto key_stats = [&](uint32_t key0, u64& n_above, u64& n_ties, u64& mass_above) {
-        u64 a = 0ull, t = 0ull, m = 0ull;
+    int buf = 0, phase = 0;
+    // The highest key such that the counts (`masses` false) or masses of the keys from it upwards reach `need_of(sum)`, of the
+    // tokens whose key is at least `lower` (`sum`: the mass of all those above `lower`, 0 for counts).  `above`: what lies
+    // above it, `inside`: what equals it.  `known`: how many tokens there are at `lower` and above, if known.
+    auto select = [&](auto need_of, bool masses, uint32_t lower, u64 known, u64& above, u64& inside) -> uint32_t {
+        uint32_t hi = top_key, lo = lower;         // the threshold lies in lo .. hi
+        int shift = TOP_SHIFT;
+        u64 need = 0ull;
+        above = 0ull;
+        bool first = true;                         // `need` is not known yet
+        for (bool try_list = known <= LIST;;) {
+            if (try_list && !any_nan) {
+                // few tokens may be left: all of them in one list, where each is compared with each
+                if (tid == 0) sh.n_list = 0u;
+                __syncthreads();
 #pragma unroll
-        for (int i = 0; i < E; ++i) {
-            if (i < n_mine) {
-                if (key[i] > key0) { ++a; m += fixed(i); }
-                else if (key[i] == key0) ++t;
+                for (int i = 0; i < E; ++i) {
+                    if (key[i] >= lo && key[i] <= hi && i < n_mine) {
+                        const uint32_t at = atomicAdd(&sh.n_list, 1u);
+                        if (at < LIST) sh.list[at] = key[i];
+                    }
+                }
+                if (tid == 0) sh.best_key = 0u;
+                cluster_sync_all();
+                uint32_t n = 0u, mine = 0u;
+                for (uint32_t c = 0; c < cc; ++c) {
+                    const uint32_t nc = ld_dsmem_u32(&sh.n_list, c);
+                    if (n <= LIST && nc <= LIST && tid >= n && tid < n + nc) mine = ld_dsmem_u32(&sh.list[tid - n], c);
+                    n = min(n + nc, LIST + 1u);
+                }
+                if (n <= LIST) {
+                    const u64 v = tid < n ? (masses ? fixed_weight(key_value(mine), mx, inv_t) : 1ull) : 0ull;
+                    if (tid < n) { sh.all_keys[tid] = mine; sh.all_values[tid] = v; }
+                    __syncthreads();
+                    u64 higher = 0ull, equal = 0ull;
+                    for (uint32_t j = 0; j < (warp * 32 < (int)n ? n : 0u); ++j) {
+                        const uint32_t k = sh.all_keys[j];
+                        const u64 w = sh.all_values[j];
+                        if (k > mine) higher += w;
+                        if (k == mine) equal += w;
+                    }
+                    if (first) {
+                        u64 sum;
+                        cta_prefix_u64(mine > lower ? v : 0ull, sh.scan, sum);
+                        need = need_of(sum);
+                    }
+                    const bool here = tid < n && equal > 0ull && above + higher + equal >= need;
+                    if (here) atomicMax(&sh.best_key, mine);
+                    __syncthreads();
+                    const uint32_t best = sh.best_key;
+                    if (here && mine == best) { sh.above = above + higher; sh.inside = equal; }     // (the same of all that are equal)
+                    if (tid == 0 && best == 0u) sh.inside = 0ull;                                       // nothing reaches the need
+                    __syncthreads();
+                    if (best != 0u) above = sh.above;
+                    inside = sh.inside;
+                    cluster_sync_all();             // (the lists have been read before another one is made)
+                    return best != 0u ? best : lower;
+                }
+                cluster_sync_all();
             }
-        }
-        cluster_sums(a, t, m);
-        n_above = a; n_ties = t; mass_above = m;
-    };
-
-    int pass_no = 0;
-    // the key of the k-th highest logit, by radix search on counts
-    auto count_select = [&](u64 k_rem) -> uint32_t {
-        uint32_t prefix = 0u;
-        for (int pass = 0; pass < 4; ++pass, ++pass_no) {
-            const int shift = 24 - 8 * pass;
-            uint32_t* hist = sh.hist_c[pass_no & 1];
-            for (int i = tid; i < 256; i += CT) hist[i] = 0u;
-            __syncthreads();
-            // (logits of one row crowd into a few bins: the lanes of a warp that meet in a bin add up
-            // among themselves first, and one of them goes to shared memory)
+            uint32_t (*hist)[BINS] = sh.hist[buf];
+            u64 sum = 0ull;
 #pragma unroll
             for (int i = 0; i < E; ++i) {
-                const bool in = i < n_mine && (pass == 0 || (key[i] >> (shift + 8)) == (prefix >> (shift + 8)));
-                if (!__any_sync(0xffffffffu, in)) continue;
-                const uint32_t bin = in ? (key[i] >> shift) & 255u : 256u;
-                const uint32_t peers = __match_any_sync(0xffffffffu, bin);
-                if (in && lane == __ffs(peers) - 1) atomicAdd(&hist[bin], (uint32_t)__popc(peers));
+                const uint32_t bin = (hi - key[i]) >> shift;
+                const bool in = key[i] <= hi && key[i] >= lo && bin < BINS && i < n_mine;
+                if (!masses) {
+                    if (in) atomicAdd(&hist[0][bin], 1u);
+                } else if (in || (first && key[i] >= lower && i < n_mine)) {
+                    const u64 w = weight(i);
+                    if (in && w != 0ull) {
+                        atomicAdd(&hist[0][bin], (uint32_t)w & 0x3FFFu);
+                        atomicAdd(&hist[1][bin], (uint32_t)(w >> 14) & 0x3FFFu);
+                        atomicAdd(&hist[2][bin], (uint32_t)(w >> 28));
+                    }
+                    if (key[i] > lower || lower == 0u) sum += w;
+                }
             }
+            const int next = buf == 2 ? 0 : buf + 1;
+            for (int i = tid; i < 3 * BINS; i += CT) sh.hist[next][0][i] = 0u;      // (read last before the cluster barrier before this one)
+            if (masses && first) {
+                u64 own_sum;
+                cta_prefix_u64(sum, sh.scan, own_sum);
+                if (tid == 0) sh.xch[phase] = own_sum;
+            }
+            if (tid == 0) sh.best = BINS;
             cluster_sync_all();
-            const u64 tot = tid < 256 ? cluster_total_u32(&hist[tid], cc) : 0ull;
-            pick_bin(tot, 0ull, k_rem, false, sh.warp_tot, &sh.best, &sh.above, &sh.bin);
-            prefix |= sh.bin << shift;
-            k_rem -= sh.above;
+            // bins 2 tid and 2 tid + 1 of all CTAs
+            u64 t0 = 0ull, t1 = 0ull;
+            for (uint32_t c = 0; c < cc; ++c) {
+                const uint2 a = ld_dsmem_2u32(&hist[0][2 * tid], c);
+                t0 += a.x;
+                t1 += a.y;
+                if (masses) {
+                    const uint2 b = ld_dsmem_2u32(&hist[1][2 * tid], c), d = ld_dsmem_2u32(&hist[2][2 * tid], c);
+                    t0 += ((u64)b.x << 14) + ((u64)d.x << 28);
+                    t1 += ((u64)b.y << 14) + ((u64)d.y << 28);
+                }
+            }
+            if (first) {
+                need = need_of(masses ? cluster_total_u64(&sh.xch[phase], cc) : 0ull);
+                phase += masses ? 1 : 0;
+                first = false;
+            }
+            u64 all;
+            const u64 incl = above + cta_prefix_u64(t0 + t1, sh.scan, all);      // sum down to the second of this thread's bins
+            if (t0 > 0ull && incl - t1 >= need) atomicMin(&sh.best, 2 * tid);
+            else if (t1 > 0ull && incl >= need) atomicMin(&sh.best, 2 * tid + 1);
             __syncthreads();
+            const int best = sh.best;
+            if (best < BINS && tid == best >> 1) {
+                sh.above = (best & 1) ? incl - t1 : incl - t1 - t0;
+                sh.inside = (best & 1) ? t1 : t0;
+            }
+            __syncthreads();
+            buf = next;
+            if (best < BINS) {
+                above = sh.above;
+                hi -= (uint32_t)best << shift;
+                const uint32_t wide = (1u << shift) - 1u;
+                lo = max(lo, hi > wide ? hi - wide : 0u);
+                if (shift == 0) { inside = sh.inside; return hi; }
+                try_list = true;
+            } else {                                // further down than the bins reach (never within an interval narrowed before)
+                above += all;
+                const uint32_t covered = shift >= 22 ? 0xFFFFFFFFu : ((uint32_t)BINS << shift) - 1u;
+                if (hi - lo <= covered) { inside = 0ull; return lower; }      // nothing reaches the need
+                hi -= covered + 1u;
+                try_list = false;
+            }
+            shift = max(0, 22 - __clz(hi - lo | 1u));       // the next level's bins cover the interval
         }
-        return prefix;
     };
-    const uint32_t kth = use_k ? count_select((u64)top_k) : 0u;
-    u64 n_above_k, n_ties_k, mass_above_k;
-    key_stats(kth, n_above_k, n_ties_k, mass_above_k);
-    const u64 keep_k = use_k ? (u64)top_k - n_above_k : n_ties_k;
-    const u64 w_k = fixed_weight(key_value(kth), mx, inv_t);
-    const u64 mass = mass_above_k + keep_k * w_k;
 
-    // top-p: the largest threshold whose upper mass reaches top_p * mass
+    // the top-k set: everything above `kth` and the first `keep_k` (in token order) of the logits equal to it
+    uint32_t kth = 0u;
+    u64 n_above_k = 0ull, n_ties_k = 0ull, keep_k = ~0ull;
+    if (use_k) {
+        kth = select([&](u64) { return (u64)top_k; }, false, 0u, ~0ull, n_above_k, n_ties_k);
+        keep_k = (u64)top_k - n_above_k;
+    }
     uint32_t thr = kth;
-    u64 tie_keep = keep_k;
+    u64 tie_keep = keep_k, n_ties = use_k ? n_ties_k : 0ull;
     if (use_p) {
-        const u64 target = (u64)((double)top_p * (double)mass);
-        // Without a top-k the search over masses would put every token of the row into histograms
-        // of 64-bit sums.  Counting is cheaper: if the PRE highest logits already hold the target
-        // mass, the nucleus lies among them and only they take part (the result is the same:
-        // the threshold depends on the masses above it alone).
-        uint32_t lower = kth;
-        constexpr int PRE = 1024;
-        if (!use_k && vocab > 4 * PRE) {
-            const uint32_t kpre = count_select((u64)PRE);
-            u64 n_above, n_ties, mass_above;
-            key_stats(kpre, n_above, n_ties, mass_above);
-            if (mass_above + n_ties * fixed_weight(key_value(kpre), mx, inv_t) >= target) lower = kpre;
-        }
-        uint32_t prefix = 0u;
-        u64 above = 0ull;
-        for (int pass = 0; pass < 4; ++pass, ++pass_no) {
-            const int shift = 24 - 8 * pass;
-            u64* hist = sh.hist_w[pass_no & 1];
-            for (int i = tid; i < 256; i += CT) hist[i] = 0ull;
-            __syncthreads();
-#pragma unroll
-            for (int i = 0; i < E; ++i) {
-                const u64 w = fixed(i);
-                const bool in = i < n_mine && key[i] >= lower && w != 0ull &&
-                                (pass == 0 || (key[i] >> (shift + 8)) == (prefix >> (shift + 8)));
-                if (!__any_sync(0xffffffffu, in)) continue;
-                const uint32_t bin = in ? (key[i] >> shift) & 255u : 256u;
-                const uint32_t peers = __match_any_sync(0xffffffffu, bin);
-                // the weights (below 2^41) of the lanes that meet in a bin, added in two 32-bit halves
-                const uint32_t lo = __reduce_add_sync(peers, (uint32_t)(w & 0xFFFFFFull));
-                const uint32_t hi = __reduce_add_sync(peers, (uint32_t)(w >> 24));
-                if (in && lane == __ffs(peers) - 1) atomicAdd(&hist[bin], (u64)lo + ((u64)hi << 24));
-            }
-            cluster_sync_all();
-            const u64 tot = tid < 256 ? cluster_total_u64(&hist[tid], cc) : 0ull;
-            pick_bin(tot, above, target, true, sh.warp_tot, &sh.best, &sh.above, &sh.bin);
-            prefix |= sh.bin << shift;
-            above = sh.above;
-            __syncthreads();
-        }
-        thr = prefix > kth ? prefix : kth;
-        u64 n_above, n_ties, mass_above;
-        key_stats(thr, n_above, n_ties, mass_above);
+        // the largest threshold whose upper mass reaches top_p * mass
+        const u64 w_k = use_k ? fixed_weight(key_value(kth), mx, inv_t) : 0ull;
+        u64 target = 0ull, above, inside;
+        thr = select([&](u64 mass_above_k) {
+            const u64 mass = mass_above_k + (use_k ? keep_k * w_k : 0ull);
+            target = (u64)((double)top_p * (double)mass);
+            return target;
+        }, true, kth, use_k ? n_above_k + n_ties_k : ~0ull, above, inside);
         const u64 w_t = fixed_weight(key_value(thr), mx, inv_t);
+        n_ties = thr == kth && use_k ? n_ties_k : w_t > 0ull ? inside / w_t : 0ull;
         u64 need = 1ull;
-        if (target > mass_above && w_t > 0ull) need = (target - mass_above + w_t - 1ull) / w_t;
-        if (need < 1ull) need = 1ull;
-        const u64 room = thr == kth ? keep_k : n_ties;
+        if (target > above && w_t > 0ull) need = (target - above + w_t - 1ull) / w_t;
+        const u64 room = thr == kth && use_k ? keep_k : n_ties;
         tie_keep = need < room ? need : room;
     }
 
     // An exclusive prefix over the vocabulary order (CTA after CTA, thread after thread) of a value
     // per thread; also the cluster's total.
     auto ordered_prefix = [&](u64 mine, u64& total) -> u64 {
-        u64 incl = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const u64 n = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += n;
-        }
-        if (lane == 31) sh.scan[warp] = incl;
-        __syncthreads();
-        u64 before = incl - mine, cta_total = 0ull;
-        for (int i = 0; i < CT / 32; ++i) {
-            if (i < warp) before += sh.scan[i];
-            cta_total += sh.scan[i];
-        }
-        u64* slot = sh.xch[phase & 15];
+        u64 cta_total;
+        u64 before = cta_prefix_u64(mine, sh.scan, cta_total) - mine;
+        u64* slot = &sh.xch[phase];
         ++phase;
-        if (tid == 0) slot[0] = cta_total;
+        if (tid == 0) *slot = cta_total;
         cluster_sync_all();
         total = 0ull;
         for (uint32_t c = 0; c < cc; ++c) {
@@ -550,17 +583,21 @@ __global__ __launch_bounds__(CT) void sample_filtered_cluster_kernel(const float
         }
         return before;
     };
-    // rank of this thread's first tie among all logits equal to the threshold
-    u64 my_ties = 0ull;
+    // rank of this thread's first tie among all logits equal to the threshold (all of them kept: no matter)
+    u64 tie_rank = 0ull;
+    if (tie_keep < n_ties) {
+        u64 my_ties = 0ull, all_ties;
 #pragma unroll
-    for (int i = 0; i < E; ++i) my_ties += (i < n_mine && key[i] == thr) ? 1ull : 0ull;
-    u64 all_ties;
-    const u64 tie_rank = ordered_prefix(my_ties, all_ties);
+        for (int i = 0; i < E; ++i) my_ties += (i < n_mine && key[i] == thr) ? 1ull : 0ull;
+        tie_rank = ordered_prefix(my_ties, all_ties);
+    } else {
+        tie_keep = ~0ull;
+    }
     // kept mass of this thread's tokens
     u64 mine = 0ull, rk = tie_rank;
 #pragma unroll
     for (int i = 0; i < E; ++i)
-        if (i < n_mine && (key[i] > thr || (key[i] == thr && rk++ < tie_keep))) mine += fixed(i);
+        if (i < n_mine && (key[i] > thr || (key[i] == thr && rk++ < tie_keep))) mine += weight(i);
     u64 kept;
     const u64 before = ordered_prefix(mine, kept);
     const u64 target_r = __umul64hi(u53 << 11, kept);          // floor(u * kept), u = u53 / 2^53
@@ -570,7 +607,7 @@ __global__ __launch_bounds__(CT) void sample_filtered_cluster_kernel(const float
 #pragma unroll
         for (int i = 0; i < E; ++i) {
             if (i < n_mine && (key[i] > thr || (key[i] == thr && rk2++ < tie_keep))) {
-                cum += fixed(i);
+                cum += weight(i);
                 if (cum > target_r) { pick = v0 + i; break; }
             }
         }
