@@ -4,7 +4,7 @@
 // calls of its tensor library (crates/model/src/layers.rs:82,181-184); here it is a hand-written
 // sm_100a kernel so that SwiGLU never makes a round trip through HBM.
 //
-// One persistent CTA per SM walks over 128 x 256 tiles.  Six warps, by role:
+// One persistent CTA per SM walks over 128 x 256 tiles.  Ten warps, by role:
 //   warp 0, one lane: TMA producer.  Per k-block of 64 it asks for the 128 x 64 tile of x and the
 //           256 x 64 tile of W (cp.async.bulk.tensor, 128-byte swizzle) into a ring of 4 stages;
 //           an mbarrier per stage counts the bytes.
@@ -14,7 +14,7 @@
 //           tells the epilogue when the accumulator is complete.  The warp also owns the TMEM
 //           allocation: all 512 columns, two accumulators, so that a tile's epilogue overlaps the
 //           next tile's products.
-//   warps 2-5: epilogue.  Each reads its quarter of the accumulator's lanes with tcgen05.ld, 32
+//   warps 2-9: epilogue.  Each reads half the columns of its quarter of the accumulator's lanes with tcgen05.ld, 32
 //           columns at a time, and stores bf16 (or float32) rows, or silu(gate) * up for a gate|up
 //           matrix whose rows are interleaved in blocks of 4.
 // Rows and columns past M, N and K are zero-filled by TMA and never stored.
@@ -31,8 +31,10 @@ using namespace tc;
 constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4;
 constexpr int UMMA_K = 16;
 constexpr int A_STAGE_BYTES = BM * BK * 2, B_STAGE_BYTES = BN * BK * 2;
-constexpr int GT_THREADS = 192;
+constexpr int GT_THREADS = 320;
+constexpr int TURN_BYTES = 8 * 32 * 32 * 4;      // float32 rows: a block of 32 x 32 sums for each epilogue warp
 constexpr size_t GT_SMEM = (size_t)STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 1024 /* alignment */ + 256;
+constexpr size_t GT_SMEM_F32 = GT_SMEM + TURN_BYTES;
 
 struct Ctrl {
     uint64_t full[STAGES];
@@ -43,6 +45,7 @@ struct Ctrl {
     int abort;
 };
 
+static_assert(sizeof(Ctrl) <= 256, "the control block, and after it the blocks in which float32 rows turn");
 constexpr uint32_t IDESC = idesc_bf16(BM, BN);
 
 // EPI 0: bf16 y [M, N].  EPI 1: SwiGLU, y [M, N / 2] bf16.  EPI 2: float32 y [M, N].  EPI 3: the gated epilogue
@@ -86,7 +89,7 @@ __global__ __launch_bounds__(GT_THREADS) void gemm_tcgen05_kernel(const __grid_c
         }
         for (int i = 0; i < 2; ++i) {
             bar_init(&ctrl->acc_full[i], 1);
-            bar_init(&ctrl->acc_empty[i], 4);      // the four epilogue warps
+            bar_init(&ctrl->acc_empty[i], 8);      // the eight epilogue warps
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -145,8 +148,8 @@ __global__ __launch_bounds__(GT_THREADS) void gemm_tcgen05_kernel(const __grid_c
             }
         }
     } else {
-        // epilogue: warp w may touch TMEM lanes 32 * (w % 4) .. + 31
-        const int q = warp & 3;
+        // epilogue: warp w may touch TMEM lanes 32 * (w % 4) .. + 31; two warps share them, a half of the columns each
+        const int q = warp & 3, cb0 = (warp - 2) / 4 * (BN / 64);
         int t = 0;
         for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
             if (tile_expert != nullptr && tile_expert[tile % m_tiles] < 0) continue;
@@ -156,12 +159,33 @@ __global__ __launch_bounds__(GT_THREADS) void gemm_tcgen05_kernel(const __grid_c
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = m0 + q * 32 + lane;
             const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * BN) + ((uint32_t)(q * 32) << 16);
-            for (int cb = 0; cb < BN / 32; ++cb) {
+            for (int cb = cb0; cb < cb0 + BN / 64; ++cb) {
                 const int col = n0 + cb * 32;
                 const float bias = EPI == 3 ? bias_of_lane(gp, col, lane, N) : 0.f;
                 uint32_t r[32];
                 tmem_ld32(tmem_acc + (uint32_t)(cb * 32), r);
                 if (EPI == 3 && gp.bias != nullptr) add_bias32(r, bias);
+                if (EPI == 2) {
+                    // A lane holds 128 bytes of a row; stored as it is, an instruction wrote 16 bytes of 32 rows.  Turned
+                    // through shared memory (rows in 16-byte pieces, their places swapped by the row, so that neither
+                    // side meets in a bank) it writes the 128 bytes of 4 rows (84 MB of sums: 72 us, now
+                    // 56).
+                    float4* turn = reinterpret_cast<float4*>(base + (size_t)STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 256) + (warp - 2) * 256;
+                    __syncwarp();
+#pragma unroll
+                    for (int v = 0; v < 8; ++v)
+                        turn[lane * 8 + (v ^ (lane & 7))] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
+                                                                        __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
+                    __syncwarp();
+                    const int piece = lane & 7, at = col + piece * 4;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const int lr = j * 4 + (lane >> 3), gr = m0 + q * 32 + lr;
+                        if (ok && gr < M && at < N)
+                            *reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + (size_t)gr * N + at) = turn[lr * 8 + (piece ^ (lr & 7))];
+                    }
+                    continue;
+                }
                 if (!ok || row >= M || col >= N) continue;
                 store_sums32<EPI>(r, y, row, col, N, gp);
             }
@@ -208,7 +232,7 @@ static int gemm_tcgen05_impl(const void* x, const void* W, void* y, int M, int N
     if (!attr_done) {
         cudaFuncSetAttribute(gemm_tcgen05_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM);
         cudaFuncSetAttribute(gemm_tcgen05_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM);
-        cudaFuncSetAttribute(gemm_tcgen05_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM);
+        cudaFuncSetAttribute(gemm_tcgen05_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM_F32);
         cudaFuncSetAttribute(gemm_tcgen05_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM);
         attr_done = true;
     }
@@ -221,7 +245,7 @@ static int gemm_tcgen05_impl(const void* x, const void* W, void* y, int M, int N
     else if (epilogue == 1)
         rlis_launch(gemm_tcgen05_kernel<1>, grid, GT_THREADS, GT_SMEM, stream, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp, (const int*)nullptr, 0);
     else if (epilogue == 2)
-        rlis_launch(gemm_tcgen05_kernel<2>, grid, GT_THREADS, GT_SMEM, stream, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp, (const int*)nullptr, 0);
+        rlis_launch(gemm_tcgen05_kernel<2>, grid, GT_THREADS, GT_SMEM_F32, stream, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp, (const int*)nullptr, 0);
     else
         rlis_launch(gemm_tcgen05_kernel<3>, grid, GT_THREADS, GT_SMEM, stream, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp, (const int*)nullptr, 0);
     return RLIS_LAUNCH_CHECK();
@@ -246,7 +270,7 @@ extern "C" int rlis_gemm_tcgen05_grouped(const void* x, const void* W, void* y, 
     static bool attr_done = false;
     if (!attr_done) {
         cudaFuncSetAttribute(gemm_tcgen05_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM);
-        cudaFuncSetAttribute(gemm_tcgen05_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM);
+        cudaFuncSetAttribute(gemm_tcgen05_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM_F32);
         cudaFuncSetAttribute(gemm_tcgen05_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM);
         attr_done = true;
     }
@@ -259,7 +283,7 @@ extern "C" int rlis_gemm_tcgen05_grouped(const void* x, const void* W, void* y, 
         rlis_launch(gemm_tcgen05_kernel<0>, grid, GT_THREADS, GT_SMEM, stream, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp,
                     tile_expert, N);
     else if (epilogue == 2)
-        rlis_launch(gemm_tcgen05_kernel<2>, grid, GT_THREADS, GT_SMEM, stream, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp,
+        rlis_launch(gemm_tcgen05_kernel<2>, grid, GT_THREADS, GT_SMEM_F32, stream, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp,
                     tile_expert, N);
     else
         rlis_launch(gemm_tcgen05_kernel<3>, grid, GT_THREADS, GT_SMEM, stream, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp,

@@ -12,7 +12,7 @@
 // the bytes of both CTAs are counted by CTA 0's barrier of the stage, `cp.async.bulk.tensor` with
 // `.cta_group::2` and the barrier's address in the cluster's window); warp 1 of CTA 0 issues the
 // instructions, `tcgen05.commit` with a mask of both CTAs hands a stage back to both producers and
-// tells both epilogues when an accumulator is complete; warps 2-5 are the epilogue of their CTA's
+// tells both epilogues when an accumulator is complete; warps 2-9 are the epilogue of their CTA's
 // 128 rows (gemm_epilogue.cuh), and tell CTA 0 when they have read an accumulator.  Tensor memory:
 // both CTAs' warp 1 allocate all 512 columns together (two accumulators of 256), and free them
 // after the two CTAs have met at the end.
@@ -31,14 +31,14 @@ using namespace tc;
 constexpr int PM = 128;                 // rows of a CTA: the pair's tile is 2 PM x PN
 constexpr int PN = 256, PK = 64, P_STAGES = 6;
 constexpr int A_BYTES = PM * PK * 2, B_BYTES = (PN / 2) * PK * 2;       // 16 KB each a CTA and stage
-constexpr int GP_THREADS = 192;
+constexpr int GP_THREADS = 320;
 constexpr size_t GP_SMEM = (size_t)P_STAGES * (A_BYTES + B_BYTES) + 1024 /* alignment */ + 256;
 
 struct PairCtrl {
     uint64_t full[P_STAGES];        // CTA 0's: both CTAs' bytes of a stage have arrived
     uint64_t empty[P_STAGES];       // each CTA's: the products that read the stage are done
     uint64_t acc_full[2];           // each CTA's: an accumulator is complete
-    uint64_t acc_empty[2];          // CTA 0's: the eight epilogue warps of the pair have read it
+    uint64_t acc_empty[2];          // CTA 0's: the sixteen epilogue warps of the pair have read it
     uint32_t tmem_base;
     int abort;
 };
@@ -113,7 +113,7 @@ __global__ __launch_bounds__(GP_THREADS) void gemm_tcgen05_pair_kernel(const __g
         }
         for (int i = 0; i < 2; ++i) {
             bar_init(&ctrl->acc_full[i], 1);
-            bar_init(&ctrl->acc_empty[i], 8);      // the four epilogue warps of each CTA
+            bar_init(&ctrl->acc_empty[i], 16);     // the eight epilogue warps of each CTA
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -181,8 +181,8 @@ __global__ __launch_bounds__(GP_THREADS) void gemm_tcgen05_pair_kernel(const __g
             }
         }
     } else {
-        // epilogue: warp w may touch TMEM lanes 32 * (w % 4) .. + 31
-        const int q = warp & 3;
+        // epilogue: warp w may touch TMEM lanes 32 * (w % 4) .. + 31; two warps share them, a half of the columns each
+        const int q = warp & 3, cb0 = (warp - 2) / 4 * (PN / 64);
         int t = 0;
         for (int tile = pair; tile < num_tiles; tile += pairs, ++t) {
             const int buf = t & 1;
@@ -191,7 +191,7 @@ __global__ __launch_bounds__(GP_THREADS) void gemm_tcgen05_pair_kernel(const __g
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = m0 + q * 32 + lane;
             const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * PN) + ((uint32_t)(q * 32) << 16);
-            for (int cb = 0; cb < PN / 32; ++cb) {
+            for (int cb = cb0; cb < cb0 + PN / 64; ++cb) {
                 const int col = n0 + cb * 32;
                 const float bias = EPI == 3 ? bias_of_lane(gp, col, lane, N) : 0.f;
                 uint32_t r[32];
