@@ -41,11 +41,13 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// A CTA takes TOK tokens and has a warp for every row of W_r (up to 32 warps): a warp forms its row against
-// all of the CTA's tokens, so the matrix is read once a CTA (the tokens' rows come back from the first-level
-// cache) and the rows' sums run side by side; then one warp a token chooses.
-template <typename T, int TOK>
-__global__ __launch_bounds__(1024) void moe_route_kernel(
+// A CTA takes TOK tokens; a warp forms ROWS rows of W_r against all of the CTA's tokens, so the matrix is read once a CTA (the
+// tokens' rows come back from the first-level cache, once for ROWS rows) and the rows' sums run side by side; then
+// one warp a token chooses.  With 8 tokens the reads of the tokens' rows are the bound, so a warp takes four rows of W_r at
+// once, and two CTAs share an SM (2,048 tokens of 2,048, 32 experts and a shared gate: 57 us with a warp a row, whose 33rd
+// row was a second round, 44 with two rows a warp, 31 with four).
+template <typename T, int TOK, int ROWS>
+__global__ __launch_bounds__(TOK == 8 ? 512 : 1024) void moe_route_kernel(
     const T* __restrict__ x, const float* __restrict__ w_router, const float* __restrict__ correction,
     int* __restrict__ top_idx, float* __restrict__ top_w, float* __restrict__ shared_gate,
     int n_tokens, int width, int n_experts, int top, float route_scale,
@@ -57,41 +59,54 @@ __global__ __launch_bounds__(1024) void moe_route_kernel(
     const int t0 = blockIdx.x * TOK;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int n_rows = n_experts + (shared_gate != nullptr ? 1 : 0);
-    for (int e = warp; e < n_rows; e += nwarps) {
-        const float* w = w_router + (size_t)e * width;
-        float dot[TOK];
+    for (int e0 = warp * ROWS; e0 < n_rows; e0 += nwarps * ROWS) {
+        const float* w[ROWS];
+        float dot[ROWS][TOK];
 #pragma unroll
-        for (int i = 0; i < TOK; ++i) dot[i] = 0.f;
+        for (int j = 0; j < ROWS; ++j) {
+            w[j] = w_router + (size_t)min(e0 + j, n_rows - 1) * width;
+#pragma unroll
+            for (int i = 0; i < TOK; ++i) dot[j][i] = 0.f;
+        }
         if ((width & 3) == 0) {
             // four elements a lane and step (16-byte loads of the matrix, four of a token's row)
-#pragma unroll 4
+#pragma unroll 2
             for (int k = lane * 4; k < width; k += 128) {
-                const float4 wv = *reinterpret_cast<const float4*>(w + k);
+                float4 wv[ROWS];
+#pragma unroll
+                for (int j = 0; j < ROWS; ++j) wv[j] = *reinterpret_cast<const float4*>(w[j] + k);
 #pragma unroll
                 for (int i = 0; i < TOK; ++i) {
                     const int t = min(t0 + i, n_tokens - 1);
                     const float4 xv = load4(x + (size_t)t * width + k);
-                    dot[i] = fmaf(wv.x, xv.x, dot[i]);
-                    dot[i] = fmaf(wv.y, xv.y, dot[i]);
-                    dot[i] = fmaf(wv.z, xv.z, dot[i]);
-                    dot[i] = fmaf(wv.w, xv.w, dot[i]);
+#pragma unroll
+                    for (int j = 0; j < ROWS; ++j) {
+                        dot[j][i] = fmaf(wv[j].x, xv.x, dot[j][i]);
+                        dot[j][i] = fmaf(wv[j].y, xv.y, dot[j][i]);
+                        dot[j][i] = fmaf(wv[j].z, xv.z, dot[j][i]);
+                        dot[j][i] = fmaf(wv[j].w, xv.w, dot[j][i]);
+                    }
                 }
             }
         } else {
 #pragma unroll 4
             for (int k = lane; k < width; k += 32) {
-                const float wv = w[k];
 #pragma unroll
                 for (int i = 0; i < TOK; ++i) {
                     const int t = min(t0 + i, n_tokens - 1);
-                    dot[i] = fmaf(wv, to_f<T>(x[(size_t)t * width + k]), dot[i]);
+                    const float xv = to_f<T>(x[(size_t)t * width + k]);
+#pragma unroll
+                    for (int j = 0; j < ROWS; ++j) dot[j][i] = fmaf(w[j][k], xv, dot[j][i]);
                 }
             }
         }
 #pragma unroll
-        for (int i = 0; i < TOK; ++i) {
-            const float d = warp_sum(dot[i]);
-            if (lane == 0) sm[i * stride + e] = d;
+        for (int j = 0; j < ROWS; ++j) {
+#pragma unroll
+            for (int i = 0; i < TOK; ++i) {
+                const float d = warp_sum(dot[j][i]);
+                if (lane == 0 && e0 + j < n_rows) sm[i * stride + e0 + j] = d;
+            }
         }
     }
     __syncthreads();
@@ -190,41 +205,81 @@ __global__ __launch_bounds__(1024) void moe_route_kernel(
 // One CTA.  pairs = tokens * top.  sorted_pair [max_tiles * tile]: the pair in a slot or -1; pair_slot [pairs];
 // tile_expert [max_tiles + 1]: the expert of a tile of `tile` slots or -1 (no such tile: they are the last
 // ones), and after them the number of tiles that have one.
+// Bound by the latency of its passes over the pairs and by counters that many pairs want.  `copies` sets of counters, one for every
+// warp while they fit: a pair's count before it in its set is its place there, so that one pass of atomics
+// serves both the counting and the placing.  A thread keeps its first KEEP pairs in registers in between; the others'
+// places wait in pair_slot.  8,192 pairs on 32 experts: 39 us with one set, two passes and a scan by one
+// thread, 23 now (34 with the lanes that meet in an expert gathered by match_any).
 __global__ __launch_bounds__(1024) void moe_align_kernel(
     const int* __restrict__ top_idx, int* __restrict__ sorted_pair, int* __restrict__ pair_slot,
-    int* __restrict__ tile_expert, int n_pairs, int n_experts, int max_tiles, int tile_rows) {
+    int* __restrict__ tile_expert, int n_pairs, int n_experts, int max_tiles, int tile_rows, int copies) {
+    constexpr int KEEP = 8;
     pdl_wait_and_trigger();
     extern __shared__ int smi[];
-    int* count = smi;                    // [n_experts]
-    int* start = smi + n_experts;        // [n_experts]
-    for (int e = threadIdx.x; e < n_experts; e += blockDim.x) count[e] = 0;
-    for (int i = threadIdx.x; i < max_tiles * tile_rows; i += blockDim.x) sorted_pair[i] = -1;
+    int* total = smi;                    // [n_experts]: an expert's pairs, then its first slot
+    int* count = smi + n_experts;        // [copies][n_experts]: a set's pairs of an expert, then how many other sets' come before them
+    const int tid = threadIdx.x, lane = tid & 31, threads = blockDim.x;
+    int* mine = count + (tid >> 5) % copies * n_experts;
+    auto expert_of = [&](int i) {
+        const int e = i < n_pairs ? top_idx[i] : -1;
+        return e < n_experts ? e : -1;
+    };
+    int kept[KEEP], place[KEEP];
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) kept[j] = expert_of(tid + j * threads);
+    for (int e = tid; e < copies * n_experts; e += threads) count[e] = 0;
+    for (int i = tid; i < max_tiles * tile_rows; i += threads) sorted_pair[i] = -1;
+    for (int i = tid; i < max_tiles; i += threads) tile_expert[i] = -1;
     __syncthreads();
-    for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-        const int e = top_idx[i];
-        if (e >= 0 && e < n_experts) atomicAdd(&count[e], 1);
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) place[j] = kept[j] >= 0 ? atomicAdd(&mine[kept[j]], 1) : 0;
+    for (int i = tid + KEEP * threads; i < n_pairs; i += threads) {
+        const int e = expert_of(i);
+        pair_slot[i] = e >= 0 ? atomicAdd(&mine[e], 1) : 0;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int tile = 0;
-        for (int e = 0; e < n_experts; ++e) {
-            start[e] = tile * tile_rows;
-            const int tiles = (count[e] + tile_rows - 1) / tile_rows;
-            for (int i = 0; i < tiles && tile < max_tiles; ++i) tile_expert[tile++] = e;
-            count[e] = 0;                // from here on: the next free slot of the expert's run
+    for (int e = tid; e < n_experts; e += threads) {
+        int before = 0;
+        for (int c = 0; c < copies; ++c) {
+            const int n = count[c * n_experts + e];
+            count[c * n_experts + e] = before;
+            before += n;
         }
-        tile_expert[max_tiles] = tile;
-        for (; tile < max_tiles; ++tile) tile_expert[tile] = -1;
+        total[e] = before;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
-        const int e = top_idx[i];
-        if (e < 0 || e >= n_experts) { pair_slot[i] = -1; continue; }
-        const int slot = start[e] + atomicAdd(&count[e], 1);
-        if (slot >= max_tiles * tile_rows) { pair_slot[i] = -1; continue; }    // the host sizes max_tiles so that this never happens
-        sorted_pair[slot] = i;
-        pair_slot[i] = slot;
+    if (tid < 32) {
+        // where every expert's tiles start: 32 experts at a time
+        int tile = 0;
+        for (int e0 = 0; e0 < n_experts; e0 += 32) {
+            const int e = e0 + lane;
+            const int tiles = e < n_experts ? (total[e] + tile_rows - 1) / tile_rows : 0;
+            int incl = tiles;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int n = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += n;
+            }
+            const int first = tile + incl - tiles;
+            if (e < n_experts) {
+                total[e] = first * tile_rows;
+                for (int i = first; i < min(first + tiles, max_tiles); ++i) tile_expert[i] = e;
+            }
+            tile += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) tile_expert[max_tiles] = min(tile, max_tiles);
     }
+    __syncthreads();
+    auto put = [&](int i, int e, int at) {
+        if (i >= n_pairs) return;
+        const int slot = e < 0 ? -1 : total[e] + mine[e] + at;
+        const bool fits = slot >= 0 && slot < max_tiles * tile_rows;          // the host sizes max_tiles so that it does
+        if (fits) sorted_pair[slot] = i;
+        pair_slot[i] = fits ? slot : -1;
+    };
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j) put(tid + j * threads, kept[j], place[j]);
+    for (int i = tid + KEEP * threads; i < n_pairs; i += threads) put(i, expert_of(i), pair_slot[i]);
 }
 
 // GLU true:  out[slot, n] = glu(A[token(slot), :] . Wg[e][n, :], A[token(slot), :] . Wu[e][n, :]), out in T
@@ -394,8 +449,10 @@ extern "C" int rlis_moe_route(const void* x, const float* w_router, const float*
     if (smem > 48 * 1024) return RLIS_ERR_UNSUPPORTED;
     const unsigned blocks = (unsigned)((n_tokens + tok - 1) / tok);
     const int rows = n_experts + (shared_gate != nullptr ? 1 : 0);
-    const unsigned threads = 32u * (unsigned)(rows < 32 ? (rows < tok ? tok : rows) : 32);
-#define RLIS_ROUTE(T, TOK) rlis_launch(moe_route_kernel<T, TOK>, blocks, threads, smem, stream, (const T*)x, w_router, correction, \
+    // a warp four rows of the matrix with eight tokens, one otherwise; at least a warp a token
+    const int warps = tok == 8 ? (rows + 3) / 4 : rows, most = tok == 8 ? 16 : 32;
+    const unsigned threads = 32u * (unsigned)(warps < most ? (warps < tok ? tok : warps) : most);
+#define RLIS_ROUTE(T, TOK) rlis_launch(moe_route_kernel<T, TOK, (TOK == 8 ? 4 : 1)>, blocks, threads, smem, stream, (const T*)x, w_router, correction, \
                                        top_idx, top_w, shared_gate, n_tokens, width, n_experts, top, route_scale, \
                                        router_bias, scoring, n_groups, keep_groups, normalize)
     if (dtype == RLIS_F32) { if (tok == 8) RLIS_ROUTE(float, 8); else RLIS_ROUTE(float, 1); }
@@ -411,8 +468,10 @@ extern "C" int rlis_moe_align(const int* top_idx, int* sorted_pair, int* pair_sl
     if (n_experts <= 0 || n_experts > 4096 || tile_rows <= 0 || tile_rows % BM != 0 ||
         max_tiles < (n_pairs + tile_rows - 1) / tile_rows)
         return RLIS_ERR_UNSUPPORTED;
-    rlis_launch(moe_align_kernel, 1, 1024, (size_t)2 * n_experts * sizeof(int), stream, top_idx, sorted_pair, pair_slot,
-                tile_expert, n_pairs, n_experts, max_tiles, tile_rows);
+    // a set of counters a warp up to 256 experts (32 KB of them), fewer sets beyond (4,096 experts: 2)
+    const int copies = n_experts <= 256 ? 32 : 8192 / n_experts;
+    rlis_launch(moe_align_kernel, 1, 1024, (size_t)(copies + 1) * n_experts * sizeof(int), stream, top_idx, sorted_pair, pair_slot,
+                tile_expert, n_pairs, n_experts, max_tiles, tile_rows, copies);
     return RLIS_LAUNCH_CHECK();
 }
 
