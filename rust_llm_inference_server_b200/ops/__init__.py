@@ -794,6 +794,38 @@ def attention_latent(qa: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, s
 LIGHTNING_SILU_PASS_TOKENS = 64
 
 
+@functools.lru_cache(maxsize=4096)
+def _lightning_chunks_pay(n_tokens: int, n_seqs: int, longest: int, columns: int, sms: int) -> bool:
+    """Whether the decayed recurrence runs faster 64 tokens at a time than token by token, for `columns` = heads x dv columns of state
+    and a longest portion of `longest` tokens.  The walk takes 0.145 us a token of a request while its CTAs (a request's 16 columns each)
+    have an SM each, and that much longer the more of them share one (the CTAs of a few requests clump: a long portion beside three
+    short ones runs as if all were long); the chunks take 25 us and 2.9 us for each of 1,024 columns' 64 tokens.  Measured at heads of
+    128 x 128, walk and chunks in us: one prompt of 2,048 with 16 heads 310 and 205, with 8 heads 290 and 108; four of 512 255 and 197;
+    130, 700, 65 and 3 tokens 314 and 140; one of 256 44 and 60; one of 128 26 and 50; sixteen of 128 230 and 232."""
+    per_sm = columns / 16 / sms
+    walk = 0.145 * max(longest * max(1.0, min(n_seqs, 4) * per_sm), n_tokens / n_seqs * max(1.0, n_seqs * per_sm))
+    return 25.0 + 2.9 * (n_tokens / 64 + n_seqs) * columns / 1024 < walk
+
+
+def _lightning_in_chunks(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, out: torch.Tensor, state: torch.Tensor, decay: torch.Tensor,
+                         step, n_heads: int, d: int, dv: int, silu: bool) -> bool:
+    """The recurrence with a constant decay a head by chunks (`rlis_lightning_chunks`), if this step's portions are long enough and the
+    rows lie on 16-byte boundaries; False: nothing was launched."""
+    T, vec = rows.shape[0], 16 // rows.element_size()
+    longest = getattr(step, "max_q_len", 0) or -(-T // step.n_seqs)
+    if (not _lightning_chunks_pay(T, step.n_seqs, longest, n_heads * dv, num_sms()) or not hasattr(step, "buffer")
+            or not lib().rlis_lightning_chunks_takes(d, dv)
+            or rows.stride(1) != 1 or any(n % vec for n in (rows.stride(0), q_off, k_off, v_off))
+            or any(t.data_ptr() % 16 for t in (rows, out, state))):
+        return False
+    chunks = T // lib().rlis_lightning_chunk_tokens() + step.n_seqs          # at least what the requests' portions come to
+    states = step.buffer("recurrence_chunks", (chunks, n_heads, dv, d), torch.float32)
+    check(lib().rlis_lightning_chunks(rows.data_ptr(), rows.stride(0), q_off, k_off, v_off, out.data_ptr(), states.data_ptr(), state.data_ptr(),
+                                      decay.data_ptr(), step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(), step.state_slots.data_ptr(),
+                                      step.n_seqs, chunks, n_heads, d, dv, 1 if silu else 0, _code(rows.dtype), _stream()), "lightning_chunks")
+    return True
+
+
 def lightning_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, out: torch.Tensor, state: torch.Tensor,
                    decay: torch.Tensor, step, n_heads: int, d: int, dv: int) -> torch.Tensor:
     """The decayed linear-attention recurrence over the step's tokens: per request and head
@@ -807,6 +839,9 @@ def lightning_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, out: 
     _req(decay, "decay", torch.float32, (n_heads,))
     if max(q_off, k_off) + n_heads * d > proj.shape[1] or v_off + n_heads * dv > proj.shape[1]:
         raise KernelError("lightning_scan: the column offsets reach beyond the projection's rows")
+    if _lightning_in_chunks(proj, q_off, k_off, v_off, out, state, decay, step, n_heads, d, dv, True):
+        _count("lightning_scan.chunks")
+        return out
     # Steps of many tokens: silu is applied once, into a float32 buffer that every CTA of a head then
     # reads (each would otherwise apply it to the head's q and k again).
     activated = None
@@ -871,6 +906,9 @@ def recurrence_scan(rows: torch.Tensor, out: torch.Tensor, state: torch.Tensor, 
     _req(state, "state", torch.float32, (None, n_heads, dv, d))
     if decay is not None:
         _req(decay, "decay", torch.float32, (n_heads,))
+        if _lightning_in_chunks(rows, 0, qk, 2 * qk, out, state, decay, step, n_heads, d, dv, False):
+            _count("recurrence_scan.chunks")
+            return out
     check(lib().rlis_recurrence_scan(rows.data_ptr(), W, 0, qk, 2 * qk, 2 * qk + hv, out.data_ptr(), state.data_ptr(),
                                      decay.data_ptr() if decay is not None else None, step.cu_seqlens.data_ptr(),
                                      step.ctx_lens.data_ptr(), step.state_slots.data_ptr(), step.n_seqs, n_heads, d, dv,

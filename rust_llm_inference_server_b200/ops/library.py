@@ -51,6 +51,9 @@ SIGNATURES = {
     "rlis_per_head_small": [P, LL, LL, P, P, LL, LL, I, I, I, I, P],
     "rlis_latent_step": [P, LL, P, LL, P, P, P, P, P, P, P, I, I, I, I, I, I, F, F, P],
     "rlis_lightning_scan": [P, LL, I, I, I, P, P, P, P, P, P, I, I, I, I, I, P, I, P],
+    "rlis_lightning_chunks": [P, LL, I, I, I, P, P, P, P, P, P, P, I, I, I, I, I, I, I, P],
+    "rlis_lightning_chunk_tokens": [],
+    "rlis_lightning_chunks_takes": [I, I],
     "rlis_recurrence_inputs": [P, LL, I, I, I, P, I, I, I, I, P, I, P, F, I, P, P, I, P],
     "rlis_recurrence_scan_rows": [P, LL, I, I, I, P, P, P, P, P, P, I, I, I, I, P, I, F, P, P, I, P],
     "rlis_recurrence_scan": [P, LL, I, I, I, I, P, P, P, P, P, P, I, I, I, I, I, P],
