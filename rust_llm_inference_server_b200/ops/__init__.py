@@ -791,6 +791,63 @@ def attention_latent(qa: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, s
     return out
 
 
+LATENT_HEADS_BYTES = 1 << 28     # of formed keys and values in a step's scratch memory; longer contexts stay on the latent rows
+
+
+def latent_heads_takes(step, dtype, n_heads: int, dim: int, rot: int, v_dim: int, rank: int) -> bool:
+    """Whether this step's attention over latents goes to `attention_latent_heads`: bfloat16 portions of prompts and nothing else, in
+    sizes that the kernel has.  It was the faster one at every size tried (a layer's mixer, 16 heads, on the rows and with heads formed, us: one
+    prompt of 17 tokens 42 and 38, 128 54 and 41, 512 97 and 63, 2,048 460 and 190; 16 portions of 20 behind 1,000 cached 234 and 157; 17
+    behind 4,096 408 and 187, 64 behind 16,384 1510 and 634), so only the memory that the formed keys and values take limits it."""
+    starts, lens = getattr(step, "starts", None), getattr(step, "q_lens", None)
+    if not LATENT_MMA or dtype != torch.bfloat16 or not starts or not lens or step.n_decode or not step.n_prefill_tiles:
+        return False
+    keys = sum(starts) + sum(lens)
+    return bool(_latent_heads_sizes(dim, rot, v_dim, rank)) and 2 * keys * n_heads * (dim + v_dim) <= LATENT_HEADS_BYTES
+
+
+@functools.lru_cache(maxsize=None)
+def _latent_heads_sizes(dim: int, rot: int, v_dim: int, rank: int) -> bool:
+    return bool(lib().rlis_latent_heads_takes(dim, rot, v_dim, rank))
+
+
+def attention_latent_heads(q: torch.Tensor, q_rot: torch.Tensor, cache: torch.Tensor, w_kv: torch.Tensor, out: torch.Tensor, step, group: int,
+                           n_heads: int, dim: int, rot: int, v_dim: int, rank: int, page_size: int, scale: float, sinks: torch.Tensor | None = None,
+                           window: int = 0, gate: torch.Tensor | None = None) -> torch.Tensor:
+    """`attention_latent` and the value map behind it for a step of prompt portions, with the heads' keys and values formed from the cached
+    latents: out[t, h] = sum_j softmax_j(scale * (q_plain . (W_k_h c_j) + q_rot . k_rot_j)) W_v_h c_j.  q [T, nh (dim + rot)], of which the plain parts
+    are read (may be a column slice of wider rows); q_rot [T, nh rot], the rotated parts; w_kv [nh dim + nh v_dim, rank], the key maps of all heads and
+    then the value maps; out [T, nh v_dim]; all bfloat16."""
+    T, dk = q.shape[0], rank + rot
+    if not q.is_cuda or q.dtype != torch.bfloat16 or tuple(q.shape) != (T, n_heads * (dim + rot)) or q.stride(1) != 1:
+        raise KernelError("attention_latent_heads: q must be bfloat16 rows [T, nh (dim + rot)] with unit stride")
+    _req(q_rot, "q_rot", torch.bfloat16, (T, n_heads * rot))
+    _req(cache, "cache", torch.bfloat16, (None, 1, page_size, dk))
+    _req(w_kv, "w_kv", torch.bfloat16, (n_heads * (dim + v_dim), rank))
+    _req(out, "out", torch.bfloat16, (T, n_heads * v_dim))
+    if sinks is not None:
+        _req(sinks, "sinks", torch.float32, (n_heads,))
+    gp, gs = None, 0
+    if gate is not None:
+        if gate.dtype != torch.bfloat16 or tuple(gate.shape) != (T, n_heads) or gate.stride(1) != 1 or not gate.is_cuda:
+            raise KernelError("attention_latent_heads: the gate must be [T, nh] rows with unit stride in bfloat16")
+        gp, gs = gate.data_ptr(), gate.stride(0)
+    tables = step.block_tables[group]
+    keys = sum(s + n for s, n in zip(step.starts, step.q_lens))
+    rows = step.buffer("latent_rows", (keys, dk), torch.bfloat16)
+    check(lib().rlis_latent_rows(cache.data_ptr(), rows.data_ptr(), step.ctx_lens.data_ptr(), tables.data_ptr(), tables.shape[1], step.n_seqs, page_size, dk,
+                                 keys, _stream()), "latent_rows")
+    _count("latent_rows")
+    kv = step.buffer("latent_kv", (keys, n_heads * (dim + v_dim)), torch.bfloat16)
+    torch.mm(rows[:, :rank], w_kv.t(), out=kv)
+    check(lib().rlis_attention_latent_heads(
+        q.data_ptr(), q.stride(0), q_rot.data_ptr(), kv.data_ptr(), rows.data_ptr(), out.data_ptr(), sinks.data_ptr() if sinks is not None else None,
+        step.prefill_tiles.data_ptr(), step.n_prefill_tiles, step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(), n_heads, dim, rot, v_dim, rank,
+        float(scale), int(window), gp, gs, _stream()), "attention_latent_heads")
+    _count("attention_latent.prefill.heads")
+    return out
+
+
 LIGHTNING_SILU_PASS_TOKENS = 64
 
 

@@ -76,7 +76,10 @@ class LatentAttention(ProjectedMixer):
         self.w_q_up = src.get(s.q_up).contiguous() if self.q_latent else None
         # [head, kv_rank, dim]: the key map transposed, so that it applies to queries
         self.w_k_fold = src.get(s.k_up).view(s.n_heads, s.dim, s.kv_rank).transpose(1, 2).contiguous()
-        self.w_v_up = src.get(s.v_up).view(s.n_heads, s.v_dim, s.kv_rank).contiguous()
+        # the key maps of all heads and the value maps below them: long portions of prompts form the heads' keys and values
+        # (`ops.attention_latent_heads`); the value maps alone are a view of it
+        self.w_kv_up = torch.cat([src.get(s.k_up), src.get(s.v_up)], dim=0).contiguous()
+        self.w_v_up = self.w_kv_up[s.n_heads * s.dim:].view(s.n_heads, s.v_dim, s.kv_rank)
         self.w_o = src.get(s.o_proj).contiguous()
         self.sinks = src.get(s.sink, "vector").contiguous() if s.sink is not None else None
 
@@ -108,20 +111,29 @@ class LatentAttention(ProjectedMixer):
         T, H = proj.shape[0], s.n_heads
         dk = s.kv_rank + s.rot_dim
         stores = self.own_kv and writes_cache
+        z = proj[:, self.kv_off:self.kv_off + dk]
+        q = proj[:, :self.kv_off]
+        gate = proj[:, self.g_off:self.g_off + H] if s.head_gate is not None else None
+        if ops.latent_heads_takes(step, self.dtype, H, s.dim, s.rot_dim, s.v_dim, s.kv_rank):
+            q = self._store_and_project(q, z, step, cache, stores)
+            with span("q rope"):
+                q_rot = step.buffer("latent_q_rot", (T, H * s.rot_dim), self.dtype)
+                ops.latent_q_rope(q, q_rot, self.inv_freq, self.rot_dims, self.magnitude, step.positions, H, s.dim, s.rot_dim, 0)
+            o = step.buffer("attn_o", (T, H * s.v_dim), self.dtype)
+            with span("k, v up proj + attention"):
+                return ops.attention_latent_heads(q, q_rot, cache.k, self.w_kv_up, o, step, cache.group, H, s.dim, s.rot_dim, s.v_dim, s.kv_rank,
+                                                  cache.page_size, self.scale, self.sinks, self.window, gate=gate)
         # float32, or bfloat16 when the whole step goes to the tensor-core attention kernels
         qa_dtype = ops.latent_attention_queries_dtype(step, self.dtype, dk, s.kv_rank)
         qa = step.buffer("latent_qa" if qa_dtype == torch.float32 else "latent_qa16", (T, H * dk), qa_dtype)
-        z = proj[:, self.kv_off:self.kv_off + dk]
-        q = proj[:, :self.kv_off]
         if not self.q_latent and self.own_kv and ops.latent_step_takes(q, qa_dtype, self.w_k_fold, H, s.dim, s.rot_dim):
             with span("latent norm + rope + cache write, q fold + rope"):
                 ops.latent_step(q, z, self.w_k_fold, self.kv_norm, self.eps, self.inv_freq, self.rot_dims, self.magnitude,
                                 step.positions, step.slots[cache.group] if stores else None, cache.k, qa, H, s.dim, s.kv_rank,
                                 cache.page_size)
         else:
-            self._queries(proj, q, z, qa, step, cache, stores)
+            self._queries(q, z, qa, step, cache, stores)
         lat = step.buffer("latent_o", (T, H * s.kv_rank), self.dtype)
-        gate = proj[:, self.g_off:self.g_off + H] if s.head_gate is not None else None
         with span("attention"):
             ops.attention_latent(qa, cache.k, lat, step, cache.group, H, s.kv_rank, cache.page_size, self.scale,
                                  self.sinks, self.window, gate=gate)
@@ -130,11 +142,10 @@ class LatentAttention(ProjectedMixer):
             ops.per_head_linear(lat.view(T, H, s.kv_rank), self.w_v_up, o.view(T, H, s.v_dim))
         return o
 
-    def _queries(self, proj, q, z, qa, step, cache, stores) -> None:
-        """The cached row of every token, and `qa`, operation by operation."""
+    def _store_and_project(self, q, z, step, cache, stores):
+        """The cached row of every token; returns the queries [T, H (dim + rot_dim)] before their rotation."""
         s = self.spec
-        T, H = proj.shape[0], s.n_heads
-        cq = step.buffer("latent_cq", (T, s.q_rank), self.dtype) if self.q_latent else None
+        cq = step.buffer("latent_cq", (q.shape[0], s.q_rank), self.dtype) if self.q_latent else None
         if stores:
             # one launch: the kv latent's norm, the shared key part's rotation, the paged write, and the
             # query latent's norm
@@ -148,6 +159,13 @@ class LatentAttention(ProjectedMixer):
         if self.q_latent:
             with span("q up proj"):
                 q = ops.linear(cq, self.w_q_up)
+        return q
+
+    def _queries(self, q, z, qa, step, cache, stores) -> None:
+        """The cached row of every token, and `qa`, operation by operation."""
+        s = self.spec
+        T, H = q.shape[0], s.n_heads
+        q = self._store_and_project(q, z, step, cache, stores)
         with span("q fold + rope"):
             ops.per_head_linear(q.unflatten(1, (H, s.dim + s.rot_dim))[:, :, :s.dim], self.w_k_fold,
                                 qa.view(T, H, -1)[:, :, :s.kv_rank])
