@@ -90,37 +90,52 @@ __device__ __forceinline__ float conv_input(const T* __restrict__ x, long long s
     return fresh ? 0.f : tail[(size_t)(taps - 1 + src) * C + c];
 }
 
+// Four neighbouring entries of a row, in one load.
+__device__ __forceinline__ float4 load_quad(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load_quad(const bf16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
 // ln g, kept finite so that differences of its sums are defined (e^x is 0 long before)
 __device__ __forceinline__ float log_decay(float a_log, float step) { return fmaxf(-expf(a_log) * step, -1e30f); }
 
 // x: the convolved columns of the projection's rows; b: the logits a head of the same rows; a: the decay logits (HEAD_DECAY:
 // one a head; CHANNEL_DECAY: d a head), rows a_stride apart.
-template <int MODE, typename T>
+// A warp takes TOKS tokens of a head, so that the head's taps are read once for them.  QUADS (four taps, everything on
+// boundaries of four entries): a lane has four neighbouring channels, a tap's inputs in one load.  Bound by the reads and writes of the rows:
+// 1,501 tokens of 4,096 channels 69 us channel by channel, 35 so.
+template <int MODE, typename T, int TOKS, bool QUADS>
 __global__ __launch_bounds__(PREP_WARPS * 32) void prepare_kernel(
     const T* __restrict__ x, long long stride, const T* __restrict__ bl, const T* __restrict__ al, long long a_stride,
     const float* __restrict__ conv_w, const float* __restrict__ conv_b, const float* __restrict__ a_log,
     const float* __restrict__ dt_bias, const float* __restrict__ state, long long state_stride, long long tail_off, Seqs sq,
-    float* __restrict__ act, int n_units, Shape z, float unit_eps, float q_scale) {
+    float* __restrict__ act, int n_units, int n_tokens, Shape z, float unit_eps, float q_scale) {
     pdl_wait_and_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int unit = blockIdx.x * PREP_WARPS + warp;
     if (unit >= n_units) return;
-    const int nh = z.nh, n_qk = z.n_qk, d = z.d, taps = z.taps;
+    const int nh = z.nh, n_qk = z.n_qk, d = z.d, taps = QUADS ? 4 : z.taps;
     const int per = 2 * n_qk + nh + (MODE == CHANNEL_DECAY ? nh : 0) + 1;
-    const int t = unit / per, u = unit - t * per;
+    const int t0 = unit / per * TOKS, u = unit % per, t1 = min(t0 + TOKS, n_tokens);
     const int C = z.channels();
-    float* arow = act + (size_t)t * act_width<MODE>(z);
+    const size_t width_of_row = act_width<MODE>(z);
     if (u == per - 1) {
-        for (int h = lane; h < nh; h += 32) {
-            const float b = to_f<T>(bl[(size_t)t * stride + h]);
-            if (MODE == STATE_SPACE) {
-                const float dt = softplus_f(b + dt_bias[h]);
-                arow[C + h] = dt;
-                arow[C + nh + h] = log_decay(a_log[h], dt);
-            } else {
-                arow[C + h] = 1.0f / (1.0f + expf(-b));
-                if (MODE == HEAD_DECAY)
-                    arow[C + nh + h] = log_decay(a_log[h], softplus_f(to_f<T>(al[(size_t)t * a_stride + h]) + dt_bias[h]));
+        for (int t = t0; t < t1; ++t) {
+            float* arow = act + t * width_of_row;
+            for (int h = lane; h < nh; h += 32) {
+                const float b = to_f<T>(bl[(size_t)t * stride + h]);
+                if (MODE == STATE_SPACE) {
+                    const float dt = softplus_f(b + dt_bias[h]);
+                    arow[C + h] = dt;
+                    arow[C + nh + h] = log_decay(a_log[h], dt);
+                } else {
+                    arow[C + h] = 1.0f / (1.0f + expf(-b));
+                    if (MODE == HEAD_DECAY)
+                        arow[C + nh + h] = log_decay(a_log[h], softplus_f(to_f<T>(al[(size_t)t * a_stride + h]) + dt_bias[h]));
+                }
             }
         }
         return;
@@ -128,35 +143,87 @@ __global__ __launch_bounds__(PREP_WARPS * 32) void prepare_kernel(
     if (MODE == CHANNEL_DECAY && u >= 2 * n_qk + nh) {
         const int h = u - 2 * n_qk - nh;
         const float alog = a_log[h];
-        for (int j = lane; j < d; j += 32)
-            arow[C + nh + h * d + j] =
-                log_decay(alog, softplus_f(to_f<T>(al[(size_t)t * a_stride + h * d + j]) + dt_bias[h * d + j]));
+        for (int t = t0; t < t1; ++t)
+            for (int j = lane; j < d; j += 32)
+                act[t * width_of_row + C + nh + h * d + j] =
+                    log_decay(alog, softplus_f(to_f<T>(al[(size_t)t * a_stride + h * d + j]) + dt_bias[h * d + j]));
         return;
     }
-    const int b = sq.seq_of_token[t];
-    const int row0 = sq.cu_seqlens[b], n = sq.cu_seqlens[b + 1] - row0;
-    const int li = t - row0;
-    const bool fresh = sq.ctx_lens[b] - n == 0;
-    const float* tail = state + (size_t)sq.state_slots[b] * state_stride + tail_off;
     const bool of_qk = u < 2 * n_qk;
     const bool unit_norm = of_qk && MODE != STATE_SPACE;
     const int width = of_qk ? d : z.dv;
     const int c0 = u < n_qk ? z.q_at + u * d : of_qk ? z.k_at + (u - n_qk) * d : z.v_at + (u - 2 * n_qk) * z.dv;
-    float ss = 0.f;
-    for (int j = lane; j < width; j += 32) {
-        const int c = c0 + j;
-        float acc = 0.f;
-        for (int k = 0; k < taps; ++k)
-            acc = fmaf(conv_w[(size_t)c * taps + k], conv_input<T>(x, stride, row0, li - (taps - 1 - k), c, C, tail, taps, fresh), acc);
-        if (conv_b != nullptr) acc += conv_b[c];
-        const float y = silu_f(acc);
-        ss = fmaf(y, y, ss);
-        arow[c] = y;
+    // where each token's inputs lie
+    int row0[TOKS], li[TOKS];
+    const float* tail[TOKS];               // null: the request starts in this step
+    float ss[TOKS];
+#pragma unroll
+    for (int i = 0; i < TOKS; ++i) {
+        const int t = min(t0 + i, n_tokens - 1), b = sq.seq_of_token[t];
+        row0[i] = sq.cu_seqlens[b];
+        li[i] = t - row0[i];
+        const bool fresh = sq.ctx_lens[b] - (sq.cu_seqlens[b + 1] - row0[i]) == 0;
+        tail[i] = fresh ? nullptr : state + (size_t)sq.state_slots[b] * state_stride + tail_off;
+        ss[i] = 0.f;
+    }
+    if (QUADS) {
+        for (int j = lane * 4; j < width; j += 128) {
+            const int c = c0 + j;
+            float w[4][4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) load16<float>(conv_w + (size_t)(c + v) * 4, w[v]);
+            const float4 bias = conv_b != nullptr ? *reinterpret_cast<const float4*>(conv_b + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < TOKS; ++i) {
+                if (t0 + i >= t1) break;
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int src = li[i] - (3 - k);
+                    float4 in = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (src >= 0) in = load_quad(x + (size_t)(row0[i] + src) * stride + c);
+                    else if (tail[i] != nullptr) in = *reinterpret_cast<const float4*>(tail[i] + (size_t)(3 + src) * C + c);
+                    acc[0] = fmaf(w[0][k], in.x, acc[0]);
+                    acc[1] = fmaf(w[1][k], in.y, acc[1]);
+                    acc[2] = fmaf(w[2][k], in.z, acc[2]);
+                    acc[3] = fmaf(w[3][k], in.w, acc[3]);
+                }
+                const float4 y = make_float4(silu_f(acc[0] + bias.x), silu_f(acc[1] + bias.y), silu_f(acc[2] + bias.z), silu_f(acc[3] + bias.w));
+                ss[i] = fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, fmaf(y.w, y.w, ss[i]))));
+                *reinterpret_cast<float4*>(act + (t0 + i) * width_of_row + c) = y;
+            }
+        }
+    } else {
+        for (int i = 0; i < TOKS && t0 + i < t1; ++i) {
+            float* arow = act + (t0 + i) * width_of_row;
+            for (int j = lane; j < width; j += 32) {
+                const int c = c0 + j;
+                float acc = 0.f;
+                for (int k = 0; k < taps; ++k)
+                    acc = fmaf(conv_w[(size_t)c * taps + k],
+                               conv_input<T>(x, stride, row0[i], li[i] - (taps - 1 - k), c, C, tail[i], taps, tail[i] == nullptr), acc);
+                if (conv_b != nullptr) acc += conv_b[c];
+                const float y = silu_f(acc);
+                ss[i] = fmaf(y, y, ss[i]);
+                arow[c] = y;
+            }
+        }
     }
     if (unit_norm) {                               // every lane scales what it wrote itself
-        ss = warp_sum(ss);
-        const float r = (u < n_qk ? q_scale : 1.0f) / sqrtf(ss + unit_eps);
-        for (int j = lane; j < width; j += 32) arow[c0 + j] *= r;
+#pragma unroll
+        for (int i = 0; i < TOKS; ++i) {
+            const float r = (u < n_qk ? q_scale : 1.0f) / sqrtf(warp_sum(ss[i]) + unit_eps);
+            if (t0 + i >= t1) break;
+            float* arow = act + (t0 + i) * width_of_row + c0;
+            if (QUADS) {
+                for (int j = lane * 4; j < width; j += 128) {
+                    const float4 y = *reinterpret_cast<const float4*>(arow + j);
+                    *reinterpret_cast<float4*>(arow + j) = make_float4(y.x * r, y.y * r, y.z * r, y.w * r);
+                }
+            } else {
+                for (int j = lane; j < width; j += 32) arow[j] *= r;
+            }
+        }
     }
 }
 
@@ -884,11 +951,22 @@ template <int MODE, typename T>
 static int launch_typed(const Args& g, cudaStream_t stream) {
     const Shape& z = g.z;
     const long long tail_off = (long long)z.nh * z.dv * z.d;
-    const long long units = (long long)g.n_tokens * (2 * z.n_qk + z.nh + (MODE == CHANNEL_DECAY ? z.nh : 0) + 1);
+    // four tokens a warp in long steps; single tokens and short portions want a warp each
+    const int toks = g.n_tokens >= 64 ? 4 : 1;
+    const long long units = (long long)((g.n_tokens + toks - 1) / toks) * (2 * z.n_qk + z.nh + (MODE == CHANNEL_DECAY ? z.nh : 0) + 1);
     if (units > 0x7fffffffLL) return RLIS_ERR_UNSUPPORTED;
-    rlis_launch(prepare_kernel<MODE, T>, (unsigned)((units + PREP_WARPS - 1) / PREP_WARPS), PREP_WARPS * 32, 0, stream,
-                (const T*)g.x, g.stride, (const T*)g.b, (const T*)g.a, g.a_stride, g.conv_w, g.conv_b, g.a_log, g.dt_bias,
-                (const float*)g.state, g.state_stride, tail_off, g.sq, g.act, (int)units, z, g.unit_eps, g.q_scale);
+    // four channels a lane need every row, head, tap and tail to start on a boundary of four entries
+    const bool quads = z.taps == 4 && z.d % 4 == 0 && z.dv % 4 == 0 && z.q_at % 4 == 0 && z.k_at % 4 == 0 && z.v_at % 4 == 0 &&
+                       g.stride % 4 == 0 && act_width<MODE>(z) % 4 == 0 && g.state_stride % 4 == 0 && tail_off % 4 == 0 &&
+                       reinterpret_cast<uintptr_t>(g.x) % (4 * sizeof(T)) == 0 &&
+                       ((reinterpret_cast<uintptr_t>(g.conv_w) | reinterpret_cast<uintptr_t>(g.conv_b) | reinterpret_cast<uintptr_t>(g.state) |
+                         reinterpret_cast<uintptr_t>(g.act)) & 15) == 0;
+#define RLIS_PREPARE(TOKS, QUADS) rlis_launch(prepare_kernel<MODE, T, TOKS, QUADS>, (unsigned)((units + PREP_WARPS - 1) / PREP_WARPS), PREP_WARPS * 32, 0, \
+                stream, (const T*)g.x, g.stride, (const T*)g.b, (const T*)g.a, g.a_stride, g.conv_w, g.conv_b, g.a_log, g.dt_bias,                   \
+                (const float*)g.state, g.state_stride, tail_off, g.sq, g.act, (int)units, g.n_tokens, z, g.unit_eps, g.q_scale)
+    if (quads) { if (toks == 4) RLIS_PREPARE(4, true); else RLIS_PREPARE(1, true); }
+    else { if (toks == 4) RLIS_PREPARE(4, false); else RLIS_PREPARE(1, false); }
+#undef RLIS_PREPARE
     dim3 grid(g.n_seqs, z.nh, (z.dv + COLS - 1) / COLS);
     // few CTAs that run long: shared memory asked for beyond the need keeps them one an SM
     static int sms = 0;
