@@ -10,8 +10,8 @@
 //
 // With a token row list only those tokens of the step are computed (n_tokens = length of the list).
 //
-// This is the kernel of the float32 path and the fallback of the bfloat16 path for shapes that the
-// tensor-core kernels refuse.  Head sizes: multiples of 16 up to 256.
+// This is the fallback of the float32 path for shapes that attention_f32.cu refuses, and of the bfloat16 path for shapes that
+// the tensor-core kernels refuse.  Head sizes: multiples of 16 up to 256.
 #include "common.cuh"
 #include <math.h>
 
