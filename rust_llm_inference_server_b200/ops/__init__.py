@@ -1621,7 +1621,7 @@ def attention(q, k_cache, v_cache, out, step, group: int, n_heads: int, n_kv_hea
     fit the step.  bfloat16: single decoded tokens go to the split decode kernel, portions of
     prompts to the flash kernel (head sizes 64 and 128).  float32: `attention_f32` for the sizes it takes.  Everything else
     goes to the kernel for any query length.  The choice never changes the result beyond rounding."""
-    if attention_f32_takes(q.dtype, n_heads, n_kv_heads, head_dim):
+    if attention_f32_takes(q.dtype, n_heads, n_kv_heads, head_dim) and q.shape[0] <= 65535:      # (its grids' limit)
         return attention_f32(q, k_cache, v_cache, out, step, group, n_heads, n_kv_heads, head_dim, page_size, scale, window)
     tables = step.block_tables[group]
     bf = q.dtype == torch.bfloat16
