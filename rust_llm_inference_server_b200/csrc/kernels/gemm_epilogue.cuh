@@ -28,10 +28,11 @@ __device__ __forceinline__ void add_bias32(uint32_t (&r)[32], float bias) {
 // EPI 0: bf16 y [M, N].  EPI 1: SwiGLU over a gate|up matrix whose rows are interleaved in blocks of
 // 4 (columns 8 t .. 8 t + 3 gate, 8 t + 4 .. 8 t + 7 up), y [M, N / 2] bf16.  EPI 2: float32 y [M, N].
 // EPI 3: the layout of EPI 1 with the clipped gating of GluParams.
-// The gates' results are rounded to bfloat16, so the fast exponential and division serve.  They matter: a tile's 32,768
-// gates with expf and a division, on four warps, took longer than its products (a scheduler runs one warp of the epilogue,
-// so nothing hides a chain of 40 instructions).  With these and eight epilogue warps: SwiGLU of 2,048 rows, 2048 x 16384, 97 -> 90
-// us; 8,192 pairs on 32 experts of 2048 x 2 x 1024, clipped, 154 -> 92 us.
+// Gates are the function of `glu_gate` to the last bit (expf and a division; gelu's form without limits excepted), so that a token
+// gets the same numbers here, in the streaming products of a decode step and in the gating kernels.  They matter: a tile has
+// 32,768 of them, and on four warps they took longer than its products (a scheduler runs one warp of the epilogue, so nothing
+// hides a chain of 40 instructions).  With eight epilogue warps and one form a launch: 4,096 rows, K 512, N 8192: SwiGLU 76 -> 47 us,
+// clipped 90 -> 58 us; 2,048 rows, K 2048, N 16384: 104 -> 101 and 111 -> 104 us.
 // r: the sums of columns col .. col + 31 of row `row`; columns from N on are not stored.
 template <int EPI>
 __device__ __forceinline__ void store_sums32(const uint32_t (&r)[32], void* __restrict__ y, int row, int col, int N,
@@ -55,7 +56,7 @@ __device__ __forceinline__ void store_sums32(const uint32_t (&r)[32], void* __re
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const float g = __uint_as_float(r[(i >> 2) * 8 + (i & 3)]), u = __uint_as_float(r[(i >> 2) * 8 + 4 + (i & 3)]);
-                res[i] = __fdividef(g, 1.0f + __expf(-g)) * u;
+                res[i] = g / (1.0f + expf(-g)) * u;
             }
         } else {
             // One form for all 16, chosen once: with the choice inside `glu_gate` every gate was a chain of its own behind two
@@ -69,15 +70,19 @@ __device__ __forceinline__ void store_sums32(const uint32_t (&r)[32], void* __re
             if (gp.slope == INFINITY) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) res[i] = fmaxf(g[i], 0.f) * u[i];
-            } else if (gp.cubic != 0.f) {
+            } else if (gp.cubic != 0.f && gp.limit == INFINITY && gp.shift == 0.f) {
+                // gelu's tanh form, whose own error is far above that of the fast exponential and division
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const float z = fmaf(gp.cubic * g[i] * g[i], g[i], g[i]);
                     res[i] = __fdividef(g[i], 1.0f + __expf(-gp.slope * z)) * u[i];
                 }
+            } else if (gp.cubic != 0.f) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) res[i] = g[i] / (1.0f + expf(-gp.slope * fmaf(gp.cubic * g[i] * g[i], g[i], g[i]))) * u[i];
             } else {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) res[i] = __fdividef(g[i], 1.0f + __expf(-gp.slope * g[i])) * u[i];
+                for (int i = 0; i < 16; ++i) res[i] = g[i] / (1.0f + expf(-gp.slope * g[i])) * u[i];
             }
         }
 #pragma unroll
