@@ -64,8 +64,19 @@ __device__ __forceinline__ void store_sums32(const uint32_t (&r)[32], void* __re
             float g[16], u[16];
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-                g[i] = fminf(__uint_as_float(r[(i >> 2) * 8 + (i & 3)]), gp.limit);
-                u[i] = fminf(fmaxf(__uint_as_float(r[(i >> 2) * 8 + 4 + (i & 3)]), -gp.limit), gp.limit) + gp.shift;
+                g[i] = __uint_as_float(r[(i >> 2) * 8 + (i & 3)]);
+                u[i] = __uint_as_float(r[(i >> 2) * 8 + 4 + (i & 3)]);
+            }
+            if (gp.limit != INFINITY) {         // (min and max with an infinity change nothing but a NaN, which has to stay one)
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    g[i] = fminf(g[i], gp.limit);
+                    u[i] = fminf(fmaxf(u[i], -gp.limit), gp.limit);
+                }
+            }
+            if (gp.shift != 0.f) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) u[i] += gp.shift;
             }
             if (gp.slope == INFINITY) {
 #pragma unroll

@@ -45,3 +45,20 @@ def test_a_gate_is_the_same_number_in_the_grouped_product():
     ops.glu_act(w.t().contiguous(), want, 1.702, 7.0, 1.0, 4)
     ops.check_device_errors()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M", [128, 300])
+@pytest.mark.parametrize("glu", [None, (1.0, None, 0.0), (1.2, None, 0.5), (1.5957691, None, 0.0, 0.044715)])
+def test_what_is_not_a_number_stays_so_behind_a_gate_without_limits(M, glu):
+    from rust_llm_inference_server_b200 import ops
+    I = 256
+    x, w = selected(M, I, torch.Generator().manual_seed(3))
+    clean = ops.gemm_tcgen05(x, w, "swiglu4" if glu is None else "glu4", glu=glu)
+    w[8 * 5 + 2] = float("nan")                                         # the gate of column 4 * 5 + 2
+    w[8 * 9 + 4 + 1] = float("nan")                                     # the linear branch of column 4 * 9 + 1
+    out = ops.gemm_tcgen05(x, w, "swiglu4" if glu is None else "glu4", glu=glu)
+    ops.check_device_errors()
+    lost = [22, 37]
+    others = [c for c in range(I) if c not in lost]
+    assert bool(torch.isnan(out[:, lost]).all())
+    assert torch.equal(out[:, others], clean[:, others])
