@@ -106,15 +106,26 @@ __device__ __forceinline__ void store_sums32(const uint32_t (&r)[32], void* __re
             pk.w = pack_bf16(res[v * 8 + 6], res[v * 8 + 7]);
             *reinterpret_cast<uint4*>(o + v * 8) = pk;
         }
-    } else {
-        float* o = reinterpret_cast<float*>(y) + (size_t)row * N + col;
+    }
+}
+
+// The float32 rows of EPI 2: columns col .. col + 31 of rows row0 .. row0 + 31, a row's sums a lane, by a whole warp.  Stored as they
+// lie, an instruction would write 16 bytes of 32 rows; turned through 4 KB of shared memory (rows in 16-byte pieces, their
+// places swapped by the row, so that neither side meets in a bank) it writes the 128 bytes of 4 rows.
+constexpr int TURN_BYTES = 32 * 32 * 4;           // a warp's
+__device__ __forceinline__ void store_rows_turned(const uint32_t (&r)[32], float4* turn, float* __restrict__ y, int row0, int col, int M, int N, bool ok) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
 #pragma unroll
-        for (int v = 0; v < 8; ++v) {
-            if (col + v * 4 >= N) break;
-            *reinterpret_cast<float4*>(o + v * 4) = make_float4(
-                __uint_as_float(r[v * 4]), __uint_as_float(r[v * 4 + 1]), __uint_as_float(r[v * 4 + 2]),
-                __uint_as_float(r[v * 4 + 3]));
-        }
+    for (int v = 0; v < 8; ++v)
+        turn[lane * 8 + (v ^ (lane & 7))] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]), __uint_as_float(r[4 * v + 2]),
+                                                        __uint_as_float(r[4 * v + 3]));
+    __syncwarp();
+    const int piece = lane & 7, at = col + piece * 4;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int lr = j * 4 + (lane >> 3);
+        if (ok && row0 + lr < M && at < N) *reinterpret_cast<float4*>(y + (size_t)(row0 + lr) * N + at) = turn[lr * 8 + (piece ^ (lr & 7))];
     }
 }
 

@@ -32,9 +32,8 @@ constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4;
 constexpr int UMMA_K = 16;
 constexpr int A_STAGE_BYTES = BM * BK * 2, B_STAGE_BYTES = BN * BK * 2;
 constexpr int GT_THREADS = 320;
-constexpr int TURN_BYTES = 8 * 32 * 32 * 4;      // float32 rows: a block of 32 x 32 sums for each epilogue warp
 constexpr size_t GT_SMEM = (size_t)STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 1024 /* alignment */ + 256;
-constexpr size_t GT_SMEM_F32 = GT_SMEM + TURN_BYTES;
+constexpr size_t GT_SMEM_F32 = GT_SMEM + 8 * TURN_BYTES;       // float32 rows turn in a block for each epilogue warp
 
 struct Ctrl {
     uint64_t full[STAGES];
@@ -165,25 +164,9 @@ __global__ __launch_bounds__(GT_THREADS) void gemm_tcgen05_kernel(const __grid_c
                 uint32_t r[32];
                 tmem_ld32(tmem_acc + (uint32_t)(cb * 32), r);
                 if (EPI == 3 && gp.bias != nullptr) add_bias32(r, bias);
-                if (EPI == 2) {
-                    // A lane holds 128 bytes of a row; stored as it is, an instruction wrote 16 bytes of 32 rows.  Turned
-                    // through shared memory (rows in 16-byte pieces, their places swapped by the row, so that neither
-                    // side meets in a bank) it writes the 128 bytes of 4 rows (84 MB of sums: 72 us, now
-                    // 56).
-                    float4* turn = reinterpret_cast<float4*>(base + (size_t)STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 256) + (warp - 2) * 256;
-                    __syncwarp();
-#pragma unroll
-                    for (int v = 0; v < 8; ++v)
-                        turn[lane * 8 + (v ^ (lane & 7))] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
-                                                                        __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-                    __syncwarp();
-                    const int piece = lane & 7, at = col + piece * 4;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const int lr = j * 4 + (lane >> 3), gr = m0 + q * 32 + lr;
-                        if (ok && gr < M && at < N)
-                            *reinterpret_cast<float4*>(reinterpret_cast<float*>(y) + (size_t)gr * N + at) = turn[lr * 8 + (piece ^ (lr & 7))];
-                    }
+                if (EPI == 2) {         // (84 MB of sums: 72 us stored as they lie, 56 turned)
+                    store_rows_turned(r, reinterpret_cast<float4*>(base + (size_t)STAGES * (A_STAGE_BYTES + B_STAGE_BYTES) + 256 + (warp - 2) * TURN_BYTES),
+                                      reinterpret_cast<float*>(y), m0 + q * 32, col, M, N, ok);
                     continue;
                 }
                 if (!ok || row >= M || col >= N) continue;

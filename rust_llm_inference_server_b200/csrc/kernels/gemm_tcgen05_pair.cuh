@@ -33,6 +33,7 @@ constexpr int PN = 256, PK = 64, P_STAGES = 6;
 constexpr int A_BYTES = PM * PK * 2, B_BYTES = (PN / 2) * PK * 2;       // 16 KB each a CTA and stage
 constexpr int GP_THREADS = 320;
 constexpr size_t GP_SMEM = (size_t)P_STAGES * (A_BYTES + B_BYTES) + 1024 /* alignment */ + 256;
+constexpr size_t GP_SMEM_F32 = GP_SMEM + 8 * TURN_BYTES;       // float32 rows turn in a block for each epilogue warp
 
 struct PairCtrl {
     uint64_t full[P_STAGES];        // CTA 0's: both CTAs' bytes of a stage have arrived
@@ -197,6 +198,12 @@ __global__ __launch_bounds__(GP_THREADS) void gemm_tcgen05_pair_kernel(const __g
                 uint32_t r[32];
                 tmem_ld32(tmem_acc + (uint32_t)(cb * 32), r);
                 if (EPI == 3 && gp.bias != nullptr) add_bias32(r, bias);
+                if (EPI == 2) {         // (us with four warps storing sums as they lie, with eight, and turned: 2,048 x 16,384 of K 2048 110, 123, 105;
+                                        // 4,096 x 8,192 of K 512 73, 79, 42)
+                    store_rows_turned(r, reinterpret_cast<float4*>(base + (size_t)P_STAGES * (A_BYTES + B_BYTES) + 256 + (warp - 2) * TURN_BYTES),
+                                      reinterpret_cast<float*>(y), m0 + q * 32, col, M, N, ok);
+                    continue;
+                }
                 if (!ok || row >= M || col >= N) continue;
                 store_sums32<EPI>(r, y, row, col, N, gp);
             }
@@ -231,7 +238,7 @@ static int launch_gemm_pair(const void* x, const void* W, void* y, int M, int N,
     if (!attr_done) {
         cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
         cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
-        cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
+        cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM_F32);
         cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
         attr_done = true;
     }
@@ -246,7 +253,7 @@ static int launch_gemm_pair(const void* x, const void* W, void* y, int M, int N,
     else if (epilogue == 1)
         rlis_launch_cluster(gemm_tcgen05_pair_kernel<1>, dim3(grid), dim3(GP_THREADS), GP_SMEM, stream, cluster, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp);
     else if (epilogue == 2)
-        rlis_launch_cluster(gemm_tcgen05_pair_kernel<2>, dim3(grid), dim3(GP_THREADS), GP_SMEM, stream, cluster, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp);
+        rlis_launch_cluster(gemm_tcgen05_pair_kernel<2>, dim3(grid), dim3(GP_THREADS), GP_SMEM_F32, stream, cluster, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp);
     else
         rlis_launch_cluster(gemm_tcgen05_pair_kernel<3>, dim3(grid), dim3(GP_THREADS), GP_SMEM, stream, cluster, map_x, map_w, y, M, N, K, m_tiles, num_tiles, gp);
     return RLIS_LAUNCH_CHECK();

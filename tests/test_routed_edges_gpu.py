@@ -93,3 +93,20 @@ def test_gates_in_the_epilogue_at_large_and_small_arguments(M, glu):
     e = 2.0 ** -24 * K * (x.abs().double() @ w.abs().double().t()).view(M, I // 4, 2, 4).amax(2).reshape(M, I)
     bound = 2.0 ** -8 * want.abs() + 4 * e * (1 + (up + shift).abs() + gate.abs()) * (1 + 3 * cubic * gt ** 2) + 1e-30
     assert bool(((out - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 264, 64), (300, 520, 72), (257, 1032, 200), (2000, 2056, 512)])
+def test_float32_rows_of_a_pair_of_ctas_end_inside_a_block(M, N, K):
+    """Rows and columns that end inside a turned block of 32 x 32 sums, several tiles a pair: the sums of one CTA a tile, bit for bit."""
+    from rust_llm_inference_server_b200 import ops
+    g = torch.Generator().manual_seed(M)
+    x, w = (torch.randn(n, K, generator=g).bfloat16() for n in (M, N))
+    out = ops.gemm_tcgen05(x.cuda(), w.cuda(), "float32")
+    ops.debug_set("gemm_pair", 0)
+    try:
+        assert torch.equal(out, ops.gemm_tcgen05(x.cuda(), w.cuda(), "float32"))
+    finally:
+        ops.debug_set("gemm_pair", -1)
+    ops.check_device_errors()
+    bound = 2.0 ** -24 * K * (x.abs().double() @ w.abs().double().t())              # float32 sums of exact products
+    assert bool(((out.cpu().double() - x.double() @ w.double().t()).abs() <= bound).all())
