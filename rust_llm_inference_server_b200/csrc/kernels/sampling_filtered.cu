@@ -5,7 +5,8 @@
 // the mass reaches top_p, an inverse-CDF draw); the rule is the same here, arranged so that no
 // sort is needed and every sum is exact:
 //   * weights are fixed-point integers, w = floor(exp((l - max) / T) * 2^40), added with integer
-//     atomics, so sums do not depend on the order of addition and a draw is reproducible;
+//     atomics, so sums do not depend on the order of addition and a draw is reproducible; a logit that is not a
+//     number weighs nothing and ranks last, and infinite ones share the mass;
 //   * the k-th highest logit, and then the nucleus threshold (the largest value t with
 //     mass{l >= t} >= top_p * mass), are found by a radix search over the order-preserving 32-bit
 //     image of the floats: four passes of 8 bits, a 256-bin histogram each (counts for top-k,
@@ -23,16 +24,17 @@ namespace {
 constexpr int FT = 1024;
 typedef unsigned long long u64;
 
-// Every bit flipped below zero, the sign alone otherwise.  A NaN without a sign stands beside zero, so that it does not push a
-// token out of a top-k set (`u | 0x80000000` came to that by itself: the compiler takes it for -|f|, a canonical NaN).
+// Every bit flipped below zero, the sign alone otherwise.  A NaN of either sign ranks below -inf, so that it pushes no token out of
+// a top-k set (the key is a NaN's, which key_value gives back as one).
 __device__ __forceinline__ uint32_t order_key(float f) {
     const uint32_t u = __float_as_uint(f);
-    if (u - 0x7f800001u < 0x007fffffu) return 0x7fffffffu;
+    if ((u & 0x7fffffffu) > 0x7f800000u) return 0x007ffffeu;
     return u ^ ((uint32_t)((int)u >> 31) | 0x80000000u);
 }
+// The row's highest logits weigh 2^40 each, also where they are infinite; a NaN weighs nothing.
 __device__ __forceinline__ u64 fixed_weight(float logit, float mx, float inv_t) {
-    const float w = expf((logit - mx) * inv_t);           // in (0, 1]
-    return (u64)(w * 1099511627776.0f);                    // * 2^40
+    const float w = logit == mx ? 1.0f : expf((logit - mx) * inv_t);           // in [0, 1], or NaN
+    return w >= 0.f ? (u64)(w * 1099511627776.0f) : 0ull;                      // * 2^40
 }
 __device__ __forceinline__ u64 block_sum_u64(u64 v, u64* scratch) {
 #pragma unroll
@@ -298,7 +300,7 @@ struct ClusterShared {
                                  // may still be read by other CTAs, the one after it is emptied
     u64 xch[8];                  // a CTA's sum of a phase, read by the whole cluster
     float xmax;
-    uint32_t xkey, xnan;
+    uint32_t xkey;
     float fmax_of[CT / 32];
     uint32_t kmax_of[CT / 32];
     u64 scan[CT / 32];
@@ -364,14 +366,12 @@ __global__ __launch_bounds__(CT, 2) void sample_filtered_cluster_kernel(const fl
     uint32_t key[E];
     float mx = -INFINITY;
     uint32_t top_key = 0u;
-    uint32_t nans = 0u;                              // which of them are NaN: their weight is what a NaN becomes as an integer
     if (((reinterpret_cast<uintptr_t>(row) & 15) == 0) && n_mine == E) {
 #pragma unroll
         for (int i = 0; i < E; i += 4) {
             const float4 x = *reinterpret_cast<const float4*>(row + v0 + i);
             mx = fmaxf(fmaxf(mx, fmaxf(x.x, x.y)), fmaxf(x.z, x.w));
             key[i] = order_key(x.x); key[i + 1] = order_key(x.y); key[i + 2] = order_key(x.z); key[i + 3] = order_key(x.w);
-            nans |= ((x.x != x.x ? 1u : 0u) | (x.y != x.y ? 2u : 0u) | (x.z != x.z ? 4u : 0u) | (x.w != x.w ? 8u : 0u)) << i;
         }
     } else {
 #pragma unroll
@@ -379,32 +379,28 @@ __global__ __launch_bounds__(CT, 2) void sample_filtered_cluster_kernel(const fl
             const float l = i < n_mine ? row[v0 + i] : -INFINITY;
             mx = fmaxf(mx, l);
             key[i] = i < n_mine ? order_key(l) : 0u;
-            nans |= l != l ? 1u << i : 0u;
         }
     }
 #pragma unroll
     for (int i = 0; i < E; ++i) top_key = max(top_key, key[i]);
 
-    // the row's maximum, and its highest key (a NaN's, where there is one)
+    // the row's maximum, and its highest key
     mx = warp_max(mx);
     top_key = __reduce_max_sync(0xffffffffu, top_key);
     if (lane == 0) { sh.fmax_of[warp] = mx; sh.kmax_of[warp] = top_key; }
     for (int i = tid; i < 3 * BINS; i += CT) sh.hist[0][0][i] = 0u;
-    const bool cta_nan = __syncthreads_or(nans != 0u);
+    __syncthreads();
     if (tid == 0) {
-        sh.xnan = cta_nan ? 1u : 0u;
         for (int i = 1; i < CT / 32; ++i) { mx = fmaxf(mx, sh.fmax_of[i]); top_key = max(top_key, sh.kmax_of[i]); }
         sh.xmax = mx;
         sh.xkey = top_key;
     }
     cluster_sync_all();
-    uint32_t any_nan = 0u;
     for (uint32_t c = 0; c < cc; ++c) {
         mx = fmaxf(mx, ld_dsmem(&sh.xmax, c));
         top_key = max(top_key, ld_dsmem_u32(&sh.xkey, c));
-        any_nan |= ld_dsmem_u32(&sh.xnan, c);
     }
-    auto weight = [&](int i) -> u64 { return (nans >> i) & 1u ? 1ull << 63 : fixed_weight(key_value(key[i]), mx, inv_t); };
+    auto weight = [&](int i) -> u64 { return fixed_weight(key_value(key[i]), mx, inv_t); };
 
     int buf = 0, phase = 0;
     // The highest key such that the counts (`masses` false) or masses of the keys from it upwards reach `need_of(sum)`, of the
@@ -417,7 +413,7 @@ __global__ __launch_bounds__(CT, 2) void sample_filtered_cluster_kernel(const fl
         above = 0ull;
         bool first = true;                         // `need` is not known yet
         for (bool try_list = known <= LIST;;) {
-            if (try_list && !any_nan) {
+            if (try_list) {
                 // few tokens may be left: all of them in one list, where each is compared with each
                 if (tid == 0) sh.n_list = 0u;
                 __syncthreads();
