@@ -5,8 +5,8 @@
 // the mass reaches top_p, an inverse-CDF draw); the rule is the same here, arranged so that no
 // sort is needed and every sum is exact:
 //   * weights are fixed-point integers, w = floor(exp((l - max) / T) * 2^40), added with integer
-//     atomics, so sums do not depend on the order of addition and a draw is reproducible; a logit that is not a
-//     number weighs nothing and ranks last, and infinite ones share the mass;
+//     atomics, so sums do not depend on the order of addition and a draw is reproducible; a NaN counts
+//     as -inf, infinite logits share the mass;
 //   * the k-th highest logit, and then the nucleus threshold (the largest value t with
 //     mass{l >= t} >= top_p * mass), are found by a radix search over the order-preserving 32-bit
 //     image of the floats: four passes of 8 bits, a 256-bin histogram each (counts for top-k,
@@ -24,17 +24,20 @@ namespace {
 constexpr int FT = 1024;
 typedef unsigned long long u64;
 
-// Every bit flipped below zero, the sign alone otherwise.  A NaN of either sign ranks below -inf, so that it pushes no token out of
-// a top-k set (the key is a NaN's, which key_value gives back as one).
+// Every bit flipped below zero, the sign alone otherwise.  A NaN of either sign counts as -inf: it pushes no token out of a top-k
+// set and weighs nothing.
 __device__ __forceinline__ uint32_t order_key(float f) {
     const uint32_t u = __float_as_uint(f);
-    if ((u & 0x7fffffffu) > 0x7f800000u) return 0x007ffffeu;
+    if ((u & 0x7fffffffu) > 0x7f800000u) return 0x007fffffu;
     return u ^ ((uint32_t)((int)u >> 31) | 0x80000000u);
 }
-// The row's highest logits weigh 2^40 each, also where they are infinite; a NaN weighs nothing.
-__device__ __forceinline__ u64 fixed_weight(float logit, float mx, float inv_t) {
-    const float w = logit == mx ? 1.0f : expf((logit - mx) * inv_t);           // in [0, 1], or NaN
-    return w >= 0.f ? (u64)(w * 1099511627776.0f) : 0ull;                      // * 2^40
+__device__ __forceinline__ float key_value(uint32_t key) {
+    return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
+}
+// `mx` is not -inf.  (inf - inf is a NaN, of which and of 1 the smaller is 1: infinite logits share the mass.)
+__device__ __forceinline__ u64 fixed_weight(uint32_t key, float mx, float inv_t) {
+    const float w = fminf(expf((key_value(key) - mx) * inv_t), 1.0f);           // in [0, 1]
+    return (u64)(w * 1099511627776.0f);                                          // * 2^40
 }
 __device__ __forceinline__ u64 block_sum_u64(u64 v, u64* scratch) {
 #pragma unroll
@@ -54,18 +57,13 @@ __device__ __forceinline__ u64 block_sum_u64(u64 v, u64* scratch) {
     return r;
 }
 
-__device__ __forceinline__ float key_value(uint32_t key) {
-    return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
-}
-
 // Over the row: how many keys exceed `key0`, how many equal it, and the mass of those that exceed it.
 __device__ __forceinline__ void key_stats(const float* row, int vocab, uint32_t key0, float mx, float inv_t,
                                           u64* scratch, u64& n_above, u64& n_ties, u64& mass_above) {
     u64 a = 0ull, t = 0ull, m = 0ull;
     for (int v = threadIdx.x; v < vocab; v += FT) {
-        const float l = row[v];
-        const uint32_t key = order_key(l);
-        if (key > key0) { ++a; m += fixed_weight(l, mx, inv_t); }
+        const uint32_t key = order_key(row[v]);
+        if (key > key0) { ++a; m += fixed_weight(key, mx, inv_t); }
         else if (key == key0) ++t;
     }
     n_above = block_sum_u64(a, scratch);
@@ -103,6 +101,7 @@ __global__ __launch_bounds__(FT) void sample_filtered_kernel(const float* __rest
     mx = s_max[0];
     for (int i = 1; i < FT / 32; ++i) mx = fmaxf(mx, s_max[i]);
     __syncthreads();
+    if (mx == -INFINITY) mx = 0.f;          // nothing to draw: no token weighs anything
 
     // top-k: the k-th highest key by radix search on counts
     uint32_t kth = 0u;
@@ -141,7 +140,7 @@ __global__ __launch_bounds__(FT) void sample_filtered_kernel(const float* __rest
     u64 n_above_k, n_ties_k, mass_above_k;
     key_stats(row, vocab, kth, mx, inv_t, scratch, n_above_k, n_ties_k, mass_above_k);
     const u64 keep_k = use_k ? (u64)top_k - n_above_k : n_ties_k;
-    const u64 w_k = fixed_weight(key_value(kth), mx, inv_t);
+    const u64 w_k = fixed_weight(kth, mx, inv_t);
     const u64 mass = mass_above_k + keep_k * w_k;        // of the top-k set (or of everything)
 
     // top-p: the largest threshold whose upper mass reaches top_p * mass, by radix search on masses
@@ -156,10 +155,9 @@ __global__ __launch_bounds__(FT) void sample_filtered_kernel(const float* __rest
             for (int i = threadIdx.x; i < 256; i += FT) hist[i] = 0ull;
             __syncthreads();
             for (int v = threadIdx.x; v < vocab; v += FT) {
-                const float l = row[v];
-                const uint32_t key = order_key(l);
+                const uint32_t key = order_key(row[v]);
                 if (key >= kth && (pass == 0 || (key >> (shift + 8)) == (prefix >> (shift + 8))))
-                    atomicAdd(&hist[(key >> shift) & 255u], fixed_weight(l, mx, inv_t));
+                    atomicAdd(&hist[(key >> shift) & 255u], fixed_weight(key, mx, inv_t));
             }
             __syncthreads();
             if (threadIdx.x == 0) {
@@ -182,7 +180,7 @@ __global__ __launch_bounds__(FT) void sample_filtered_kernel(const float* __rest
         // (the crossing token included; sampler.rs:200-209)
         u64 n_above, n_ties, mass_above;
         key_stats(row, vocab, thr, mx, inv_t, scratch, n_above, n_ties, mass_above);
-        const u64 w_t = fixed_weight(key_value(thr), mx, inv_t);
+        const u64 w_t = fixed_weight(thr, mx, inv_t);
         u64 need = 1ull;
         if (target > mass_above && w_t > 0ull) need = (target - mass_above + w_t - 1ull) / w_t;
         if (need < 1ull) need = 1ull;
@@ -210,9 +208,8 @@ __global__ __launch_bounds__(FT) void sample_filtered_kernel(const float* __rest
     // kept mass of this piece
     u64 mine = 0ull, rank = tie_rank;
     for (int v = v0; v < v1; ++v) {
-        const float l = row[v];
-        const uint32_t key = order_key(l);
-        if (key > thr || (key == thr && rank++ < tie_keep)) mine += fixed_weight(l, mx, inv_t);
+        const uint32_t key = order_key(row[v]);
+        if (key > thr || (key == thr && rank++ < tie_keep)) mine += fixed_weight(key, mx, inv_t);
     }
     u64 incl = mine;
 #pragma unroll
@@ -237,16 +234,15 @@ __global__ __launch_bounds__(FT) void sample_filtered_kernel(const float* __rest
         u64 cum = before, rk = tie_rank;
         int pick = v1 - 1;
         for (int v = v0; v < v1; ++v) {
-            const float l = row[v];
-            const uint32_t key = order_key(l);
+            const uint32_t key = order_key(row[v]);
             if (key > thr || (key == thr && rk++ < tie_keep)) {
-                cum += fixed_weight(l, mx, inv_t);
+                cum += fixed_weight(key, mx, inv_t);
                 if (cum > target_r) { pick = v; break; }
             }
         }
         out[r] = pick;
     }
-    if (s_owner < 0 && threadIdx.x == 0) out[r] = 0;   // nothing kept (a row of NaNs): id 0, as the greedy path
+    if (s_owner < 0 && threadIdx.x == 0) out[r] = 0;   // nothing kept (a row of NaNs or -inf): id 0, as the greedy path
     pdl_trigger();   // the next kernel of the stream may start its launch
 }
 
@@ -400,7 +396,8 @@ __global__ __launch_bounds__(CT, 2) void sample_filtered_cluster_kernel(const fl
         mx = fmaxf(mx, ld_dsmem(&sh.xmax, c));
         top_key = max(top_key, ld_dsmem_u32(&sh.xkey, c));
     }
-    auto weight = [&](int i) -> u64 { return fixed_weight(key_value(key[i]), mx, inv_t); };
+    if (mx == -INFINITY) mx = 0.f;              // nothing to draw: no token weighs anything
+    auto weight = [&](int i) -> u64 { return fixed_weight(key[i], mx, inv_t); };
 
     int buf = 0, phase = 0;
     // The highest key such that the counts (`masses` false) or masses of the keys from it upwards reach `need_of(sum)`, of the
@@ -433,7 +430,7 @@ __global__ __launch_bounds__(CT, 2) void sample_filtered_cluster_kernel(const fl
                     n = min(n + nc, LIST + 1u);
                 }
                 if (n <= LIST) {
-                    const u64 v = tid < n ? (masses ? fixed_weight(key_value(mine), mx, inv_t) : 1ull) : 0ull;
+                    const u64 v = tid < n ? (masses ? fixed_weight(mine, mx, inv_t) : 1ull) : 0ull;
                     if (tid < n) { sh.all_keys[tid] = mine; sh.all_values[tid] = v; }
                     __syncthreads();
                     u64 higher = 0ull, equal = 0ull;
@@ -547,14 +544,14 @@ __global__ __launch_bounds__(CT, 2) void sample_filtered_cluster_kernel(const fl
     u64 tie_keep = keep_k, n_ties = use_k ? n_ties_k : 0ull;
     if (use_p) {
         // the largest threshold whose upper mass reaches top_p * mass
-        const u64 w_k = use_k ? fixed_weight(key_value(kth), mx, inv_t) : 0ull;
+        const u64 w_k = use_k ? fixed_weight(kth, mx, inv_t) : 0ull;
         u64 target = 0ull, above, inside;
         thr = select([&](u64 mass_above_k) {
             const u64 mass = mass_above_k + (use_k ? keep_k * w_k : 0ull);
             target = (u64)((double)top_p * (double)mass);
             return target;
         }, true, kth, use_k ? n_above_k + n_ties_k : ~0ull, above, inside);
-        const u64 w_t = fixed_weight(key_value(thr), mx, inv_t);
+        const u64 w_t = fixed_weight(thr, mx, inv_t);
         n_ties = thr == kth && use_k ? n_ties_k : w_t > 0ull ? inside / w_t : 0ull;
         u64 need = 1ull;
         if (target > above && w_t > 0ull) need = (target - above + w_t - 1ull) / w_t;
@@ -609,7 +606,7 @@ __global__ __launch_bounds__(CT, 2) void sample_filtered_cluster_kernel(const fl
         }
         out[r] = pick;
     }
-    if (kept == 0ull && rank == 0 && tid == 0) out[r] = 0;     // nothing kept (a row of NaNs): id 0, as the greedy path
+    if (kept == 0ull && rank == 0 && tid == 0) out[r] = 0;     // nothing kept (a row of NaNs or -inf): id 0, as the greedy path
     cluster_sync_all();          // nobody leaves while its shared memory may still be read
     pdl_trigger();
 }
