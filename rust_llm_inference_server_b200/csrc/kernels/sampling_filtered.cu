@@ -521,7 +521,9 @@ __global__ __launch_bounds__(CT, 2) void sample_filtered_cluster_kernel(const fl
                 const uint32_t wide = (1u << shift) - 1u;
                 lo = max(lo, hi > wide ? hi - wide : 0u);
                 if (shift == 0) { inside = sh.inside; return hi; }
-                try_list = true;
+                // (counts say how many are left: thousands of equal tokens would queue up at the list's counter for nothing;
+                // 64 rows of 32,000 logits in steps of one, top-k 5,000: 61 us with the attempt, 46 without)
+                try_list = masses || sh.inside <= LIST;
             } else {                                // further down than the bins reach (never within an interval narrowed before)
                 above += all;
                 const uint32_t covered = shift >= 22 ? 0xFFFFFFFFu : ((uint32_t)BINS << shift) - 1u;
