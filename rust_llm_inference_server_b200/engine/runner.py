@@ -110,7 +110,7 @@ class ModelRunner:
         self._meta_host = None
         self._meta_dev = None
         # CUDA graphs of decode-only steps, by (batch, wanted rows, split plan); dropped whenever
-        # a buffer they point into is replaced by a larger one
+        # a buffer they point into is replaced by a larger one: one that was asked for while a graph was recorded
         self.use_graphs = True
         self._graphs: dict = {}
         self._graph_seen: dict = {}     # key -> times seen before its capture
@@ -118,6 +118,7 @@ class ModelRunner:
         self._upload_done = None
         self._graph_launches = 0
         self._capturing = False
+        self._recorded: set = set()     # names of those buffers
 
     # ---- scratch memory that keeps its address while it is large enough ----
 
@@ -125,6 +126,8 @@ class ModelRunner:
         n = 1
         for s in shape:
             n *= int(s)
+        if self._capturing:
+            self._recorded.add(name)
         buf = self._ws.get(name)
         if buf is None or buf.dtype != dtype or buf.numel() < n:
             if self._capturing:
@@ -132,13 +135,15 @@ class ModelRunner:
                 # which sizes the buffer, and the shape is captured the next time it comes)
                 raise _CaptureAbort(name)
             cap = max(n, 2 * buf.numel() if buf is not None and buf.dtype == dtype else n)
-            self._drop_graphs()         # captured graphs point at the old buffer
+            if name in self._recorded:
+                self._drop_graphs()     # captured graphs point at the old buffer
             buf = torch.empty((cap,), dtype=dtype, device=self.device)
             self._ws[name] = buf
         return buf[:n].view(*shape)
 
     def _drop_graphs(self) -> None:
         self._graphs.clear()
+        self._recorded.clear()
         self._graph_pool = None         # a pool dies with its last graph; the next capture opens a new one
 
     def _meta(self, n: int):
