@@ -77,20 +77,31 @@ template <typename T, bool SILU> __device__ __forceinline__ void load_piece(cons
     }
 }
 
-// rows x cols of x into shared memory as they lie, [row][cols + 4]; rows from n on become zeros; `scale` a row.
-template <typename T, bool SILU, int COLS, typename Scale>
-__device__ __forceinline__ void stage(float* dst, const T* x, long long stride, int n, Scale scale) {
+// rows x cols of x into shared memory as they lie, [row][cols + 4]; rows from n on become zeros; `scale` a row.  FINITE: what is
+// not finite becomes 0 there; whether this thread met some.
+template <typename T, bool SILU, int COLS, bool FINITE = false, typename Scale>
+__device__ __forceinline__ bool stage(float* dst, const T* x, long long stride, int n, Scale scale) {
     constexpr int N = 16 / sizeof(T), P = COLS / N;
+    bool spoilt = false;
 #pragma unroll 4
     for (int i = threadIdx.x; i < CHUNK * P; i += THREADS) {
         const int r = i / P, c = i % P * N;
         float v[N];
         load_piece<T, SILU>(x + (size_t)r * stride + c, r < n, v);
+        if (FINITE) {
+#pragma unroll
+            for (int u = 0; u < N; ++u) {
+                const bool finite = fabsf(v[u]) < INFINITY;
+                spoilt |= !finite;
+                v[u] = finite ? v[u] : 0.f;
+            }
+        }
         const float f = scale(r);
 #pragma unroll
         for (int u = 0; u < N; u += 4)
             *reinterpret_cast<float4*>(dst + r * (COLS + 4) + c + u) = make_float4(v[u] * f, v[u + 1] * f, v[u + 2] * f, v[u + 3] * f);
     }
+    return spoilt;
 }
 // The same turned: [col][64 rows + 4].  A warp takes 16 rows x 2 pieces (bf16) or 8 x 4 (float): whole sectors of memory, and
 // no more than two of its writes in a bank.
@@ -232,8 +243,9 @@ __global__ __launch_bounds__(THREADS) void chunk_outputs_kernel(const Rows in, c
         if (threadIdx.x <= CHUNK) pw[threadIdx.x] = power(g, threadIdx.x);
         stage_turned<T, SILU, D>(qt, x + in.q_off + h * D, in.stride, n);
         stage_turned<T, SILU, D>(xt, x + in.k_off + h * D, in.stride, n);
-        stage<T, SILU, VT>(vs, x + in.v_off + h * dv + v0, in.stride, n, [](int) { return 1.0f; });
-        __syncthreads();
+        // (the weights of later keys are zeros, and a zero times what is not finite would reach tokens that came before it)
+        const bool met = stage<T, SILU, VT, true>(vs, x + in.v_off + h * dv + v0, in.stride, n, [](int) { return 1.0f; });
+        const bool spoilt = __syncthreads_or(met);
         const int ty = thread_row(), tx = thread_col();
         u64 acc[8][2];
         clear(acc);
@@ -267,6 +279,22 @@ __global__ __launch_bounds__(THREADS) void chunk_outputs_kernel(const Rows in, c
         for (int i = 0; i < 8; ++i) {
             const int q = i / 4 * 32 + ty * 4 + i % 4;
             if (q < n) *reinterpret_cast<ulonglong2*>(out + (size_t)(rows.x + q) * nh * dv + h * dv + v0 + tx * 4) = *reinterpret_cast<ulonglong2*>(acc[i]);
+        }
+        if (spoilt) {           // values that are not finite, for the tokens from theirs on
+            __syncthreads();
+            stage<T, SILU, VT>(vs, x + in.v_off + h * dv + v0, in.stride, n, [](int) { return 1.0f; });
+            __syncthreads();
+#pragma unroll 1
+            for (int i = threadIdx.x; i < n * VT; i += THREADS) {
+                const int q = i / VT, c = i % VT;
+                float more = 0.f;
+#pragma unroll 1
+                for (int k = 0; k <= q; ++k) {
+                    const float v = vs[k * (VT + 4) + c];
+                    if (!(fabsf(v) < INFINITY)) more = fmaf(pt[k * LDT + q], v, more);
+                }
+                if (more != 0.f) out[(size_t)(rows.x + q) * nh * dv + h * dv + v0 + c] += more;      // (after the block's barriers)
+            }
         }
     }
     pdl_trigger();   // the next kernel of the stream may start its launch

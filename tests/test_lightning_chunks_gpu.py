@@ -66,3 +66,31 @@ def test_long_portions_go_by_chunks_and_short_ones_token_by_token():
     from rust_llm_inference_server_b200.ops import _lightning_chunks_pay as pays
     assert pays(2048, 1, 2048, 2048, 148) and pays(2048, 4, 512, 2048, 148) and pays(898, 4, 700, 2048, 148)
     assert not pays(128, 1, 128, 2048, 148) and not pays(8, 8, 1, 2048, 148) and not pays(540, 41, 500, 2048, 148)
+
+
+@pytest.mark.parametrize("at", [0, 5, 63, 64, 70])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("part", ["q", "k", "v"])
+def test_a_token_sees_nothing_of_what_comes_after_it(monkeypatch, at, value, part):
+    """A number that is not finite in a token's query, key or value: the outputs before it are those without it, bit for bit."""
+    from rust_llm_inference_server_b200 import ops
+    monkeypatch.setattr(ops, "_lightning_chunks_pay", lambda *a: True)
+    H, d, T = 2, 64, 100
+    st, g = Step([T], [0]), torch.Generator().manual_seed(at)
+    rows = torch.randn(T, 3 * H * d, generator=g).cuda()
+    decay = torch.tensor([0.9, 0.5], device="cuda")
+    outs = []
+    for spoilt in (False, True):
+        if spoilt:
+            rows[at, {"q": 0, "k": H * d, "v": 2 * H * d}[part] + 3] = value              # (an entry of the first head)
+        out, state = torch.zeros(T, H * d, device="cuda"), torch.zeros(3, H, d, d, device="cuda")
+        ops.recurrence_scan(rows, out, state, decay, st, H, d, d)
+        outs.append(out)
+    clean, out = outs
+    assert torch.equal(out[:at], clean[:at]) and torch.equal(out[:, d:], clean[:, d:])
+    assert not bool(torch.isfinite(out[at, :d]).all())
+    if part == "q":
+        assert torch.equal(out[at + 1:], clean[at + 1:])
+    elif part == "v":               # one column of the values
+        others = [c for c in range(d) if c != 3]
+        assert torch.equal(out[:, others], clean[:, others])
