@@ -39,9 +39,13 @@ struct Args {
 
 __device__ __forceinline__ int first_key(int pos, int window) { return window > 0 ? max(0, pos - window + 1) : 0; }
 
+// What scores are taken from before expf: their running maximum, or 0 while all of them are -inf (whose weights are 0 then, not the NaN
+// of -inf - -inf).
+__device__ __forceinline__ float reference_score(float top) { return top == -INFINITY ? 0.f : top; }
+
 // Folds the piece (m, l, a) into the ones before it (M, L, A).
 template <int DL> __device__ __forceinline__ void fold(float& M, float& L, float (&A)[DL], float m, float l, const float (&a)[DL]) {
-    const float top = fmaxf(M, m), c0 = expf(M - top), c1 = expf(m - top);
+    const float top = fmaxf(M, m), from = reference_score(top), c0 = expf(M - from), c1 = expf(m - from);
     L = __fmaf_rn(L, c0, __fmul_rn(l, c1));
 #pragma unroll
     for (int i = 0; i < DL; ++i) A[i] = __fmaf_rn(A[i], c0, __fmul_rn(a[i], c1));
@@ -173,9 +177,9 @@ __global__ __launch_bounds__((SPLIT ? MAX_GROUP : PROMPT_WARPS) * 32) void attn_
                     const bool valid = key >= row_lo[r] && key <= row_pos[r];
                     // a page the host did not map: make it visible
                     const float sc = !valid ? -INFINITY : there ? __fmul_rn(s[r], p.scale) : NAN;
-                    const float m_new = fmaxf(m[r], warp_max(sc));
-                    w[r] = valid ? expf(sc - m_new) : 0.f;
-                    const float corr = expf(m[r] - m_new);
+                    const float m_new = fmaxf(m[r], warp_max(sc)), from = reference_score(m_new);
+                    w[r] = valid ? expf(sc - from) : 0.f;
+                    const float corr = expf(m[r] - from);
                     l[r] = __fmaf_rn(l[r], corr, warp_sum(w[r]));
 #pragma unroll
                     for (int i = 0; i < DL; ++i) acc[r][i] *= corr;
@@ -198,7 +202,7 @@ __global__ __launch_bounds__((SPLIT ? MAX_GROUP : PROMPT_WARPS) * 32) void attn_
             if (!SPLIT && ((kb + BLOCK) % PIECE == 0 || b == blocks - 1)) {
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
-                    if (m[r] == -INFINITY && l[r] == 0.f) continue;             // the row sees nothing of this piece
+                    if (m[r] == -INFINITY && l[r] == 0.f) continue;             // the row sees nothing of this piece, or only scores of -inf
                     if (begun[r]) {
                         fold<DL>(M[r], L[r], A[r], m[r], l[r], acc[r]);
                     } else {

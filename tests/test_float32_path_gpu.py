@@ -114,3 +114,24 @@ def test_pieces_cover_every_context():
             touched = max(p // piece - (max(0, p - window + 1) if window else 0) // piece + 1 for p in range(ctx))
             n = ops.attention_f32_pieces(ctx, window)
             assert n >= touched and n & (n - 1) == 0 and n < 2 * touched + 2
+
+
+@pytest.mark.parametrize("lo,hi", [(0, 32), (256, 288), (256, 512), (200, 300), (0, 512)])
+def test_float32_attention_passes_by_keys_whose_scores_are_minus_infinity(lo, hi):
+    """Whole blocks and pieces of such keys, at the start and behind others: what is left is the softmax over the other keys."""
+    from rust_llm_inference_server_b200 import ops
+    n = 600
+    g = torch.Generator().manual_seed(lo + hi)
+    tables = torch.arange(40, dtype=torch.int32).view(1, 40)
+    kc, vc, q = torch.randn(40, 1, 16, 64, generator=g), torch.randn(40, 1, 16, 64, generator=g), torch.randn(n, 64, generator=g)
+    q[:, 0] = 1.0
+    kc.view(640, 64)[lo:hi, 0] = -torch.inf
+    rows = list(range(hi, n))                                   # (the queries before them may see nothing else)
+    outs = [ops.attention(q.cuda(), kc.cuda(), vc.cuda(), torch.zeros(n, 64, device="cuda"), Step([n], [n], tables, single), 0, 1, 1, 64, 16, 0.125, 0)
+            for single in (False, True)]
+    s = (q.double() @ kc.view(640, 64)[:n].double().t()) * 0.125
+    s = s.masked_fill(torch.arange(n)[:, None] < torch.arange(n)[None], -torch.inf)
+    want = torch.softmax(s[rows], dim=1) @ vc.view(640, 64)[:n].double()
+    for out in outs:
+        assert (out.cpu().double()[rows] - want).abs().max() <= 2e-5
+    assert torch.equal(outs[0][rows], outs[1][rows])
