@@ -43,9 +43,9 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
 
 // A CTA takes TOK tokens; a warp forms ROWS rows of W_r against all of the CTA's tokens, so the matrix is read once a CTA (the
 // tokens' rows come back from the first-level cache, once for ROWS rows) and the rows' sums run side by side; then
-// one warp a token chooses.  With 8 tokens the reads of the tokens' rows are the bound, so a warp takes four rows of W_r at
+// one warp a token chooses.  With 8 tokens the reads of the tokens' rows are the bound, so a warp takes up to four rows of W_r at
 // once, and two CTAs share an SM (2,048 tokens of 2,048, 32 experts and a shared gate: 57 us with a warp a row, whose 33rd
-// row was a second round, 44 with two rows a warp, 31 with four).
+// row was a second round, 44 with two rows a warp, 31 with four); as many as leave each of its eight warps some.
 template <typename T, int TOK, int ROWS>
 __global__ __launch_bounds__(TOK == 8 ? 512 : 1024) void moe_route_kernel(
     const T* __restrict__ x, const float* __restrict__ w_router, const float* __restrict__ correction,
@@ -449,15 +449,25 @@ extern "C" int rlis_moe_route(const void* x, const float* w_router, const float*
     if (smem > 48 * 1024) return RLIS_ERR_UNSUPPORTED;
     const unsigned blocks = (unsigned)((n_tokens + tok - 1) / tok);
     const int rows = n_experts + (shared_gate != nullptr ? 1 : 0);
-    // a warp four rows of the matrix with eight tokens, one otherwise; at least a warp a token
-    const int warps = tok == 8 ? (rows + 3) / 4 : rows, most = tok == 8 ? 16 : 32;
+    // Rows of the matrix a warp: with eight tokens four, two or one, so that at least eight warps (one a token is launched in
+    // any case) have some; with four, 8 experts left six of eight warps idle (8,192 tokens of 1,024: router and sort 29 us before, 32 with four rows a warp).
+    const int per = tok == 8 ? (rows >= 32 ? 4 : rows >= 16 ? 2 : 1) : 1;
+    const int warps = (rows + per - 1) / per, most = tok == 8 ? 16 : 32;
     const unsigned threads = 32u * (unsigned)(warps < most ? (warps < tok ? tok : warps) : most);
-#define RLIS_ROUTE(T, TOK) rlis_launch(moe_route_kernel<T, TOK, (TOK == 8 ? 4 : 1)>, blocks, threads, smem, stream, (const T*)x, w_router, correction, \
+#define RLIS_ROUTE(T, TOK, ROWS) rlis_launch(moe_route_kernel<T, TOK, ROWS>, blocks, threads, smem, stream, (const T*)x, w_router, correction, \
                                        top_idx, top_w, shared_gate, n_tokens, width, n_experts, top, route_scale, \
                                        router_bias, scoring, n_groups, keep_groups, normalize)
-    if (dtype == RLIS_F32) { if (tok == 8) RLIS_ROUTE(float, 8); else RLIS_ROUTE(float, 1); }
-    else if (dtype == RLIS_BF16) { if (tok == 8) RLIS_ROUTE(bf16, 8); else RLIS_ROUTE(bf16, 1); }
+#define RLIS_ROUTE_T(T)                             \
+    do {                                            \
+        if (tok != 8) RLIS_ROUTE(T, 1, 1);          \
+        else if (per == 4) RLIS_ROUTE(T, 8, 4);     \
+        else if (per == 2) RLIS_ROUTE(T, 8, 2);     \
+        else RLIS_ROUTE(T, 8, 1);                   \
+    } while (0)
+    if (dtype == RLIS_F32) RLIS_ROUTE_T(float);
+    else if (dtype == RLIS_BF16) RLIS_ROUTE_T(bf16);
     else return RLIS_ERR_UNSUPPORTED;
+#undef RLIS_ROUTE_T
 #undef RLIS_ROUTE
     return RLIS_LAUNCH_CHECK();
 }
@@ -468,8 +478,10 @@ extern "C" int rlis_moe_align(const int* top_idx, int* sorted_pair, int* pair_sl
     if (n_experts <= 0 || n_experts > 4096 || tile_rows <= 0 || tile_rows % BM != 0 ||
         max_tiles < (n_pairs + tile_rows - 1) / tile_rows)
         return RLIS_ERR_UNSUPPORTED;
-    // a set of counters a warp up to 256 experts (32 KB of them), fewer sets beyond (4,096 experts: 2)
-    const int copies = n_experts <= 256 ? 32 : 8192 / n_experts;
+    // Sets of counters: one for 64 pairs, as far as there are warps and 32 KB (256 experts: 32 sets, 4,096: 2).  Few pairs do not
+    // meet often, and every set has to be emptied and added up; 2 pairs on 8 experts: router and sort 5.7 us with one set, 7.8 with 32.
+    const int room = n_experts <= 256 ? 32 : 8192 / n_experts, sets = (n_pairs + 63) / 64;
+    const int copies = sets < room ? sets : room;
     rlis_launch(moe_align_kernel, 1, 1024, (size_t)(copies + 1) * n_experts * sizeof(int), stream, top_idx, sorted_pair, pair_slot,
                 tile_expert, n_pairs, n_experts, max_tiles, tile_rows, copies);
     return RLIS_LAUNCH_CHECK();

@@ -14,9 +14,11 @@ class Step:
 
 
 # pairs below, at and beyond what the sort's threads keep in registers (8,192); one set of counters a warp up to 256 experts
-# and fewer beyond; router rows (with and without a shared gate's) that fill a warp's four or do not
+# and fewer beyond; router rows (with and without a shared gate's) one, two and four a warp, that fill
+# the last warp's or do not; few pairs, with fewer sets
 @pytest.mark.parametrize("T,W,E,top,shared,crowd", [(64, 64, 3, 2, True, False), (2048, 64, 32, 4, True, False), (2049, 68, 31, 4, False, False),
-                                                    (5000, 36, 255, 6, False, False), (900, 40, 512, 10, False, False), (3000, 30, 5, 3, True, True),
+                                                    (5000, 36, 255, 6, False, False), (900, 40, 512, 10, False, False), (3000, 30, 5, 3, True, True), (300, 64, 16, 4, False, False),
+                                                    (200, 36, 30, 5, True, False), (64, 32, 15, 3, False, False), (70, 32, 4096 // 16, 1, False, False),
                                                     (63, 32, 300, 2, False, False), (1, 64, 32, 4, True, False)])
 def test_every_pair_has_a_slot_of_its_expert_and_every_tile_one_expert(T, W, E, top, shared, crowd):
     from rust_llm_inference_server_b200 import ops
