@@ -951,9 +951,16 @@ template <int MODE, typename T>
 static int launch_typed(const Args& g, cudaStream_t stream) {
     const Shape& z = g.z;
     const long long tail_off = (long long)z.nh * z.dv * z.d;
-    // four tokens a warp in long steps; single tokens and short portions want a warp each
-    const int toks = g.n_tokens >= 64 ? 4 : 1;
-    const long long units = (long long)((g.n_tokens + toks - 1) / toks) * (2 * z.n_qk + z.nh + (MODE == CHANNEL_DECAY ? z.nh : 0) + 1);
+    // Four tokens a warp where that leaves 16 warps and more an SM, one otherwise: 64 single tokens of 8 heads of 64 took 14.2 us one by one and 17.6 in fours, 256 tokens of 32 heads of 128 118 and 107.
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    const long long per_token = 2 * z.n_qk + z.nh + (MODE == CHANNEL_DECAY ? z.nh : 0) + 1;
+    const int toks = (g.n_tokens + 3LL) / 4 * per_token >= 16LL * sms ? 4 : 1;
+    const long long units = (g.n_tokens + toks - 1LL) / toks * per_token;
     if (units > 0x7fffffffLL) return RLIS_ERR_UNSUPPORTED;
     // four channels a lane need every row, head, tap and tail to start on a boundary of four entries
     const bool quads = z.taps == 4 && z.d % 4 == 0 && z.dv % 4 == 0 && z.q_at % 4 == 0 && z.k_at % 4 == 0 && z.v_at % 4 == 0 &&
@@ -969,12 +976,6 @@ static int launch_typed(const Args& g, cudaStream_t stream) {
 #undef RLIS_PREPARE
     dim3 grid(g.n_seqs, z.nh, (z.dv + COLS - 1) / COLS);
     // few CTAs that run long: shared memory asked for beyond the need keeps them one an SM
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    }
     const bool spread = (long long)grid.x * grid.y * grid.z <= sms;
     const int e = (z.d + SLICES - 1) / SLICES;
 #define RLIS_SCAN(E)                                                                                                     \
