@@ -5,7 +5,8 @@
 // latents go through the key and value maps once (one library product over all heads), and a pair costs dim + rot + v_dim = 320.
 // 2,048 tokens, 16 heads: 362 us on the rows, 93 us here and 16 for the rows' copy and the maps.
 //
-//   latent_rows: the cached rows of all the step's contexts, one request after the other, out of the pages
+//   latent_rows: the cached rows that the step's tokens see (whole contexts, or from the window's first key on), one request after the
+//     other, out of the pages
 //   latent_heads: one head x 64 tokens of one request a CTA of 4 warps x 16 rows, mma.sync m16n8k16 with float32 sums, keys and values in
 //     tiles of 64 through two stages of 16-byte asynchronous copies: a key is its head's `dim` columns of the mapped rows
 //     and the row's rotated part, which all heads share.  Rows padded by 8 elements, so that ldmatrix is free of bank
@@ -26,17 +27,33 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-// out[i, :] = row of the i-th key of the step's contexts, which stand one after the other; a warp a row, 16 bytes a lane.
-__global__ __launch_bounds__(256) void latent_rows_kernel(const uint4* __restrict__ cache, uint4* __restrict__ out, const int* __restrict__ ctx_lens,
-                                                          const int* __restrict__ block_tables, int max_blocks, int n_seqs, int page_size, int vecs, int total) {
+// A request's first key that a token of the step sees (the one before it by `window` - 1 keys, or key 0).
+__device__ __forceinline__ int first_formed(int ctx, int q_len, int window) { return window > 0 ? max(0, ctx - q_len - window + 1) : 0; }
+
+// The i-th key that the step sees, requests one after the other: its latent to lat[i], its rotated part to rot[i]; a warp a row,
+// 16 bytes a lane.
+__global__ __launch_bounds__(256) void latent_rows_kernel(const uint4* __restrict__ cache, uint4* __restrict__ lat, uint4* __restrict__ rot,
+                                                          const int* __restrict__ cu_seqlens, const int* __restrict__ ctx_lens,
+                                                          const int* __restrict__ block_tables, int max_blocks, int n_seqs, int page_size, int lat_vecs, int rot_vecs,
+                                                          int window, int total) {
     pdl_wait();
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (i < total) {
-        int key = i, b = 0;
-        while (b < n_seqs - 1 && key >= ctx_lens[b]) key -= ctx_lens[b++];
-        const int page = key < ctx_lens[b] ? block_tables[(size_t)b * max_blocks + key / page_size] : -1;
-        const uint4* src = cache + ((size_t)(page < 0 ? 0 : page) * page_size + key % page_size) * vecs;
-        for (int v = lane; v < vecs; v += 32) out[(size_t)i * vecs + v] = page < 0 ? make_uint4(0u, 0u, 0u, 0u) : src[v];
+        int key = i, b = 0, lo, n;
+        for (;; key -= n, ++b) {
+            const int ctx = ctx_lens[b];
+            lo = first_formed(ctx, cu_seqlens[b + 1] - cu_seqlens[b], window);
+            n = ctx - lo;
+            if (key < n || b == n_seqs - 1) break;
+        }
+        const int page = key < n ? block_tables[(size_t)b * max_blocks + (lo + key) / page_size] : -1;
+        const int vecs = lat_vecs + rot_vecs;
+        const uint4* src = cache + ((size_t)(page < 0 ? 0 : page) * page_size + (lo + key) % page_size) * vecs;
+        for (int v = lane; v < vecs; v += 32) {
+            const uint4 x = page < 0 ? make_uint4(0u, 0u, 0u, 0u) : src[v];
+            if (v < lat_vecs) lat[(size_t)i * lat_vecs + v] = x;
+            else rot[(size_t)i * rot_vecs + v - lat_vecs] = x;
+        }
     }
     pdl_trigger();
 }
@@ -45,14 +62,14 @@ struct Args {
     const bf16* q;              // [T, nh * (DIM + ROT)], q_stride apart: the plain parts are read here
     long long q_stride;
     const bf16* q_rot;          // [T, nh * ROT]: the rotated parts
-    const bf16* kv;             // [context keys, nh * DIM | nh * DV]
-    const bf16* rows;           // [context keys, rank + ROT]
+    const bf16* kv;             // [keys that the step sees, nh * DIM | nh * DV]
+    const bf16* rot;            // [keys that the step sees, ROT]
     bf16* out;                  // [T, nh * DV]
     const float* sinks;
     const int* tiles;
     const int* cu_seqlens;
     const int* ctx_lens;
-    int nh, rank;
+    int nh;
     float scale;
     int window;
     const bf16* gate;
@@ -69,8 +86,8 @@ __global__ __launch_bounds__(THREADS, 2) void latent_heads_kernel(const Args p) 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
     const int b = p.tiles[2 * blockIdx.y], t0 = p.tiles[2 * blockIdx.y + 1], head = blockIdx.x, nh = p.nh;
     const int q_start = p.cu_seqlens[b], q_len = p.cu_seqlens[b + 1] - q_start, start_pos = p.ctx_lens[b] - q_len;
-    size_t key_base = 0;
-    for (int o = 0; o < b; ++o) key_base += p.ctx_lens[o];
+    long long key_base = -first_formed(p.ctx_lens[b], q_len, p.window);          // where the request's key 0 would lie
+    for (int o = 0; o < b; ++o) key_base += p.ctx_lens[o] - first_formed(p.ctx_lens[o], p.cu_seqlens[o + 1] - p.cu_seqlens[o], p.window);
 
     const int r0 = warp * 16 + g, ti0 = t0 + r0, ti1 = ti0 + 8;       // this lane's two rows of the tile
     const bool rv0 = ti0 < q_len, rv1 = ti1 < q_len;
@@ -93,25 +110,23 @@ __global__ __launch_bounds__(THREADS, 2) void latent_heads_kernel(const Args p) 
     const int k_hi = start_pos + min(t0 + BM, q_len);                                  // exclusive
     const int k_lo = p.window > 0 ? max(0, start_pos + t0 - p.window + 1) : 0;
     const int kt0 = k_lo / BN, kt1 = (k_hi + BN - 1) / BN;
-    const size_t kv_row = (size_t)nh * (DIM + DV);
-    const int row_width = p.rank + ROT;
-    const bf16* kbase = p.kv + key_base * kv_row + head * DIM;
-    const bf16* vbase = p.kv + key_base * kv_row + (size_t)nh * DIM + head * DV;
-    const bf16* rbase = p.rows + key_base * row_width + p.rank;
+    const long long kv_row = (long long)nh * (DIM + DV);
+    const bf16* kbase = p.kv + head * DIM;
+    const bf16* vbase = p.kv + (size_t)nh * DIM + head * DV;
 
     auto issue = [&](int kt, int stage) {
         bf16* ks_ = sbase + stage * STAGE;
         bf16* vs_ = ks_ + BN * SK;
-        auto copy = [&](bf16* dst, int pitch, const bf16* src, size_t src_row, int pieces) {
+        auto copy = [&](bf16* dst, int pitch, const bf16* src, long long src_row, int pieces) {
 #pragma unroll
             for (int i = 0; i < BN * pieces / THREADS; ++i) {
                 const int idx = threadIdx.x + i * THREADS, kin = idx / pieces, c16 = idx % pieces * 8, key = kt * BN + kin;
                 const bool valid = key < k_hi && key >= k_lo;
-                cp_async16(dst + kin * pitch + c16, src + (valid ? (size_t)key * src_row + c16 : 0), valid);
+                cp_async16(dst + kin * pitch + c16, src + (key_base + (valid ? key : k_lo)) * src_row + c16, valid);
             }
         };
         copy(ks_, SK, kbase, kv_row, DIM / 8);
-        copy(ks_ + DIM, SK, rbase, row_width, ROT / 8);
+        copy(ks_ + DIM, SK, p.rot, ROT, ROT / 8);
         copy(vs_, SV, vbase, kv_row, DV / 8);
         cp_async_commit();
     };
@@ -237,30 +252,33 @@ __global__ __launch_bounds__(THREADS, 2) void latent_heads_kernel(const Args p) 
 
 extern "C" int rlis_latent_heads_takes(int dim, int rot, int v_dim, int rank) { return dim == 128 && rot == 64 && v_dim == 128 && rank > 0 && rank % 8 == 0; }
 
-// cache [pages, page_size, width] -> out [total, width] (bfloat16, width a multiple of 8): the first ctx_lens[b] rows of every request b in turn.
-extern "C" int rlis_latent_rows(const void* cache, void* out, const int* ctx_lens, const int* block_tables, int max_blocks, int n_seqs, int page_size,
-                                int width, int total, cudaStream_t stream) {
+// cache [pages, page_size, rank + rot_width] -> lat [total, rank] and rot [total, rot_width] (bfloat16, both widths multiples of 8): for every request in
+// turn the cached rows from the first one on that its first token of the step sees (with a window W: W - 1 keys back).
+extern "C" int rlis_latent_rows(const void* cache, void* lat, void* rot, const int* cu_seqlens, const int* ctx_lens, const int* block_tables, int max_blocks,
+                                int n_seqs, int page_size, int rank, int rot_width, int window, int total, cudaStream_t stream) {
     if (total <= 0 || n_seqs <= 0) return 0;
-    if (width % 8 || page_size <= 0 || ((reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) & 15)) return RLIS_ERR_UNSUPPORTED;
-    rlis_launch(latent_rows_kernel, (total + 7) / 8, 256, 0, stream, (const uint4*)cache, (uint4*)out, ctx_lens, block_tables, max_blocks, n_seqs, page_size,
-                width / 8, total);
+    if (rank <= 0 || rank % 8 || rot_width % 8 || page_size <= 0 ||
+        ((reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(lat) | reinterpret_cast<uintptr_t>(rot)) & 15))
+        return RLIS_ERR_UNSUPPORTED;
+    rlis_launch(latent_rows_kernel, (total + 7) / 8, 256, 0, stream, (const uint4*)cache, (uint4*)lat, (uint4*)rot, cu_seqlens, ctx_lens, block_tables, max_blocks,
+                n_seqs, page_size, rank / 8, rot_width / 8, window, total);
     return RLIS_LAUNCH_CHECK();
 }
 
-// tiles: int32 [n_tiles][2] = (batch entry, first token of the tile within the entry's portion); kv [context keys, nh * dim | nh * v_dim] and rows
-// [context keys, rank + rot] in the order of rlis_latent_rows; gate (null: none): logits, head h of token t at gate[t * gate_stride + h].
-extern "C" int rlis_attention_latent_heads(const void* q, long long q_stride, const void* q_rot, const void* kv, const void* rows, void* out,
+// tiles: int32 [n_tiles][2] = (batch entry, first token of the tile within the entry's portion); kv [keys, nh * dim | nh * v_dim] and rot
+// [keys, rot] in the order of rlis_latent_rows with the same window; gate (null: none): logits, head h of token t at gate[t * gate_stride + h].
+extern "C" int rlis_attention_latent_heads(const void* q, long long q_stride, const void* q_rot, const void* kv, const void* rot_keys, void* out,
                                            const float* sinks, const int* tiles, int n_tiles, const int* cu_seqlens, const int* ctx_lens, int nh, int dim,
                                            int rot, int v_dim, int rank, float scale, int window, const void* gate, long long gate_stride, cudaStream_t stream) {
     if (n_tiles <= 0) return 0;
     if (!rlis_latent_heads_takes(dim, rot, v_dim, rank) || nh <= 0 || n_tiles > 65535 || q_stride % 2 || (reinterpret_cast<uintptr_t>(q) & 3) ||
-        ((reinterpret_cast<uintptr_t>(kv) | reinterpret_cast<uintptr_t>(rows)) & 15))
+        ((reinterpret_cast<uintptr_t>(kv) | reinterpret_cast<uintptr_t>(rot_keys)) & 15))
         return RLIS_ERR_UNSUPPORTED;
     constexpr int DIM = 128, ROT = 64, DV = 128, smem = 2 * BN * (DIM + ROT + 8 + DV + 8) * 2;
     const cudaError_t e = cudaFuncSetAttribute(latent_heads_kernel<DIM, ROT, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
-    const Args p = {(const bf16*)q, q_stride, (const bf16*)q_rot, (const bf16*)kv, (const bf16*)rows, (bf16*)out, sinks, tiles, cu_seqlens, ctx_lens,
-                    nh, rank, scale, window, (const bf16*)gate, gate_stride};
+    const Args p = {(const bf16*)q, q_stride, (const bf16*)q_rot, (const bf16*)kv, (const bf16*)rot_keys, (bf16*)out, sinks, tiles, cu_seqlens, ctx_lens,
+                    nh, scale, window, (const bf16*)gate, gate_stride};
     rlis_launch(latent_heads_kernel<DIM, ROT, DV>, dim3(nh, n_tiles), THREADS, smem, stream, p);
     return RLIS_LAUNCH_CHECK();
 }

@@ -794,16 +794,22 @@ def attention_latent(qa: torch.Tensor, cache: torch.Tensor, out: torch.Tensor, s
 LATENT_HEADS_BYTES = 1 << 28     # of formed keys and values in a step's scratch memory; longer contexts stay on the latent rows
 
 
-def latent_heads_takes(step, dtype, n_heads: int, dim: int, rot: int, v_dim: int, rank: int) -> bool:
+def _latent_heads_keys(step, window: int) -> int:
+    """The keys that the step's tokens see, all requests together: whole contexts, or what a window leaves of them."""
+    return sum(n + (min(s, window - 1) if window else s) for s, n in zip(step.starts, step.q_lens))
+
+
+def latent_heads_takes(step, dtype, n_heads: int, dim: int, rot: int, v_dim: int, rank: int, window: int = 0) -> bool:
     """Whether this step's attention over latents goes to `attention_latent_heads`: bfloat16 portions of prompts and nothing else, in
     sizes that the kernel has.  It was the faster one at every size tried (a layer's mixer, 16 heads, on the rows and with heads formed, us: one
     prompt of 17 tokens 42 and 38, 128 54 and 41, 512 97 and 63, 2,048 460 and 190; 16 portions of 20 behind 1,000 cached 234 and 157; 17
-    behind 4,096 408 and 187, 64 behind 16,384 1510 and 634), so only the memory that the formed keys and values take limits it."""
+    behind 4,096 408 and 187, 64 behind 16,384 1510 and 634), so only
+    the memory that the formed keys and values take limits it: those in reach of the window, as the rows' kernel reads them."""
     starts, lens = getattr(step, "starts", None), getattr(step, "q_lens", None)
     if not LATENT_MMA or dtype != torch.bfloat16 or not starts or not lens or step.n_decode or not step.n_prefill_tiles:
         return False
-    keys = sum(starts) + sum(lens)
-    return bool(_latent_heads_sizes(dim, rot, v_dim, rank)) and 2 * keys * n_heads * (dim + v_dim) <= LATENT_HEADS_BYTES
+    return (bool(_latent_heads_sizes(dim, rot, v_dim, rank))
+            and 2 * _latent_heads_keys(step, int(window)) * n_heads * (dim + v_dim) <= LATENT_HEADS_BYTES)
 
 
 @functools.lru_cache(maxsize=None)
@@ -833,15 +839,16 @@ def attention_latent_heads(q: torch.Tensor, q_rot: torch.Tensor, cache: torch.Te
             raise KernelError("attention_latent_heads: the gate must be [T, nh] rows with unit stride in bfloat16")
         gp, gs = gate.data_ptr(), gate.stride(0)
     tables = step.block_tables[group]
-    keys = sum(s + n for s, n in zip(step.starts, step.q_lens))
-    rows = step.buffer("latent_rows", (keys, dk), torch.bfloat16)
-    check(lib().rlis_latent_rows(cache.data_ptr(), rows.data_ptr(), step.ctx_lens.data_ptr(), tables.data_ptr(), tables.shape[1], step.n_seqs, page_size, dk,
-                                 keys, _stream()), "latent_rows")
+    keys = _latent_heads_keys(step, int(window))
+    lat = step.buffer("latent_rows", (keys, rank), torch.bfloat16)
+    rot_keys = step.buffer("latent_rot", (keys, rot), torch.bfloat16)
+    check(lib().rlis_latent_rows(cache.data_ptr(), lat.data_ptr(), rot_keys.data_ptr(), step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(), tables.data_ptr(),
+                                 tables.shape[1], step.n_seqs, page_size, rank, rot, int(window), keys, _stream()), "latent_rows")
     _count("latent_rows")
     kv = step.buffer("latent_kv", (keys, n_heads * (dim + v_dim)), torch.bfloat16)
-    torch.mm(rows[:, :rank], w_kv.t(), out=kv)
+    torch.mm(lat, w_kv.t(), out=kv)
     check(lib().rlis_attention_latent_heads(
-        q.data_ptr(), q.stride(0), q_rot.data_ptr(), kv.data_ptr(), rows.data_ptr(), out.data_ptr(), sinks.data_ptr() if sinks is not None else None,
+        q.data_ptr(), q.stride(0), q_rot.data_ptr(), kv.data_ptr(), rot_keys.data_ptr(), out.data_ptr(), sinks.data_ptr() if sinks is not None else None,
         step.prefill_tiles.data_ptr(), step.n_prefill_tiles, step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(), n_heads, dim, rot, v_dim, rank,
         float(scale), int(window), gp, gs, _stream()), "attention_latent_heads")
     _count("attention_latent.prefill.heads")

@@ -45,7 +45,7 @@ SIGNATURES = {
     "rlis_latent_q_rope": [P, LL, P, P, P, I, I, I, I, I, I, F, I, I, P],
     "rlis_attention_latent": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, I, P, LL, I, P],
     "rlis_latent_heads_takes": [I, I, I, I],
-    "rlis_latent_rows": [P, P, P, P, I, I, I, I, I, P],
+    "rlis_latent_rows": [P, P, P, P, P, P, I, I, I, I, I, I, I, P],
     "rlis_attention_latent_heads": [P, LL, P, P, P, P, P, P, I, P, P, I, I, I, I, I, F, I, P, LL, P],
     "rlis_attention_latent_mma_takes": [I, I],
     "rlis_attention_latent_prefill": [P, I, P, P, P, P, I, P, P, P, I, I, I, I, I, F, I, P, LL, P],

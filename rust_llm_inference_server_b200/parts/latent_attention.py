@@ -114,7 +114,7 @@ class LatentAttention(ProjectedMixer):
         z = proj[:, self.kv_off:self.kv_off + dk]
         q = proj[:, :self.kv_off]
         gate = proj[:, self.g_off:self.g_off + H] if s.head_gate is not None else None
-        if ops.latent_heads_takes(step, self.dtype, H, s.dim, s.rot_dim, s.v_dim, s.kv_rank):
+        if ops.latent_heads_takes(step, self.dtype, H, s.dim, s.rot_dim, s.v_dim, s.kv_rank, self.window):
             q = self._store_and_project(q, z, step, cache, stores)
             with span("q rope"):
                 q_rot = step.buffer("latent_q_rot", (T, H * s.rot_dim), self.dtype)

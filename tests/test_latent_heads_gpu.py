@@ -77,3 +77,50 @@ def test_prompts_form_heads_within_a_bound_of_memory():
     assert not takes(st)
     st.n_decode, st.starts = 0, [0, 40000]          # 328 MB of keys and values
     assert not takes(st) and takes(st, heads=8)
+
+
+@pytest.mark.parametrize("starts,lens,window,page", [([5000, 40, 0], [70, 3, 130], 100, 16), ([4096, 7000], [64, 2], 1, 32), ([3000], [200], 64, 24)])
+def test_a_window_forms_only_the_keys_in_its_reach(starts, lens, window, page):
+    """Long contexts behind a window, their early pages released: the scratch rows are those that some token of the step sees, and the outputs those
+    of attention over the rows themselves with the maps behind it."""
+    from rust_llm_inference_server_b200 import ops
+    H, dim, rot, dv, rank, scale = 2, 128, 64, 128, 64, 192 ** -0.5
+    g = torch.Generator().manual_seed(window)
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    st, T = Step(starts, lens, page), sum(lens)
+    cache = rnd(st.pages, 1, page, rank + rot).bfloat16().cuda()
+    for b, s in enumerate(starts):
+        released = max(0, s - window + 1) // page
+        cache[st.tables[b][:released].cuda()] = float("nan")              # (another request's by now)
+        st.block_tables[0][b, :released] = -1
+    sizes = {}
+    def buffer(name, shape, dtype):
+        sizes[name] = tuple(shape)
+        return torch.full(tuple(shape), float("nan"), dtype=dtype, device="cuda")
+    st.buffer = buffer
+    q, q_rot = rnd(T, H * (dim + rot)).bfloat16().cuda(), rnd(T, H * rot).bfloat16().cuda()
+    w = (rnd(H * (dim + dv), rank) * rank ** -0.5).bfloat16().cuda()
+    out = torch.full((T, H * dv), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.attention_latent_heads(q, q_rot, cache, w, out, st, 0, H, dim, rot, dv, rank, page, scale, None, window)
+    seen = sum(n + min(s, window - 1) for s, n in zip(starts, lens))
+    assert sizes["latent_kv"][0] <= max(seen, 128) and sizes["latent_rows"][0] <= max(seen, 128)
+    at = 0
+    for b, (s, n) in enumerate(zip(starts, lens)):
+        lo = max(0, s - window + 1)
+        rows = cache[st.tables[b].cuda()].reshape(-1, rank + rot)[lo:s + n]
+        kv = (rows[:, :rank] @ w.t()).double()
+        k, v = kv[:, :H * dim].view(-1, H, dim), kv[:, H * dim:].view(-1, H, dv)
+        qp, qr = q[at:at + n].double().view(n, H, dim + rot)[..., :dim], q_rot[at:at + n].double().view(n, H, rot)
+        sc = (torch.einsum("nhd,khd->hnk", qp, k) + torch.einsum("nhd,kd->hnk", qr, rows[:, rank:].double())) * scale
+        back = (s + torch.arange(n, device="cuda"))[:, None] - torch.arange(lo, s + n, device="cuda")[None]
+        want = torch.einsum("hnk,khd->nhd", torch.softmax(sc.masked_fill((back < 0) | (back >= window), -torch.inf), dim=2), v)
+        got = out[at:at + n].double().view(n, H, dv)
+        assert bool(torch.isfinite(got).all()) and (got - want).norm() <= 2.0 ** -8 * 1.5 * want.norm() + 1e-6, b
+        at += n
+
+
+def test_a_window_bounds_the_memory_of_formed_heads():
+    from rust_llm_inference_server_b200 import ops
+    st = Step([32000, 70], [64, 65], 16)
+    sizes = (torch.bfloat16, 32, 128, 64, 128, 512)
+    assert not ops.latent_heads_takes(st, *sizes) and ops.latent_heads_takes(st, *sizes, window=1024)
