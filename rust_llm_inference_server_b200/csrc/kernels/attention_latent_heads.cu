@@ -2,7 +2,7 @@
 //
 // attention_latent_mma.cu scores against the cached rows themselves, [c | k_rot], with the key map folded into the query: 576 +
 // 512 multiply-adds a (token, key, head) at a latent of 512 and 64 rotated entries, and nothing to prepare.  Here the context's
-// latents go through the key and value maps once (one library product over all heads), and a pair costs dim + rot + v_dim = 320.
+// latents go through the key and value maps once (one tcgen05 product over all heads), and a pair costs dim + rot + v_dim = 320.
 // 2,048 tokens, 16 heads: 362 us on the rows, 93 us here and 16 for the rows' copy and the maps.
 //
 //   latent_rows: the cached rows that the step's tokens see (whole contexts, or from the window's first key on), one request after the

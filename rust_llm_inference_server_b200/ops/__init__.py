@@ -840,13 +840,13 @@ def attention_latent_heads(q: torch.Tensor, q_rot: torch.Tensor, cache: torch.Te
         gp, gs = gate.data_ptr(), gate.stride(0)
     tables = step.block_tables[group]
     keys = _latent_heads_keys(step, int(window))
-    lat = step.buffer("latent_rows", (keys, rank), torch.bfloat16)
+    held = max(keys, 128)           # (the product takes 128 rows and more; those beyond the keys are never read)
+    lat = step.buffer("latent_rows", (held, rank), torch.bfloat16)
     rot_keys = step.buffer("latent_rot", (keys, rot), torch.bfloat16)
     check(lib().rlis_latent_rows(cache.data_ptr(), lat.data_ptr(), rot_keys.data_ptr(), step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(), tables.data_ptr(),
                                  tables.shape[1], step.n_seqs, page_size, rank, rot, int(window), keys, _stream()), "latent_rows")
     _count("latent_rows")
-    kv = step.buffer("latent_kv", (keys, n_heads * (dim + v_dim)), torch.bfloat16)
-    torch.mm(lat, w_kv.t(), out=kv)
+    kv = gemm_tcgen05(lat, w_kv, out=step.buffer("latent_kv", (held, n_heads * (dim + v_dim)), torch.bfloat16))
     check(lib().rlis_attention_latent_heads(
         q.data_ptr(), q.stride(0), q_rot.data_ptr(), kv.data_ptr(), rot_keys.data_ptr(), out.data_ptr(), sinks.data_ptr() if sinks is not None else None,
         step.prefill_tiles.data_ptr(), step.n_prefill_tiles, step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(), n_heads, dim, rot, v_dim, rank,
@@ -1191,12 +1191,12 @@ def stream_gemm(x, w: torch.Tensor, out_dtype=torch.bfloat16, swiglu4: bool = Fa
 
 
 def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, epilogue: str = "plain", glu: tuple | None = None,
-                 bias: torch.Tensor | None = None) -> torch.Tensor:
+                 bias: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """y = x @ w^T on the tcgen05 tensor cores (TMA-fed, accumulator in tensor memory), bfloat16
     operands.  epilogue "plain": bf16 [M, N]; "float32": float32 [M, N]; "swiglu4": w is a gate|up
     matrix interleaved in blocks of 4 rows and the result is silu(gate) * up, bf16 [M, N / 2]; "glu4":
     the same layout with the gating of `glu` = (slope, limit or None, up_shift[, cubic]), see `glu_act`, after `bias` (float32 [N]
-    in the order of w's rows; this epilogue only) is added."""
+    in the order of w's rows; this epilogue only) is added.  `out`: where the result goes (default: a new tensor)."""
     M, K = x.shape
     N = w.shape[0]
     _req(x, "x", torch.bfloat16)
@@ -1210,8 +1210,11 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, epilogue: str = "plain", glu:
     if M < 128 or N < 256 or K % 8 or N % (16 if gated else 8):
         raise KernelError(f"gemm_tcgen05: takes M >= 128, N >= 256, K a multiple of 8 and N a multiple of 8 "
                           f"(16 with a gated epilogue); got M={M}, N={N}, K={K}")
-    out = torch.empty((M, N // 2 if gated else N), dtype=torch.float32 if code == 2 else torch.bfloat16,
-                      device=x.device)
+    shape, dtype = (M, N // 2 if gated else N), torch.float32 if code == 2 else torch.bfloat16
+    if out is None:
+        out = torch.empty(shape, dtype=dtype, device=x.device)
+    else:
+        _req(out, "out", dtype, shape)
     if code == 3:
         slope, limit, shift, *cubic = glu
         check(lib().rlis_gemm_tcgen05_glu(x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, float(slope),
