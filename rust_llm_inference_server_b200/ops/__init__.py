@@ -806,15 +806,16 @@ def latent_heads_takes(step, dtype, n_heads: int, dim: int, rot: int, v_dim: int
     behind 4,096 408 and 187, 64 behind 16,384 1510 and 634), so only
     the memory that the formed keys and values take limits it: those in reach of the window, as the rows' kernel reads them."""
     starts, lens = getattr(step, "starts", None), getattr(step, "q_lens", None)
-    if not LATENT_MMA or dtype != torch.bfloat16 or not starts or not lens or step.n_decode or not step.n_prefill_tiles:
+    if not LATENT_MMA or not starts or not lens or step.n_decode or not step.n_prefill_tiles:
         return False
-    return (bool(_latent_heads_sizes(dim, rot, v_dim, rank))
+    return (latent_heads_exist(dtype, dim, rot, v_dim, rank)
             and 2 * _latent_heads_keys(step, int(window)) * n_heads * (dim + v_dim) <= LATENT_HEADS_BYTES)
 
 
 @functools.lru_cache(maxsize=None)
-def _latent_heads_sizes(dim: int, rot: int, v_dim: int, rank: int) -> bool:
-    return bool(lib().rlis_latent_heads_takes(dim, rot, v_dim, rank))
+def latent_heads_exist(dtype, dim: int, rot: int, v_dim: int, rank: int) -> bool:
+    """Whether `attention_latent_heads` exists for these sizes, whatever the step."""
+    return dtype == torch.bfloat16 and bool(lib().rlis_latent_heads_takes(dim, rot, v_dim, rank))
 
 
 def attention_latent_heads(q: torch.Tensor, q_rot: torch.Tensor, cache: torch.Tensor, w_kv: torch.Tensor, out: torch.Tensor, step, group: int,

@@ -76,10 +76,14 @@ class LatentAttention(ProjectedMixer):
         self.w_q_up = src.get(s.q_up).contiguous() if self.q_latent else None
         # [head, kv_rank, dim]: the key map transposed, so that it applies to queries
         self.w_k_fold = src.get(s.k_up).view(s.n_heads, s.dim, s.kv_rank).transpose(1, 2).contiguous()
-        # the key maps of all heads and the value maps below them: long portions of prompts form the heads' keys and values
-        # (`ops.attention_latent_heads`); the value maps alone are a view of it
-        self.w_kv_up = torch.cat([src.get(s.k_up), src.get(s.v_up)], dim=0).contiguous()
-        self.w_v_up = self.w_kv_up[s.n_heads * s.dim:].view(s.n_heads, s.v_dim, s.kv_rank)
+        self.w_kv_up = None
+        if ops.latent_heads_exist(self.dtype, s.dim, s.rot_dim, s.v_dim, s.kv_rank):
+            # the key maps of all heads and the value maps below them: portions of prompts form the heads' keys and values
+            # (`ops.attention_latent_heads`); the value maps alone are a view of it
+            self.w_kv_up = torch.cat([src.get(s.k_up), src.get(s.v_up)], dim=0).contiguous()
+            self.w_v_up = self.w_kv_up[s.n_heads * s.dim:].view(s.n_heads, s.v_dim, s.kv_rank)
+        else:
+            self.w_v_up = src.get(s.v_up).view(s.n_heads, s.v_dim, s.kv_rank).contiguous()
         self.w_o = src.get(s.o_proj).contiguous()
         self.sinks = src.get(s.sink, "vector").contiguous() if s.sink is not None else None
 
