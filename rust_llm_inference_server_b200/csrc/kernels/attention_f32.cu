@@ -12,7 +12,10 @@
 // 16-byte asynchronous copies, once for all of them.
 //   single tokens (SPLIT): a CTA a (request, kv head, piece), a warp a query head; a second kernel folds the pieces.  Bound
 //     by the cache's bytes: a group of four heads reads them once where the kernel with a warp a head read them four
-//     times, and a context of 2,048 offers eight times as many CTAs.
+//     times, and a context of 2,048 offers eight times as many CTAs.  The pieces that exist stand one after the other, request by
+//     request, and a CTA looks its own up from the positions, so that neither launch nor scratch memory is sized by the longest context
+//     times the requests (64 requests of 200 keys beside one of 131,072, 32 heads of 128: 545 MB by the longest, 17 by the pieces).  Beyond
+//     SPLIT_ROWS requests, which are many waves of CTAs by themselves, a CTA takes a whole context.
 //   prompts: 8 warps of R = 4 rows, a row a (token, query head); lanes are keys for the scores and dimensions for
 //     the value sum, so a key's 16 bytes in shared memory serve four rows.
 #include "common.cuh"
@@ -20,24 +23,58 @@
 #include <math.h>
 
 namespace {
-constexpr int PIECE = 256, BLOCK = 32, PROMPT_WARPS = 8, PROMPT_ROWS = 4, MAX_GROUP = 8, STAGES = 3;
+constexpr int PIECE = 256, BLOCK = 32, PROMPT_WARPS = 8, PROMPT_ROWS = 4, MAX_GROUP = 8, STAGES = 3, SPLIT_ROWS = 1024;
 
 struct Args {
     const float* q;
     const float* k_cache;
     const float* v_cache;
     float* out;
-    float* partial;               // [rows, nh, pieces, d + 2]: value sum, maximum, denominator of a piece
+    float* partial;               // [pieces of all rows, nh, d + 2]: value sum, maximum, denominator of a piece
     const int* seq_of_token;
     const int* positions;
     const int* block_tables;
     const int* token_rows;        // the step's tokens this launch computes, or null for all
-    int max_blocks, n_rows, tokens_per_cta, pieces, nh, nkv, d, page_size;
+    int max_blocks, n_rows, tokens_per_cta, slots, nh, nkv, d, page_size;
     float scale;
     int window;
 };
 
 __device__ __forceinline__ int first_key(int pos, int window) { return window > 0 ? max(0, pos - window + 1) : 0; }
+__device__ __forceinline__ int row_token_of(const Args& p, int row) { return p.token_rows != nullptr ? p.token_rows[row] : row; }
+__device__ __forceinline__ int row_pieces(const Args& p, int row) {
+    const int pos = p.positions[row_token_of(p, row)];
+    return pos / PIECE - first_key(pos, p.window) / PIECE + 1;
+}
+
+// Whose piece number `slot` is, and which of that row's it is: all threads of the block; row -1 beyond the last.
+__device__ __forceinline__ int2 piece_at(const Args& p, int slot) {
+    __shared__ int totals[MAX_GROUP];
+    __shared__ int2 found;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, per = (p.n_rows + blockDim.x - 1) / blockDim.x;
+    const int row0 = tid * per, row1 = min(row0 + per, p.n_rows);
+    int own = 0;
+#pragma unroll 4
+    for (int row = row0; row < row1; ++row) own += row_pieces(p, row);
+    int incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += n;
+    }
+    if (lane == 31) totals[warp] = incl;
+    if (tid == 0) found = make_int2(-1, 0);
+    __syncthreads();
+    int before = incl - own;
+    for (int w = 0; w < warp; ++w) before += totals[w];
+    if (slot >= before && slot < before + own) {
+        int row = row0, at = slot - before;
+        for (int n; at >= (n = row_pieces(p, row)); ++row) at -= n;
+        found = make_int2(row, at);
+    }
+    __syncthreads();
+    return found;
+}
 
 // What scores are taken from before expf: their running maximum, or 0 while all of them are -inf (whose weights are 0 then, not the NaN
 // of -inf - -inf).
@@ -57,15 +94,17 @@ __global__ __launch_bounds__((SPLIT ? MAX_GROUP : PROMPT_WARPS) * 32) void attn_
     extern __shared__ __align__(16) float smem[];
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    const int group = p.nh / p.nkv, kvh = blockIdx.x, d = p.d, ld = d + 4;
+    const int group = p.nh / p.nkv, kvh = SPLIT ? blockIdx.y : blockIdx.x, d = p.d, ld = d + 4;
     float* qs = smem + warp * R * d;                                        // this warp's rows of q
     float* ring = smem + warps * R * d;
     const int stage_floats = 2 * BLOCK * ld;
     int* mapped = reinterpret_cast<int*>(ring + STAGES * stage_floats);     // [stage][key]: whether its page is there
+    const int2 piece = SPLIT ? piece_at(p, blockIdx.x) : make_int2(0, 0);
+    if (SPLIT && piece.x < 0) return;
     // long tiles first: the last tokens of a prompt see the most keys
-    const int t0 = SPLIT ? blockIdx.y : (gridDim.y - 1 - blockIdx.y) * p.tokens_per_cta;
+    const int t0 = SPLIT ? piece.x : (gridDim.y - 1 - blockIdx.y) * p.tokens_per_cta;
     const int nt = SPLIT ? 1 : min(p.tokens_per_cta, p.n_rows - t0);
-    auto token = [&](int i) { return p.token_rows != nullptr ? p.token_rows[t0 + i] : t0 + i; };
+    auto token = [&](int i) { return row_token_of(p, t0 + i); };
 
     // this warp's rows: token of the tile and query head
     int row_token[R], row_head[R], row_pos[R], row_lo[R];
@@ -96,10 +135,8 @@ __global__ __launch_bounds__((SPLIT ? MAX_GROUP : PROMPT_WARPS) * 32) void attn_
         int kb0 = lo & ~(BLOCK - 1), end = last + 1;            // keys kb0 .. end - 1, block by block
         const int piece0 = lo / PIECE, pieces = last / PIECE - piece0 + 1;
         if (SPLIT) {
-            const int z = blockIdx.z;
-            if (z >= pieces) break;
-            kb0 = max(kb0, (piece0 + z) * PIECE);
-            end = min(end, (piece0 + z + 1) * PIECE);
+            kb0 = max(kb0, (piece0 + piece.y) * PIECE);
+            end = min(end, (piece0 + piece.y + 1) * PIECE);
         }
         const int blocks = (end - kb0 + BLOCK - 1) / BLOCK;
 
@@ -222,8 +259,8 @@ __global__ __launch_bounds__((SPLIT ? MAX_GROUP : PROMPT_WARPS) * 32) void attn_
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             if (row_token[r] < s0 || row_token[r] >= s1) continue;
-            if (SPLIT && pieces > 1) {
-                float* dst = p.partial + (((size_t)t0 * p.nh + row_head[r]) * p.pieces + blockIdx.z) * (d + 2);
+            if (SPLIT && pieces > 1 && p.partial != nullptr) {
+                float* dst = p.partial + ((size_t)blockIdx.x * p.nh + row_head[r]) * (d + 2);
 #pragma unroll
                 for (int i = 0; i < DL; ++i)
                     if (lane + 32 * i < d) dst[lane + 32 * i] = acc[r][i];
@@ -246,12 +283,16 @@ template <int DL> __global__ __launch_bounds__(128) void attn_f32_fold_kernel(co
     pdl_wait();
     const int lane = threadIdx.x & 31, row = blockIdx.x * 4 + (threadIdx.x >> 5), d = p.d;
     if (row < p.n_rows * p.nh) {
-        const int i = row / p.nh, t = p.token_rows != nullptr ? p.token_rows[i] : i;
-        const int pos = p.positions[t], pieces = pos / PIECE - first_key(pos, p.window) / PIECE + 1;
+        const int i = row / p.nh, t = row_token_of(p, i), pieces = row_pieces(p, i);
         if (pieces > 1) {
-            const float* src = p.partial + (size_t)row * p.pieces * (d + 2);
+            int slot = 0;                   // of its first piece
+            for (int o = lane; o < i; o += 32) slot += row_pieces(p, o);
+            slot = __reduce_add_sync(0xffffffffu, slot);
+            if (slot + pieces > p.slots) return;            // (the host counts them; never read beyond what it made room for)
+            const size_t step = (size_t)p.nh * (d + 2);
+            const float* src = p.partial + slot * step + (size_t)(row % p.nh) * (d + 2);
             float M = 0.f, L = 0.f, A[DL];
-            for (int z = 0; z < pieces; ++z, src += d + 2) {
+            for (int z = 0; z < pieces; ++z, src += step) {
                 float a[DL];
 #pragma unroll
                 for (int u = 0; u < DL; ++u) a[u] = lane + 32 * u < d ? src[lane + 32 * u] : 0.f;
@@ -275,16 +316,25 @@ template <int DL> __global__ __launch_bounds__(128) void attn_f32_fold_kernel(co
     pdl_trigger();
 }
 
-template <int DL> int run(Args p, cudaStream_t stream) {
+template <int DL> int run(Args p, bool folds, bool single, cudaStream_t stream) {
     const int group = p.nh / p.nkv;
     auto smem = [&](int rows) { return (rows * p.d + STAGES * 2 * BLOCK * (p.d + 4)) * (int)sizeof(float) + STAGES * BLOCK * (int)sizeof(int); };
-    if (p.partial != nullptr) {
+    if (p.slots > 0) {
         auto kernel = attn_f32_kernel<DL, 1, true>;
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(MAX_GROUP));
         if (e != cudaSuccess) return (int)e;
-        if (p.n_rows > 65535 || p.pieces > 65535) return RLIS_ERR_UNSUPPORTED;
-        rlis_launch(kernel, dim3(p.nkv, p.n_rows, p.pieces), group * 32, smem(group), stream, p);
-        if (p.pieces > 1) rlis_launch(attn_f32_fold_kernel<DL>, (p.n_rows * p.nh + 3) / 4, 128, 0, stream, p);
+        if (p.nkv > 65535) return RLIS_ERR_UNSUPPORTED;
+        rlis_launch(kernel, dim3(p.slots, p.nkv), group * 32, smem(group), stream, p);
+        if (folds) rlis_launch(attn_f32_fold_kernel<DL>, (p.n_rows * p.nh + 3) / 4, 128, 0, stream, p);
+        return RLIS_LAUNCH_CHECK();
+    }
+    if (single) {
+        auto kernel = attn_f32_kernel<DL, 1, false>;
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(MAX_GROUP));
+        if (e != cudaSuccess) return (int)e;
+        if (p.n_rows > 65535) return RLIS_ERR_UNSUPPORTED;
+        p.tokens_per_cta = 1;
+        rlis_launch(kernel, dim3(p.nkv, p.n_rows), group * 32, smem(group), stream, p);
         return RLIS_LAUNCH_CHECK();
     }
     auto kernel = attn_f32_kernel<DL, PROMPT_ROWS, false>;
@@ -299,22 +349,25 @@ template <int DL> int run(Args p, cudaStream_t stream) {
 }
 }  // namespace
 
-// Keys of a piece: what the host sizes `partial` by.
+// Keys of a piece, and up to how many single tokens' contexts are cut into them: what the host sizes `partial` by.
 extern "C" int rlis_attention_f32_piece(void) { return PIECE; }
+extern "C" int rlis_attention_f32_split_rows(void) { return SPLIT_ROWS; }
 extern "C" int rlis_attention_f32_takes(int nh, int nkv, int d) {
     return d > 0 && d % 16 == 0 && d <= 128 && nkv > 0 && nh % nkv == 0 && nh / nkv <= MAX_GROUP;
 }
 
-// `partial` null: any query lengths, a CTA a tile of tokens.  Otherwise every row is a token on its own, and `pieces` is at
-// least the number of pieces of the longest context (further CTAs find nothing to do); float32
-// [n_rows, nh, pieces, d + 2] (not written or read with one piece).
+// `single` 0: any query lengths, a CTA a tile of tokens.  Otherwise every row is a token on its own: with `slots` their contexts are cut into
+// pieces, of which there are at most that many (further CTAs find nothing to do), and `partial` is float32 [slots, nh, d + 2] if some context has
+// more than one (`folds`); with 0 slots a CTA takes a whole context.
 extern "C" int rlis_attention_f32(const float* q, const float* k_cache, const float* v_cache, float* out, float* partial,
                                   const int* seq_of_token, const int* positions, const int* block_tables, const int* token_rows,
-                                  int max_blocks, int n_rows, int pieces, int nh, int nkv, int d, int page_size, float scale,
+                                  int max_blocks, int n_rows, int single, int slots, int folds, int nh, int nkv, int d, int page_size, float scale,
                                   int window, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
-    if (!rlis_attention_f32_takes(nh, nkv, d) || page_size <= 0 || pieces <= 0) return RLIS_ERR_UNSUPPORTED;
+    if (!rlis_attention_f32_takes(nh, nkv, d) || page_size <= 0 || slots < 0 || (slots > 0 && (!single || n_rows > SPLIT_ROWS)) ||
+        (folds && (slots == 0 || partial == nullptr)))
+        return RLIS_ERR_UNSUPPORTED;
     const Args p = {q, k_cache, v_cache, out, partial, seq_of_token, positions, block_tables, token_rows, max_blocks, n_rows, 1,
-                    pieces, nh, nkv, d, page_size, scale, window};
-    return d <= 32 ? run<1>(p, stream) : d <= 64 ? run<2>(p, stream) : run<4>(p, stream);
+                    slots, nh, nkv, d, page_size, scale, window};
+    return d <= 32 ? run<1>(p, folds != 0, single != 0, stream) : d <= 64 ? run<2>(p, folds != 0, single != 0, stream) : run<4>(p, folds != 0, single != 0, stream);
 }

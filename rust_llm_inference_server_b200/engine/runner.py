@@ -63,6 +63,7 @@ class StepContext:
         self.n_decode = 0
         self.dec_rows = self.dec_seqs = None      # int32 [n_decode]: token row, batch entry
         self.max_decode_ctx = 0
+        self.decode_ctxs: list = []               # keys of every single token's context (host)
         self.n_prefill_tokens = 0
         self.prefill_rows = None                  # int32: rows of the tokens of longer entries
         self.n_prefill_tiles = 0
@@ -269,7 +270,8 @@ class ModelRunner:
         st.n_prefill_tokens = Tp
         st.n_prefill_tiles = Nt
         if Bd:
-            st.max_decode_ctx = max(starts[b] + 1 for b in dec_seqs)
+            st.decode_ctxs = [starts[b] + 1 for b in dec_seqs]
+            st.max_decode_ctx = max(st.decode_ctxs)
 
         def views():
             # The step's arrays as views of the uploaded block.  A step replayed from a graph never

@@ -13,6 +13,7 @@ from __future__ import annotations
 import ctypes
 import functools
 
+import numpy as np
 import torch
 
 from . import library
@@ -1401,14 +1402,34 @@ def attention_f32_takes(dtype, n_heads: int, n_kv_heads: int, head_dim: int) -> 
 
 
 def attention_f32_pieces(max_ctx: int, window: int = 0) -> int:
-    """For how many pieces of a context `attention_f32` launches CTAs for single tokens: the most that a context of up to
-    `max_ctx` keys has, rounded up to a power of two, so that a recorded decode step serves while contexts double
-    (a CTA without a piece returns at once)."""
+    """Into how many pieces `attention_f32` cuts the context of a single token with up to `max_ctx` keys at most, rounded up to
+    a power of two."""
     piece = lib().rlis_attention_f32_piece()
     most = -(-max_ctx // piece)
     if window:          # a window's first and last key lie in pieces of their own
         most = min(most, -(-window // piece) + 1)
     return 1 << (max(1, most) - 1).bit_length()
+
+
+def attention_f32_split(step, window: int = 0) -> tuple:
+    """(slots, whether some context has several pieces) for the single tokens of a step: slots for all the pieces that their contexts
+    come to, rounded up to a power of two, so that a recorded decode step serves while contexts double (a CTA without a
+    piece returns at once); (0, False) where every CTA takes a whole context."""
+    if step.n_decode > lib().rlis_attention_f32_split_rows():
+        return 0, False
+    piece, window = lib().rlis_attention_f32_piece(), int(window)
+    most = attention_f32_pieces(step.max_decode_ctx, window)
+    ctxs = getattr(step, "decode_ctxs", None)
+    if ctxs is None:            # (a step whose contexts are known by the longest alone)
+        return 1 << (step.n_decode * most - 1).bit_length(), most > 1
+    known = step.carry.setdefault("attention_f32_split", {})
+    if window not in known:
+        last = np.asarray(ctxs, dtype=np.int64) - 1
+        pieces = last // piece + 1
+        if window:
+            pieces -= np.maximum(last - window + 1, 0) // piece
+        known[window] = 1 << (int(pieces.sum()) - 1).bit_length(), most > 1
+    return known[window]
 
 
 def attention_f32(q, k_cache, v_cache, out, step, group: int, n_heads: int, n_kv_heads: int, head_dim: int, page_size: int,
@@ -1422,20 +1443,20 @@ def attention_f32(q, k_cache, v_cache, out, step, group: int, n_heads: int, n_kv
     _req(v_cache, "v_cache", torch.float32, (None, n_kv_heads, page_size, head_dim))
     tables = step.block_tables[group]
 
-    def launch(rows, n_rows, partial, pieces):
+    def launch(name, rows, n_rows, single, slots, folds, partial):
         check(lib().rlis_attention_f32(
             q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), partial.data_ptr() if partial is not None else None,
             step.seq_of_token.data_ptr(), step.positions.data_ptr(), tables.data_ptr(), rows.data_ptr() if rows is not None else None,
-            tables.shape[1], n_rows, pieces, n_heads, n_kv_heads, head_dim, page_size, float(scale), int(window), _stream()),
+            tables.shape[1], n_rows, int(single), slots, int(folds), n_heads, n_kv_heads, head_dim, page_size, float(scale), int(window), _stream()),
             "attention_f32")
-        _count("attention_f32.pieces" if partial is not None else "attention_f32")
+        _count(name)
 
     if step.n_decode:
-        pieces = attention_f32_pieces(step.max_decode_ctx, window)
-        partial = step.buffer("attn_partial", (step.n_decode * n_heads * pieces * (head_dim + 2),), torch.float32)
-        launch(step.dec_rows, step.n_decode, partial, pieces)
+        slots, folds = attention_f32_split(step, window)
+        partial = step.buffer("attn_partial", (slots * n_heads * (head_dim + 2),), torch.float32) if folds else None
+        launch("attention_f32.pieces" if slots else "attention_f32.single", step.dec_rows, step.n_decode, True, slots, folds, partial)
     if step.n_prefill_tokens:
-        launch(step.prefill_rows if step.n_decode else None, step.n_prefill_tokens, None, 1)
+        launch("attention_f32", step.prefill_rows if step.n_decode else None, step.n_prefill_tokens, False, 0, False, None)
     return out
 
 

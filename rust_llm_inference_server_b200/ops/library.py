@@ -85,7 +85,8 @@ SIGNATURES = {
     "rlis_glu_act": [P, P, I, I, F, F, F, F, I, P, I, P],
     "rlis_rope_cache": [P, P, P, P, P, P, P, I, I, I, I, I, I, P],
     "rlis_attention_generic": [P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, I, I, P],
-    "rlis_attention_f32": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, P],
+    "rlis_attention_f32": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P],
+    "rlis_attention_f32_split_rows": [],
     "rlis_attention_f32_piece": [],
     "rlis_attention_f32_takes": [I, I, I],
     "rlis_attention_decode": [P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, F, I, I, I, P],

@@ -62,7 +62,7 @@ class GQAAttention(Mixer):
         if not step.n_decode:
             return None
         if ops.attention_f32_takes(self.dtype, s.n_heads, s.n_kv_heads, s.head_dim):
-            return ops.attention_f32_pieces(step.max_decode_ctx, self.window)
+            return ops.attention_f32_split(step, self.window)
         return ops.decode_splits(step.n_decode, s.n_kv_heads, step.max_decode_ctx)
 
     def fuses_norms(self, step) -> bool:

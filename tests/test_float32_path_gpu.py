@@ -135,3 +135,41 @@ def test_float32_attention_passes_by_keys_whose_scores_are_minus_infinity(lo, hi
     for out in outs:
         assert (out.cpu().double()[rows] - want).abs().max() <= 2e-5
     assert torch.equal(outs[0][rows], outs[1][rows])
+
+
+def decode_step(lens, tables):
+    """A step of one token for each of `lens` that knows every context, and what scratch memory it was asked for."""
+    st = Step(lens, [1] * len(lens), tables, True)
+    st.decode_ctxs, st.carry, st.asked = list(lens), {}, []
+    def buffer(name, shape, dtype):
+        st.asked.append(math.prod(shape))
+        return torch.full(tuple(shape), float("nan"), dtype=dtype, device="cuda")
+    st.buffer = buffer
+    return st
+
+
+@pytest.mark.parametrize("lens,nh,nkv,d,window", [([9000] + [20] * 40, 8, 2, 64, 0), ([300, 20000, 1, 256, 257], 4, 4, 32, 0), ([9000] * 3 + [5] * 90, 16, 2, 128, 700),
+                                                  ([100] * 9, 8, 1, 64, 0), ([4097], 6, 2, 80, 0), ([513] * 300, 2, 2, 16, 0), ([600] + [3] * 1100, 4, 2, 16, 0)])
+def test_float32_decode_asks_for_the_pieces_that_exist(lens, nh, nkv, d, window):
+    """Ragged contexts: scratch memory by the sum of the pieces, not by the longest context for each; the bits of every request on its own."""
+    from rust_llm_inference_server_b200 import ops
+    page = 16
+    g = torch.Generator().manual_seed(len(lens) + nh)
+    used = [-(-n // page) for n in lens]
+    tables = torch.full((len(lens), max(used)), -1, dtype=torch.int32)
+    order = torch.randperm(sum(used), generator=g).to(torch.int32)
+    for b, n in enumerate(used):
+        tables[b, :n] = order[sum(used[:b]):sum(used[:b]) + n]
+    kc, vc = (torch.randn(sum(used), nkv, page, d, generator=g).cuda() for _ in range(2))
+    q = torch.randn(len(lens), nh * d, generator=g).cuda()
+    args = (0, nh, nkv, d, page, 1 / math.sqrt(d), window)
+    st = decode_step(lens, tables)
+    out = ops.attention(q, kc, vc, torch.full_like(q, 7.0), st, *args)
+    pieces = sum((n - 1) // 256 + 1 - (max(0, n - window) // 256 if window else 0) for n in lens)
+    assert sum(st.asked) <= 2 * pieces * nh * (d + 2)
+    for b in sorted({0, 1, len(lens) // 2, len(lens) - 1} & set(range(len(lens)))):
+        one = Step([lens[b]], [1], tables[b:b + 1], True)
+        assert torch.equal(ops.attention(q[b:b + 1].contiguous(), kc, vc, torch.zeros(1, nh * d, device="cuda"), one, *args)[0], out[b]), b
+    want = ops.attention_generic(q, kc, vc, torch.empty_like(q), st.seq_of_token, st.positions, st.block_tables[0], *args[1:])
+    # sums of weights that add up to one and values around one
+    assert (out - want).abs().max() <= 2e-5
