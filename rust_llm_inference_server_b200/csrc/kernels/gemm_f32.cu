@@ -280,6 +280,24 @@ inline double cta_time(long long ctas, int sms, double alone, double shared) {
     return per <= 1 ? alone : alone * shared * per;
 }
 
+// Which kernel a product goes to.  FEW: a step's few rows; else the split of the outputs that takes least time on this many SMs, by what a CTA of each
+// kind was measured to take (us at K 2048 alone on an SM; all are proportional to K).  The more outputs a CTA has, the less it
+// takes for each, and the fewer SMs a small product occupies.
+enum Shape { FEW, ROWS_32x64, ROWS_32x32, TILE_128x128, TILE_128x64, TILE_64x64, SHAPES };
+
+Shape choose(int M, int N, int batch, bool vec, int sms) {
+    if (vec && M <= 32) return FEW;
+    auto ctas = [&](int bm, int bn) { return (((long long)M + bm - 1) / bm) * (((long long)N + bn - 1) / bn) * batch; };
+    const double t128 = cta_time(ctas(128, 128), sms, 211, 0.9), t128x64 = cta_time(ctas(128, 64), sms, 137, 0.83),
+                 t64 = cta_time(ctas(64, 64), sms, 92, 0.97);
+    if (vec && M <= 32 * 65535) {
+        const double f64 = cta_time(ctas(32, 64), sms, 57, 1.0), f32 = cta_time(ctas(32, 32), sms, 35, 1.0);
+        if (f64 < t128 && f64 < t128x64 && f64 < t64 && f64 <= f32) return ROWS_32x64;
+        if (f32 < t128 && f32 < t128x64 && f32 < t64) return ROWS_32x32;
+    }
+    return t128 <= t128x64 && t128 <= t64 ? TILE_128x128 : t128x64 <= t64 ? TILE_128x64 : TILE_64x64;
+}
+
 int run(const Product& p, int batch, cudaStream_t stream) {
     if (p.M <= 0 || p.N <= 0 || batch <= 0) return 0;
     if (batch > 65535) return RLIS_ERR_UNSUPPORTED;
@@ -289,27 +307,19 @@ int run(const Product& p, int batch, cudaStream_t stream) {
     // 16-byte loads need rows and pieces of k on 16-byte boundaries
     const bool vec = p.K > 0 && p.K % 4 == 0 && p.lda % 4 == 0 && p.ldw % 4 == 0 && p.sa % 4 == 0 && p.sw % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(p.A) | reinterpret_cast<uintptr_t>(p.W)) & 15) == 0;
-    auto ctas = [&](int bm, int bn) { return (long long)((p.M + bm - 1) / bm) * ((p.N + bn - 1) / bn) * batch; };
-    if (vec && p.M <= 32) {
-        if (p.M == 1) return run_few_rows<1>(p, batch, sms, stream);
-        if (p.M <= 4) return run_few_rows<4>(p, batch, sms, stream);
-        if (p.M <= 8) return run_few_rows<8>(p, batch, sms, stream);
-        if (p.M <= 16) return run_few_rows<16>(p, batch, sms, stream);
-        return run_few_rows<32>(p, batch, sms, stream);
+    switch (choose(p.M, p.N, batch, vec, sms)) {
+        case FEW:
+            if (p.M == 1) return run_few_rows<1>(p, batch, sms, stream);
+            if (p.M <= 4) return run_few_rows<4>(p, batch, sms, stream);
+            if (p.M <= 8) return run_few_rows<8>(p, batch, sms, stream);
+            if (p.M <= 16) return run_few_rows<16>(p, batch, sms, stream);
+            return run_few_rows<32>(p, batch, sms, stream);
+        case ROWS_32x64: return launch_few_rows<64, 32, 8, 32, 6>(p, batch, stream);
+        case ROWS_32x32: return launch_few_rows<32, 32, 4, 64, 6>(p, batch, stream);
+        case TILE_128x128: return launch_tiles<128, 128>(p, batch, vec, stream);
+        case TILE_128x64: return launch_tiles<128, 64>(p, batch, vec, stream);
+        default: return launch_tiles<64, 64>(p, batch, vec, stream);
     }
-    // More rows: the split of the outputs that takes least time on this many SMs, by what a CTA of each kind was measured
-    // to take (us at K 2048 alone on an SM; all are proportional to K).  The more outputs a CTA has, the less it
-    // takes for each, and the fewer SMs a small product occupies.
-    const double t128 = cta_time(ctas(128, 128), sms, 211, 0.9), t128x64 = cta_time(ctas(128, 64), sms, 137, 0.83),
-                 t64 = cta_time(ctas(64, 64), sms, 92, 0.97);
-    if (vec && p.M <= 32 * 65535) {
-        const double f64 = cta_time(ctas(32, 64), sms, 57, 1.0), f32 = cta_time(ctas(32, 32), sms, 35, 1.0);
-        if (f64 < t128 && f64 < t128x64 && f64 < t64 && f64 <= f32) return launch_few_rows<64, 32, 8, 32, 6>(p, batch, stream);
-        if (f32 < t128 && f32 < t128x64 && f32 < t64) return launch_few_rows<32, 32, 4, 64, 6>(p, batch, stream);
-    }
-    if (t128 <= t128x64 && t128 <= t64) return launch_tiles<128, 128>(p, batch, vec, stream);
-    if (t128x64 <= t64) return launch_tiles<128, 64>(p, batch, vec, stream);
-    return launch_tiles<64, 64>(p, batch, vec, stream);
 }
 }  // namespace
 
@@ -325,3 +335,10 @@ extern "C" int rlis_gemm_f32_nt_batched(const float* A, const float* W, float* C
                                         long long sw, long long sc, cudaStream_t stream) {
     return run({A, W, C, M, N, K, lda, ldw, ldc, sa, sw, sc}, batch, stream);
 }
+
+// The kernel that a product of M x N outputs goes to on a device of `sms` SMs (`aligned`: rows and k on 16-byte boundaries), as a number below
+// rlis_gemm_f32_shapes(): what tests cover the kernels by.
+extern "C" int rlis_gemm_f32_shape(int M, int N, int batch, int aligned, int sms) {
+    return M <= 0 || N <= 0 || batch <= 0 || sms <= 0 ? -1 : (int)choose(M, N, batch, aligned != 0, sms);
+}
+extern "C" int rlis_gemm_f32_shapes(void) { return (int)SHAPES; }

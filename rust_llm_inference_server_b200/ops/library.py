@@ -29,6 +29,8 @@ SIGNATURES = {
     "rlis_layer_norm": [P, P, P, P, P, P, I, I, F, I, P],
     "rlis_swiglu": [P, P, I, I, I, I, P],
     "rlis_gemm_f32_nt": [P, P, P, I, I, I, P],
+    "rlis_gemm_f32_shape": [I, I, I, I, I],
+    "rlis_gemm_f32_shapes": [],
     "rlis_gemm_f32_nt_batched": [P, P, P, I, I, I, LL, LL, LL, I, LL, LL, LL, P],
     "rlis_post_norm_residual": [P, P, P, P, P, P, P, I, I, F, F, F, I, P],
     "rlis_sum_norm": [P, P, F, P, P, F, P, F, P, P, I, I, F, F, I, P],

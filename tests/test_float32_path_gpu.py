@@ -24,8 +24,25 @@ def chained(a, w):
                                    (9, 30, 128), (16, 2369, 200), (16, 9480, 40), (17, 2000, 300), (32, 9473, 36), (33, 300, 52), (64, 2048, 256),
                                    (65, 9500, 44), (129, 3000, 84), (200, 16390, 24), (700, 2048, 72), (130, 260, 257), (31, 77, 129)])
 def test_every_float32_product_is_one_chain_over_k(shape):
+    product_is_one_chain(*shape)
+
+
+# what the shapes above leave out: the kernels of many rows in every form, whole and ragged, each with 16-byte and with single
+# loads where it has both (the numbers are those of `rlis_gemm_f32_shape` on 148 SMs)
+MANY_ROWS = [((250, 3070, 72), 4), ((256, 3072, 64), 4), ((250, 3070, 73), 4), ((256, 3072, 30), 4), ((1000, 4096, 36), 3), ((700, 2050, 33), 3),
+             ((1030, 4000, 130), 3), ((40, 4001, 44), 1), ((64, 2048, 256), 2), ((33, 5001, 40), 5), ((33, 5001, 41), 5)]
+
+
+@pytest.mark.parametrize("shape,kernel", MANY_ROWS)
+def test_float32_products_of_many_rows_in_every_form(shape, kernel):
     from rust_llm_inference_server_b200 import ops
-    M, N, K = shape
+    product_is_one_chain(*shape)
+    if ops.num_sms() == 148:
+        assert ops.lib().rlis_gemm_f32_shape(shape[0], shape[1], 1, int(shape[2] % 4 == 0), 148) == kernel
+
+
+def product_is_one_chain(M, N, K):
+    from rust_llm_inference_server_b200 import ops
     g = torch.Generator().manual_seed(M * 31 + N)
     a, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g)
     ad, wd = a.cuda(), w.cuda()

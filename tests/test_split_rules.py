@@ -1,4 +1,4 @@
-"""The host-side rule that cuts a decode step's contexts into pieces (no GPU needed)."""
+"""The host-side rules that cut a decode step's contexts into pieces and choose between kernels (no GPU needed)."""
 
 from rust_llm_inference_server_b200 import ops
 
@@ -25,3 +25,59 @@ def test_decode_attention_pieces_by_batch_and_context():
     assert splits(3, 2, 7000) == splits(3, 2, 7000)
     # a smaller part fills up with fewer pieces
     assert ops.decode_splits(8, kv, 4096, 32) <= splits(8, kv, 4096)
+
+
+def test_float32_attention_counts_the_pieces_that_exist():
+    class Step:
+        def __init__(self, ctxs):
+            self.decode_ctxs, self.n_decode, self.max_decode_ctx, self.carry = ctxs, len(ctxs), max(ctxs), {}
+
+    piece, rows = ops.lib().rlis_attention_f32_piece(), ops.lib().rlis_attention_f32_split_rows()
+    for ctxs in ([1], [piece], [piece + 1], [131072] + [200] * 63, [4096] * 8, [1, 255, 256, 257, 513, 5000]):
+        for window in (0, 1, 255, 256, 257, 1000):
+            exist = sum((c - 1) // piece - (max(0, c - window) // piece if window else 0) + 1 for c in ctxs)
+            for _ in range(2):              # (the second time from the step)
+                step = Step(ctxs)
+                slots, folds = ops.attention_f32_split(step, window)
+                assert exist <= slots < 2 * exist and slots & (slots - 1) == 0
+                assert folds or exist == len(ctxs)
+            step.decode_ctxs = None         # contexts known by the longest alone
+            assert ops.attention_f32_split(step, window)[0] >= exist
+    assert ops.attention_f32_split(Step([300] * (rows + 1)), 0) == (0, False)
+
+
+def test_every_float32_product_kernel_is_reached_by_the_shapes_it_is_tested_with():
+    from tests.test_float32_path_gpu import MANY_ROWS
+    lib = ops.lib()
+    chosen = {(lib.rlis_gemm_f32_shape(M, N, 1, int(K % 4 == 0), 148), K % 4 == 0) for (M, N, K), _ in MANY_ROWS}
+    for (M, N, K), kernel in MANY_ROWS:
+        assert lib.rlis_gemm_f32_shape(M, N, 1, int(K % 4 == 0), 148) == kernel
+    # number 0 (few rows) has tests of its own; 1 and 2 exist for aligned rows only
+    assert chosen == {(k, True) for k in range(1, lib.rlis_gemm_f32_shapes())} | {(k, False) for k in (3, 4, 5)}
+    assert all(lib.rlis_gemm_f32_shape(M, N, 1, 1, 148) == 0 for M in (1, 32) for N in (16, 100000))
+    assert lib.rlis_gemm_f32_shape(0, 4, 1, 1, 148) == -1
+
+
+def test_formed_heads_by_step_and_memory():
+    import torch
+
+    class Step:
+        n_decode, n_prefill_tiles = 0, 1
+
+        def __init__(self, starts, lens):
+            self.starts, self.q_lens = starts, lens
+
+    takes = lambda step, window=0, heads=16, dtype=torch.bfloat16, dim=128: ops.latent_heads_takes(step, dtype, heads, dim, 64, 128, 512, window)
+    assert takes(Step([0, 70], [130, 65]))
+    assert not takes(Step([0], [64]), dtype=torch.float32) and not takes(Step([0], [64]), dim=96)
+    long = Step([40000], [64])              # 328 MB of keys and values
+    assert not takes(long) and takes(long, heads=8) and takes(long, window=1024)
+    mixed = Step([0], [64])
+    mixed.n_decode = 1
+    assert not takes(mixed)
+
+
+def test_long_portions_go_by_chunks_and_short_ones_token_by_token():
+    from rust_llm_inference_server_b200.ops import _lightning_chunks_pay as pays
+    assert pays(2048, 1, 2048, 2048, 148) and pays(2048, 4, 512, 2048, 148) and pays(898, 4, 700, 2048, 148)
+    assert not pays(128, 1, 128, 2048, 148) and not pays(8, 8, 1, 2048, 148) and not pays(540, 41, 500, 2048, 148)
