@@ -70,10 +70,12 @@ template <typename T, bool SILU> __device__ __forceinline__ void load_piece(cons
     constexpr int N = 16 / sizeof(T);
 #pragma unroll
     for (int i = 0; i < N; ++i) v[i] = 0.f;
-    if (valid) load16<T>(p, v);
-    if (SILU) {
+    if (valid) {
+        load16<T>(p, v);
+        if (SILU) {
 #pragma unroll
-        for (int i = 0; i < N; ++i) v[i] = silu_f(v[i]);            // (silu(0) = 0)
+            for (int i = 0; i < N; ++i) v[i] = silu_f(v[i]);
+        }
     }
 }
 

@@ -860,17 +860,28 @@ def attention_latent_heads(q: torch.Tensor, q_rot: torch.Tensor, cache: torch.Te
 LIGHTNING_SILU_PASS_TOKENS = 64
 
 
+# The recurrence by chunks, us: before the first chunk, for 1,024 columns' 64 tokens while there are up to 64 of these, and for those beyond; by
+# the heads' key size and the rows' form.
+LIGHTNING_CHUNKS_US = {(128, "silu bf16"): (45.0, 2.2, 3.4), (128, "silu f32"): (47.0, 2.3, 4.0), (128, "plain"): (28.0, 1.9, 3.2),
+                       (64, "silu bf16"): (27.5, 1.2, 1.8), (64, "silu f32"): (34.0, 1.5, 2.3), (64, "plain"): (19.0, 1.0, 1.4)}
+
+
 @functools.lru_cache(maxsize=4096)
-def _lightning_chunks_pay(n_tokens: int, n_seqs: int, longest: int, columns: int, sms: int) -> bool:
+def _lightning_chunks_pay(n_tokens: int, n_seqs: int, longest: int, columns: int, sms: int, d: int = 128, form: str = "silu bf16") -> bool:
     """Whether the decayed recurrence runs faster 64 tokens at a time than token by token, for `columns` = heads x dv columns of state
-    and a longest portion of `longest` tokens.  The walk takes 0.145 us a token of a request while its CTAs (a request's 16 columns each)
-    have an SM each, and that much longer the more of them share one (the CTAs of a few requests clump: a long portion beside three
-    short ones runs as if all were long); the chunks take 25 us and 2.9 us for each of 1,024 columns' 64 tokens.  Measured at heads of
-    128 x 128, walk and chunks in us: one prompt of 2,048 with 16 heads 310 and 205, with 8 heads 290 and 108; four of 512 255 and 197;
-    130, 700, 65 and 3 tokens 314 and 140; one of 256 44 and 60; one of 128 26 and 50; sixteen of 128 230 and 232."""
+    and a longest portion of `longest` tokens.  The walk takes 0.12 (heads of 64) or 0.14 us a token of a request while its CTAs (a request's 16
+    columns each) have an SM each, that much longer the more of a request's share one (up to 2.6 times as long: the CTAs of a few requests clump),
+    and 0.9 of it a token and CTA of an SM once all are full; the chunks take LIGHTNING_CHUNKS_US.  Measured, walk and chunks in us: heads of 128 x
+    128, bfloat16 with silu, one prompt of 2,048 with 16 heads 310 and 202, with 2 heads 284 and 53, one of 256 42 and 60, four of 512 256 and 196,
+    sixteen of 256 449 and 501; the same in float32 312 and 255, 284 and 58, 41 and 66, 256 and 247, 453 and 617; without silu 280 and 155, 278 and 36, 37 and 46,
+    230 and 155, 390 and 418; heads of 64 x 64, sixteen, one prompt of 256: 35 and 32, 35 and 37, 32 and 21."""
+    plain = form == "plain"
+    a_token = (0.134 if plain else 0.138) if d > 64 else (0.118 if plain else 0.121)
     per_sm = columns / 16 / sms
-    walk = 0.145 * max(longest * max(1.0, min(n_seqs, 4) * per_sm), n_tokens / n_seqs * max(1.0, n_seqs * per_sm))
-    return 25.0 + 2.9 * (n_tokens / 64 + n_seqs) * columns / 1024 < walk
+    walk = a_token * max(longest * max(1.0, per_sm, min(2.6, min(n_seqs, 4) * per_sm)), 0.9 * n_tokens * per_sm)
+    first, few, many = LIGHTNING_CHUNKS_US[128 if d > 64 else 64, form]
+    load = (n_tokens / 64 + n_seqs) * columns / 1024
+    return first + few * min(load, 64.0) + many * max(load - 64.0, 0.0) < walk
 
 
 def _lightning_in_chunks(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, out: torch.Tensor, state: torch.Tensor, decay: torch.Tensor,
@@ -879,7 +890,8 @@ def _lightning_in_chunks(rows: torch.Tensor, q_off: int, k_off: int, v_off: int,
     rows lie on 16-byte boundaries; False: nothing was launched."""
     T, vec = rows.shape[0], 16 // rows.element_size()
     longest = getattr(step, "max_q_len", 0) or -(-T // step.n_seqs)
-    if (not _lightning_chunks_pay(T, step.n_seqs, longest, n_heads * dv, num_sms()) or not hasattr(step, "buffer")
+    form = "plain" if not silu else "silu bf16" if rows.dtype == torch.bfloat16 else "silu f32"
+    if (not _lightning_chunks_pay(T, step.n_seqs, longest, n_heads * dv, num_sms(), d, form) or not hasattr(step, "buffer")
             or not lib().rlis_lightning_chunks_takes(d, dv)
             or rows.stride(1) != 1 or any(n % vec for n in (rows.stride(0), q_off, k_off, v_off))
             or any(t.data_ptr() % 16 for t in (rows, out, state))):

@@ -81,3 +81,8 @@ def test_long_portions_go_by_chunks_and_short_ones_token_by_token():
     from rust_llm_inference_server_b200.ops import _lightning_chunks_pay as pays
     assert pays(2048, 1, 2048, 2048, 148) and pays(2048, 4, 512, 2048, 148) and pays(898, 4, 700, 2048, 148)
     assert not pays(128, 1, 128, 2048, 148) and not pays(8, 8, 1, 2048, 148) and not pays(540, 41, 500, 2048, 148)
+    # by the heads' key size and the rows' form: measured on both sides of the lines
+    for d, form, faster, slower in [(128, "silu f32", (2048, 1, 2048, 2048), (4096, 16, 256, 2048)), (128, "plain", (256, 1, 256, 256), (128, 1, 128, 256)),
+                                    (64, "plain", (256, 1, 256, 512), (128, 1, 128, 512)), (64, "silu bf16", (512, 1, 512, 1024), (192, 1, 192, 128)),
+                                    (64, "silu f32", (512, 1, 512, 1024), (192, 1, 192, 128)), (128, "silu bf16", (2048, 4, 512, 2048), (8000, 8, 1000, 2048))]:
+        assert pays(*faster, 148, d, form) and not pays(*slower, 148, d, form), (d, form)
