@@ -444,10 +444,9 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
             if (it >= 1 && !load_tile(it - 1, true)) break;
         }
       } else if (warp == 1) {
-        // The whole warp walks the loop and waits; one lane issues.  (With the loop inside
+        // The whole warp walks the loop and waits; the elected lane issues.  (With the loop inside
         // `if (lane == 0)` a product's eight instructions took 800 cycles to issue and every wait on
-        // a barrier that was long complete 250: the block's chain P ready -> P V done was 1200
-        // cycles for 256 of tensor work.)
+        // a barrier that was long complete 250; with the instructions alone inside it 56 each.)
         {
             bool ok = bar_wait(&ctrl->q_full, 0, &ctrl->abort);
             uint64_t qdesc[HALVES];
@@ -460,7 +459,7 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
                 if (it > 0 && !bar_wait(&ctrl->s_empty, (it - 1) & 1, &ctrl->abort)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned char* kt = kv_tiles + (size_t)s * 2 * KV_TILE_BYTES;
-                if (lane == 0) {
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < HD / 16; ++k) {
                         // four k-steps of 32 bytes inside a sub-tile of 64 columns, then the next sub-tile
@@ -482,14 +481,13 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
                 if (!bar_wait(&ctrl->v_full[s], (it / KV_STAGES) & 1, &ctrl->abort)) break;
                 const unsigned char* vt = kv_tiles + (size_t)s * 2 * KV_TILE_BYTES + KV_TILE_BYTES;
                 // O += P V in two bursts: the first half of the keys while the softmax warps are in the
-                // exponentials of the second (a burst costs 300 cycles before its first instruction
-                // is through and 50 an instruction; after the last exponential only four are left)
+                // exponentials of the second (after the last exponential only half of the instructions are left)
                 bool fine = true;
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
                     if (!bar_wait(&ctrl->p_full[hf], it & 1, &ctrl->abort)) { fine = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (lane == 0) {
+                    if (elect_one()) {
 #pragma unroll
                         for (int k = hf * (TN / 32); k < (hf + 1) * (TN / 32); ++k) {
                             // P: 16 keys are 8 columns of tensor memory; V: 16 keys = 2 KB further in each of

@@ -122,29 +122,32 @@ __global__ __launch_bounds__(GT_THREADS) void gemm_tcgen05_kernel(const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            int it = 0, t = 0;      // t counts the tiles this CTA works on (a tile that is left out is not one)
-            for (int tile = blockIdx.x; tile < num_tiles && !ctrl->abort; tile += gridDim.x) {
-                if (tile_expert != nullptr && tile_expert[tile % m_tiles] < 0) continue;
-                const int buf = t & 1;
-                if (t >= 2 && !bar_wait(&ctrl->acc_empty[buf], ((t >> 1) - 1) & 1, &ctrl->abort)) break;
+        // the whole warp walks the loop and waits; one lane issues
+        int it = 0, t = 0;          // t counts the tiles this CTA works on (a tile that is left out is not one)
+        for (int tile = blockIdx.x; tile < num_tiles && !ctrl->abort; tile += gridDim.x) {
+            if (tile_expert != nullptr && tile_expert[tile % m_tiles] < 0) continue;
+            const int buf = t & 1;
+            if (t >= 2 && !bar_wait(&ctrl->acc_empty[buf], ((t >> 1) - 1) & 1, &ctrl->abort)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * BN);
+            for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                const int s = it % STAGES;
+                if (!bar_wait(&ctrl->full[s], (it / STAGES) & 1, &ctrl->abort)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * BN);
-                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!bar_wait(&ctrl->full[s], (it / STAGES) & 1, &ctrl->abort)) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t adesc = smem_desc_sw128(a_tiles + (size_t)s * A_STAGE_BYTES);
-                    const uint64_t bdesc = smem_desc_sw128(b_tiles + (size_t)s * B_STAGE_BYTES);
+                const uint64_t adesc = smem_desc_sw128(a_tiles + (size_t)s * A_STAGE_BYTES);
+                const uint64_t bdesc = smem_desc_sw128(b_tiles + (size_t)s * B_STAGE_BYTES);
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k)      // 32 bytes further along K in the swizzled row
                         umma_bf16(tmem_acc, adesc + (uint64_t)(k * UMMA_K * 2 >> 4), bdesc + (uint64_t)(k * UMMA_K * 2 >> 4),
                                   IDESC, (kb | k) != 0 ? 1u : 0u);
                     umma_commit(&ctrl->empty[s]);              // the stage is free once these products are done
                 }
-                umma_commit(&ctrl->acc_full[buf]);
-                ++t;
+                __syncwarp();
             }
+            if (elect_one()) umma_commit(&ctrl->acc_full[buf]);
+            __syncwarp();
+            ++t;
         }
     } else {
         // epilogue: warp w may touch TMEM lanes 32 * (w % 4) .. + 31; two warps share them, a half of the columns each

@@ -165,7 +165,7 @@ __global__ __launch_bounds__(GP_THREADS) void gemm_tcgen05_pair_kernel(const __g
                     const int s = it % P_STAGES;
                     if (!bar_wait(&ctrl->full[s], (it / P_STAGES) & 1, &ctrl->abort)) { fine = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (lane == 0) {
+                    if (elect_one()) {
                         const uint64_t adesc = smem_desc_sw128(a_tiles + (size_t)s * A_BYTES);
                         const uint64_t bdesc = smem_desc_sw128(b_tiles + (size_t)s * B_BYTES);
 #pragma unroll
@@ -177,7 +177,7 @@ __global__ __launch_bounds__(GP_THREADS) void gemm_tcgen05_pair_kernel(const __g
                     __syncwarp();
                 }
                 if (!fine) break;
-                if (lane == 0) umma_commit_pair(&ctrl->acc_full[buf]);
+                if (elect_one()) umma_commit_pair(&ctrl->acc_full[buf]);
                 __syncwarp();
             }
         }

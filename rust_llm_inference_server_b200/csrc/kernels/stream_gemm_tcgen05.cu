@@ -363,20 +363,24 @@ __global__ __launch_bounds__(S_THREADS) void stream_gemm_kernel(const __grid_con
             load_x(s, kb);
         }
         pdl_trigger();     // everything this CTA reads is requested: the next kernel may start its own requests
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
+        // the whole warp walks the loop and waits; one lane issues
         for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
             const int s = it % STG;
             if (!bar_wait(&ctrl->full[s], (it / STG) & 1, &ctrl->abort)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint64_t adesc = smem_desc_sw128(w_tiles + (size_t)s * W_STAGE_BYTES);
             const uint64_t bdesc = smem_desc_sw128(x_tiles + (size_t)s * X_STAGE_BYTES);
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < SK / 16; ++k)          // 32 bytes further along K in the swizzled row
-                umma_bf16(tmem_base, adesc + (uint64_t)(k * 32 >> 4), bdesc + (uint64_t)(k * 32 >> 4), IDESC,
-                          (it | k) != 0 ? 1u : 0u);
-            umma_commit(&ctrl->empty[s]);
+                for (int k = 0; k < SK / 16; ++k)          // 32 bytes further along K in the swizzled row
+                    umma_bf16(tmem_base, adesc + (uint64_t)(k * 32 >> 4), bdesc + (uint64_t)(k * 32 >> 4), IDESC,
+                              (it | k) != 0 ? 1u : 0u);
+                umma_commit(&ctrl->empty[s]);
+            }
+            __syncwarp();
         }
-        if (has_work) umma_commit(&ctrl->acc_full);
+        if (has_work && elect_one()) umma_commit(&ctrl->acc_full);
     }
     __syncwarp();
     pdl_wait();            // nothing is stored before the kernels before this one have finished

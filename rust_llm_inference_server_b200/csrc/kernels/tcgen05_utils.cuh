@@ -72,6 +72,20 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// True in one lane of a whole warp, always the same one: the lane that issues products and commits.  Under `lane == 0` the compiler does
+// not know that one lane is left, and moves every operand of every instruction to uniform registers by way of a loop: a burst of
+// twelve tcgen05.mma of 128 x 16 takes its thread 730 cycles that way and 183 this way.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(one));
+    return one != 0;
+}
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate) {
     asm volatile(
