@@ -1,0 +1,642 @@
+// 32-bit matrix product on the fifth-generation tensor cores: C[M, N] = A[M, K] * W[N, K]^T for float32 matrices with k of 1,024 and more.
+//
+// A float32 number is exactly the sum of three bf16 numbers (8 bits each of its 24): x = x1 + x2 + x3.  Six of the nine products of two such
+// sums carry everything above 2^-26 of x w; each is exact in the tensor core's float32 accumulator, and what an accumulator loses is its own
+// truncation (measured: 0.37 of 2^-24 of it for every 16 of k).  So w1 x1 has an accumulator of its own and the five small products share another;
+// both are read out and added in float32, rounded to nearest, every 256 of k (a segment):
+//     C = ((s0 + s1) + s2) + ..,   s = (w1 x1) + (w3 x1 + w2 x2 + w1 x3 + w2 x1 + w1 x2)
+// Off float64 by 2.5e-7 of the result at K 2048 and 8192 (normal numbers), where one chain of K FMAs is 8e-7 and 1.6e-6.  The segments and the order in
+// them are the same in both kernels below and for any number of rows, so a row's result does not depend on what else is in the batch.
+// A result that is not finite is worked out again as a chain of FMAs from the float32 operands: infinities and NaN, and numbers that
+// round to infinity in 8 bits, come out as that chain gives them.
+//
+// W is the M side of the instruction (128 features a tile), split on the way: TMA brings 128 x 32 floats, warps turn a row of 32 into three
+// planes of bf16 and put them into tensor memory as the A operand.  The rows of A are the N side, from shared memory in three planes.
+//
+// Every mbarrier wait is bounded by a fifth of a second of wall time; one that runs out sets an error word, lets every role run to its end
+// without further waiting, and the CTA still frees its tensor memory.
+// Role in the reference: `x.matmul(w.t())`, crates/model/src/layers.rs:82.
+#include "tcgen05_utils.cuh"
+#include <float.h>
+
+namespace {
+using namespace tc;
+
+constexpr int FT = 128;                     // features a tile
+constexpr int KS = 32;                      // k of a stage
+constexpr int SEG_STAGES = 8;               // stages of a segment
+constexpr int RAW_BYTES = FT * KS * 4;      // float32 weights of a stage
+constexpr int A_COLS = 3 * KS / 2;          // columns of tensor memory that the three planes of a stage's weights take
+constexpr int MAX_RINGS = 12, MAX_A = 6;    // stages of a ring in shared memory, and of the planes of weights in tensor memory
+
+struct Ctrl {
+    uint64_t raw_full[MAX_RINGS], raw_empty[MAX_RINGS], b_full[MAX_RINGS], b_empty[MAX_RINGS], a_full[MAX_A], a_empty[MAX_A], acc_full[2], acc_empty[2];
+    uint32_t tmem_base;
+    int abort;
+};
+
+struct SplitArgs {
+    const float* A;
+    const float* W;
+    float* C;
+    long long lda, ldw, ldc;
+    int M, N, K;
+    int bn;             // rows of A a tile
+    int stages;         // of k in all
+    int raw_ring;       // stages of the ring of float32 weights (few rows: and of float32 rows)
+    int rings;          // stages of the ring of A's planes (many rows)
+    int m_tiles;
+    int per;            // segments of a CTA of the cluster (few rows)
+    int early;          // the weights may be read before the kernel before has finished
+};
+
+// Two floats as three pairs of bf16 whose sum they are, low half first.
+__device__ __forceinline__ void split2(float a, float b, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+    p1 = pack_bf16(a, b);
+    a -= __uint_as_float(p1 << 16);
+    b -= __uint_as_float(p1 & 0xffff0000u);
+    p2 = pack_bf16(a, b);
+    a -= __uint_as_float(p2 << 16);
+    b -= __uint_as_float(p2 & 0xffff0000u);
+    p3 = pack_bf16(a, b);
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                 "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+// Shared-memory matrix descriptor of a K-major tile whose rows are 64 bytes wide, 64-byte swizzle (layout type 4, 512 bytes between groups of 8 rows).
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
+    return ((uint64_t)(addr >> 4) & 0x3FFFull) | (1ull << 16) | ((uint64_t)(512 >> 4) << 32) | (1ull << 46) | (4ull << 61);
+}
+
+// A value that is the same in all lanes, in a way that the compiler sees: what descriptors are made from stays in uniform registers, which
+// is where tcgen05.mma takes them.
+template <typename T> __device__ __forceinline__ T uniform(T v) { return __shfl_sync(0xffffffffu, v, 0); }
+
+// A stage's products over `n` rows of A: planes of the weights from tensor memory column `a`, of the rows from shared memory at `b`, planes
+// `plane` bytes apart; sums of w1 x1 in columns `main`, of the others in `small`.
+__device__ __forceinline__ void stage_products(uint32_t main, uint32_t small, uint32_t a, uint32_t b, uint32_t plane, int n, bool first) {
+    const uint32_t idesc = idesc_bf16(FT, n);
+    const uint64_t b1 = smem_desc_sw64(b), b2 = smem_desc_sw64(b + plane), b3 = smem_desc_sw64(b + 2 * plane);
+    const uint32_t a1 = a, a2 = a + KS / 2, a3 = a + KS;
+#pragma unroll
+    for (int k = 0; k < KS / 16; ++k) {         // 8 columns, or 32 bytes of a swizzled row, further along k
+        const uint32_t on = first && k == 0 ? 0u : 1u;
+        umma_bf16_ts(small, a3 + k * 8, b1 + k * 2, idesc, on);
+        umma_bf16_ts(small, a2 + k * 8, b2 + k * 2, idesc, 1u);
+        umma_bf16_ts(small, a1 + k * 8, b3 + k * 2, idesc, 1u);
+        umma_bf16_ts(small, a2 + k * 8, b1 + k * 2, idesc, 1u);
+        umma_bf16_ts(small, a1 + k * 8, b2 + k * 2, idesc, 1u);
+        umma_bf16_ts(main, a1 + k * 8, b1 + k * 2, idesc, on);
+    }
+}
+
+// One row of 32 float32 weights (128 bytes, 128-byte swizzle) into its three planes in tensor memory.
+__device__ __forceinline__ void split_weights(const unsigned char* raw, int row, uint32_t taddr) {
+    const unsigned char* src = raw + row * (KS * 4);
+#pragma unroll
+    for (int kk = 0; kk < 2; ++kk) {
+        uint32_t p1[8], p2[8], p3[8];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float4 v = *reinterpret_cast<const float4*>(src + (((kk * 4 + c) ^ (row & 7)) << 4));
+            split2(v.x, v.y, p1[2 * c], p2[2 * c], p3[2 * c]);
+            split2(v.z, v.w, p1[2 * c + 1], p2[2 * c + 1], p3[2 * c + 1]);
+        }
+        tmem_st8(taddr + kk * 8, p1);
+        tmem_st8(taddr + KS / 2 + kk * 8, p2);
+        tmem_st8(taddr + KS + kk * 8, p3);
+    }
+    tmem_st_wait();
+}
+
+// An output that did not come out finite, as a chain of FMAs.
+__device__ __noinline__ float chain(const float* __restrict__ a, const float* __restrict__ w, int K) {
+    float acc = 0.f;
+    for (int k = 0; k < K; ++k) acc = fmaf(a[k], w[k], acc);
+    return acc;
+}
+__device__ __forceinline__ void store(const SplitArgs& p, int m, int n, float v) {
+    if (!(fabsf(v) <= FLT_MAX)) v = chain(p.A + (size_t)m * p.lda, p.W + (size_t)n * p.ldw, p.K);
+    p.C[(size_t)m * p.ldc + n] = v;
+}
+
+// The rows of A in three planes: planes[p][m][0 .. pitch), zeros beyond K.
+__global__ __launch_bounds__(256) void split_rows_kernel(const float* __restrict__ A, long long lda, bf16* __restrict__ planes, int M, int K, int pitch) {
+    pdl_wait_and_trigger();
+    const int per_row = pitch / 4, vec = ((reinterpret_cast<uintptr_t>(A) & 15) == 0 && lda % 4 == 0);
+    const size_t plane = (size_t)M * pitch;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)M * per_row; i += (size_t)gridDim.x * blockDim.x) {
+        const int m = (int)(i / per_row), k = (int)(i % per_row) * 4;
+        const float* src = A + (size_t)m * lda + k;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (vec && k + 3 < K) v = *reinterpret_cast<const float4*>(src);
+        else {
+            if (k < K) v.x = src[0];
+            if (k + 1 < K) v.y = src[1];
+            if (k + 2 < K) v.z = src[2];
+            if (k + 3 < K) v.w = src[3];
+        }
+        uint2 p1, p2, p3;
+        split2(v.x, v.y, p1.x, p2.x, p3.x);
+        split2(v.z, v.w, p1.y, p2.y, p3.y);
+        bf16* dst = planes + (size_t)m * pitch + k;
+        *reinterpret_cast<uint2*>(dst) = p1;
+        *reinterpret_cast<uint2*>(dst + plane) = p2;
+        *reinterpret_cast<uint2*>(dst + 2 * plane) = p3;
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Many rows.  700 rows, us here and in FFMA tiles: K 2048 N 16384 228 / 1139, N 3072 50 / 218, N 2048 44 / 218; K 8192 N 2048 142 / 858; 2,048 rows of K 2048 N 16384
+// 649 / 2648 (212 TFLOP/s, six times that on the tensor cores: 1.27 PFLOP/s).  Bound by the pipe for whole tiles of 176 and 192 rows (1,700 cycles a
+// stage for 1,056 of products; bytes through shared memory are close behind), by about 800 cycles of a stage's waits for small ones.
+// A tile of 128 features x bn rows of A a CTA (bn up to 192), in two halves of the rows with accumulators, an issuing warp and four adding
+// warps of their own: one warp alone spends more cycles between the bursts of two stages than the pipe has instructions queued.
+// The rings have an even number of stages: a set meets the same ones every time, and so sees every phase of their barriers.
+// Twenty warps, by role: 0-7 add the segments up and store, 8-15 split weights (two sets, taking turns at the stages), 16 and 17 ask for weights
+// and for A's planes, 18 and 19 issue the products.
+constexpr int MANY_THREADS = 640, MAX_BN = 192, HALF = MAX_BN / 2;
+constexpr int MANY_RING_BYTES = 225 * 1024;         // both rings (tiles of 192 rows: four stages each)
+constexpr int MANY_SMEM = 1024 + MANY_RING_BYTES + (int)sizeof(Ctrl);
+static_assert(MANY_SMEM <= 227 * 1024, "shared memory");
+
+__global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
+                                                                         const SplitArgs p) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* raw = base;
+    unsigned char* planes = base + p.raw_ring * RAW_BYTES;
+    Ctrl* ctrl = reinterpret_cast<Ctrl*>(base + MANY_RING_BYTES);
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int f0 = (int)(blockIdx.x / p.m_tiles) * FT, m0 = (int)(blockIdx.x % p.m_tiles) * p.bn;
+    const int n0 = (p.bn / 2 + 15) / 16 * 16, n1 = p.bn - n0;      // rows of the halves (the second has none where bn is 16)
+    const uint32_t plane = (uint32_t)p.bn * (KS * 2), b_bytes = 3 * plane;
+    const int a_ring = min(MAX_A, (512 - 4 * n0) / A_COLS) & ~1;
+
+    if (threadIdx.x == 0) {
+        ctrl->abort = 0;
+        for (int i = 0; i < MAX_RINGS; ++i) {
+            bar_init(&ctrl->raw_full[i], 1);
+            bar_init(&ctrl->raw_empty[i], 4);
+            bar_init(&ctrl->b_full[i], 1);
+            bar_init(&ctrl->b_empty[i], n1 > 0 ? 2 : 1);
+        }
+        for (int i = 0; i < MAX_A; ++i) {
+            bar_init(&ctrl->a_full[i], 4);
+            bar_init(&ctrl->a_empty[i], n1 > 0 ? 2 : 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            bar_init(&ctrl->acc_full[i], 1);
+            bar_init(&ctrl->acc_empty[i], 4);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 18) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctrl->tmem_base)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = uniform(ctrl->tmem_base), a_base = tmem + 4 * n0;     // halves of [w1 x1 | the rest], n0 columns each; planes of weights
+
+    if (warp >= 16) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+        if (warp == 16) {
+            if (lane == 0) {
+                if (!p.early) pdl_wait();
+                for (int it = 0, s = 0, turn = 0; it < p.stages; ++it) {
+                    if (turn > 0 && !bar_wait(&ctrl->raw_empty[s], (turn - 1) & 1, &ctrl->abort)) break;
+                    bar_expect_tx(&ctrl->raw_full[s], RAW_BYTES);
+                    tma_load_2d(raw + s * RAW_BYTES, &map_w, it * KS, f0, &ctrl->raw_full[s]);
+                    if (++s == p.raw_ring) { s = 0; ++turn; }
+                }
+            }
+        } else if (warp == 17) {
+            if (lane == 0) {
+                pdl_wait();
+                for (int it = 0, s = 0, turn = 0; it < p.stages; ++it) {
+                    if (turn > 0 && !bar_wait(&ctrl->b_empty[s], (turn - 1) & 1, &ctrl->abort)) break;
+                    bar_expect_tx(&ctrl->b_full[s], b_bytes);
+                    tma_load_3d(planes + (size_t)s * b_bytes, &map_a, it * KS, m0, 0, &ctrl->b_full[s]);
+                    if (++s == p.rings) { s = 0; ++turn; }
+                }
+            }
+        } else if (warp == 18 || n1 > 0) {
+            const int h = warp - 18, n = h ? n1 : n0;
+            const uint32_t main = tmem + (uint32_t)(h * 2 * n0), rows = smem_u32(planes) + (uint32_t)(h * n0) * (KS * 2);
+            int s = 0, a = 0;
+            uint32_t a_turn = 0;
+            for (int it = 0; it < p.stages; ++it) {
+                const bool first = it % SEG_STAGES == 0, last = it % SEG_STAGES == SEG_STAGES - 1 || it == p.stages - 1;
+                if (first && it > 0 && !bar_wait_warp(&ctrl->acc_empty[h], (it / SEG_STAGES - 1) & 1, &ctrl->abort)) break;
+                if (!bar_wait_warp(&ctrl->a_full[a], a_turn, &ctrl->abort)) break;           // the rows' planes are there, too
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (elect_one()) {
+                    stage_products(main, main + n0, a_base + (uint32_t)(a * A_COLS), rows + (uint32_t)s * b_bytes, plane, n, first);
+                    umma_commit(&ctrl->a_empty[a]);
+                    umma_commit(&ctrl->b_empty[s]);
+                    if (last) umma_commit(&ctrl->acc_full[h]);
+                }
+                __syncwarp();
+                if (++s == p.rings) s = 0;
+                if (++a == a_ring) { a = 0; a_turn ^= 1; }
+            }
+        }
+    } else if (warp >= 8) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+        const int set = (warp - 8) / 4, row = (warp & 3) * 32 + lane;
+        const uint32_t taddr = a_base + ((uint32_t)((warp & 3) * 32) << 16);
+        int s = set, a = set, b = set % p.rings;
+        uint32_t turn = 0, a_turn = 0, b_turn = set / p.rings;
+        for (int it = set; it < p.stages; it += 2) {
+            if (!bar_wait_warp(&ctrl->raw_full[s], turn & 1, &ctrl->abort)) break;
+            if (a_turn > 0 && !bar_wait_warp(&ctrl->a_empty[a], (a_turn - 1) & 1, &ctrl->abort)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            split_weights(raw + s * RAW_BYTES, row, taddr + (uint32_t)(a * A_COLS));
+            if (!bar_wait_warp(&ctrl->b_full[b], b_turn & 1, &ctrl->abort)) break;
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                bar_arrive(&ctrl->a_full[a]);
+                bar_arrive(&ctrl->raw_empty[s]);
+            }
+            s += 2;
+            if (s >= p.raw_ring) { s -= p.raw_ring; ++turn; }
+            a += 2;
+            if (a >= a_ring) { a -= a_ring; ++a_turn; }
+            b += 2;
+            if (b >= p.rings) { b -= p.rings; ++b_turn; }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
+        const int h = warp >> 2, q = warp & 3, cols = h ? n1 : n0, segs = cols == 0 ? 0 : (p.stages + SEG_STAGES - 1) / SEG_STAGES;
+        const uint32_t main = tmem + (uint32_t)(h * 2 * n0) + ((uint32_t)(q * 32) << 16);
+        float sum[HALF];
+#pragma unroll
+        for (int c = 0; c < HALF; ++c) sum[c] = 0.f;
+        for (int seg = 0; seg < segs; ++seg) {
+            if (!bar_wait_warp(&ctrl->acc_full[h], seg & 1, &ctrl->abort)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < HALF / 16; ++c) {
+                if (c * 16 < cols) {
+                    uint32_t a[16], b[16];
+                    tmem_ld16_nowait(main + c * 16, a);
+                    tmem_ld16_nowait(main + n0 + c * 16, b);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) sum[c * 16 + j] += __uint_as_float(a[j]) + __uint_as_float(b[j]);
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(&ctrl->acc_empty[h]);
+        }
+        const int n = f0 + q * 32 + lane, m1 = m0 + h * n0;
+        pdl_wait();         // (C may still be read by the kernel before, whose end the producers alone have waited for)
+        if (n < p.N && !ctrl->abort) {
+#pragma unroll
+            for (int c = 0; c < HALF; ++c)
+                if (c < cols && m1 + c < p.M) store(p, m1 + c, n, sum[c]);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 18) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+    pdl_trigger();
+}
+
+// ------------------------------------------------------------------------------------------------
+// Few rows (a decode step): bound by the memory's rate over W, and below it by a stage's way through the roles (raw weights, planes, products: about
+// 900 cycles with one CTA on an SM, 600 a stage with two).  8 rows, us here and as chains of FMAs: K 2048 N 2048 8.9 / 11.3, N 3072 9.8 / 16, N 16384 28 / 42,
+// N 32000 47 / 81 (5.6 TB/s); K 8192 N 2048 26 / 37.  A tile of 128 features a cluster, whose CTAs take whole segments of k and leave their
+// sums in shared memory; the cluster then adds them up in the order of k, each CTA for a share of the features.  The rows of A are split
+// where the weights are.  Fourteen warps: 0-3 read the accumulators, 4-11 split (two sets), 12 asks for weights and rows, 13 issues the products.
+constexpr int FEW_THREADS = 448, FEW_A = 4;
+
+template <int BN> struct Few {
+    static constexpr int ROWS_BYTES = BN * KS * 4, STAGE = RAW_BYTES + ROWS_BYTES, PLANES = 3 * BN * KS * 2, ROW = FT * 4;
+    static constexpr int ACC = BN == 16 ? 2 : 1;                // accumulators: of two segments where there is room for them
+    static_assert(ACC * 2 * BN + FEW_A * A_COLS <= 256, "two CTAs an SM share its tensor memory");
+    static constexpr int smem(int rings, int rows) { return 1024 + rings * STAGE + FEW_A * PLANES + rows * ROW + (int)sizeof(Ctrl); }
+};
+
+template <int BN>
+__global__ __launch_bounds__(FEW_THREADS, 2) void f32_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
+                                                                       const SplitArgs p, int parts) {
+    using F = Few<BN>;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* ring = base;                                             // weights, then rows
+    unsigned char* planes = base + p.raw_ring * F::STAGE;
+    float* sums = reinterpret_cast<float*>(planes + FEW_A * F::PLANES);     // [segment of this CTA][row][feature]
+    Ctrl* ctrl = reinterpret_cast<Ctrl*>(reinterpret_cast<unsigned char*>(sums) + (parts == 1 ? 1 : p.per) * p.M * F::ROW);
+    const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int f0 = (int)(blockIdx.x / parts) * FT, part = (int)(blockIdx.x % parts);
+    const int segs = (p.stages + SEG_STAGES - 1) / SEG_STAGES;
+    const int seg0 = min(part * p.per, segs), mine = min(segs - seg0, p.per);
+    const int st0 = seg0 * SEG_STAGES, stages = max(0, min(p.stages, (seg0 + mine) * SEG_STAGES) - st0);
+
+    if (threadIdx.x == 0) {
+        ctrl->abort = 0;
+        for (int i = 0; i < MAX_RINGS; ++i) {
+            bar_init(&ctrl->raw_full[i], 1);
+            bar_init(&ctrl->raw_empty[i], 8);
+        }
+        for (int i = 0; i < FEW_A; ++i) {
+            bar_init(&ctrl->a_full[i], 8);
+            bar_init(&ctrl->a_empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            bar_init(&ctrl->acc_full[i], 1);
+            bar_init(&ctrl->acc_empty[i], 4);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 13) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctrl->tmem_base)), "r"(256) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = uniform(ctrl->tmem_base), a_base = tmem + F::ACC * 2 * BN;
+
+    if (warp == 12) {
+        if (lane == 0) {
+            // weights that no kernel of a step writes are asked for before the wait; the rows after it
+            if (!p.early) pdl_wait();
+            const int early = min(stages, p.raw_ring);
+            for (int it = 0; it < early; ++it) {
+                bar_expect_tx(&ctrl->raw_full[it], F::STAGE);
+                tma_load_2d(ring + it * F::STAGE, &map_w, (st0 + it) * KS, f0, &ctrl->raw_full[it]);
+            }
+            pdl_wait();
+            for (int it = 0; it < early; ++it) tma_load_2d(ring + it * F::STAGE + RAW_BYTES, &map_a, (st0 + it) * KS, 0, &ctrl->raw_full[it]);
+            for (int it = early, s = 0, turn = 1; it < stages; ++it) {
+                if (!bar_wait(&ctrl->raw_empty[s], (turn - 1) & 1, &ctrl->abort)) break;
+                unsigned char* dst = ring + s * F::STAGE;
+                bar_expect_tx(&ctrl->raw_full[s], F::STAGE);
+                tma_load_2d(dst, &map_w, (st0 + it) * KS, f0, &ctrl->raw_full[s]);
+                tma_load_2d(dst + RAW_BYTES, &map_a, (st0 + it) * KS, 0, &ctrl->raw_full[s]);
+                if (++s == p.raw_ring) { s = 0; ++turn; }
+            }
+            pdl_trigger();
+        }
+    } else if (warp == 13) {
+        for (int it = 0; it < stages; ++it) {
+            const int seg = it / SEG_STAGES, buf = seg % F::ACC, a = it % FEW_A;
+            const bool first = it % SEG_STAGES == 0, last = it % SEG_STAGES == SEG_STAGES - 1 || it == stages - 1;
+            if (first && seg >= F::ACC && !bar_wait_warp(&ctrl->acc_empty[buf], (seg / F::ACC - 1) & 1, &ctrl->abort)) break;
+            if (!bar_wait_warp(&ctrl->a_full[a], (it / FEW_A) & 1, &ctrl->abort)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one()) {
+                const uint32_t main = tmem + (uint32_t)(buf * 2 * BN);
+                stage_products(main, main + BN, a_base + (uint32_t)(a * A_COLS), smem_u32(planes) + (uint32_t)(a * F::PLANES), BN * KS * 2, BN, first);
+                umma_commit(&ctrl->a_empty[a]);
+                if (last) umma_commit(&ctrl->acc_full[buf]);
+            }
+            __syncwarp();
+        }
+    } else if (warp >= 4) {
+        const int set = (warp - 4) / 4, row = (warp & 3) * 32 + lane;
+        const uint32_t taddr = a_base + ((uint32_t)((warp & 3) * 32) << 16);
+        int s = set, turn = 0;
+        for (int it = set; it < stages; it += 2) {
+            const int a = it % FEW_A;
+            if (!bar_wait_warp(&ctrl->raw_full[s], turn & 1, &ctrl->abort)) break;
+            if (it >= FEW_A && !bar_wait_warp(&ctrl->a_empty[a], (it / FEW_A - 1) & 1, &ctrl->abort)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            split_weights(ring + s * F::STAGE, row, taddr + (uint32_t)(a * A_COLS));
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                bar_arrive(&ctrl->a_full[a]);
+                bar_arrive(&ctrl->raw_empty[s]);
+            }
+            s += 2;
+            if (s >= p.raw_ring) { s -= p.raw_ring; ++turn; }
+        }
+    } else {
+        // the rows' planes, stage by stage, and behind each segment its sums
+        const int f = threadIdx.x;
+        auto take = [&](int seg) {
+            const int buf = seg % F::ACC;
+            if (!bar_wait_warp(&ctrl->acc_full[buf], (seg / F::ACC) & 1, &ctrl->abort)) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t main = tmem + (uint32_t)(buf * 2 * BN) + ((uint32_t)(warp * 32) << 16);
+            float* dst = sums + (parts == 1 ? 0 : seg * p.M * FT) + f;
+#pragma unroll
+            for (int c = 0; c < BN / 16; ++c) {
+                uint32_t a[16], b[16];
+                tmem_ld16_nowait(main + c * 16, a);
+                tmem_ld16_nowait(main + BN + c * 16, b);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (c * 16 + j >= p.M) break;
+                    const float v = __uint_as_float(a[j]) + __uint_as_float(b[j]);
+                    float* at = dst + (c * 16 + j) * FT;
+                    *at = parts == 1 ? (seg == 0 ? 0.f : *at) + v : v;
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(&ctrl->acc_empty[buf]);
+            return true;
+        };
+        int s = 0, turn = 0, taken = 0;
+        bool fine = true;
+        for (int it = 0; it < stages; ++it) {
+            const int a = it % FEW_A;
+            // a segment's sums are due before the products that wait for their accumulator, and not before its last products are on their way
+            if (it / SEG_STAGES >= taken + F::ACC && !(fine = take(taken++))) break;
+            if (!(fine = bar_wait_warp(&ctrl->raw_full[s], turn & 1, &ctrl->abort))) break;
+            if (it >= FEW_A && !(fine = bar_wait_warp(&ctrl->a_empty[a], (it / FEW_A - 1) & 1, &ctrl->abort))) break;
+            const unsigned char* src = ring + s * F::STAGE + RAW_BYTES;
+            unsigned char* dst = planes + a * F::PLANES;
+#pragma unroll
+            for (int i = 0; i < BN / 16; ++i) {         // four numbers of a row of A into 64-byte rows, 64-byte swizzle
+                const int r = i * 16 + (f >> 3), c = f & 7;
+                const float4 v = *reinterpret_cast<const float4*>(src + r * (KS * 4) + ((c ^ (r & 7)) << 4));
+                uint2 p1, p2, p3;
+                split2(v.x, v.y, p1.x, p2.x, p3.x);
+                split2(v.z, v.w, p1.y, p2.y, p3.y);
+                unsigned char* d = dst + r * (KS * 2) + (((c >> 1) ^ ((r >> 1) & 3)) << 4) + (c & 1) * 8;
+                *reinterpret_cast<uint2*>(d) = p1;
+                *reinterpret_cast<uint2*>(d + BN * KS * 2) = p2;
+                *reinterpret_cast<uint2*>(d + 2 * BN * KS * 2) = p3;
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                bar_arrive(&ctrl->a_full[a]);
+                bar_arrive(&ctrl->raw_empty[s]);
+            }
+            if (++s == p.raw_ring) { s = 0; ++turn; }
+        }
+        while (fine && taken < mine) fine = take(taken++);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 13) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
+    }
+    pdl_wait();             // (C may still be read by the kernel before, whose end one thread alone has waited for)
+    if (parts == 1) {
+        for (int i = threadIdx.x; i < p.M * FT; i += FEW_THREADS)
+            if (f0 + i % FT < p.N && !ctrl->abort) store(p, i / FT, f0 + i % FT, sums[i]);
+    } else {
+        cluster_sync_all();
+        const int share = (FT + parts - 1) / parts, lo = part * share, width = max(0, min(FT - lo, share));
+        for (int i = threadIdx.x; i < p.M * width; i += FEW_THREADS) {
+            const int m = i / width, f = lo + i % width;
+            float v = 0.f;
+            for (int s0 = 0; s0 < segs; s0 += 8) {
+                float x[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int seg = min(s0 + j, segs - 1);
+                    x[j] = ld_dsmem(sums + (seg % p.per) * p.M * FT + m * FT + f, (uint32_t)(seg / p.per));
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (s0 + j < segs) v += x[j];
+            }
+            if (f0 + f < p.N && !ctrl->abort) store(p, m, f0 + f, v);
+        }
+        cluster_sync_all();         // nobody leaves while another CTA reads its sums
+    }
+    pdl_trigger();
+}
+
+// A float32 [rows, K] matrix with boxes of 32 k x box_rows rows, 128-byte swizzle.
+bool map_f32(CUtensorMap* map, const float* ptr, int rows, int K, long long ld, int box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (fn == nullptr) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld * 4};
+    const cuuint32_t box[2] = {(cuuint32_t)KS, (cuuint32_t)box_rows}, estr[2] = {1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// The three planes of `rows` rows, pitch apart, with boxes of 32 k x box_rows rows x 3 planes, 64-byte swizzle.
+bool map_planes(CUtensorMap* map, const bf16* ptr, int rows, int pitch, int box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (fn == nullptr) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)pitch, (cuuint64_t)rows, 3}, strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)pitch * rows * 2};
+    const cuuint32_t box[3] = {(cuuint32_t)KS, (cuuint32_t)box_rows, 3}, estr[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+int sm_count() {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+constexpr int FEW_ROWS = 32, MAX_PARTS = 8;
+int g_bn = 0, g_parts = 0;      // held fixed by a measurement (0: automatic)
+
+template <int BN> int launch_few(SplitArgs p, cudaStream_t stream) {
+    using F = Few<BN>;
+    const int sms = sm_count(), tiles = (p.N + FT - 1) / FT, segs = (p.stages + SEG_STAGES - 1) / SEG_STAGES;
+    // CTAs a tile: by what a segment takes a CTA alone on its SM (about 7,200 cycles) and beside another (9,600), and by what a CTA takes beside its segments.
+    // 8 rows, us with 1, 2, 4 and 8 CTAs a tile: N 16384 K 2048 33, 29, 32, 39; N 32000 48, 55, 61, 72; N 3072 27, 16, 11, 9.5; N 2048 K 8192 101, 61, 29, 26.
+    int parts = 1;
+    long long best = -1;
+    for (int c = 1; c <= MAX_PARTS && c <= segs; ++c) {
+        const int per = (segs + c - 1) / c;
+        if (c > 1 && F::smem(4, per * p.M) > 227 * 1024) continue;
+        const long long ctas = (long long)tiles * c;
+        const long long cost = (ctas <= sms ? 7200LL : 9600LL) * per + (c > 1 ? 5000 : 2500), total = (ctas + 2 * sms - 1) / (2 * sms) * cost;
+        if (best < 0 || total < best) { best = total; parts = c; }
+    }
+    if (g_parts > 0 && g_parts <= segs && F::smem(4, (segs + g_parts - 1) / g_parts * p.M) <= 227 * 1024) parts = g_parts;
+    p.per = (segs + parts - 1) / parts;
+    const int rows = (parts == 1 ? 1 : p.per) * p.M;
+    p.raw_ring = F::smem(6, rows) <= 113 * 1024 ? 6 : 4;       // (even, see above; room for a second CTA on the SM, of this product or of the kernel after it)
+    CUtensorMap map_w, map_a;
+    if (!map_f32(&map_w, p.W, p.N, p.K, p.ldw, FT) || !map_f32(&map_a, p.A, p.M, p.K, p.lda, BN)) return RLIS_ERR_UNSUPPORTED;
+    const int smem = F::smem(p.raw_ring, rows);
+    const cudaError_t e = cudaFuncSetAttribute(f32_split_few_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    rlis_launch_cluster(f32_split_few_kernel<BN>, dim3((unsigned)(tiles * parts)), dim3(FEW_THREADS), (size_t)smem, stream, dim3((unsigned)parts, 1, 1), map_w, map_a, p, parts);
+    return RLIS_LAUNCH_CHECK();
+}
+
+// Rows of A a tile: what takes the SMs least time.  Measured on 700 rows, in cycles a stage: 16 rows 850, 64 990, 96 1180, 128 1330, 176 1700, 192 1860;
+// a tile takes about 6,000 cycles beside its stages.
+int choose_bn(int M, int N, int stages, int sms) {
+    if (g_bn > 0) return g_bn;
+    const long long f_tiles = (N + FT - 1) / FT;
+    int best = 16;
+    double least = -1;
+    for (int bn = 16; bn <= MAX_BN; bn += 16) {
+        const long long waves = (f_tiles * ((M + bn - 1) / bn) + sms - 1) / sms;
+        const double t = (double)waves * (stages * (750 + 5.5 * bn) + 6000);
+        if (least < 0 || t < least) { least = t; best = bn; }
+    }
+    return best;
+}
+}  // namespace
+
+extern "C" int rlis_gemm_f32_split_few_rows(void) { return FEW_ROWS; }
+extern "C" void rlis_gemm_f32_split_set_rows(int n) { g_bn = n >= 16 && n <= MAX_BN && n % 16 == 0 ? n : 0; }
+extern "C" void rlis_gemm_f32_split_set_parts(int n) { g_parts = n >= 0 && n <= MAX_PARTS ? n : 0; }
+
+// C[M, N] = A[M, K] W[N, K]^T, rows lda, ldw, ldc floats apart; A, W, lda and ldw on 16-byte boundaries, K >= 1.  More than
+// rlis_gemm_f32_split_few_rows() rows: `planes` is scratch of 3 * M * (K rounded up to 8) bf16 on a 16-byte boundary.  `early`: no kernel
+// that is still running writes W, so that its first tiles may be asked for before those before in the stream have finished.
+extern "C" int rlis_gemm_f32_split(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc, int M, int N, int K, void* planes,
+                                   int early, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K <= 0 || lda % 4 || ldw % 4 || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15)) return RLIS_ERR_UNSUPPORTED;
+    SplitArgs p = {A, W, C, lda, ldw, ldc, M, N, K, 0, (K + KS - 1) / KS, 0, 0, 1, 0, early};
+    if (M <= 16) return launch_few<16>(p, stream);
+    if (M <= FEW_ROWS) return launch_few<32>(p, stream);
+    if (planes == nullptr || (reinterpret_cast<uintptr_t>(planes) & 15)) return RLIS_ERR_UNSUPPORTED;
+    const int sms = sm_count(), pitch = (K + 7) / 8 * 8;
+    const long long pieces = (long long)M * (pitch / 4);
+    rlis_launch(split_rows_kernel, dim3((unsigned)(pieces / 256 + 1 < 8LL * sms ? pieces / 256 + 1 : 8LL * sms)), dim3(256), 0, stream, A, lda,
+                reinterpret_cast<bf16*>(planes), M, K, pitch);
+    int rc = RLIS_LAUNCH_CHECK();
+    if (rc != 0) return rc;
+    p.bn = choose_bn(M, N, p.stages, sms);
+    p.m_tiles = (M + p.bn - 1) / p.bn;
+    const int b_bytes = 3 * p.bn * KS * 2;
+    p.rings = p.bn > 64 ? 4 : 6;
+    p.raw_ring = (MANY_RING_BYTES - p.rings * b_bytes) / RAW_BYTES & ~1;
+    if (p.raw_ring > 8) p.raw_ring = 8;
+    CUtensorMap map_w, map_a;
+    if (!map_f32(&map_w, W, N, K, ldw, FT) || !map_planes(&map_a, reinterpret_cast<const bf16*>(planes), M, pitch, p.bn)) return RLIS_ERR_UNSUPPORTED;
+    const cudaError_t e = cudaFuncSetAttribute(f32_split_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MANY_SMEM);
+    if (e != cudaSuccess) return (int)e;
+    const long long tiles = (long long)((N + FT - 1) / FT) * p.m_tiles;
+    rlis_launch(f32_split_many_kernel, dim3((unsigned)tiles), dim3(MANY_THREADS), (size_t)MANY_SMEM, stream, map_w, map_a, p);
+    return RLIS_LAUNCH_CHECK();
+}
+
+extern "C" int rlis_gemm_f32_split_error(void) { return tc::read_error_word(); }
+extern "C" int* rlis_gemm_f32_split_error_addr(void) { return tc::error_word_addr(); }

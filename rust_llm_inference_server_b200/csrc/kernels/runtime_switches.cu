@@ -24,7 +24,11 @@ extern "C" int rlis_get_pdl(void) { return g_rlis_pdl; }
 //   prefill_splits   0,1,2,4   CTAs that share a tile's keys in the tcgen05 prefill attention (0: automatic)
 //   gemm_pair        -1 / 0    two SMs to a tile in the tcgen05 product of many rows (-1: where it applies)
 //   filtered_cluster 0 / 1     the cluster kernel of top-k / top-p sampling where the vocabulary fits
+//   f32_split_rows   0, 16..192 rows a tile of the float32 product on tensor cores (0: automatic)
+//   f32_split_parts  0, 1..8   CTAs that share a tile's k there when the rows are few (0: automatic)
 extern "C" void rlis_stream_gemm_set_target(int);
+extern "C" void rlis_gemm_f32_split_set_rows(int);
+extern "C" void rlis_gemm_f32_split_set_parts(int);
 extern "C" void rlis_stream_gemm_set_min_stages(int);
 extern "C" void rlis_gemm_tcgen05_set_pair(int);
 extern "C" void rlis_attention_decode_set_stages(int);
@@ -43,6 +47,8 @@ extern "C" int rlis_debug_set(const char* name, int value) {
     else if (!strcmp(name, "decode_tma")) rlis_attention_decode_set_tma(value);
     else if (!strcmp(name, "prefill_splits")) rlis_attention_prefill_tc_set_splits(value);
     else if (!strcmp(name, "gemm_pair")) rlis_gemm_tcgen05_set_pair(value);
+    else if (!strcmp(name, "f32_split_rows")) rlis_gemm_f32_split_set_rows(value);
+    else if (!strcmp(name, "f32_split_parts")) rlis_gemm_f32_split_set_parts(value);
     else if (!strcmp(name, "filtered_cluster")) rlis_sample_filtered_set_cluster(value);
     else return RLIS_ERR_UNSUPPORTED;
     return 0;
@@ -57,9 +63,10 @@ extern "C" int* rlis_stream_gemm_error_addr(void);
 extern "C" int* rlis_attention_prefill_tc_error_addr(void);
 extern "C" int* rlis_attention_decode_error_addr(void);
 extern "C" int* rlis_attention_difference_decode_error_addr(void);
+extern "C" int* rlis_gemm_f32_split_error_addr(void);
 
 namespace {
-constexpr int kWords = 5;
+constexpr int kWords = 6;
 struct ErrorWords { int* w[kWords]; };
 
 __global__ void take_errors_kernel(ErrorWords words, int* __restrict__ out) {
@@ -82,7 +89,7 @@ extern "C" int rlis_take_errors(int* out, cudaStream_t stream) {
     if (!g_words_known[dev]) {
         ErrorWords w = {{rlis_gemm_tcgen05_error_addr(), rlis_stream_gemm_error_addr(),
                          rlis_attention_prefill_tc_error_addr(), rlis_attention_decode_error_addr(),
-                         rlis_attention_difference_decode_error_addr()}};
+                         rlis_attention_difference_decode_error_addr(), rlis_gemm_f32_split_error_addr()}};
         for (int i = 0; i < kWords; ++i)
             if (w.w[i] == nullptr) return RLIS_ERR_UNSUPPORTED;
         g_words[dev] = w;

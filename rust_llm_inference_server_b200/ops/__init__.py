@@ -4,7 +4,7 @@ Every function takes CUDA tensors, checks element types, shapes and contiguity, 
 the current stream.  A size that a kernel does not take is refused with an error; nothing here
 falls back to a tensor library's model code or to the CPU.  Matrix products in bfloat16 go to the
 library GEMM (cuBLAS through `torch.mm`), as the reference's go to its tensor library
-(crates/model/src/layers.rs:82); in float32 they go to this package's own FFMA kernel so that
+(crates/model/src/layers.rs:82); in float32 they go to this package's own kernels so that
 no reduced-precision matrix mode can enter.
 """
 
@@ -186,8 +186,37 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor, interleave: int = 0) -> tor
     return out
 
 
+# Products over this much of k and more go to the tensor cores.  A row has the same bits with any other rows beside it, so the rule asks for the matrix and not for the
+# rows.  us on the tensor cores and as chains of FMAs, 1, 8 and 300 rows: N 576 K 2048 6.3 / 10.1, 6.2 / 10.1, 33 / 56; N 2048 K 14336 52 / 68, 54 / 64,
+# 188 / 1164; but N 4096 K 1024 8.3 / 7.0 at one row, and a chain of 1,024 is closer to float64 than one of 8,192 by three times.
+SPLIT_MIN_K = 2048
+_SPLIT_PLANES = 128 << 20       # bytes of scratch that a product's rows are cut to
+
+
+def _gemm_f32_splits(a: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether a [M, K] @ w[N, K]^T in float32 is done as six products of bfloat16 parts on the tensor cores: long rows on 16-byte boundaries."""
+    return w.shape[1] >= SPLIT_MIN_K and w.shape[1] % 4 == 0 and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+
+
+def _gemm_f32_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, early: bool = False) -> torch.Tensor:
+    """The product of `gemm_f32` on the tensor cores; rows of a and out may lie in wider ones.  `early`: w is a weight, whose first tiles may be read
+    before the kernels before have finished, as `stream_gemm` does."""
+    (M, K), N = a.shape, w.shape[0]
+    few = lib().rlis_gemm_f32_split_few_rows()
+    rows = M if M <= few else max(few + 1, _SPLIT_PLANES // (6 * K))
+    planes = torch.empty((3 * min(M, rows) * ((K + 7) // 8 * 8),), dtype=torch.bfloat16, device=a.device) if M > few else None
+    for m in range(0, M, max(1, rows)):
+        n = min(rows, M - m)
+        check(lib().rlis_gemm_f32_split(a[m:].data_ptr(), a.stride(0), w.data_ptr(), K, out[m:].data_ptr(), out.stride(0), n, N, K,
+                                        planes.data_ptr() if n > few else None, int(early), _stream()), "gemm_f32")
+    _count("gemm_f32.split")
+    return out
+
+
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """out[M, N] = a[M, K] @ w[N, K]^T in true float32 (FFMA, fixed order over K)."""
+    """out[M, N] = a[M, K] @ w[N, K]^T in true float32: rows of `SPLIT_MIN_K` and more on the tensor cores, every operand as the exact sum of three
+    bfloat16 numbers (`csrc/kernels/gemm_f32_split.cu`), others as chains of FMAs in the order of k.  A row has the same bits whatever other
+    rows there are."""
     M, K = a.shape
     N = w.shape[0]
     _req(a, "a", torch.float32)
@@ -195,6 +224,8 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) 
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=a.device)
     _req(out, "out", torch.float32, (M, N))
+    if _gemm_f32_splits(a, w):
+        return _gemm_f32_split(a, w, out)
     check(lib().rlis_gemm_f32_nt(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, _stream()),
           "gemm_f32")
     _count("gemm_f32")
@@ -202,7 +233,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) 
 
 
 def gemm_f32_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-    """out[:, b, :] = a[:, b, :] @ w[b]^T for every b, in true float32 (the same kernel and k order as
+    """out[:, b, :] = a[:, b, :] @ w[b]^T for every b, in true float32 (the same kernels as
     `gemm_f32`).  a [M, B, K], out [M, B, N]: views whose last axis has unit stride (the per-head
     slices of wider rows); w [B, N, K] contiguous."""
     M, B, K = a.shape
@@ -213,6 +244,9 @@ def gemm_f32_batched(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> tor
     _req(w, "w", torch.float32, (B, N, K))
     if tuple(out.shape) != (M, B, N):
         raise KernelError(f"gemm_f32_batched: expected out of shape {(M, B, N)}, got {tuple(out.shape)}")
+    if B == 1 and _gemm_f32_splits(a[:, 0], w[0]):
+        _gemm_f32_split(a[:, 0], w[0], out[:, 0])
+        return out
     check(lib().rlis_gemm_f32_nt_batched(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), K,
                                          out.stride(0), B, a.stride(1), N * K, out.stride(1), _stream()),
           "gemm_f32_batched")
@@ -1288,7 +1322,7 @@ def check_device_errors() -> None:
     """Raises if a bounded wait inside a kernel ever ran out on this device (the kernel then
     finished without its data; results since are not to be trusted).  Synchronises the device."""
     code = (lib().rlis_gemm_tcgen05_error() or lib().rlis_stream_gemm_error() or lib().rlis_attention_prefill_tc_error()
-            or lib().rlis_attention_decode_error() or lib().rlis_attention_difference_decode_error())
+            or lib().rlis_attention_decode_error() or lib().rlis_attention_difference_decode_error() or lib().rlis_gemm_f32_split_error())
     if code != 0:
         raise KernelError(f"a bounded mbarrier wait of a tcgen05 kernel ran out on the device (code {code})")
 
@@ -1301,7 +1335,7 @@ def fuses_norms(n_rows: int, dtype, *widths: int) -> bool:
 
 
 def linear(x, w: torch.Tensor, out_dtype=None, sink=None, bias: torch.Tensor | None = None, second: tuple | None = None):
-    """y = x @ w^T for w stored (out, in); x may be a column slice of wider rows.  float32: this package's FFMA kernel.
+    """y = x @ w^T for w stored (out, in); x may be a column slice of wider rows.  float32: this package's kernels (`gemm_f32`).
     bfloat16: up to 16 rows go to this package's weight-streaming tcgen05 kernel, more to the library GEMM; both
     accumulate in float32, and `out_dtype=torch.float32` keeps that precision (used for logits).
     ScaledRows as x, a `sink` (with an optional `bias` of the product) and a `second` source = (x2, w2), whose product is
@@ -1313,6 +1347,8 @@ def linear(x, w: torch.Tensor, out_dtype=None, sink=None, bias: torch.Tensor | N
     if bias is not None:
         raise KernelError("linear: a bias is taken with a sink")
     if x.dtype == torch.float32:
+        if w.dtype == torch.float32 and x.is_cuda and x.dim() == 2 and x.is_contiguous() and w.is_contiguous() and x.shape[1] == w.shape[1] and _gemm_f32_splits(x, w):
+            return _gemm_f32_split(x, w, torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device), early=True)
         if not x.is_contiguous() and x.dim() == 2 and x.stride(1) == 1:
             out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
             gemm_f32_batched(x.unsqueeze(1), w.unsqueeze(0), out.unsqueeze(1))

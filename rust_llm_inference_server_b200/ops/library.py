@@ -29,6 +29,8 @@ SIGNATURES = {
     "rlis_layer_norm": [P, P, P, P, P, P, I, I, F, I, P],
     "rlis_swiglu": [P, P, I, I, I, I, P],
     "rlis_gemm_f32_nt": [P, P, P, I, I, I, P],
+    "rlis_gemm_f32_split": [P, LL, P, LL, P, LL, I, I, I, P, I, P],
+    "rlis_gemm_f32_split_few_rows": [],
     "rlis_gemm_f32_shape": [I, I, I, I, I],
     "rlis_gemm_f32_shapes": [],
     "rlis_gemm_f32_nt_batched": [P, P, P, I, I, I, LL, LL, LL, I, LL, LL, LL, P],
@@ -150,7 +152,7 @@ def lib():
             fn.argtypes = args
             fn.restype = c_int
         for name in ("rlis_gemm_tcgen05_error", "rlis_stream_gemm_error", "rlis_attention_prefill_tc_error",
-                     "rlis_attention_decode_error", "rlis_attention_difference_decode_error"):
+                     "rlis_attention_decode_error", "rlis_attention_difference_decode_error", "rlis_gemm_f32_split_error"):
             fn = getattr(handle, name)
             fn.argtypes = []
             fn.restype = c_int

@@ -1,0 +1,79 @@
+"""float32 products of long rows on the tensor cores: edges of tiles, segments and rings, the same bits in any step, and numbers that do not split."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def operands(M, N, K, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(M * 31 + N + K + seed)
+    return torch.randn(M, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+
+
+def product(a, w):
+    from rust_llm_inference_server_b200 import ops
+    n0 = ops.launches_by_kernel.get("gemm_f32.split", 0)
+    out = ops.gemm_f32(a, w)
+    assert ops.launches_by_kernel["gemm_f32.split"] == n0 + 1
+    return out
+
+
+# rows at the ends of the kernels of few rows (16, 32) and of many, whose tiles have 16 to 192 rows in halves that are multiples of 16; features that end inside a
+# tile of 128; k that ends with, inside and one float4 into a stage of 32 and a segment of 256; k cut over 1 to 8 CTAs
+@pytest.mark.parametrize("M,N,K", [(1, 128, 2048), (3, 40, 2052), (8, 2048, 2048), (8, 20000, 2304), (16, 300, 8192), (17, 129, 2300), (31, 3000, 4096), (32, 16400, 2052),
+                                   (33, 128, 2048), (50, 2048, 2084), (97, 300, 2560), (180, 2900, 2048), (193, 9500, 2052), (700, 2048, 2336), (800, 19000, 2048)])
+def test_products_of_long_rows(M, N, K):
+    from rust_llm_inference_server_b200 import ops
+    a, w = operands(M, N, K)
+    out = product(a, w)
+    want, size = a.double() @ w.double().t(), a.abs().double() @ w.abs().double().t()
+    # an accumulator truncates (a unit of 2^-23) 16 times a segment, the small products' 80 times at 2^-8 of it, the segments are added with
+    # half a unit each, and three products below 2^-26 are left out
+    assert bool(((out.double() - want).abs() <= (18 + K / 512) * 2.0 ** -23 * size).all())
+    assert float((out.double() - want).norm() / want.norm()) <= 4e-7            # (a chain of 2,048 FMAs is 8e-7 off)
+    for m in sorted({1, 8, 16, 17, 32, 33, 100, 200} & set(range(M))):          # whatever else is in the batch
+        assert torch.equal(product(a[:m].contiguous(), w), out[:m])
+    assert torch.equal(product(a[M // 2:].contiguous(), w), out[M // 2:])
+    wide = torch.zeros(M, K + 12, device="cuda")
+    wide[:, 8:8 + K] = a
+    assert torch.equal(ops.linear(wide[:, 8:8 + K], w), out)                    # rows inside wider ones
+    ops.check_device_errors()
+
+
+@pytest.mark.parametrize("M", [4, 40])
+def test_numbers_that_do_not_split_come_out_as_a_chain_gives_them(M):
+    a, w = operands(M, 200, 2048)
+    a[0, 5], a[1, 9], w[9, 100] = float("inf"), float("nan"), float("-inf")
+    a[2, 0], a[2, 1:] = 3.4e38, 0.0                   # rounds to infinity in 8 bits; alone in its row
+    a[3] *= 1e30
+    w[30] *= 1e30
+    got, chain = product(a, w), torch.zeros(M, 200, dtype=torch.float64, device="cuda")
+    for k in range(a.shape[1]):         # the range of float32, step by step
+        chain = (chain + a[:, k:k + 1].double() * w[:, k].double()).float().double()
+    assert torch.equal(got.isnan(), chain.isnan()) and torch.equal(got.isinf(), chain.isinf()) and torch.equal(got[got.isinf()], chain[chain.isinf()].float())
+    fine = chain.isfinite()
+    size = a.abs().double() @ w.abs().double().t()
+    assert bool(((got.double() - chain).abs()[fine] <= 2048 * 2.0 ** -23 * size[fine]).all()) and bool(fine.any())
+
+
+def test_rows_beyond_the_scratch_go_in_portions(monkeypatch):
+    from rust_llm_inference_server_b200 import ops
+    a, w = operands(300, 200, 2048)
+    out = product(a, w)
+    monkeypatch.setattr(ops, "_SPLIT_PLANES", 100 * 6 * 2048)
+    assert torch.equal(product(a, w), out)
+    monkeypatch.setattr(ops, "_SPLIT_PLANES", 0)          # (33 rows at a time, the last portion of a few)
+    assert torch.equal(product(a, w), out)
+
+
+def test_the_rule_asks_for_the_matrix_and_the_alignment():
+    from rust_llm_inference_server_b200 import ops
+    a, w = operands(4, 64, 2052)
+    assert ops._gemm_f32_splits(a, w) and ops._gemm_f32_splits(a[:1], w)
+    assert not ops._gemm_f32_splits(a[:, :2044].contiguous(), w[:, :2044].contiguous())
+    assert not ops._gemm_f32_splits(a[:, 1:2050], w[:, 1:2050])
+    odd = torch.zeros(4 * 2052 + 1, device="cuda")[1:].view(4, 2052)
+    assert not ops._gemm_f32_splits(odd, w)
+    odd.copy_(a)
+    assert torch.allclose(ops.gemm_f32(odd, w), ops.gemm_f32(a, w), rtol=0, atol=1e-3)
