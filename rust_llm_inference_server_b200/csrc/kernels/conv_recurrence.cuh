@@ -43,8 +43,10 @@
 //          (token, tokens back).  With a decay a channel the factors e^{L_t - L_i} sit inside the dot products, so gram
 //          forms them there, and also leaves e^{L_t} q_t, e^{L_t} k_t and e^{L_15 - L_t} k_t for the walk.  Every
 //          exponent is a sum of ln g over tokens in between, so <= 0.
+// HEAD_DECAY with heads of 128 x 128 and long portions: 64 tokens at a time, see delta_chunks.cuh.
 #pragma once
 #include "common.cuh"
+#include "mma_utils.cuh"
 #include <math.h>
 
 namespace convrec {
@@ -925,10 +927,15 @@ __global__ __launch_bounds__(CTHREADS) void chunk_kernel(
         if (live[x]) store_column<E>(s[x], S[x], slice * E, d, quads);
     pdl_trigger();
 }
+}  // namespace convrec
 
+#include "delta_chunks.cuh"
+
+namespace convrec {
 // What a launch gets.  x, b, a: the convolved columns, the logits a head and the decay logits of the first token, in the
 // element type.  act float32 [T, act_width]; gram null: token by token, else float32 [T, gram_width] and 16 tokens at a
-// time; scaled float32 [T, nh, 4 d] (CHANNEL_DECAY in chunks); out float32 [T, nh dv].
+// time; scaled float32 [T, nh, 4 d] (CHANNEL_DECAY in chunks); out float32 [T, nh dv].  wide (HEAD_DECAY, instead of gram): scratch of `wide_chunks`
+// chunks, at least the sum over the requests of their tokens / 64, rounded up, for the kernels that take 64 tokens at a time.
 struct Args {
     const void *x, *b, *a;
     long long stride, a_stride;
@@ -940,7 +947,35 @@ struct Args {
     int n_tokens, n_seqs;
     Shape z;
     float unit_eps, q_scale;
+    float* wide;
+    int wide_chunks;
 };
+
+// What the kernels of delta_chunks.cuh take: heads of 128 x 128 (or more columns in blocks of 64), everything on 16-byte boundaries.
+static inline bool wide_takes(const Shape& z) {
+    return z.d == wide::D && z.dv > 0 && z.dv % wide::VT == 0 && z.q_at % 4 == 0 && z.k_at % 4 == 0 && z.v_at % 4 == 0 && act_width<HEAD_DECAY>(z) % 4 == 0;
+}
+static inline size_t wide_floats(int nh, int dv) { return nh * wide::Unit::size(dv); }
+
+template <typename T> static int launch_wide(const Args& g, long long tail_off, cudaStream_t stream) {
+    using namespace wide;
+    const Shape& z = g.z;
+    if (!wide_takes(z) || g.state_stride % 4 ||
+        ((reinterpret_cast<uintptr_t>(g.act) | reinterpret_cast<uintptr_t>(g.state) | reinterpret_cast<uintptr_t>(g.wide) | reinterpret_cast<uintptr_t>(g.out)) & 15))
+        return RLIS_ERR_UNSUPPORTED;
+    constexpr int prepare_smem = (2 * D * LDT + 2 * CHUNK * LDT + 3 * 16 * 17) * 4, walk_smem = (D * LDT + CHUNK * LDR + (D + CHUNK) * (WC + 4)) * 4,
+                  output_smem = (2 * D * LDT + 2 * CHUNK * LDT) * 4;
+    static_assert(CHUNK * LDR <= D * LDT, "rows take the place of turned ones");
+    cudaError_t e = cudaFuncSetAttribute(delta_chunk_prepare<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, prepare_smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_walk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, walk_smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_outputs<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, output_smem);
+    if (e != cudaSuccess) return (int)e;
+    rlis_launch(delta_chunk_prepare<0>, dim3(g.wide_chunks, z.nh), PREPARE_THREADS, prepare_smem, stream, (const float*)g.act, g.wide, g.sq, g.n_seqs, z);
+    rlis_launch(delta_chunk_walk<T>, dim3(g.n_seqs, z.nh, z.dv / WC), WALK_THREADS, walk_smem, stream, (const float*)g.act, g.wide, g.state, g.state_stride, tail_off,
+                (const T*)g.x, g.stride, g.sq, z);
+    rlis_launch(delta_chunk_outputs<0>, dim3(g.wide_chunks, z.nh, z.dv / VT), OUTPUT_THREADS, output_smem, stream, (const float*)g.act, g.wide, g.out, g.sq, g.n_seqs, z);
+    return RLIS_LAUNCH_CHECK();
+}
 
 // Floats of a request's state slot: S of every head, then the convolution's tail, rounded up to whole 16-byte vectors.
 static inline int state_floats(int nh, int n_qk, int d, int dv, int taps) {
@@ -974,6 +1009,8 @@ static int launch_typed(const Args& g, cudaStream_t stream) {
     if (quads) { if (toks == 4) RLIS_PREPARE(4, true); else RLIS_PREPARE(1, true); }
     else { if (toks == 4) RLIS_PREPARE(4, false); else RLIS_PREPARE(1, false); }
 #undef RLIS_PREPARE
+    if constexpr (MODE == HEAD_DECAY)
+        if (g.wide != nullptr) return launch_wide<T>(g, tail_off, stream);
     dim3 grid(g.n_seqs, z.nh, (z.dv + COLS - 1) / COLS);
     // few CTAs that run long: shared memory asked for beyond the need keeps them one an SM
     const bool spread = (long long)grid.x * grid.y * grid.z <= sms;

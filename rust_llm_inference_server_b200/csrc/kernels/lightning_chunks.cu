@@ -18,23 +18,14 @@
 //
 // Everything is float32 (FFMA, two at a time), as in the walk; powers of g are made in float64 and rounded once, where the walk
 // rounds at every token.  Bound by the FMA pipes and by reads of shared memory: a thread has 8 x 4 or 8 x 8 outputs, so
-// three or four 16-byte reads feed 32 or 64 FMAs.  205 us (45, 25 and 135) at the sizes above, silu included (inputs are activated on their way
-// into shared memory).
-#include "common.cuh"
-#include <math.h>
+// three or four 16-byte reads feed 32 or 64 FMAs.  200 us (43, 25 and 132; 47, 25 and 151 with pairs of columns in the FMAs) at the sizes above, silu
+// included (inputs are activated on their way into shared memory).
+#include "chunk_products.cuh"
 
 namespace {
-constexpr int CHUNK = 64, VT = 64, THREADS = 128, LDT = CHUNK + 4;
-typedef unsigned long long u64;
+using namespace chunkprod;
+constexpr int VT = 64, THREADS = 128;
 
-__device__ __forceinline__ u64 pack2(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void fma2(u64& acc, u64 a, u64 b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
 
 struct Rows {
@@ -121,55 +112,6 @@ __device__ __forceinline__ void stage_turned(float* dst, const T* x, long long s
     }
 }
 
-// acc[i][j] += sum_k A[k][row i] B[k][column j]: 8 rows (ty * 4 + {0..3}, 32 on) and NC columns (tx * 4 + {0..3}, 64 on) a thread.
-// BLOCK > 0: a sum of its own every BLOCK terms, added to acc (with one chain of 128 the outputs were 2.0e-7 off 64 bits, the
-// walk's, in shares of 8, are 0.8e-7).
-template <int NC, int BLOCK>
-__device__ __forceinline__ void product(u64 (&acc)[8][NC / 2], const float* A, int lda, const float* B, int ldb, int K, int ty, int tx) {
-    u64 part[8][NC / 2];
-    auto step = [&](int k, u64 (&into)[8][NC / 2]) {
-        float a[8];
-        u64 b[NC / 2];
-#pragma unroll
-        for (int i = 0; i < 8; i += 4) *reinterpret_cast<float4*>(&a[i]) = *reinterpret_cast<const float4*>(A + k * lda + i * 8 + ty * 4);
-#pragma unroll
-        for (int j = 0; j < NC; j += 4) *reinterpret_cast<ulonglong2*>(&b[j / 2]) = *reinterpret_cast<const ulonglong2*>(B + k * ldb + j * 16 + tx * 4);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const u64 aa = pack2(a[i], a[i]);
-#pragma unroll
-            for (int j = 0; j < NC / 2; ++j) fma2(into[i][j], aa, b[j]);
-        }
-    };
-    if (BLOCK == 0) {
-#pragma unroll 8
-        for (int k = 0; k < K; ++k) step(k, acc);
-        return;
-    }
-    for (int k0 = 0; k0 < K; k0 += BLOCK) {         // (K is a multiple of BLOCK)
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < NC / 2; ++j) part[i][j] = 0ull;
-#pragma unroll
-        for (int k = 0; k < BLOCK; ++k) step(k0 + k, part);
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < NC / 2; ++j) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][j]) : "l"(part[i][j]));
-    }
-}
-template <int N> __device__ __forceinline__ void clear(u64 (&acc)[8][N]) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < N; ++j) acc[i][j] = 0ull;
-}
-
-// 8 x 16 threads, a warp 4 x 8 of them.
-__device__ __forceinline__ int thread_row() { return (threadIdx.x >> 6) * 4 + ((threadIdx.x & 31) >> 3); }
-__device__ __forceinline__ int thread_col() { return ((threadIdx.x >> 5) & 1) * 8 + (threadIdx.x & 7); }
-
 template <typename T, bool SILU, int D>
 __global__ __launch_bounds__(THREADS) void chunk_update_kernel(const Rows in, float* __restrict__ states, const float* __restrict__ decay,
                                                                const Seqs seqs, int nh, int dv) {
@@ -188,16 +130,17 @@ __global__ __launch_bounds__(THREADS) void chunk_update_kernel(const Rows in, fl
         stage<T, SILU, VT>(vs, x + in.v_off + h * dv + v0, in.stride, n, [](int) { return 1.0f; });
         stage<T, SILU, D>(ks, x + in.k_off + h * D, in.stride, n, [&](int r) { return pw[r]; });
         __syncthreads();
-        const int ty = thread_row(), tx = thread_col();
-        u64 acc[8][D / 32];
-        clear(acc);
+        const int ty = thread_row(threadIdx.x), tx = thread_col(threadIdx.x);
+        Tile<D / 16> acc;
+        acc.clear();
         product<D / 16, 0>(acc, vs, VT + 4, ks, D + 4, n, ty, tx);
         float* out = states + (((size_t)blockIdx.x * nh + h) * dv + v0) * D;
 #pragma unroll
         for (int i = 0; i < 8; ++i)
 #pragma unroll
             for (int j = 0; j < D / 16; j += 4)
-                *reinterpret_cast<ulonglong2*>(out + (size_t)(i / 4 * 32 + ty * 4 + i % 4) * D + j * 16 + tx * 4) = *reinterpret_cast<ulonglong2*>(&acc[i][j / 2]);
+                *reinterpret_cast<float4*>(out + (size_t)(i / 4 * 32 + ty * 4 + i % 4) * D + j * 16 + tx * 4) =
+                    make_float4(acc.at(i, j), acc.at(i, j + 1), acc.at(i, j + 2), acc.at(i, j + 3));
     }
     pdl_trigger();
 }
@@ -248,39 +191,35 @@ __global__ __launch_bounds__(THREADS) void chunk_outputs_kernel(const Rows in, c
         // (the weights of later keys are zeros, and a zero times what is not finite would reach tokens that came before it)
         const bool met = stage<T, SILU, VT, true>(vs, x + in.v_off + h * dv + v0, in.stride, n, [](int) { return 1.0f; });
         const bool spoilt = __syncthreads_or(met);
-        const int ty = thread_row(), tx = thread_col();
-        u64 acc[8][2];
-        clear(acc);
+        const int ty = thread_row(threadIdx.x), tx = thread_col(threadIdx.x);
+        Tile<4> acc;
+        acc.clear();
         product<4, 8>(acc, qt, LDT, xt, LDT, D, ty, tx);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int q = i / 4 * 32 + ty * 4 + i % 4;
-            float p[4];
-            *reinterpret_cast<ulonglong2*>(p) = *reinterpret_cast<ulonglong2*>(acc[i]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int k = tx * 4 + j;
-                pt[k * LDT + q] = q >= k ? p[j] * pw[q - k] : 0.f;
+                pt[k * LDT + q] = q >= k ? acc.at(i, j) * pw[q - k] : 0.f;
             }
         }
         __syncthreads();
         stage_turned<float, false, D>(xt, states + (((size_t)blockIdx.x * nh + h) * dv + v0) * D, D, VT);
         __syncthreads();
-        clear(acc);
+        acc.clear();
         product<4, 8>(acc, qt, LDT, xt, LDT, D, ty, tx);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float f = pw[i / 4 * 32 + ty * 4 + i % 4 + 1];
-            float p[4];
-            *reinterpret_cast<ulonglong2*>(p) = *reinterpret_cast<ulonglong2*>(acc[i]);
-            acc[i][0] = pack2(p[0] * f, p[1] * f);
-            acc[i][1] = pack2(p[2] * f, p[3] * f);
+        for (int i = 0; i < 4; ++i) {
+            const int q = i / 2 * 32 + ty * 4 + i % 2 * 2;
+            acc.scale(i, pw[q + 1], pw[q + 2]);
         }
         product<4, 8>(acc, pt, LDT, vs, VT + 4, (n + 7) & ~7, ty, tx);     // (rows of zeros beyond n)
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int q = i / 4 * 32 + ty * 4 + i % 4;
-            if (q < n) *reinterpret_cast<ulonglong2*>(out + (size_t)(rows.x + q) * nh * dv + h * dv + v0 + tx * 4) = *reinterpret_cast<ulonglong2*>(acc[i]);
+            if (q < n)
+                *reinterpret_cast<float4*>(out + (size_t)(rows.x + q) * nh * dv + h * dv + v0 + tx * 4) = make_float4(acc.at(i, 0), acc.at(i, 1), acc.at(i, 2), acc.at(i, 3));
         }
         if (spoilt) {           // values that are not finite, for the tokens from theirs on
             __syncthreads();

@@ -484,23 +484,61 @@ def gated_delta(proj: torch.Tensor, qkv_off: int, b_off: int, a_off: int, conv_w
     the convolution's tail between steps; out float32 [T, nh dv].
 
     A step of long portions of few requests (GATED_DELTA_CHUNKS_FROM) goes through the kernels that take 16 tokens
-    of a request at a time; other steps walk token by token (`chunks` says which, for any step)."""
+    of a request at a time, or 64 (`_gated_delta_wide_pays`); other steps walk token by token (`chunks` says whether by chunks or not, for any step)."""
     T, N = proj.shape
     C = _recurrence_operands("gated_delta", proj, qkv_off, b_off, conv_w, a_log, dt_bias, state, out, n_heads, n_qk_heads,
                              d, dv, taps, n_heads)
     if a_off + n_heads > N:
         raise KernelError("gated_delta: the column offsets reach beyond the projection's rows")
     act = step.buffer("recurrence_act", (T, C + 2 * n_heads), torch.float32)
-    if chunks is None:
+    by_rule = chunks is None
+    if by_rule:
         chunks = _recurrence_in_chunks(step, T, n_heads, dv, proj.device)
-    gram = step.buffer("recurrence_gram", (T, n_qk_heads * 32 + n_heads * 16), torch.float32).data_ptr() if chunks else 0
+    wide = _gated_delta_wide(step, T, n_heads, n_qk_heads, d, dv, taps, state, act, out, chunks) if by_rule or chunks else None
+    gram = step.buffer("recurrence_gram", (T, n_qk_heads * 32 + n_heads * 16), torch.float32).data_ptr() if chunks and wide is None else 0
     check(lib().rlis_gated_delta(proj.data_ptr(), proj.stride(0), int(qkv_off), int(b_off), int(a_off), conv_w.data_ptr(),
                                  a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), state.stride(0),
-                                 *_step_pointers(step), act.data_ptr(), gram, out.data_ptr(), T, step.n_seqs, n_heads,
+                                 *_step_pointers(step), act.data_ptr(), gram,
+                                 wide.data_ptr() if wide is not None else 0, wide.shape[0] if wide is not None else 0, out.data_ptr(), T, step.n_seqs, n_heads,
                                  n_qk_heads, d, dv, taps, float(unit_eps), float(q_scale), _code(proj.dtype), _stream()),
           "gated_delta")
-    _count_recurrence("gated_delta", chunks, True)
+    if wide is not None:
+        _count("gated_delta.prepare")
+        _count("gated_delta.wide")
+    else:
+        _count_recurrence("gated_delta", chunks, True)
     return out
+
+
+@functools.lru_cache(maxsize=4096)
+def _gated_delta_wide_pays(n_tokens: int, n_seqs: int, longest: int, columns: int, sms: int, sixteen: bool) -> bool:
+    """Whether the gated delta rule runs faster 64 tokens at a time than 16 at a time (`sixteen`) or token by token, for `columns` = heads x dv columns of
+    state and a longest portion of `longest` tokens.  Measured, 16 and 64 at a time in us (the inputs behind the convolutions included): one prompt of 2,048
+    with 16 heads 440 and 317, with 8 heads 402 and 219, of 1,024 228 and 166, of 512 124 and 109, of 256 73 and 89, of 64 33 and 70; 409 and 1,092
+    tokens 384 and 280; four of 512 with 8 heads 203 and 160; token by token and 64 at a time, four of 512 with 16 heads 333 and 313, of 256 170 and
+    164, of 128 90 and 109, 341, 910, 455 and 342 tokens 553 and 358, two of 2,048 with 32 heads 1,328 and 1,120."""
+    load = n_tokens * columns / 2048
+    if sixteen:
+        before = 18 + 0.206 * max(longest, 0.9 * load)
+    else:
+        before = 15 + max(0.6 * longest, 0.155 * load)
+    after = 50 + (0.095 if n_seqs * columns <= 16 * sms else 0.125) * (load + 48 * (n_seqs - 1) * columns / 2048) + 0.02 * longest
+    return longest >= 64 and after < 0.98 * before
+
+
+GATED_DELTA_WIDE_BYTES = 512 << 20      # of scratch; steps that would take more go 16 tokens at a time
+
+
+def _gated_delta_wide(step, T: int, n_heads: int, n_qk_heads: int, d: int, dv: int, taps: int, state: torch.Tensor, act: torch.Tensor,
+                      out: torch.Tensor, sixteen: bool) -> torch.Tensor | None:
+    """The scratch of the kernels that take 64 tokens of a request at a time (csrc/kernels/delta_chunks.cuh), or None where they do not apply or do not pay."""
+    longest = getattr(step, "max_q_len", 0) or -(-T // step.n_seqs)
+    if not _gated_delta_wide_pays(T, step.n_seqs, longest, n_heads * dv, num_sms(), sixteen):
+        return None
+    floats, chunks = lib().rlis_gated_delta_wide_floats(n_heads, n_qk_heads, d, dv, taps), T // 64 + step.n_seqs
+    if floats <= 0 or 4 * floats * chunks > GATED_DELTA_WIDE_BYTES or state.stride(0) % 4 or any(t.data_ptr() % 16 for t in (state, act, out)):
+        return None
+    return step.buffer("recurrence_wide", (chunks, floats), torch.float32)
 
 
 def channel_delta(proj: torch.Tensor, qkv_off: int, b_off: int, decay: torch.Tensor, conv_w: torch.Tensor,
