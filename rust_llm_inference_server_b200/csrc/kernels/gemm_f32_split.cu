@@ -23,10 +23,10 @@ namespace {
 using namespace tc;
 
 constexpr int FT = 128;                     // features a tile
-constexpr int KS = 32;                      // k of a stage
-constexpr int SEG_STAGES = 8;               // stages of a segment
-constexpr int RAW_BYTES = FT * KS * 4;      // float32 weights of a stage
-constexpr int A_COLS = 3 * KS / 2;          // columns of tensor memory that the three planes of a stage's weights take
+constexpr int SEG = 256;                    // k of a segment
+// k of a stage, and for it: stages of a segment, bytes of float32 weights, columns of tensor memory that their three planes take
+constexpr int KS = 32, SEG_STAGES = SEG / KS, RAW_BYTES = FT * KS * 4, A_COLS = 3 * KS / 2;             // few rows
+constexpr int KM = 64, SEG_STAGES_M = SEG / KM, RAW_BYTES_M = FT * KM * 4, A_COLS_M = 3 * KM / 2;       // many
 constexpr int MAX_RINGS = 12, MAX_A = 6;    // stages of a ring in shared memory, and of the planes of weights in tensor memory
 
 struct Ctrl {
@@ -79,23 +79,25 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
-// Shared-memory matrix descriptor of a K-major tile whose rows are 64 bytes wide, 64-byte swizzle (layout type 4, 512 bytes between groups of 8 rows).
-__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
-    return ((uint64_t)(addr >> 4) & 0x3FFFull) | (1ull << 16) | ((uint64_t)(512 >> 4) << 32) | (1ull << 46) | (4ull << 61);
+// Shared-memory matrix descriptor of a K-major tile whose rows are 32 k (64 bytes, 64-byte swizzle: layout type 4, 512 bytes between groups of 8 rows)
+// or 64 k (128 bytes, 128-byte swizzle) wide.
+template <int KT> __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
+    static_assert(KT == 32 || KT == 64, "stage");
+    return ((uint64_t)(addr >> 4) & 0x3FFFull) | (1ull << 16) | ((uint64_t)(KT * 16 >> 4) << 32) | (1ull << 46) | ((KT == 32 ? 4ull : 2ull) << 61);
 }
 
 // A value that is the same in all lanes, in a way that the compiler sees: what descriptors are made from stays in uniform registers, which
 // is where tcgen05.mma takes them.
 template <typename T> __device__ __forceinline__ T uniform(T v) { return __shfl_sync(0xffffffffu, v, 0); }
 
-// A stage's products over `n` rows of A: planes of the weights from tensor memory column `a`, of the rows from shared memory at `b`, planes
+// A stage's products (KT of k) over `n` rows of A: planes of the weights from tensor memory column `a`, of the rows from shared memory at `b`, planes
 // `plane` bytes apart; sums of w1 x1 in columns `main`, of the others in `small`.
-__device__ __forceinline__ void stage_products(uint32_t main, uint32_t small, uint32_t a, uint32_t b, uint32_t plane, int n, bool first) {
+template <int KT> __device__ __forceinline__ void stage_products(uint32_t main, uint32_t small, uint32_t a, uint32_t b, uint32_t plane, int n, bool first) {
     const uint32_t idesc = idesc_bf16(FT, n);
-    const uint64_t b1 = smem_desc_sw64(b), b2 = smem_desc_sw64(b + plane), b3 = smem_desc_sw64(b + 2 * plane);
-    const uint32_t a1 = a, a2 = a + KS / 2, a3 = a + KS;
+    const uint64_t b1 = smem_desc<KT>(b), b2 = smem_desc<KT>(b + plane), b3 = smem_desc<KT>(b + 2 * plane);
+    const uint32_t a1 = a, a2 = a + KT / 2, a3 = a + KT;
 #pragma unroll
-    for (int k = 0; k < KS / 16; ++k) {         // 8 columns, or 32 bytes of a swizzled row, further along k
+    for (int k = 0; k < KT / 16; ++k) {         // 8 columns, or 32 bytes of a swizzled row, further along k
         const uint32_t on = first && k == 0 ? 0u : 1u;
         umma_bf16_ts(small, a3 + k * 8, b1 + k * 2, idesc, on);
         umma_bf16_ts(small, a2 + k * 8, b2 + k * 2, idesc, 1u);
@@ -106,21 +108,21 @@ __device__ __forceinline__ void stage_products(uint32_t main, uint32_t small, ui
     }
 }
 
-// One row of 32 float32 weights (128 bytes, 128-byte swizzle) into its three planes in tensor memory.
-__device__ __forceinline__ void split_weights(const unsigned char* raw, int row, uint32_t taddr) {
-    const unsigned char* src = raw + row * (KS * 4);
+// One row of KT float32 weights (boxes of 32: 128 bytes, 128-byte swizzle) into its three planes in tensor memory.
+template <int KT> __device__ __forceinline__ void split_weights(const unsigned char* raw, int row, uint32_t taddr) {
 #pragma unroll
-    for (int kk = 0; kk < 2; ++kk) {
+    for (int kk = 0; kk < KT / 16; ++kk) {
+        const unsigned char* src = raw + kk / 2 * (FT * 32 * 4) + row * (32 * 4);
         uint32_t p1[8], p2[8], p3[8];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const float4 v = *reinterpret_cast<const float4*>(src + (((kk * 4 + c) ^ (row & 7)) << 4));
+            const float4 v = *reinterpret_cast<const float4*>(src + (((kk % 2 * 4 + c) ^ (row & 7)) << 4));
             split2(v.x, v.y, p1[2 * c], p2[2 * c], p3[2 * c]);
             split2(v.z, v.w, p1[2 * c + 1], p2[2 * c + 1], p3[2 * c + 1]);
         }
         tmem_st8(taddr + kk * 8, p1);
-        tmem_st8(taddr + KS / 2 + kk * 8, p2);
-        tmem_st8(taddr + KS + kk * 8, p3);
+        tmem_st8(taddr + KT / 2 + kk * 8, p2);
+        tmem_st8(taddr + KT + kk * 8, p3);
     }
     tmem_st_wait();
 }
@@ -163,16 +165,16 @@ __global__ __launch_bounds__(256) void split_rows_kernel(const float* __restrict
 }
 
 // ------------------------------------------------------------------------------------------------
-// Many rows.  700 rows, us here and in FFMA tiles: K 2048 N 16384 228 / 1139, N 3072 50 / 218, N 2048 44 / 218; K 8192 N 2048 142 / 858; 2,048 rows of K 2048 N 16384
-// 649 / 2648 (212 TFLOP/s, six times that on the tensor cores: 1.27 PFLOP/s).  Bound by the pipe for whole tiles of 176 and 192 rows (1,700 cycles a
-// stage for 1,056 of products; bytes through shared memory are close behind), by about 800 cycles of a stage's waits for small ones.
-// A tile of 128 features x bn rows of A a CTA (bn up to 192), in two halves of the rows with accumulators, an issuing warp and four adding
+// Many rows.  700 rows, us here and in FFMA tiles: K 2048 N 16384 238 / 1139, N 3072 50 / 218, N 2048 39 / 218; K 8192 N 2048 127 / 858; 2,048 rows of K 2048 N 16384
+// 625 / 2648 (220 TFLOP/s, six times that on the tensor cores: 1.3 PFLOP/s).  A stage takes the products' time (12 cycles a row) and about 1,100 cycles
+// beside it, whatever the depth of the rings, so stages of 64 k are better than stages of 32 for tiles of few rows (48 rows 27 / 33 us, 200 39 / 50).
+// A tile of 128 features x bn rows of A a CTA (bn up to 160), in two halves of the rows with accumulators, an issuing warp and four adding
 // warps of their own: one warp alone spends more cycles between the bursts of two stages than the pipe has instructions queued.
 // The rings have an even number of stages: a set meets the same ones every time, and so sees every phase of their barriers.
 // Twenty warps, by role: 0-7 add the segments up and store, 8-15 split weights (two sets, taking turns at the stages), 16 and 17 ask for weights
 // and for A's planes, 18 and 19 issue the products.
-constexpr int MANY_THREADS = 640, MAX_BN = 192, HALF = MAX_BN / 2;
-constexpr int MANY_RING_BYTES = 225 * 1024;         // both rings (tiles of 192 rows: four stages each)
+constexpr int MANY_THREADS = 640, MAX_BN = 160, HALF = MAX_BN / 2;
+constexpr int MANY_RING_BYTES = 225 * 1024;         // both rings
 constexpr int MANY_SMEM = 1024 + MANY_RING_BYTES + (int)sizeof(Ctrl);
 static_assert(MANY_SMEM <= 227 * 1024, "shared memory");
 
@@ -181,13 +183,13 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* raw = base;
-    unsigned char* planes = base + p.raw_ring * RAW_BYTES;
+    unsigned char* planes = base + p.raw_ring * RAW_BYTES_M;
     Ctrl* ctrl = reinterpret_cast<Ctrl*>(base + MANY_RING_BYTES);
     const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int f0 = (int)(blockIdx.x / p.m_tiles) * FT, m0 = (int)(blockIdx.x % p.m_tiles) * p.bn;
     const int n0 = (p.bn / 2 + 15) / 16 * 16, n1 = p.bn - n0;      // rows of the halves (the second has none where bn is 16)
-    const uint32_t plane = (uint32_t)p.bn * (KS * 2), b_bytes = 3 * plane;
-    const int a_ring = min(MAX_A, (512 - 4 * n0) / A_COLS) & ~1;
+    const uint32_t plane = (uint32_t)p.bn * (KM * 2), b_bytes = 3 * plane;
+    const int a_ring = min(MAX_A, (512 - 4 * n0) / A_COLS_M) & ~1;
 
     if (threadIdx.x == 0) {
         ctrl->abort = 0;
@@ -223,8 +225,9 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
                 if (!p.early) pdl_wait();
                 for (int it = 0, s = 0, turn = 0; it < p.stages; ++it) {
                     if (turn > 0 && !bar_wait(&ctrl->raw_empty[s], (turn - 1) & 1, &ctrl->abort)) break;
-                    bar_expect_tx(&ctrl->raw_full[s], RAW_BYTES);
-                    tma_load_2d(raw + s * RAW_BYTES, &map_w, it * KS, f0, &ctrl->raw_full[s]);
+                    bar_expect_tx(&ctrl->raw_full[s], RAW_BYTES_M);
+                    tma_load_2d(raw + s * RAW_BYTES_M, &map_w, it * KM, f0, &ctrl->raw_full[s]);
+                    tma_load_2d(raw + s * RAW_BYTES_M + RAW_BYTES_M / 2, &map_w, it * KM + 32, f0, &ctrl->raw_full[s]);
                     if (++s == p.raw_ring) { s = 0; ++turn; }
                 }
             }
@@ -234,22 +237,22 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
                 for (int it = 0, s = 0, turn = 0; it < p.stages; ++it) {
                     if (turn > 0 && !bar_wait(&ctrl->b_empty[s], (turn - 1) & 1, &ctrl->abort)) break;
                     bar_expect_tx(&ctrl->b_full[s], b_bytes);
-                    tma_load_3d(planes + (size_t)s * b_bytes, &map_a, it * KS, m0, 0, &ctrl->b_full[s]);
+                    tma_load_3d(planes + (size_t)s * b_bytes, &map_a, it * KM, m0, 0, &ctrl->b_full[s]);
                     if (++s == p.rings) { s = 0; ++turn; }
                 }
             }
         } else if (warp == 18 || n1 > 0) {
             const int h = warp - 18, n = h ? n1 : n0;
-            const uint32_t main = tmem + (uint32_t)(h * 2 * n0), rows = smem_u32(planes) + (uint32_t)(h * n0) * (KS * 2);
+            const uint32_t main = tmem + (uint32_t)(h * 2 * n0), rows = smem_u32(planes) + (uint32_t)(h * n0) * (KM * 2);
             int s = 0, a = 0;
             uint32_t a_turn = 0;
             for (int it = 0; it < p.stages; ++it) {
-                const bool first = it % SEG_STAGES == 0, last = it % SEG_STAGES == SEG_STAGES - 1 || it == p.stages - 1;
-                if (first && it > 0 && !bar_wait_warp(&ctrl->acc_empty[h], (it / SEG_STAGES - 1) & 1, &ctrl->abort)) break;
+                const bool first = it % SEG_STAGES_M == 0, last = it % SEG_STAGES_M == SEG_STAGES_M - 1 || it == p.stages - 1;
+                if (first && it > 0 && !bar_wait_warp(&ctrl->acc_empty[h], (it / SEG_STAGES_M - 1) & 1, &ctrl->abort)) break;
                 if (!bar_wait_warp(&ctrl->a_full[a], a_turn, &ctrl->abort)) break;           // the rows' planes are there, too
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (elect_one()) {
-                    stage_products(main, main + n0, a_base + (uint32_t)(a * A_COLS), rows + (uint32_t)s * b_bytes, plane, n, first);
+                    stage_products<KM>(main, main + n0, a_base + (uint32_t)(a * A_COLS_M), rows + (uint32_t)s * b_bytes, plane, n, first);
                     umma_commit(&ctrl->a_empty[a]);
                     umma_commit(&ctrl->b_empty[s]);
                     if (last) umma_commit(&ctrl->acc_full[h]);
@@ -269,7 +272,7 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
             if (!bar_wait_warp(&ctrl->raw_full[s], turn & 1, &ctrl->abort)) break;
             if (a_turn > 0 && !bar_wait_warp(&ctrl->a_empty[a], (a_turn - 1) & 1, &ctrl->abort)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            split_weights(raw + s * RAW_BYTES, row, taddr + (uint32_t)(a * A_COLS));
+            split_weights<KM>(raw + s * RAW_BYTES_M, row, taddr + (uint32_t)(a * A_COLS_M));
             if (!bar_wait_warp(&ctrl->b_full[b], b_turn & 1, &ctrl->abort)) break;
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -286,7 +289,7 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
-        const int h = warp >> 2, q = warp & 3, cols = h ? n1 : n0, segs = cols == 0 ? 0 : (p.stages + SEG_STAGES - 1) / SEG_STAGES;
+        const int h = warp >> 2, q = warp & 3, cols = h ? n1 : n0, segs = cols == 0 ? 0 : (p.stages + SEG_STAGES_M - 1) / SEG_STAGES_M;
         const uint32_t main = tmem + (uint32_t)(h * 2 * n0) + ((uint32_t)(q * 32) << 16);
         float sum[HALF];
 #pragma unroll
@@ -412,7 +415,7 @@ __global__ __launch_bounds__(FEW_THREADS, 2) void f32_split_few_kernel(const __g
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (elect_one()) {
                 const uint32_t main = tmem + (uint32_t)(buf * 2 * BN);
-                stage_products(main, main + BN, a_base + (uint32_t)(a * A_COLS), smem_u32(planes) + (uint32_t)(a * F::PLANES), BN * KS * 2, BN, first);
+                stage_products<KS>(main, main + BN, a_base + (uint32_t)(a * A_COLS), smem_u32(planes) + (uint32_t)(a * F::PLANES), BN * KS * 2, BN, first);
                 umma_commit(&ctrl->a_empty[a]);
                 if (last) umma_commit(&ctrl->acc_full[buf]);
             }
@@ -427,7 +430,7 @@ __global__ __launch_bounds__(FEW_THREADS, 2) void f32_split_few_kernel(const __g
             if (!bar_wait_warp(&ctrl->raw_full[s], turn & 1, &ctrl->abort)) break;
             if (it >= FEW_A && !bar_wait_warp(&ctrl->a_empty[a], (it / FEW_A - 1) & 1, &ctrl->abort)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            split_weights(ring + s * F::STAGE, row, taddr + (uint32_t)(a * A_COLS));
+            split_weights<KS>(ring + s * F::STAGE, row, taddr + (uint32_t)(a * A_COLS));
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) {
@@ -540,14 +543,14 @@ bool map_f32(CUtensorMap* map, const float* ptr, int rows, int K, long long ld, 
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// The three planes of `rows` rows, pitch apart, with boxes of 32 k x box_rows rows x 3 planes, 64-byte swizzle.
+// The three planes of `rows` rows, pitch apart, with boxes of 64 k x box_rows rows x 3 planes, 128-byte swizzle.
 bool map_planes(CUtensorMap* map, const bf16* ptr, int rows, int pitch, int box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (fn == nullptr) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)pitch, (cuuint64_t)rows, 3}, strides[2] = {(cuuint64_t)pitch * 2, (cuuint64_t)pitch * rows * 2};
-    const cuuint32_t box[3] = {(cuuint32_t)KS, (cuuint32_t)box_rows, 3}, estr[3] = {1, 1, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)KM, (cuuint32_t)box_rows, 3}, estr[3] = {1, 1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 int sm_count() {
@@ -586,7 +589,7 @@ template <int BN> int launch_few(SplitArgs p, cudaStream_t stream) {
     return RLIS_LAUNCH_CHECK();
 }
 
-// Rows of A a tile: what takes the SMs least time.  Measured on 700 rows, in cycles a stage: 16 rows 850, 64 990, 96 1180, 128 1330, 176 1700, 192 1860;
+// Rows of A a tile: what takes the SMs least time.  Measured on 700 rows, in cycles a stage: 16 rows 1,300, 64 1,680, 96 2,160, 128 2,640, 160 3,050;
 // a tile takes about 6,000 cycles beside its stages.
 int choose_bn(int M, int N, int stages, int sms) {
     if (g_bn > 0) return g_bn;
@@ -595,7 +598,7 @@ int choose_bn(int M, int N, int stages, int sms) {
     double least = -1;
     for (int bn = 16; bn <= MAX_BN; bn += 16) {
         const long long waves = (f_tiles * ((M + bn - 1) / bn) + sms - 1) / sms;
-        const double t = (double)waves * (stages * (750 + 5.5 * bn) + 6000);
+        const double t = (double)waves * (stages * (1070 + 12.2 * bn) + 6000);
         if (least < 0 || t < least) { least = t; best = bn; }
     }
     return best;
@@ -623,12 +626,12 @@ extern "C" int rlis_gemm_f32_split(const float* A, long long lda, const float* W
                 reinterpret_cast<bf16*>(planes), M, K, pitch);
     int rc = RLIS_LAUNCH_CHECK();
     if (rc != 0) return rc;
-    p.bn = choose_bn(M, N, p.stages, sms);
+    p.bn = choose_bn(M, N, (K + KM - 1) / KM, sms);
     p.m_tiles = (M + p.bn - 1) / p.bn;
-    const int b_bytes = 3 * p.bn * KS * 2;
-    p.rings = p.bn > 64 ? 4 : 6;
-    p.raw_ring = (MANY_RING_BYTES - p.rings * b_bytes) / RAW_BYTES & ~1;
-    if (p.raw_ring > 8) p.raw_ring = 8;
+    const int b_bytes = 3 * p.bn * KM * 2;
+    p.stages = (K + KM - 1) / KM;
+    p.rings = p.bn > 64 ? 2 : 4;
+    p.raw_ring = p.rings * b_bytes + 4 * RAW_BYTES_M <= MANY_RING_BYTES ? 4 : 2;
     CUtensorMap map_w, map_a;
     if (!map_f32(&map_w, W, N, K, ldw, FT) || !map_planes(&map_a, reinterpret_cast<const bf16*>(planes), M, pitch, p.bn)) return RLIS_ERR_UNSUPPORTED;
     const cudaError_t e = cudaFuncSetAttribute(f32_split_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MANY_SMEM);

@@ -19,8 +19,8 @@ def product(a, w):
     return out
 
 
-# rows at the ends of the kernels of few rows (16, 32) and of many, whose tiles have 16 to 192 rows in halves that are multiples of 16; features that end inside a
-# tile of 128; k that ends with, inside and one float4 into a stage of 32 and a segment of 256; k cut over 1 to 8 CTAs
+# rows at the ends of the kernels of few rows (16, 32) and of many, whose tiles have 16 to 160 rows in halves that are multiples of 16; features that end inside a
+# tile of 128; k that ends with, inside and one float4 into a stage of 32 or 64 and a segment of 256; k cut over 1 to 8 CTAs
 @pytest.mark.parametrize("M,N,K", [(1, 128, 2048), (3, 40, 2052), (8, 2048, 2048), (8, 20000, 2304), (16, 300, 8192), (17, 129, 2300), (31, 3000, 4096), (32, 16400, 2052),
                                    (33, 128, 2048), (50, 2048, 2084), (97, 300, 2560), (180, 2900, 2048), (193, 9500, 2052), (700, 2048, 2336), (800, 19000, 2048)])
 def test_products_of_long_rows(M, N, K):
