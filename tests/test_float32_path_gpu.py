@@ -190,3 +190,15 @@ def test_float32_decode_asks_for_the_pieces_that_exist(lens, nh, nkv, d, window)
     want = ops.attention_generic(q, kc, vc, torch.empty_like(q), st.seq_of_token, st.positions, st.block_tables[0], *args[1:])
     # sums of weights that add up to one and values around one
     assert (out - want).abs().max() <= 2e-5
+
+
+@pytest.mark.parametrize("interleave", [0, 4, 8])
+def test_gates_four_at_a_time_are_the_gates_one_by_one(interleave):
+    from rust_llm_inference_server_b200 import ops
+    g = torch.Generator().manual_seed(interleave)
+    T, I = 37, 200
+    flat = torch.zeros(T * 2 * I + 1, device="cuda")
+    gu, odd = (torch.randn(T, 2 * I, generator=g) * 3).cuda(), flat[1:].view(T, 2 * I)          # rows on a boundary of 16 bytes, and not
+    odd.copy_(gu)
+    outs = [ops.swiglu(x, torch.empty(T, I, device="cuda"), interleave) for x in (gu, odd)]
+    assert torch.equal(*outs) and bool(outs[0].isfinite().all())
