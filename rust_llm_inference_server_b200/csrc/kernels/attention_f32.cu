@@ -17,7 +17,9 @@
 //     times the requests (64 requests of 200 keys beside one of 131,072, 32 heads of 128: 545 MB by the longest, 17 by the pieces).  Beyond
 //     SPLIT_ROWS requests, which are many waves of CTAs by themselves, a CTA takes a whole context.
 //   prompts: 8 warps of R = 4 rows, a row a (token, query head); lanes are keys for the scores and dimensions for
-//     the value sum, so a key's 16 bytes in shared memory serve four rows.
+//     the value sum, so a key's 16 bytes in shared memory serve four rows.  The weights of a block go through shared memory, four rows' in a
+//     read: 700 tokens, 32 heads of 64 157 us, with a shuffle a key and row 175 (eight rows a warp 225: half as many CTAs, whose longest rows are
+//     the kernel's end).
 #include "common.cuh"
 #include "mma_utils.cuh"
 #include <math.h>
@@ -91,6 +93,7 @@ template <int DL> __device__ __forceinline__ void fold(float& M, float& L, float
 
 template <int DL, int R, bool SPLIT>
 __global__ __launch_bounds__((SPLIT ? MAX_GROUP : PROMPT_WARPS) * 32) void attn_f32_kernel(const Args p) {
+    static_assert(R == 1 || R % 4 == 0, "weights go by fours");
     extern __shared__ __align__(16) float smem[];
     pdl_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -99,6 +102,7 @@ __global__ __launch_bounds__((SPLIT ? MAX_GROUP : PROMPT_WARPS) * 32) void attn_
     float* ring = smem + warps * R * d;
     const int stage_floats = 2 * BLOCK * ld;
     int* mapped = reinterpret_cast<int*>(ring + STAGES * stage_floats);     // [stage][key]: whether its page is there
+    float* ws = reinterpret_cast<float*>(mapped + STAGES * BLOCK) + warp * BLOCK * R;       // [key][row] weights of a block (R > 1)
     const int2 piece = SPLIT ? piece_at(p, blockIdx.x) : make_int2(0, 0);
     if (SPLIT && piece.x < 0) return;
     // long tiles first: the last tokens of a prompt see the most keys
@@ -223,18 +227,29 @@ __global__ __launch_bounds__((SPLIT ? MAX_GROUP : PROMPT_WARPS) * 32) void attn_
                     m[r] = m_new;
                 }
                 // p . v in the order of the keys; a key without weight takes part with nothing, whatever its row holds
+                if (R > 1) {
+#pragma unroll
+                    for (int r = 0; r < R; r += 4) *reinterpret_cast<float4*>(ws + lane * R + r) = make_float4(w[r], w[(r + 1) % R], w[(r + 2) % R], w[(r + 3) % R]);
+                    __syncwarp();
+                }
 #pragma unroll 8
                 for (int kk = 0; kk < BLOCK; ++kk) {
-                    float v[DL];
+                    float v[DL], pk[R];
 #pragma unroll
                     for (int i = 0; i < DL; ++i) v[i] = lane + 32 * i < d ? vs[kk * ld + lane + 32 * i] : 0.f;
+                    if (R > 1) {
+#pragma unroll
+                        for (int r = 0; r < R; r += 4) *reinterpret_cast<float4*>(pk + r) = *reinterpret_cast<const float4*>(ws + kk * R + r);
+                    } else {
+                        pk[0] = __shfl_sync(0xffffffffu, w[0], kk);
+                    }
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
-                        const float pk = __shfl_sync(0xffffffffu, w[r], kk);
 #pragma unroll
-                        for (int i = 0; i < DL; ++i) acc[r][i] = pk != 0.f ? fmaf(pk, v[i], acc[r][i]) : acc[r][i];
+                        for (int i = 0; i < DL; ++i) acc[r][i] = pk[r] != 0.f ? fmaf(pk[r], v[i], acc[r][i]) : acc[r][i];
                     }
                 }
+                if (R > 1) __syncwarp();            // (the weights have been read before the next block's)
             }
             if (!SPLIT && ((kb + BLOCK) % PIECE == 0 || b == blocks - 1)) {
 #pragma unroll
@@ -318,7 +333,7 @@ template <int DL> __global__ __launch_bounds__(128) void attn_f32_fold_kernel(co
 
 template <int DL> int run(Args p, bool folds, bool single, cudaStream_t stream) {
     const int group = p.nh / p.nkv;
-    auto smem = [&](int rows) { return (rows * p.d + STAGES * 2 * BLOCK * (p.d + 4)) * (int)sizeof(float) + STAGES * BLOCK * (int)sizeof(int); };
+    auto smem = [&](int rows) { return (rows * p.d + STAGES * 2 * BLOCK * (p.d + 4) + rows * BLOCK) * (int)sizeof(float) + STAGES * BLOCK * (int)sizeof(int); };
     if (p.slots > 0) {
         auto kernel = attn_f32_kernel<DL, 1, true>;
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(MAX_GROUP));
