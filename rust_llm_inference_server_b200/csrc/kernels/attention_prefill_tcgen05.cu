@@ -99,6 +99,13 @@
 // are (2^92 fits bfloat16 and the float32 sums with room for the keys), so O is never rescaled.  At the end the warps of map 2
 // leave their rows in shared memory and those of map 1 subtract, norm, gate and store.
 //
+// A bias by distance, a gate a head, a sink (BIAS; the formulas are in attention_bias.cu): the same kernel with two rings of two tiles, which leaves room
+// for both heads' biases by distance in shared memory (times log2(e); repeated past their ends so that no index needs a bound).  A block that lies wholly
+// beyond the table's reach adds the last row's constant to the exponent's offset, for nothing; one within it reads a number a score (neighbouring rows
+// read neighbouring numbers).  A sink is what the row's reference and sum start from.  2,048 tokens, 32 heads of 64, a table of 129: 55 us, with
+// mma.sync (attention_bias_mma.cu, which keeps slopes, gates a channel, other sizes and longer tables) 102; a window of 1,024 and sinks, 409 and 1,092
+// tokens 40 and 63.
+//
 // Every mbarrier wait is bounded (a fifth of a second); a wait that runs out sets the error word
 // (rlis_attention_prefill_tc_error), every role runs to its end without further waits, and the
 // CTA frees its tensor memory before it returns.
@@ -116,21 +123,27 @@ constexpr int PT_SOFTMAX_WARP0 = 4;
 constexpr int LINE_TILE = TM * 128;     // bytes of a swizzled sub-tile of 128 rows: 64 columns, 128-byte lines
 constexpr uint32_t TMEM_COLS = 256;     // S: columns 0 .. TN - 1, O: 128 .. 128 + HD - 1, P (bf16 pairs): TN / 2 columns in what is left
 
+// Entries of a head's table of biases by distance, and how many more its copy in shared memory has: 128 in front (keys after the query, hidden) and
+// 192 behind (the last one, for the block that the table ends in: up to 127 + 63 beyond).
+constexpr int BIAS_MAX_DIST = 1024, BIAS_FRONT = 128, BIAS_PAD = BIAS_FRONT + 192;
+
 // Sizes by head size HD and keys of a block TN (64, 128) or (128, 64): 16 KB of keys and of values a
 // block, three blocks in flight for head size 64 and two for 128 (112 and 96 KB a CTA, two CTAs an SM).
-template <int HD, int TN> struct PShape {
+template <int HD, int TN, bool BIAS = false> struct PShape {
     static constexpr int Q_BYTES = TM * HD * 2;             // 16 or 32 KB: HD / 64 sub-tiles [128 x 64]
     static constexpr int KV_TILE_BYTES = TN * HD * 2;       // 16 KB each for K and V: HD / 64 sub-tiles [TN x 64]
     static constexpr int KV_LINE_TILE = TN * 128;           // bytes of one such sub-tile
-    static constexpr int KV_STAGES = HD == 64 ? 3 : 2;
+    static constexpr int KV_STAGES = HD == 64 && !BIAS ? 3 : 2;
     // the tiles + the control block; with the kilobyte the system keeps per CTA, two CTAs fit the
     // 228 KB of an SM only if no alignment slack is spent: the dynamic array is declared 1024-aligned
     static constexpr size_t SMEM = Q_BYTES + KV_STAGES * 2 * KV_TILE_BYTES + 256;
+    static constexpr size_t smem_bias(int n_dist) { return SMEM + 2 * (size_t)(n_dist + BIAS_PAD) * sizeof(float); }
+    static_assert(!BIAS || 2 * (SMEM + 2 * (size_t)(BIAS_MAX_DIST + BIAS_PAD) * sizeof(float) + 1024) <= 228 * 1024, "two CTAs an SM, tables included");
     static constexpr uint32_t IDESC_S = idesc_bf16(TM, TN);
     static constexpr uint32_t IDESC_PV = idesc_bf16(TM, HD) | (1u << 16);      // B (V) is MN-major
     static constexpr uint32_t P_COL = HD == 64 ? 192u : 64u;   // where P lives in tensor memory
     static constexpr int ROW_F = HD + 4;                    // floats a row in the clusters' exchange area
-    static constexpr int MAX_SPLITS = HD == 64 ? 4 : 2;     // what that area holds: (splits - 1) * 128 rows
+    static constexpr int MAX_SPLITS = BIAS ? 1 : HD == 64 ? 4 : 2;     // what that area holds: (splits - 1) * 128 rows
     static_assert((MAX_SPLITS - 1) * TM * ROW_F * 4 <= Q_BYTES + KV_STAGES * 2 * KV_TILE_BYTES,
                   "the exchange area of the cluster merge does not fit the tiles");
     static_assert(TN == 64 || TN == 128, "a block of keys");
@@ -268,6 +281,14 @@ struct DiffArgs {
     float cap, lambda, out_scale, eps;
     int dv;
 };
+// What a bias by distance needs beyond the rest (see attention_bias.cu): bias [n_dist, nh] or null, a gate logit a head or null, sinks [nh] or null.
+struct BiasArgs {
+    const float* bias;
+    const bf16* gate;
+    const float* sinks;
+    long long gate_stride;
+    int n_dist;
+};
 constexpr float FIXED_REFERENCE_CAP = 64.0f;    // capped scores up to here are exponentiated as they are
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
@@ -307,20 +328,21 @@ __device__ __forceinline__ void cap_of_chunk(uint32_t (&v)[32], float scale, flo
     }
 }
 
-template <int HD, int TN, bool DIFF = false>
+template <int HD, int TN, bool DIFF = false, bool BIAS = false>
 __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out, const int* __restrict__ tiles,
     const int* __restrict__ cu_seqlens, const int* __restrict__ ctx_lens,
     const int* __restrict__ block_tables, int max_blocks, int nh, int nkv, int page_size,
-    int cache_rows, float scale, int window, int splits, const DiffArgs diff) {
+    int cache_rows, float scale, int window, int splits, const DiffArgs diff, const BiasArgs ba) {
+    static_assert(!(DIFF && BIAS), "one or the other");
     static_assert(!DIFF || (HD == 128 && TN == 64), "two maps of 64 are a row of 128");
     extern __shared__ __align__(1024) unsigned char pt_smem_raw[];
     if ((smem_u32(pt_smem_raw) & 1023u) != 0u) {       // the swizzled tiles need it; never seen, but checked
         if (threadIdx.x == 0) atomicExch(&g_tc_error, 2);
         return;
     }
-    using SH = PShape<HD, TN>;
+    using SH = PShape<HD, TN, BIAS>;
     constexpr int Q_BYTES = SH::Q_BYTES, KV_TILE_BYTES = SH::KV_TILE_BYTES;
     constexpr int KV_LINE_TILE = SH::KV_LINE_TILE, KV_STAGES = SH::KV_STAGES;
     constexpr int HALVES = HD / 64;                                   // sub-tiles of 64 columns in a row of Q, K, V
@@ -525,6 +547,28 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
         const float scale_log2 = capped ? 1.0f : scale * 1.4426950408889634f;      // (capping leaves scores in units of log2(e))
         const uint32_t tmem_p_row = tmem_p + lane_addr;
         bool ok = true;
+        constexpr float LOG2E = 1.4426950408889634f;
+        // this row's head's table, in front of the place of distance 0 minus this row's distance to key 0 of a block at its own position
+        const float* near_row = nullptr;
+        float far_bias = 0.f;
+        if constexpr (BIAS) {
+            const int head = srow < 64 ? head0 : head1;
+            if (ba.bias != nullptr) {
+                float* tables = reinterpret_cast<float*>(pt_smem_raw + SH::SMEM);
+                const int len = ba.n_dist + BIAS_PAD;
+                for (int i = threadIdx.x - PT_SOFTMAX_WARP0 * 32; i < 2 * len; i += 128) {
+                    const int dist = min(max(i % len - BIAS_FRONT, 0), ba.n_dist - 1);
+                    tables[i] = ba.bias[(size_t)dist * nh + (i < len ? head0 : head1)] * LOG2E;
+                }
+                near_row = tables + (srow < 64 ? 0 : len) + BIAS_FRONT;
+                far_bias = ba.bias[(size_t)(ba.n_dist - 1) * nh + head] * LOG2E;
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+            }
+            if (ba.sinks != nullptr) {
+                m_ref = ba.sinks[head] * LOG2E;
+                l_run = m_ref == -INFINITY ? 0.f : 1.f;
+            }
+        }
         for (int it = 0; it < n_blk; ++it) {
             const int key0 = (blk0 + it * splits) * TN;
             ok = bar_wait(&ctrl->s_full, it & 1, &ctrl->abort) && ok;
@@ -545,6 +589,26 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
             const bool need_mask = key0 + TN - 1 > pos0 || window > 0;
             const int kmax = pos - key0, kmin = lo - key0;           // visible: kmin <= index <= kmax
             float mx = -INFINITY;
+            float block_scale = scale_log2, block_add = 0.f;
+            if constexpr (BIAS) {
+                if (ba.bias != nullptr) {
+                    block_add = far_bias;
+                    if (pos0 - (key0 + TN - 1) < ba.n_dist - 1) {       // some of the tile's rows are within the table's reach
+                        const float* at = near_row + kmax;              // (distance of key `idx`: kmax - idx)
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            s0[i] = __float_as_uint(fmaf(__uint_as_float(s0[i]), scale_log2, at[-i]));
+                            s1[i] = __float_as_uint(fmaf(__uint_as_float(s1[i]), scale_log2, at[-32 - i]));
+                            if constexpr (TN > 64) {
+                                s2[i] = __float_as_uint(fmaf(__uint_as_float(s2[i]), scale_log2, at[-64 - i]));
+                                s3[i] = __float_as_uint(fmaf(__uint_as_float(s3[i]), scale_log2, at[-96 - i]));
+                            }
+                        }
+                        block_scale = 1.0f;
+                        block_add = 0.f;
+                    }
+                }
+            }
             if constexpr (DIFF) {
                 if (capped) {
                     cap_of_chunk(s0, scale, diff.cap);
@@ -568,7 +632,7 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
                     max_of_chunk3(s3, mx);
                 }
             }
-            const float m_new = fmaxf(m_ref, mx * scale_log2);
+            const float m_new = fmaxf(m_ref, BIAS ? fmaf(mx, block_scale, block_add) : mx * scale_log2);
             // the reference moves only when the maximum has run ahead of it (always on the first keys seen)
             const bool move = m_new - m_ref > RESCALE_AFTER || (m_ref == -INFINITY && m_new != -INFINITY);
             float corr = 1.0f;
@@ -614,7 +678,7 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
             }
             // P goes to tensor memory in two halves of the block's keys, each handed to the product
             // as soon as it is complete (O, if it was rescaled, is back there before the first)
-            const uint64_t scale2 = pair_of(scale_log2), neg_m2 = pair_of(-m_use);
+            const uint64_t scale2 = pair_of(block_scale), neg_m2 = pair_of(BIAS ? block_add - m_use : -m_use);
             uint64_t lsum2 = 0ull;
             auto hand_over = [&](int half) {
                 tmem_st_wait();
@@ -704,7 +768,12 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
                 }
             }
         } else if (splits == 1) {
-            if (n_blk > 0) store_row<HD>(tmem_o + slane_addr, 1.0f / l_run, row_ok && srow_valid, sorow);
+            float inv = 1.0f / l_run;
+            if constexpr (BIAS) {
+                if (ba.gate != nullptr && srow_valid)
+                    inv /= 1.0f + expf(-__bfloat162float(ba.gate[(size_t)(q_start + t0 + (srow & 63)) * ba.gate_stride + (srow < 64 ? head0 : head1)]));
+            }
+            if (n_blk > 0) store_row<HD>(tmem_o + slane_addr, inv, row_ok && srow_valid, sorow);
         } else {
             // The CTAs of the cluster took the blocks of keys in turn.  Once all their products are done
             // (the tiles in shared memory are free), ranks 1.. send their rows (64 unnormalised sums,
@@ -850,7 +919,7 @@ int launch_prefill_tc(const CUtensorMap& map_q, const CUtensorMap& map_k, const 
     if (splits != 1 && splits != 2 && splits != 4) return RLIS_ERR_UNSUPPORTED;
     rlis_launch_cluster(attn_prefill_tc_kernel<HD, TN>, dim3((unsigned)(pairs * splits), (unsigned)n_tiles), PT_THREADS,
                         SH::SMEM, stream, dim3((unsigned)splits, 1, 1), map_q, map_k, map_v, out, tiles, cu_seqlens,
-                        ctx_lens, block_tables, max_blocks, nh, nkv, page_size, cache_rows, scale, window, splits, DiffArgs{});
+                        ctx_lens, block_tables, max_blocks, nh, nkv, page_size, cache_rows, scale, window, splits, DiffArgs{}, BiasArgs{});
     return RLIS_LAUNCH_CHECK();
 }
 }  // namespace
@@ -930,6 +999,56 @@ extern "C" int rlis_attention_difference_prefill(const void* q, const void* k_ca
     const DiffArgs da{(const bf16*)gate, gate_stride, cap, lambda, out_scale, eps, dv};
     rlis_launch_cluster(attn_prefill_tc_kernel<128, 64, true>, dim3((unsigned)nh, (unsigned)n_tiles), PT_THREADS, SH::SMEM, stream,
                         dim3(1, 1, 1), map_q, map_k, map_v, (bf16*)out, tiles, cu_seqlens, ctx_lens, block_tables, max_blocks, nh, nkv,
-                        page_size, (int)cache_rows, scale, window, 1, da);
+                        page_size, (int)cache_rows, scale, window, 1, da, BiasArgs{});
     return RLIS_LAUNCH_CHECK();
+}
+
+// Whether the tensor-core kernel takes attention with a bias by distance of these sizes (`bias` null: n_dist 0; no slopes, a gate a head at most).
+extern "C" int rlis_attention_bias_prefill_tc_takes(int nh, int nkv, int d, int dv, int page_size, int n_dist) {
+    return d == dv && n_dist >= 0 && n_dist <= BIAS_MAX_DIST && rlis_attention_prefill_tc_takes(nh, nkv, d, page_size);
+}
+
+namespace {
+template <int HD, int TN>
+int launch_bias_tc(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v, bf16* out, const BiasArgs& ba, const int* tiles, int n_tiles,
+                   const int* cu_seqlens, const int* ctx_lens, const int* block_tables, int max_blocks, int nh, int nkv, int page_size, int cache_rows, float scale,
+                   int window, cudaStream_t stream) {
+    using SH = PShape<HD, TN, true>;
+    const size_t smem = ba.bias != nullptr ? SH::smem_bias(ba.n_dist) : SH::SMEM;
+    static bool attr_done = false;
+    if (!attr_done) {
+        cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, TN, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::smem_bias(BIAS_MAX_DIST));
+        attr_done = true;
+    }
+    rlis_launch_cluster(attn_prefill_tc_kernel<HD, TN, false, true>, dim3((unsigned)(nkv * ((nh / nkv + 1) / 2)), (unsigned)n_tiles), PT_THREADS, smem, stream,
+                        dim3(1, 1, 1), map_q, map_k, map_v, out, tiles, cu_seqlens, ctx_lens, block_tables, max_blocks, nh, nkv, page_size, cache_rows, scale, window,
+                        1, DiffArgs{}, ba);
+    return RLIS_LAUNCH_CHECK();
+}
+}  // namespace
+
+// The contract of rlis_attention_bias_prefill (no slopes; gate: a logit a head, head h of token t at gate[t * gate_stride + h]); n_tokens and n_pages: rows of q
+// and pages of the caches.
+extern "C" int rlis_attention_bias_prefill_tc(const void* q, const void* k_cache, const void* v_cache, void* out, const float* bias, int n_dist, const void* gate,
+                                              long long gate_stride, const int* tiles, int n_tiles, const int* cu_seqlens, const int* ctx_lens,
+                                              const int* block_tables, int max_blocks, int n_tokens, int n_pages, int nh, int nkv, int d, int page_size, float scale,
+                                              int window, const float* sinks, cudaStream_t stream) {
+    if (n_tiles <= 0) return 0;
+    if (!rlis_attention_bias_prefill_tc_takes(nh, nkv, d, d, page_size, bias != nullptr ? n_dist : 0) || n_tiles > 65535 || (bias != nullptr && n_dist <= 0))
+        return RLIS_ERR_UNSUPPORTED;
+    if (((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache) |
+          reinterpret_cast<uintptr_t>(out)) & 15) != 0)
+        return RLIS_ERR_UNSUPPORTED;
+    const long long cache_rows = (long long)n_pages * nkv * page_size;
+    if (cache_rows >= (1ll << 31)) return RLIS_ERR_UNSUPPORTED;
+    CUtensorMap map_q, map_k, map_v;
+    if (!make_map_2d(&map_q, q, n_tokens, (long long)nh * d, TQ) || !make_map_2d(&map_k, k_cache, cache_rows, d, page_size) ||
+        !make_map_2d(&map_v, v_cache, cache_rows, d, page_size))
+        return RLIS_ERR_UNSUPPORTED;
+    const BiasArgs ba{bias, (const bf16*)gate, sinks, gate_stride, n_dist};
+    if (d == 64)
+        return launch_bias_tc<64, 128>(map_q, map_k, map_v, (bf16*)out, ba, tiles, n_tiles, cu_seqlens, ctx_lens, block_tables, max_blocks, nh, nkv, page_size,
+                                       (int)cache_rows, scale, window, stream);
+    return launch_bias_tc<128, 64>(map_q, map_k, map_v, (bf16*)out, ba, tiles, n_tiles, cu_seqlens, ctx_lens, block_tables, max_blocks, nh, nkv, page_size,
+                                   (int)cache_rows, scale, window, stream);
 }

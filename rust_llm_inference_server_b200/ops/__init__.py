@@ -1905,6 +1905,18 @@ def biased_decode_pieces(n_decode: int, n_kv_heads: int, max_ctx: int) -> int:
     return _biased_decode_pieces(int(n_decode), int(n_kv_heads), max(1, int(max_ctx)), num_sms())
 
 
+@functools.lru_cache(maxsize=None)
+def _biased_tc_sizes(n_heads: int, n_kv_heads: int, dim: int, v_dim: int, page_size: int, n_dist: int) -> bool:
+    return bool(lib().rlis_attention_bias_prefill_tc_takes(n_heads, n_kv_heads, dim, v_dim, page_size, n_dist))
+
+
+def _biased_prefill_tc(q, k_cache, v_cache, out, bias, gate, gate_cols: int, slopes, n_heads: int, n_kv_heads: int, dim: int, v_dim: int, page_size: int) -> bool:
+    """Whether portions of prompts with these operands go to the tcgen05 kernel (csrc/kernels/attention_prefill_tcgen05.cu)."""
+    return (slopes is None and (gate is None or gate_cols == 1) and k_cache.shape[0] * n_kv_heads * page_size < 1 << 31
+            and (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | out.data_ptr()) % 16 == 0
+            and _biased_tc_sizes(n_heads, n_kv_heads, dim, v_dim, page_size, 0 if bias is None else bias.shape[0]))
+
+
 def attention_biased(q, k_cache, v_cache, out, bias, gate, step, group: int, n_heads: int, n_kv_heads: int,
                      dim: int, v_dim: int, page_size: int, scale: float, window: int = 0,
                      sinks: torch.Tensor | None = None, slopes: torch.Tensor | None = None) -> torch.Tensor:
@@ -1953,7 +1965,14 @@ def attention_biased(q, k_cache, v_cache, out, bias, gate, step, group: int, n_h
             step.dec_seqs.data_ptr(), step.ctx_lens.data_ptr(), tables.data_ptr(), tables.shape[1], n_dec, n_heads,
             n_kv_heads, dim, v_dim, page_size, float(scale), int(window), pieces, sp, lp, gc, _stream()), "attention_bias_decode")
         _count("attention_bias.decode.mma" + (".split" if pieces > 1 else ""))
-    if n_tiles:
+    if n_tiles and _biased_prefill_tc(q, k_cache, v_cache, out, bias, gate, gc, slopes, n_heads, n_kv_heads, dim, v_dim, page_size):
+        check(lib().rlis_attention_bias_prefill_tc(
+            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), bp, n_dist, gp, gs, step.prefill_tiles.data_ptr(), n_tiles,
+            step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(), tables.data_ptr(), tables.shape[1], T, k_cache.shape[0], n_heads, n_kv_heads, dim,
+            page_size, float(scale), int(window), sp, _stream()), "attention_bias_prefill_tc")
+        _count("attention_bias.prefill.mma")
+        launches_by_kernel["attention_bias.prefill.mma.tcgen05"] = launches_by_kernel.get("attention_bias.prefill.mma.tcgen05", 0) + 1
+    elif n_tiles:
         check(lib().rlis_attention_bias_prefill(
             q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), bp, n_dist, gp, gs,
             step.prefill_tiles.data_ptr(), n_tiles, step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(),

@@ -69,6 +69,8 @@ SIGNATURES = {
     "rlis_qk_row_norm_store": [P, LL, I, I, I, P, P, F, P, P, P, P, I, I, I, I, I, I, I, P],
     "rlis_attention_bias": [P, P, P, P, P, I, P, LL, P, P, P, P, I, I, I, I, I, I, I, F, I, P, P, I, I, P],
     "rlis_attention_bias_mma_takes": [I, I],
+    "rlis_attention_bias_prefill_tc": [P, P, P, P, P, I, P, LL, P, I, P, P, P, I, I, I, I, I, I, I, F, I, P, P],
+    "rlis_attention_bias_prefill_tc_takes": [I, I, I, I, I, I],
     "rlis_attention_bias_prefill": [P, P, P, P, P, I, P, LL, P, I, P, P, P, I, I, I, I, I, I, F, I, P, P, I, P],
     "rlis_attention_bias_decode": [P, P, P, P, P, P, I, P, LL, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P, P, I, P],
     "rlis_attention_difference": [P, P, P, P, P, LL, P, P, P, P, I, I, I, I, I, I, I, F, F, I, F, F, F, I, P],
