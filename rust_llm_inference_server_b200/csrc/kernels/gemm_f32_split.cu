@@ -332,7 +332,7 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
 // ------------------------------------------------------------------------------------------------
 // Few rows (a decode step): bound by the memory's rate over W, and below it by a stage's way through the roles (raw weights, planes, products: about
 // 900 cycles with one CTA on an SM, 600 a stage with two).  8 rows, us here and as chains of FMAs: K 2048 N 2048 8.9 / 11.3, N 3072 9.8 / 16, N 16384 28 / 42,
-// N 32000 47 / 81 (5.6 TB/s); K 8192 N 2048 26 / 37.  A tile of 128 features a cluster, whose CTAs take whole segments of k and leave their
+// N 32000 47 / 81 (5.6 TB/s); K 8192 N 2048 22 / 37.  A tile of 128 features a cluster, whose CTAs take whole segments of k and leave their
 // sums in shared memory; the cluster then adds them up in the order of k, each CTA for a share of the features.  The rows of A are split
 // where the weights are.  Fourteen warps: 0-3 read the accumulators, 4-11 split (two sets), 12 asks for weights and rows, 13 issues the products.
 constexpr int FEW_THREADS = 448, FEW_A = 4;
@@ -559,21 +559,22 @@ int sm_count() {
     return sms;
 }
 
-constexpr int FEW_ROWS = 32, MAX_PARTS = 8;
+constexpr int FEW_ROWS = 32, MAX_PARTS = 12;
 int g_bn = 0, g_parts = 0;      // held fixed by a measurement (0: automatic)
 
 template <int BN> int launch_few(SplitArgs p, cudaStream_t stream) {
     using F = Few<BN>;
     const int sms = sm_count(), tiles = (p.N + FT - 1) / FT, segs = (p.stages + SEG_STAGES - 1) / SEG_STAGES;
-    // CTAs a tile: by what a segment takes a CTA alone on its SM (about 7,200 cycles) and beside another (9,600), and by what a CTA takes beside its segments.
-    // 8 rows, us with 1, 2, 4 and 8 CTAs a tile: N 16384 K 2048 33, 29, 32, 39; N 32000 48, 55, 61, 72; N 3072 27, 16, 11, 9.5; N 2048 K 8192 101, 61, 29, 26.
+    // CTAs a tile: by what a segment takes a CTA alone on its SM (about 7,400 cycles) and beside another (9,600), and by what a CTA takes beside its segments.
+    // 8 rows, us with 1, 2, 4 and 8 CTAs a tile: N 16384 K 2048 33, 29, 32, 39; N 32000 48, 55, 61, 72; N 3072 27, 16, 11, 9.5; N 2048 K 8192 105, 57, 31, 25,
+    // with 12 22 and with 16, which half a GPC has to hold, 28.
     int parts = 1;
     long long best = -1;
     for (int c = 1; c <= MAX_PARTS && c <= segs; ++c) {
         const int per = (segs + c - 1) / c;
         if (c > 1 && F::smem(4, per * p.M) > 227 * 1024) continue;
         const long long ctas = (long long)tiles * c;
-        const long long cost = (ctas <= sms ? 7200LL : 9600LL) * per + (c > 1 ? 5000 : 2500), total = (ctas + 2 * sms - 1) / (2 * sms) * cost;
+        const long long cost = (ctas <= sms ? 7400LL : 9600LL) * per + (c > 1 ? 5000 : 2500), total = (ctas + 2 * sms - 1) / (2 * sms) * cost;
         if (best < 0 || total < best) { best = total; parts = c; }
     }
     if (g_parts > 0 && g_parts <= segs && F::smem(4, (segs + g_parts - 1) / g_parts * p.M) <= 227 * 1024) parts = g_parts;
@@ -583,7 +584,8 @@ template <int BN> int launch_few(SplitArgs p, cudaStream_t stream) {
     CUtensorMap map_w, map_a;
     if (!map_f32(&map_w, p.W, p.N, p.K, p.ldw, FT) || !map_f32(&map_a, p.A, p.M, p.K, p.lda, BN)) return RLIS_ERR_UNSUPPORTED;
     const int smem = F::smem(p.raw_ring, rows);
-    const cudaError_t e = cudaFuncSetAttribute(f32_split_few_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(f32_split_few_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess && parts > 8) e = cudaFuncSetAttribute(f32_split_few_kernel<BN>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return (int)e;
     rlis_launch_cluster(f32_split_few_kernel<BN>, dim3((unsigned)(tiles * parts)), dim3(FEW_THREADS), (size_t)smem, stream, dim3((unsigned)parts, 1, 1), map_w, map_a, p, parts);
     return RLIS_LAUNCH_CHECK();

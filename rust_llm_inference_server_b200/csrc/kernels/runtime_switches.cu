@@ -24,8 +24,8 @@ extern "C" int rlis_get_pdl(void) { return g_rlis_pdl; }
 //   prefill_splits   0,1,2,4   CTAs that share a tile's keys in the tcgen05 prefill attention (0: automatic)
 //   gemm_pair        -1 / 0    two SMs to a tile in the tcgen05 product of many rows (-1: where it applies)
 //   filtered_cluster 0 / 1     the cluster kernel of top-k / top-p sampling where the vocabulary fits
-//   f32_split_rows   0, 16..192 rows a tile of the float32 product on tensor cores (0: automatic)
-//   f32_split_parts  0, 1..8   CTAs that share a tile's k there when the rows are few (0: automatic)
+//   f32_split_rows   0, 16..160 rows a tile of the float32 product on tensor cores (0: automatic)
+//   f32_split_parts  0, 1..12  CTAs that share a tile's k there when the rows are few (0: automatic)
 extern "C" void rlis_stream_gemm_set_target(int);
 extern "C" void rlis_gemm_f32_split_set_rows(int);
 extern "C" void rlis_gemm_f32_split_set_parts(int);
