@@ -494,7 +494,7 @@ def gated_delta(proj: torch.Tensor, qkv_off: int, b_off: int, a_off: int, conv_w
     by_rule = chunks is None
     if by_rule:
         chunks = _recurrence_in_chunks(step, T, n_heads, dv, proj.device)
-    wide = _gated_delta_wide(step, T, n_heads, n_qk_heads, d, dv, taps, state, act, out, chunks) if by_rule or chunks else None
+    wide = _gated_delta_wide(step, T, n_heads, n_qk_heads, d, dv, taps, state, act, out, chunks) if d == 128 and T >= 64 and (by_rule or chunks) else None
     gram = step.buffer("recurrence_gram", (T, n_qk_heads * 32 + n_heads * 16), torch.float32).data_ptr() if chunks and wide is None else 0
     check(lib().rlis_gated_delta(proj.data_ptr(), proj.stride(0), int(qkv_off), int(b_off), int(a_off), conv_w.data_ptr(),
                                  a_log.data_ptr(), dt_bias.data_ptr(), state.data_ptr(), state.stride(0),
@@ -1910,9 +1910,17 @@ def _biased_tc_sizes(n_heads: int, n_kv_heads: int, dim: int, v_dim: int, page_s
     return bool(lib().rlis_attention_bias_prefill_tc_takes(n_heads, n_kv_heads, dim, v_dim, page_size, n_dist))
 
 
-def _biased_prefill_tc(q, k_cache, v_cache, out, bias, gate, gate_cols: int, slopes, n_heads: int, n_kv_heads: int, dim: int, v_dim: int, page_size: int) -> bool:
-    """Whether portions of prompts with these operands go to the tcgen05 kernel (csrc/kernels/attention_prefill_tcgen05.cu)."""
-    return (slopes is None and (gate is None or gate_cols == 1) and k_cache.shape[0] * n_kv_heads * page_size < 1 << 31
+# The longest context of a step up to which its portions stay on mma.sync, by head size: a short one is all latency, of which the tcgen05 kernel has more.
+# us on tcgen05 and mma.sync, 32 heads of 64: 64 tokens 8.4 and 4.7, 128 8.2 and 6.9, 269 (a window and sinks) 13.8 and 12.4, 384 12.1 and 15.0, 512 13.5 and 18.9;
+# 16 heads of 128: 64 7.3 and 6.9, 128 8.0 and 10.5.
+BIASED_TC_AFTER = {64: 320, 128: 96}
+
+
+def _biased_prefill_tc(q, k_cache, v_cache, out, bias, gate, gate_cols: int, slopes, n_heads: int, n_kv_heads: int, dim: int, v_dim: int, page_size: int,
+                       max_ctx: int = 1 << 30) -> bool:
+    """Whether portions of prompts with these operands, in a step whose longest context is `max_ctx`, go to the tcgen05 kernel
+    (csrc/kernels/attention_prefill_tcgen05.cu)."""
+    return (max_ctx > BIASED_TC_AFTER.get(dim, 1 << 30) and slopes is None and (gate is None or gate_cols == 1) and k_cache.shape[0] * n_kv_heads * page_size < 1 << 31
             and (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | out.data_ptr()) % 16 == 0
             and _biased_tc_sizes(n_heads, n_kv_heads, dim, v_dim, page_size, 0 if bias is None else bias.shape[0]))
 
@@ -1965,7 +1973,8 @@ def attention_biased(q, k_cache, v_cache, out, bias, gate, step, group: int, n_h
             step.dec_seqs.data_ptr(), step.ctx_lens.data_ptr(), tables.data_ptr(), tables.shape[1], n_dec, n_heads,
             n_kv_heads, dim, v_dim, page_size, float(scale), int(window), pieces, sp, lp, gc, _stream()), "attention_bias_decode")
         _count("attention_bias.decode.mma" + (".split" if pieces > 1 else ""))
-    if n_tiles and _biased_prefill_tc(q, k_cache, v_cache, out, bias, gate, gc, slopes, n_heads, n_kv_heads, dim, v_dim, page_size):
+    if n_tiles and _biased_prefill_tc(q, k_cache, v_cache, out, bias, gate, gc, slopes, n_heads, n_kv_heads, dim, v_dim, page_size,
+                                      getattr(step, "max_ctx_len", 1 << 30)):
         check(lib().rlis_attention_bias_prefill_tc(
             q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), bp, n_dist, gp, gs, step.prefill_tiles.data_ptr(), n_tiles,
             step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(), tables.data_ptr(), tables.shape[1], T, k_cache.shape[0], n_heads, n_kv_heads, dim,

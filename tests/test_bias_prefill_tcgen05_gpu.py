@@ -81,6 +81,6 @@ def test_what_goes_there():
     from rust_llm_inference_server_b200 import ops
     x, odd = torch.zeros(4, 128, dtype=torch.bfloat16, device="cuda"), torch.zeros(513, dtype=torch.bfloat16, device="cuda")[1:].view(4, 128)
     cache, table = torch.zeros(3, 1, 16, 64, dtype=torch.bfloat16, device="cuda"), torch.zeros(1025, 2, device="cuda")
-    takes = lambda q=x, bias=table[:1024], gate=None, cols=1, slopes=None, dim=64, v_dim=64: ops._biased_prefill_tc(q, cache, cache, x, bias, gate, cols, slopes, 2, 1, dim, v_dim, 16)
-    assert takes() and takes(bias=None) and takes(gate=x)
+    takes = lambda q=x, bias=table[:1024], gate=None, cols=1, slopes=None, dim=64, v_dim=64, ctx=400: ops._biased_prefill_tc(q, cache, cache, x, bias, gate, cols, slopes, 2, 1, dim, v_dim, 16, ctx)
+    assert takes() and takes(bias=None) and takes(gate=x) and not takes(ctx=128) and takes(ctx=128, dim=128, v_dim=128)
     assert not takes(q=odd) and not takes(bias=table) and not takes(gate=x, cols=64) and not takes(slopes=x) and not takes(v_dim=32) and not takes(dim=96, v_dim=96)
