@@ -440,7 +440,7 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
             const int s = it % KV_STAGES;
             uint64_t* full = is_v ? &ctrl->v_full[s] : &ctrl->k_full[s];
             if (it >= KV_STAGES &&
-                !bar_wait(is_v ? &ctrl->v_empty[s] : &ctrl->k_empty[s], ((it / KV_STAGES) - 1) & 1, &ctrl->abort))
+                !bar_wait_warp(is_v ? &ctrl->v_empty[s] : &ctrl->k_empty[s], ((it / KV_STAGES) - 1) & 1, &ctrl->abort))
                 return false;
             unsigned char* tile = kv_tiles + (size_t)s * 2 * KV_TILE_BYTES + (is_v ? KV_TILE_BYTES : 0);
             if (lane == 0) bar_expect_tx(full, KV_TILE_BYTES);
@@ -466,19 +466,19 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
             if (it >= 1 && !load_tile(it - 1, true)) break;
         }
       } else if (warp == 1) {
-        // The whole warp walks the loop and waits; the elected lane issues.  (With the loop inside
+        // The whole warp walks the loop and waits, and leaves it together; the elected lane issues.  (With the loop inside
         // `if (lane == 0)` a product's eight instructions took 800 cycles to issue and every wait on
         // a barrier that was long complete 250; with the instructions alone inside it 56 each.)
         {
-            bool ok = bar_wait(&ctrl->q_full, 0, &ctrl->abort);
+            bool ok = bar_wait_warp(&ctrl->q_full, 0, &ctrl->abort);
             uint64_t qdesc[HALVES];
 #pragma unroll
             for (int hf = 0; hf < HALVES; ++hf) qdesc[hf] = smem_desc_sw128(q_tile + hf * LINE_TILE);
             auto issue_s = [&](int it) {
                 const int s = it % KV_STAGES;
-                if (!bar_wait(&ctrl->k_full[s], (it / KV_STAGES) & 1, &ctrl->abort)) return false;
+                if (!bar_wait_warp(&ctrl->k_full[s], (it / KV_STAGES) & 1, &ctrl->abort)) return false;
                 // the softmax warps have taken the scores of the block before out of tensor memory
-                if (it > 0 && !bar_wait(&ctrl->s_empty, (it - 1) & 1, &ctrl->abort)) return false;
+                if (it > 0 && !bar_wait_warp(&ctrl->s_empty, (it - 1) & 1, &ctrl->abort)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned char* kt = kv_tiles + (size_t)s * 2 * KV_TILE_BYTES;
                 if (elect_one()) {
@@ -500,14 +500,14 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
                 const int s = it % KV_STAGES;
                 if (it + 1 < n_blk && !issue_s(it + 1)) break;         // the next block's scores, behind this block's softmax
                 // the values have been there for a while; P is what the product waits for
-                if (!bar_wait(&ctrl->v_full[s], (it / KV_STAGES) & 1, &ctrl->abort)) break;
+                if (!bar_wait_warp(&ctrl->v_full[s], (it / KV_STAGES) & 1, &ctrl->abort)) break;
                 const unsigned char* vt = kv_tiles + (size_t)s * 2 * KV_TILE_BYTES + KV_TILE_BYTES;
                 // O += P V in two bursts: the first half of the keys while the softmax warps are in the
                 // exponentials of the second (after the last exponential only half of the instructions are left)
                 bool fine = true;
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
-                    if (!bar_wait(&ctrl->p_full[hf], it & 1, &ctrl->abort)) { fine = false; break; }
+                    if (!bar_wait_warp(&ctrl->p_full[hf], it & 1, &ctrl->abort)) { fine = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (elect_one()) {
 #pragma unroll

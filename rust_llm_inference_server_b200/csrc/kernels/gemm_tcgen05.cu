@@ -122,17 +122,18 @@ __global__ __launch_bounds__(GT_THREADS) void gemm_tcgen05_kernel(const __grid_c
             }
         }
     } else if (warp == 1) {
-        // the whole warp walks the loop and waits; one lane issues
+        // the whole warp walks the loop and waits, and leaves it together; one lane issues
         int it = 0, t = 0;          // t counts the tiles this CTA works on (a tile that is left out is not one)
-        for (int tile = blockIdx.x; tile < num_tiles && !ctrl->abort; tile += gridDim.x) {
+        bool fine = true;
+        for (int tile = blockIdx.x; tile < num_tiles && fine; tile += gridDim.x) {
             if (tile_expert != nullptr && tile_expert[tile % m_tiles] < 0) continue;
             const int buf = t & 1;
-            if (t >= 2 && !bar_wait(&ctrl->acc_empty[buf], ((t >> 1) - 1) & 1, &ctrl->abort)) break;
+            if (t >= 2 && !bar_wait_warp(&ctrl->acc_empty[buf], ((t >> 1) - 1) & 1, &ctrl->abort)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * BN);
             for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                 const int s = it % STAGES;
-                if (!bar_wait(&ctrl->full[s], (it / STAGES) & 1, &ctrl->abort)) break;
+                if (!bar_wait_warp(&ctrl->full[s], (it / STAGES) & 1, &ctrl->abort)) { fine = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t adesc = smem_desc_sw128(a_tiles + (size_t)s * A_STAGE_BYTES);
                 const uint64_t bdesc = smem_desc_sw128(b_tiles + (size_t)s * B_STAGE_BYTES);
@@ -145,6 +146,7 @@ __global__ __launch_bounds__(GT_THREADS) void gemm_tcgen05_kernel(const __grid_c
                 }
                 __syncwarp();
             }
+            if (!fine) break;
             if (elect_one()) umma_commit(&ctrl->acc_full[buf]);
             __syncwarp();
             ++t;
@@ -157,7 +159,7 @@ __global__ __launch_bounds__(GT_THREADS) void gemm_tcgen05_kernel(const __grid_c
             if (tile_expert != nullptr && tile_expert[tile % m_tiles] < 0) continue;
             const int buf = t & 1;
             const int n0 = (tile / m_tiles) * BN, m0 = (tile % m_tiles) * BM;
-            const bool ok = bar_wait(&ctrl->acc_full[buf], (t >> 1) & 1, &ctrl->abort);
+            const bool ok = bar_wait_warp(&ctrl->acc_full[buf], (t >> 1) & 1, &ctrl->abort);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = m0 + q * 32 + lane;
             const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * BN) + ((uint32_t)(q * 32) << 16);

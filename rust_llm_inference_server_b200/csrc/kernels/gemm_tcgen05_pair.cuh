@@ -145,7 +145,7 @@ __global__ __launch_bounds__(GP_THREADS) void gemm_tcgen05_pair_kernel(const __g
         }
     } else if (warp == 1) {
         if (rank == 0) {
-            // The whole warp walks the loop and waits; one lane issues.  (Measured: the warp never
+            // The whole warp walks the loop and waits, and leaves it together; one lane issues.  (Measured: the warp never
             // waits for a stage after the first, and a k-block still takes it 628 cycles for 512 of
             // tensor work: the instructions queue behind the pipe, which is held up by shared memory,
             // 32 KB a block written by the copies and 32 KB read by the products at 128 bytes a
@@ -156,14 +156,14 @@ __global__ __launch_bounds__(GP_THREADS) void gemm_tcgen05_pair_kernel(const __g
             // shared memory shrink by 15 % only.)
             int it = 0, t = 0;
             bool fine = true;
-            for (int tile = pair; tile < num_tiles && fine && !ctrl->abort; tile += pairs, ++t) {
+            for (int tile = pair; tile < num_tiles && fine; tile += pairs, ++t) {
                 const int buf = t & 1;
-                if (t >= 2 && !bar_wait(&ctrl->acc_empty[buf], ((t >> 1) - 1) & 1, &ctrl->abort)) break;
+                if (t >= 2 && !bar_wait_warp(&ctrl->acc_empty[buf], ((t >> 1) - 1) & 1, &ctrl->abort)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * PN);
                 for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                     const int s = it % P_STAGES;
-                    if (!bar_wait(&ctrl->full[s], (it / P_STAGES) & 1, &ctrl->abort)) { fine = false; break; }
+                    if (!bar_wait_warp(&ctrl->full[s], (it / P_STAGES) & 1, &ctrl->abort)) { fine = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (elect_one()) {
                         const uint64_t adesc = smem_desc_sw128(a_tiles + (size_t)s * A_BYTES);
@@ -188,7 +188,7 @@ __global__ __launch_bounds__(GP_THREADS) void gemm_tcgen05_pair_kernel(const __g
         for (int tile = pair; tile < num_tiles; tile += pairs, ++t) {
             const int buf = t & 1;
             const int n0 = (tile / m_tiles) * PN, m0 = (tile % m_tiles) * 2 * PM + (int)rank * PM;
-            const bool ok = bar_wait(&ctrl->acc_full[buf], (t >> 1) & 1, &ctrl->abort);
+            const bool ok = bar_wait_warp(&ctrl->acc_full[buf], (t >> 1) & 1, &ctrl->abort);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = m0 + q * 32 + lane;
             const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * PN) + ((uint32_t)(q * 32) << 16);

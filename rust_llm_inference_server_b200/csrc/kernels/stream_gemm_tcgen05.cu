@@ -364,10 +364,10 @@ __global__ __launch_bounds__(S_THREADS) void stream_gemm_kernel(const __grid_con
         }
         pdl_trigger();     // everything this CTA reads is requested: the next kernel may start its own requests
     } else if (warp == 1) {
-        // the whole warp walks the loop and waits; one lane issues
+        // the whole warp walks the loop and waits, and leaves it together; one lane issues
         for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
             const int s = it % STG;
-            if (!bar_wait(&ctrl->full[s], (it / STG) & 1, &ctrl->abort)) break;
+            if (!bar_wait_warp(&ctrl->full[s], (it / STG) & 1, &ctrl->abort)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint64_t adesc = smem_desc_sw128(w_tiles + (size_t)s * W_STAGE_BYTES);
             const uint64_t bdesc = smem_desc_sw128(x_tiles + (size_t)s * X_STAGE_BYTES);

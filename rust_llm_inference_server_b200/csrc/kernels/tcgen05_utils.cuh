@@ -55,8 +55,9 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatil
     const uint32_t addr = smem_u32(bar);
     return bar_try(addr, parity) || bar_wait_more(addr, parity, abort);
 }
-// The same for a whole warp that waits together.  The votes make the branches uniform for the compiler: a wait on a barrier that is long complete
-// costs 94 cycles instead of 150 to 220 (in a loop that ends when a wait fails).
+// The same for a whole warp that waits together: all lanes get one answer, as elect_one and __syncwarp behind a branch on it need (bar_wait's lanes
+// each go by the clock and `abort`, so that one may give up in the try in which another is through).  The votes also make the branches uniform for the
+// compiler: a wait on a barrier that is long complete costs 94 cycles instead of 150 to 220 (in a loop that ends when a wait fails).
 __device__ __forceinline__ bool bar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort) {
     const uint32_t addr = smem_u32(bar);
     if (__all_sync(0xffffffffu, bar_try(addr, parity))) return true;
