@@ -123,9 +123,10 @@ constexpr int PT_SOFTMAX_WARP0 = 4;
 constexpr int LINE_TILE = TM * 128;     // bytes of a swizzled sub-tile of 128 rows: 64 columns, 128-byte lines
 constexpr uint32_t TMEM_COLS = 256;     // S: columns 0 .. TN - 1, O: 128 .. 128 + HD - 1, P (bf16 pairs): TN / 2 columns in what is left
 
-// Entries of a head's table of biases by distance, and how many more its copy in shared memory has: 128 in front (keys after the query, hidden) and
-// 192 behind (the last one, for the block that the table ends in: up to 127 + 63 beyond).
-constexpr int BIAS_MAX_DIST = 1024, BIAS_FRONT = 128, BIAS_PAD = BIAS_FRONT + 192;
+// Entries of a head's table of biases by distance, and how many more its copy in shared memory has in front and behind.  In front: the last block of
+// keys may begin at the tile's last token and end TN - 1 keys after it (hidden ones, whose scores are formed like the others), TQ - 1 tokens after the
+// first row.  Behind (the last entry again): the block that the table ends in has rows and keys up to as far beyond.
+constexpr int BIAS_MAX_DIST = 1024, BIAS_FRONT = 192, BIAS_BACK = 192, BIAS_PAD = BIAS_FRONT + BIAS_BACK;
 
 // Sizes by head size HD and keys of a block TN (64, 128) or (128, 64): 16 KB of keys and of values a
 // block, three blocks in flight for head size 64 and two for 128 (112 and 96 KB a CTA, two CTAs an SM).
@@ -138,6 +139,7 @@ template <int HD, int TN, bool BIAS = false> struct PShape {
     // 228 KB of an SM only if no alignment slack is spent: the dynamic array is declared 1024-aligned
     static constexpr size_t SMEM = Q_BYTES + KV_STAGES * 2 * KV_TILE_BYTES + 256;
     static constexpr size_t smem_bias(int n_dist) { return SMEM + 2 * (size_t)(n_dist + BIAS_PAD) * sizeof(float); }
+    static_assert(BIAS_FRONT >= (TN - 1) + (TQ - 1) && BIAS_BACK >= (TN - 1) + (TQ - 1), "every distance between a tile's rows and the keys of its blocks");
     static_assert(!BIAS || 2 * (SMEM + 2 * (size_t)(BIAS_MAX_DIST + BIAS_PAD) * sizeof(float) + 1024) <= 228 * 1024, "two CTAs an SM, tables included");
     static constexpr uint32_t IDESC_S = idesc_bf16(TM, TN);
     static constexpr uint32_t IDESC_PV = idesc_bf16(TM, HD) | (1u << 16);      // B (V) is MN-major

@@ -26,11 +26,11 @@ class Step:
 
 
 # portions that end inside, at and one past a tile and a block of keys, with and without tokens before them; groups of 2, 3 and 4; tables of one entry, one that ends
-# inside a block, and the longest; windows; pages of 8 to 64
+# inside a block, and the longest; windows; pages of 8 to 64; tiles whose last token begins a block of 128 keys (64 behind 65)
 @pytest.mark.parametrize("d,group,page,lens,cached,n_dist,window,gated,sunk", [
     (64, 4, 16, [130], [0], 129, 0, True, False), (64, 2, 8, [64, 1, 65], [0, 300, 127], 1, 0, True, True), (64, 3, 64, [200, 31], [70, 0], 1024, 0, False, True),
     (64, 4, 16, [257], [40], 0, 100, False, True), (128, 2, 32, [129, 70], [0, 513], 40, 0, True, True), (128, 4, 16, [300], [0], 129, 64, True, False),
-    (64, 4, 16, [700], [0], 300, 0, True, True)])
+    (64, 4, 16, [700], [0], 300, 0, True, True), (64, 4, 16, [64, 65, 63], [65, 193, 1], 129, 0, True, False), (64, 2, 8, [64, 200], [65, 449], 1024, 0, False, True)])
 def test_portions_on_tcgen05(monkeypatch, d, group, page, lens, cached, n_dist, window, gated, sunk):
     from rust_llm_inference_server_b200 import ops
     rng = torch.Generator().manual_seed(sum(lens) + d)

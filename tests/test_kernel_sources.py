@@ -49,3 +49,20 @@ def test_a_warp_that_elects_a_lane_leaves_its_waits_together(name):
         assert "bar_wait_warp(" in role
         assert not re.search(r"\bbar_wait\(", role), name
         assert not re.search(r"(?<!&)ctrl->abort", role), name
+
+
+def test_a_table_of_biases_reaches_every_distance_that_a_tile_reads():
+    """All places of a tile against blocks of keys: the entries that its rows read, hidden keys included, lie in their head's copy of the table."""
+    text = source("attention_prefill_tcgen05.cu")
+    number = lambda name: int(re.search(rf"\b{name} = (\d+)\b", text).group(1))
+    front, tq = number("BIAS_FRONT"), number("TQ")
+    back = int(re.search(r"BIAS_PAD = BIAS_FRONT \+ (\w+)", text).group(1).replace("BIAS_BACK", str(number("BIAS_BACK")) if "BIAS_BACK" in text else ""))
+    for tn in (64, 128):
+        for n_dist in (1, 40, 129, 1024):
+            for pos0 in range(0, 2 * n_dist + 3 * tn, 1 if n_dist < 1024 else 7):
+                for tokens in {1, 2, tq - 1, tq}:
+                    for key0 in range(0, pos0 + tokens, tn):
+                        if pos0 - (key0 + tn - 1) >= n_dist - 1:
+                            continue            # a block beyond the table's reach takes its last entry
+                        first, last = pos0 - key0 - (tn - 1), pos0 + tq - 1 - key0          # (rows past the portion's end read, too)
+                        assert -front <= first and last < n_dist + back, (tn, n_dist, pos0, tokens, key0)
