@@ -513,17 +513,24 @@ def gated_delta(proj: torch.Tensor, qkv_off: int, b_off: int, a_off: int, conv_w
 @functools.lru_cache(maxsize=4096)
 def _gated_delta_wide_pays(n_tokens: int, n_seqs: int, longest: int, columns: int, sms: int, sixteen: bool) -> bool:
     """Whether the gated delta rule runs faster 64 tokens at a time than 16 at a time (`sixteen`) or token by token, for `columns` = heads x dv columns of
-    state and a longest portion of `longest` tokens.  Measured, 16 and 64 at a time in us (the inputs behind the convolutions included): one prompt of 2,048
-    with 16 heads 440 and 317, with 8 heads 402 and 219, of 1,024 228 and 166, of 512 124 and 109, of 256 73 and 89, of 64 33 and 70; 409 and 1,092
-    tokens 384 and 280; four of 512 with 8 heads 203 and 160; token by token and 64 at a time, four of 512 with 16 heads 333 and 313, of 256 170 and
-    164, of 128 90 and 109, 341, 910, 455 and 342 tokens 553 and 358, two of 2,048 with 32 heads 1,328 and 1,120."""
-    load = n_tokens * columns / 2048
-    if sixteen:
-        before = 18 + 0.206 * max(longest, 0.9 * load)
-    else:
-        before = 15 + max(0.6 * longest, 0.155 * load)
-    after = 50 + (0.095 if n_seqs * columns <= 16 * sms else 0.125) * (load + 48 * (n_seqs - 1) * columns / 2048) + 0.02 * longest
-    return longest >= 64 and after < 0.98 * before
+    state and a longest portion of `longest` tokens.  The three in us (the inputs behind the convolutions included), token by token / 16 / 64 tokens: with 16
+    heads one prompt of 64 tokens 20 / 28 / 64, of 256 66 / 68 / 85, of 512 126 / 119 / 104, of 2,048 492 / 435 / 313; with 8 heads 20 / 28 / 59, 63 / 62 / 76,
+    121 / 110 / 93 and 470 / 396 / 213; with 32 heads 43 / 37 / 71, 156 / 107 / 103, 306 / 197 / 156 and 1,229 / 769 / 577; two of 53 and 140 tokens 37 / 43 / 72
+    (8 heads) and 87 / 63 / 90 (16), of 409 and 1,092 258 / 227 / 151 and 633 / 379 / 273; four of 512 306 / 198 / 155, 329 / 482 / 310 and 592 / 761 / 556; 700
+    beside eight single tokens 261 / 229 / 155, 335 / 305 / 205 and 423 / 362 / 355.  A tie stays with the kernels before."""
+    heads = columns / 2048
+    if sixteen:             # a chain a request and head; the longest one's, beside what shares its SM
+        x = n_seqs * heads
+        before = 13 + longest * (0.17 + 0.034 * x if x <= 1 else 0.204 + 0.14 * (x - 1))
+    elif n_seqs * columns <= 16 * sms:          # the same with a CTA (16 columns) alone on its SM
+        before = 6 + 0.23 * longest
+    else:                   # with several on an SM, fewer of them where the others are single tokens; or by all of them
+        rate = 0.57 if n_seqs <= 4 else min(0.57, 0.24 + 0.22 * n_tokens / longest * heads)
+        before = 5 + max(rate * longest, 0.143 * n_tokens * heads)
+    # by the chain, or by the tokens of whole chunks
+    load = (longest + 32 + max(n_tokens - longest + 32 * (n_seqs - 1), 64 * (n_seqs - 1))) * heads
+    after = 57 + max(0.075 * longest, 0.095 * min(load, 1024) + 0.14 * max(load - 1024, 0))
+    return longest >= 64 and after < 0.95 * before
 
 
 GATED_DELTA_WIDE_BYTES = 512 << 20      # of scratch; steps that would take more go 16 tokens at a time

@@ -1,5 +1,7 @@
 """The host-side rules that cut a decode step's contexts into pieces and choose between kernels (no GPU needed)."""
 
+import pytest
+
 from rust_llm_inference_server_b200 import ops
 
 
@@ -86,3 +88,24 @@ def test_long_portions_go_by_chunks_and_short_ones_token_by_token():
                                     (64, "plain", (256, 1, 256, 512), (128, 1, 128, 512)), (64, "silu bf16", (512, 1, 512, 1024), (192, 1, 192, 128)),
                                     (64, "silu f32", (512, 1, 512, 1024), (192, 1, 192, 128)), (128, "silu bf16", (2048, 4, 512, 2048), (8000, 8, 1000, 2048))]:
         assert pays(*faster, 148, d, form) and not pays(*slower, 148, d, form), (d, form)
+
+
+# (heads, tokens of the portions, us token by token, 16 at a time, 64 at a time)
+DELTA_RULE = [
+    (8, [64], 20.2, 27.8, 58.6), (8, [100], 28.4, 35.5, 67.3), (8, [193], 49.0, 52.3, 75.0), (8, [256], 62.5, 62.1, 76.2), (8, [384], 92.5, 87.0, 85.4), (8, [512], 121.1, 110.2, 92.8),
+    (8, [2048], 469.7, 396.1, 213.4), (8, [53, 140], 37.2, 42.5, 71.5), (8, [100, 100], 29.1, 36.9, 68.2), (8, [200, 56], 50.6, 54.0, 76.0), (8, [256, 256], 65.7, 68.0, 84.0),
+    (8, [409, 1092], 258.1, 227.2, 151.0), (8, [60, 30, 100], 61.3, 48.8, 74.4), (8, [100] * 4, 66.2, 53.5, 82.4), (8, [512] * 4, 305.9, 198.4, 154.9), (8, [700] + [1] * 8, 261.4, 229.0, 154.8),
+    (16, [64], 20.4, 28.1, 64.1), (16, [128], 35.3, 40.6, 70.4), (16, [193], 52.4, 57.1, 79.5), (16, [256], 66.1, 68.0, 85.3), (16, [512], 126.1, 119.3, 104.0), (16, [2048], 491.8, 435.4, 312.8),
+    (16, [53, 140], 86.7, 62.6, 90.2), (16, [200, 56], 120.8, 83.0, 97.3), (16, [409, 1092], 633.2, 378.6, 272.8), (16, [200] * 4, 131.5, 198.5, 150.8), (16, [60, 30, 100], 65.7, 63.3, 87.8),
+    (16, [700] + [1] * 8, 335.4, 304.6, 205.1), (16, [1500] + [1] * 30, 722.6, 660.5, 521.1),
+    (32, [64], 42.9, 37.4, 70.6), (32, [128], 81.1, 61.1, 85.2), (32, [193], 122.0, 90.2, 101.3), (32, [512], 306.4, 197.4, 155.7), (32, [2048], 1229.4, 768.5, 576.9),
+    (32, [53, 140], 91.7, 102.8, 107.2), (32, [409, 1092], 677.5, 700.7, 484.7), (32, [200] * 4, 228.6, 306.1, 279.4), (32, [700] + [1] * 8, 423.0, 361.7, 355.3), (32, [1500] + [1] * 30, 926.4, 814.2, 913.7)]
+
+
+@pytest.mark.parametrize("heads,lens,single,sixteen,wide", DELTA_RULE)
+def test_the_delta_rule_by_64_tokens_is_taken_where_it_is_faster(heads, lens, single, sixteen, wide):
+    """Against what the three ways were measured to take: never slower than the way that a step would go otherwise, and never far from the faster one."""
+    by_sixteen = sum(lens) >= ops.GATED_DELTA_CHUNKS_FROM * len(lens) and len(lens) * heads * 8 <= 3 * 148
+    before = sixteen if by_sixteen else single
+    took = wide if ops._gated_delta_wide_pays(sum(lens), len(lens), max(lens), heads * 128, 148, by_sixteen) else before
+    assert took <= before and took <= 1.05 * min(before, wide)
