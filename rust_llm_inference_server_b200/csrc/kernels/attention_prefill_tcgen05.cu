@@ -99,12 +99,14 @@
 // are (2^92 fits bfloat16 and the float32 sums with room for the keys), so O is never rescaled.  At the end the warps of map 2
 // leave their rows in shared memory and those of map 1 subtract, norm, gate and store.
 //
-// A bias by distance, a gate a head, a sink (BIAS; the formulas are in attention_bias.cu): the same kernel with two rings of two tiles, which leaves room
-// for both heads' biases by distance in shared memory (times log2(e); repeated past their ends so that no index needs a bound).  A block that lies wholly
-// beyond the table's reach adds the last row's constant to the exponent's offset, for nothing; one within it reads a number a score (neighbouring rows
-// read neighbouring numbers).  A sink is what the row's reference and sum start from.  2,048 tokens, 32 heads of 64, a table of 129: 55 us, with
-// mma.sync (attention_bias_mma.cu, which keeps slopes, gates a channel, other sizes and longer tables) 102; a window of 1,024 and sinks, 409 and 1,092
-// tokens 40 and 63.
+// A bias by distance, a gate a head, a sink (BIAS; the formulas are in attention_bias.cu): the same kernel with blocks of 64 keys for both head sizes and
+// both heads' biases by distance in shared memory (times log2(e); with more entries in front and behind, so that no index needs a bound).  A block that
+// lies wholly beyond the table's reach adds the last row's constant; one within it reads a number a score (neighbouring rows read neighbouring numbers).
+// The weights are the ones that attention_bias_mma.cu forms: references move to the maximum with every block of 64 keys, the sum is of the weights before
+// rounding, and the sink joins it at the end, so the results agree but for the last bit of one number in 50,000 or more and a step may use both kernels.
+// (With blocks of 128 and a reference that lags, the highest weights are not exactly 1: off 64 bits by up to 9 % more.)  2,048 tokens, 32 heads of 64, a table
+// of 129: 50 us, with mma.sync (which keeps slopes, gates a channel, other sizes and longer tables) 92; a window of 1,024 and sinks, 409 and 1,092 tokens 31 and
+// 50; 16 heads of 128, 2,048 tokens 55 and 132.
 //
 // Every mbarrier wait is bounded (a fifth of a second); a wait that runs out sets the error word
 // (rlis_attention_prefill_tc_error), every role runs to its end without further waits, and the
@@ -134,7 +136,7 @@ template <int HD, int TN, bool BIAS = false> struct PShape {
     static constexpr int Q_BYTES = TM * HD * 2;             // 16 or 32 KB: HD / 64 sub-tiles [128 x 64]
     static constexpr int KV_TILE_BYTES = TN * HD * 2;       // 16 KB each for K and V: HD / 64 sub-tiles [TN x 64]
     static constexpr int KV_LINE_TILE = TN * 128;           // bytes of one such sub-tile
-    static constexpr int KV_STAGES = HD == 64 && !BIAS ? 3 : 2;
+    static constexpr int KV_STAGES = HD == 64 ? 3 : 2;
     // the tiles + the control block; with the kilobyte the system keeps per CTA, two CTAs fit the
     // 228 KB of an SM only if no alignment slack is spent: the dynamic array is declared 1024-aligned
     static constexpr size_t SMEM = Q_BYTES + KV_STAGES * 2 * KV_TILE_BYTES + 256;
@@ -213,6 +215,12 @@ __device__ __forceinline__ void fma2(float& d0, float& d1, float a0, float a1, u
     asm("{\n.reg .b64 ra, rd;\nmov.b64 ra, {%2, %3};\nfma.rn.f32x2 rd, ra, %4, %5;\nmov.b64 {%0, %1}, rd;\n}\n"
         : "=f"(d0), "=f"(d1) : "f"(a0), "f"(a1), "l"(b), "l"(c));
 }
+__device__ __forceinline__ void scale_pair(uint32_t& a0, uint32_t& a1, uint64_t b, uint64_t c) {
+    float d0, d1;
+    fma2(d0, d1, __uint_as_float(a0), __uint_as_float(a1), b, c);
+    a0 = __float_as_uint(d0);
+    a1 = __float_as_uint(d1);
+}
 __device__ __forceinline__ void add2(uint64_t& acc, uint32_t a0, uint32_t a1) {
     asm("{\n.reg .b64 ra;\nmov.b64 ra, {%1, %2};\nadd.rn.f32x2 %0, %0, ra;\n}\n" : "+l"(acc) : "r"(a0), "r"(a1));
 }
@@ -225,7 +233,9 @@ __device__ __forceinline__ float sum_of_pair(uint64_t acc) {
 // P = exp2(s * scale - m) of 32 keys, rounded to bf16, into the row's lane of tensor memory: two
 // consecutive keys to a column, the layout in which the tensor core reads its A operand from there.
 // `lsum2`: the running sums of the even and of the odd keys.
-template <bool MASK>
+// ROUNDED: the sum is of the rounded values, the ones the product with V uses: the rounding of a dominant key then cancels between numerator and
+// denominator.  Otherwise of the weights as they are.
+template <bool MASK, bool ROUNDED>
 __device__ __forceinline__ void exp_of_chunk(const uint32_t (&v)[32], int c, int kmin, int kmax, uint64_t scale2,
                                              uint64_t neg_m2, uint32_t tmem_p_row, uint64_t& lsum2) {
     uint32_t pk[16];
@@ -239,11 +249,10 @@ __device__ __forceinline__ void exp_of_chunk(const uint32_t (&v)[32], int c, int
             if (!(idx <= kmax && idx >= kmin)) p0 = 0.f;
             if (!(idx + 1 <= kmax && idx + 1 >= kmin)) p1 = 0.f;
         }
-        // the sum is of the rounded values, the ones the product with V uses: the rounding of a
-        // dominant key then cancels between numerator and denominator
         const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
         pk[i] = *reinterpret_cast<const uint32_t*>(&h);
-        add2(lsum2, pk[i] << 16, pk[i] & 0xffff0000u);
+        if (ROUNDED) add2(lsum2, pk[i] << 16, pk[i] & 0xffff0000u);
+        else add2(lsum2, __float_as_uint(p0), __float_as_uint(p1));
     }
     tmem_st16(tmem_p_row + (uint32_t)(c * 16), pk);
 }
@@ -337,7 +346,7 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
     const int* __restrict__ cu_seqlens, const int* __restrict__ ctx_lens,
     const int* __restrict__ block_tables, int max_blocks, int nh, int nkv, int page_size,
     int cache_rows, float scale, int window, int splits, const DiffArgs diff, const BiasArgs ba) {
-    static_assert(!(DIFF && BIAS), "one or the other");
+    static_assert(!(DIFF && BIAS) && (!BIAS || TN == 64), "one or the other; with a bias two chunks of 32 scores");
     static_assert(!DIFF || (HD == 128 && TN == 64), "two maps of 64 are a row of 128");
     extern __shared__ __align__(1024) unsigned char pt_smem_raw[];
     if ((smem_u32(pt_smem_raw) & 1023u) != 0u) {       // the swizzled tiles need it; never seen, but checked
@@ -566,10 +575,6 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
                 far_bias = ba.bias[(size_t)(ba.n_dist - 1) * nh + head] * LOG2E;
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             }
-            if (ba.sinks != nullptr) {
-                m_ref = ba.sinks[head] * LOG2E;
-                l_run = m_ref == -INFINITY ? 0.f : 1.f;
-            }
         }
         for (int it = 0; it < n_blk; ++it) {
             const int key0 = (blk0 + it * splits) * TN;
@@ -591,23 +596,21 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
             const bool need_mask = key0 + TN - 1 > pos0 || window > 0;
             const int kmax = pos - key0, kmin = lo - key0;           // visible: kmin <= index <= kmax
             float mx = -INFINITY;
-            float block_scale = scale_log2, block_add = 0.f;
             if constexpr (BIAS) {
-                if (ba.bias != nullptr) {
-                    block_add = far_bias;
-                    if (pos0 - (key0 + TN - 1) < ba.n_dist - 1) {       // some of the tile's rows are within the table's reach
-                        const float* at = near_row + kmax;              // (distance of key `idx`: kmax - idx)
+                // scores with their bias, in powers of two
+                if (ba.bias != nullptr && pos0 - (key0 + TN - 1) < ba.n_dist - 1) {       // some of the tile's rows are within the table's reach
+                    const float* at = near_row + kmax;              // (distance of key `idx`: kmax - idx)
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            s0[i] = __float_as_uint(fmaf(__uint_as_float(s0[i]), scale_log2, at[-i]));
-                            s1[i] = __float_as_uint(fmaf(__uint_as_float(s1[i]), scale_log2, at[-32 - i]));
-                            if constexpr (TN > 64) {
-                                s2[i] = __float_as_uint(fmaf(__uint_as_float(s2[i]), scale_log2, at[-64 - i]));
-                                s3[i] = __float_as_uint(fmaf(__uint_as_float(s3[i]), scale_log2, at[-96 - i]));
-                            }
-                        }
-                        block_scale = 1.0f;
-                        block_add = 0.f;
+                    for (int i = 0; i < 32; ++i) {
+                        s0[i] = __float_as_uint(fmaf(__uint_as_float(s0[i]), scale_log2, at[-i]));
+                        s1[i] = __float_as_uint(fmaf(__uint_as_float(s1[i]), scale_log2, at[-32 - i]));
+                    }
+                } else {
+                    const uint64_t scale2 = pair_of(scale_log2), far2 = pair_of(far_bias);
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        scale_pair(s0[i], s0[i + 1], scale2, far2);
+                        scale_pair(s1[i], s1[i + 1], scale2, far2);
                     }
                 }
             }
@@ -634,9 +637,9 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
                     max_of_chunk3(s3, mx);
                 }
             }
-            const float m_new = fmaxf(m_ref, BIAS ? fmaf(mx, block_scale, block_add) : mx * scale_log2);
-            // the reference moves only when the maximum has run ahead of it (always on the first keys seen)
-            const bool move = m_new - m_ref > RESCALE_AFTER || (m_ref == -INFINITY && m_new != -INFINITY);
+            const float m_new = fmaxf(m_ref, BIAS ? mx : mx * scale_log2);
+            // the reference moves only when the maximum has run ahead of it (always on the first keys seen); with a bias it is the maximum
+            const bool move = m_new - m_ref > (BIAS ? 0.f : RESCALE_AFTER) || (m_ref == -INFINITY && m_new != -INFINITY);
             float corr = 1.0f;
             if (move) {
                 corr = ex2_approx(m_ref - m_new);                    // 0 when nothing was seen before
@@ -680,7 +683,7 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
             }
             // P goes to tensor memory in two halves of the block's keys, each handed to the product
             // as soon as it is complete (O, if it was rescaled, is back there before the first)
-            const uint64_t scale2 = pair_of(block_scale), neg_m2 = pair_of(BIAS ? block_add - m_use : -m_use);
+            const uint64_t scale2 = pair_of(BIAS ? 1.0f : scale_log2), neg_m2 = pair_of(-m_use);
             uint64_t lsum2 = 0ull;
             auto hand_over = [&](int half) {
                 tmem_st_wait();
@@ -689,22 +692,22 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
                 if (lane == 0) bar_arrive(&ctrl->p_full[half]);
             };
             if (need_mask) {
-                exp_of_chunk<true>(s0, 0, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                exp_of_chunk<true, !BIAS>(s0, 0, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 if constexpr (TN == 64) hand_over(0);
-                exp_of_chunk<true>(s1, 1, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                exp_of_chunk<true, !BIAS>(s1, 1, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 if constexpr (TN > 64) {
                     hand_over(0);
-                    exp_of_chunk<true>(s2, 2, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
-                    exp_of_chunk<true>(s3, 3, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                    exp_of_chunk<true, !BIAS>(s2, 2, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                    exp_of_chunk<true, !BIAS>(s3, 3, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 }
             } else {
-                exp_of_chunk<false>(s0, 0, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                exp_of_chunk<false, !BIAS>(s0, 0, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 if constexpr (TN == 64) hand_over(0);
-                exp_of_chunk<false>(s1, 1, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                exp_of_chunk<false, !BIAS>(s1, 1, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 if constexpr (TN > 64) {
                     hand_over(0);
-                    exp_of_chunk<false>(s2, 2, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
-                    exp_of_chunk<false>(s3, 3, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                    exp_of_chunk<false, !BIAS>(s2, 2, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                    exp_of_chunk<false, !BIAS>(s3, 3, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 }
             }
             l_run += sum_of_pair(lsum2);
@@ -770,10 +773,12 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
                 }
             }
         } else if (splits == 1) {
-            float inv = 1.0f / l_run;
+            // one more term of the denominator, without a key or a value (one far above every score gives inf, and 0)
+            if (BIAS && ba.sinks != nullptr) l_run += ex2_approx(ba.sinks[srow < 64 ? head0 : head1] * LOG2E - m_ref);
+            float inv = !BIAS || l_run > 0.f ? 1.0f / l_run : 0.f;
             if constexpr (BIAS) {
                 if (ba.gate != nullptr && srow_valid)
-                    inv /= 1.0f + expf(-__bfloat162float(ba.gate[(size_t)(q_start + t0 + (srow & 63)) * ba.gate_stride + (srow < 64 ? head0 : head1)]));
+                    inv *= 1.0f / (1.0f + expf(-__bfloat162float(ba.gate[(size_t)(q_start + t0 + (srow & 63)) * ba.gate_stride + (srow < 64 ? head0 : head1)])));
             }
             if (n_blk > 0) store_row<HD>(tmem_o + slane_addr, inv, row_ok && srow_valid, sorow);
         } else {
@@ -1007,7 +1012,7 @@ extern "C" int rlis_attention_difference_prefill(const void* q, const void* k_ca
 
 // Whether the tensor-core kernel takes attention with a bias by distance of these sizes (`bias` null: n_dist 0; no slopes, a gate a head at most).
 extern "C" int rlis_attention_bias_prefill_tc_takes(int nh, int nkv, int d, int dv, int page_size, int n_dist) {
-    return d == dv && n_dist >= 0 && n_dist <= BIAS_MAX_DIST && rlis_attention_prefill_tc_takes(nh, nkv, d, page_size);
+    return d == dv && n_dist >= 0 && n_dist <= BIAS_MAX_DIST && page_size <= 64 && rlis_attention_prefill_tc_takes(nh, nkv, d, page_size);
 }
 
 namespace {
@@ -1049,7 +1054,7 @@ extern "C" int rlis_attention_bias_prefill_tc(const void* q, const void* k_cache
         return RLIS_ERR_UNSUPPORTED;
     const BiasArgs ba{bias, (const bf16*)gate, sinks, gate_stride, n_dist};
     if (d == 64)
-        return launch_bias_tc<64, 128>(map_q, map_k, map_v, (bf16*)out, ba, tiles, n_tiles, cu_seqlens, ctx_lens, block_tables, max_blocks, nh, nkv, page_size,
+        return launch_bias_tc<64, 64>(map_q, map_k, map_v, (bf16*)out, ba, tiles, n_tiles, cu_seqlens, ctx_lens, block_tables, max_blocks, nh, nkv, page_size,
                                        (int)cache_rows, scale, window, stream);
     return launch_bias_tc<128, 64>(map_q, map_k, map_v, (bf16*)out, ba, tiles, n_tiles, cu_seqlens, ctx_lens, block_tables, max_blocks, nh, nkv, page_size,
                                    (int)cache_rows, scale, window, stream);

@@ -1918,8 +1918,8 @@ def _biased_tc_sizes(n_heads: int, n_kv_heads: int, dim: int, v_dim: int, page_s
 
 
 # The longest context of a step up to which its portions stay on mma.sync, by head size: a short one is all latency, of which the tcgen05 kernel has more.
-# us on tcgen05 and mma.sync, 32 heads of 64: 64 tokens 8.4 and 4.7, 128 8.2 and 6.9, 269 (a window and sinks) 13.8 and 12.4, 384 12.1 and 15.0, 512 13.5 and 18.9;
-# 16 heads of 128: 64 7.3 and 6.9, 128 8.0 and 10.5.
+# us on tcgen05 and mma.sync, 32 heads of 64: 64 tokens 6.5 and 5.3, 128 7.8 and 7.4, 256 (a window and sinks) 10.6 and 10.6, 320 12.1 and 13.3, 448 15.0 and 18.4;
+# 16 heads of 128: 64 7.6 and 7.5, 96 8.4 and 10.2, 128 8.5 and 11.0.
 BIASED_TC_AFTER = {64: 320, 128: 96}
 
 

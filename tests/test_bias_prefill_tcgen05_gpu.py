@@ -77,6 +77,51 @@ def test_portions_on_tcgen05(monkeypatch, d, group, page, lens, cached, n_dist, 
     ops.check_device_errors()
 
 
+@pytest.mark.parametrize("d,n_dist,window,gated,sunk", [(64, 129, 0, True, False), (64, 0, 256, False, True), (128, 40, 0, True, True), (64, 300, 100, False, False)])
+def test_both_kernels_form_the_same_weights(monkeypatch, d, n_dist, window, gated, sunk):
+    """The results of the tcgen05 kernel are those of the mma.sync one but for float32 sums in another order, so no further from 64 bits: sums that differ by a
+    few times 2^-24 move a result across the boundary of two bfloat16 numbers, 2^-9 apart, in about 2^-13 of the cases."""
+    from rust_llm_inference_server_b200 import ops
+    rng = torch.Generator().manual_seed(d + n_dist)
+    rnd = lambda *s: torch.randn(*s, generator=rng)
+    lens, cached, nkv, nh, page = [500, 333], [0, 100], 2, 8, 16
+    st, T = Step(lens, cached, page, rng), sum(lens)
+    q, kc, vc = (rnd(*s).bfloat16().cuda() for s in ((T, nh * d), (st.pages, nkv, page, d), (st.pages, nkv, page, d)))
+    bias = (rnd(n_dist, nh) * 2).cuda() if n_dist else None
+    gate = rnd(T, nh).bfloat16().cuda() if gated else None
+    sinks = rnd(nh).cuda() if sunk else None
+    outs = []
+    for on in (True, False):
+        monkeypatch.setattr(ops, "_biased_prefill_tc", lambda *a, on=on: on)
+        outs.append(ops.attention_biased(q, kc, vc, torch.empty(T, nh * d, dtype=torch.bfloat16, device="cuda"), bias, gate, st, 0, nh, nkv, d, d, page, d ** -0.5, window, sinks))
+    assert float((outs[0] != outs[1]).double().mean()) <= 2.0 ** -12
+    ops.check_device_errors()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_edges_come_out_as_with_the_other_kernel(monkeypatch, d):
+    """Heads whose keys are all masked by the table, with -inf and with float32's lowest number; sinks at both ends; a scale below zero."""
+    from rust_llm_inference_server_b200 import ops
+    rng = torch.Generator().manual_seed(d)
+    rnd = lambda *s: torch.randn(*s, generator=rng)
+    lens, cached, nkv, nh, page = [140, 70], [0, 33], 2, 8, 16
+    st, T = Step(lens, cached, page, rng), sum(lens)
+    q, kc, vc = (rnd(*s).bfloat16().cuda() for s in ((T, nh * d), (st.pages, nkv, page, d), (st.pages, nkv, page, d)))
+    bias = rnd(50, nh).cuda()
+    bias[:, 0], bias[:, 1], bias[10:, 2], bias[0, 3] = float("-inf"), torch.finfo(torch.float32).min, float("-inf"), float("-inf")
+    sinks = rnd(nh).cuda()
+    sinks[0], sinks[4], sinks[5] = float("-inf"), float("inf"), -1e30
+    for scale in (d ** -0.5, -2.0, 0.0):
+        for at in (None, sinks):
+            outs = []
+            for on in (True, False):
+                monkeypatch.setattr(ops, "_biased_prefill_tc", lambda *a, on=on: on)
+                outs.append(ops.attention_biased(q, kc, vc, torch.empty(T, nh * d, dtype=torch.bfloat16, device="cuda"), bias, None, st, 0, nh, nkv, d, d, page, scale, 0, at))
+            assert bool(outs[1].isfinite().all()) and not bool(outs[1][:, :2 * d].any())
+            assert bool(outs[0].isfinite().all()) and float((outs[0] != outs[1]).double().mean()) <= 2.0 ** -12
+    ops.check_device_errors()
+
+
 def test_what_goes_there():
     from rust_llm_inference_server_b200 import ops
     x, odd = torch.zeros(4, 128, dtype=torch.bfloat16, device="cuda"), torch.zeros(513, dtype=torch.bfloat16, device="cuda")[1:].view(4, 128)
