@@ -122,6 +122,44 @@ def test_edges_come_out_as_with_the_other_kernel(monkeypatch, d):
     ops.check_device_errors()
 
 
+def test_a_portion_takes_its_kernel_whatever_is_beside_it():
+    """A short portion beside a long one and beside a single token of a long context: each the kernel, and the bits, that it has alone."""
+    from rust_llm_inference_server_b200 import ops
+    from rust_llm_inference_server_b200.engine.runner import tiles_of_portions
+    rng = torch.Generator().manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=rng)
+    d, nkv, nh, page, keys = 64, 2, 8, 16, ("attention_bias.prefill.mma.tcgen05", "attention_bias.prefill.mma")
+    lens, cached = [100, 500, 1], [20, 0, 900]
+    st = Step(lens, cached, page, rng)
+    q, kc, vc = (rnd(*s).bfloat16().cuda() for s in ((sum(lens), nh * d), (st.pages, nkv, page, d), (st.pages, nkv, page, d)))
+    bias = rnd(129, nh).cuda()
+
+    def run(rows):
+        part = Step.__new__(Step)
+        n, c = [lens[b] for b in rows], [cached[b] for b in rows]
+        dev = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+        part.n_seqs, part.block_tables, part.ctx_lens = len(rows), [st.block_tables[0][rows].contiguous()], dev([x + y for x, y in zip(n, c)])
+        part.cu_seqlens = dev([0] + torch.tensor(n).cumsum(0).tolist())
+        tiles, part.tiles_beyond = tiles_of_portions(n, c, 64, (ops.BIASED_TC_AFTER[d],))
+        part.prefill_tiles, part.n_prefill_tiles = dev(tiles), len(tiles)
+        dec = [b for b, x in enumerate(n) if x == 1]
+        part.n_decode, part.dec_rows, part.dec_seqs = len(dec), dev([sum(n[:b]) for b in dec]), dev(dec)
+        part.max_ctx_len, part.max_decode_ctx = max(x + y for x, y in zip(n, c)), 901
+        part.buffer = lambda name, shape, dtype: torch.empty(shape, dtype=dtype, device="cuda")
+        at = [sum(lens[:b]) for b in range(3)]
+        x = torch.cat([q[at[b]:at[b] + lens[b]] for b in rows])
+        n0 = [ops.launches_by_kernel.get(k, 0) for k in keys]
+        out = ops.attention_biased(x, kc, vc, torch.full_like(x, 7.0), bias, None, part, 0, nh, nkv, d, d, page, d ** -0.5)
+        tc, all_ = (ops.launches_by_kernel.get(k, 0) - m for k, m in zip(keys, n0))
+        return out.split(n), (tc, all_ - tc)
+
+    (short,), (long,) = (run([b])[0] for b in (0, 1))
+    assert run([0])[1] == (0, 1) and run([1])[1] == (1, 0) and run([0, 2])[1] == (0, 1) and run([0, 1, 2])[1] == (1, 1)
+    both = run([0, 1, 2])[0]
+    assert torch.equal(both[0], short) and torch.equal(both[1], long) and torch.equal(run([0, 2])[0][0], short)
+    ops.check_device_errors()
+
+
 def test_what_goes_there():
     from rust_llm_inference_server_b200 import ops
     x, odd = torch.zeros(4, 128, dtype=torch.bfloat16, device="cuda"), torch.zeros(513, dtype=torch.bfloat16, device="cuda")[1:].view(4, 128)
