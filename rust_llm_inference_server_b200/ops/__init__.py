@@ -1193,6 +1193,7 @@ def stream_gemm(x, w: torch.Tensor, out_dtype=torch.bfloat16, swiglu4: bool = Fa
                 bias: torch.Tensor | None = None, cubic: float = 0.0, n_plain: int | None = None, second: tuple | None = None):
     """y = x @ w^T (+ bias, float32 [N]) for at most 128 rows of bfloat16 x: the decode step's weight-streaming product on
     the tcgen05 tensor cores (TMA-fed, weights as the M side, k split over CTAs).  x may be a column slice of wider rows.
+    w is a loaded weight: its first tiles may be read before the kernels before this one in the stream have finished.
     `swiglu4`: w is a gate|up matrix interleaved in blocks of 4 rows (bias in the same order) and the result is silu(gate)
     * up, [M, N / 2]; with a `slope` (and `cubic`), gate sigmoid(slope (gate + cubic gate^3)) * up (+inf: max(gate, 0) * up).
     `n_plain` (up to 16 rows): the first n_plain rows of w are an ordinary matrix and the rest such a gate|up matrix; the
@@ -1379,12 +1380,14 @@ def fuses_norms(n_rows: int, dtype, *widths: int) -> bool:
             and all(w % 8 == 0 for w in widths))
 
 
-def linear(x, w: torch.Tensor, out_dtype=None, sink=None, bias: torch.Tensor | None = None, second: tuple | None = None):
+def linear(x, w: torch.Tensor, out_dtype=None, sink=None, bias: torch.Tensor | None = None, second: tuple | None = None, *, early: bool = False):
     """y = x @ w^T for w stored (out, in); x may be a column slice of wider rows.  float32: this package's kernels (`gemm_f32`).
     bfloat16: up to 16 rows go to this package's weight-streaming tcgen05 kernel, more to the library GEMM; both
     accumulate in float32, and `out_dtype=torch.float32` keeps that precision (used for logits).
     ScaledRows as x, a `sink` (with an optional `bias` of the product) and a `second` source = (x2, w2), whose product is
-    added, are for the streaming kernel only (see `fuses_norms`)."""
+    added, are for the streaming kernel only (see `fuses_norms`).
+    `early`: w is a weight that no kernel still in flight writes, so that a float32 product of few rows may ask for its first tiles before the kernels
+    before it have finished.  (The streaming kernel always does, see `stream_gemm`.)"""
     if isinstance(x, ScaledRows) or sink is not None or second is not None:
         if not fuses_norms(x.shape[0], x.dtype, x.shape[1]):
             raise KernelError("linear: scaled rows or a sink with a product that does not take them")
@@ -1393,7 +1396,7 @@ def linear(x, w: torch.Tensor, out_dtype=None, sink=None, bias: torch.Tensor | N
         raise KernelError("linear: a bias is taken with a sink")
     if x.dtype == torch.float32:
         if w.dtype == torch.float32 and x.is_cuda and x.dim() == 2 and x.is_contiguous() and w.is_contiguous() and x.shape[1] == w.shape[1] and _gemm_f32_splits(x, w):
-            return _gemm_f32_split(x, w, torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device), early=True)
+            return _gemm_f32_split(x, w, torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device), early)
         if not x.is_contiguous() and x.dim() == 2 and x.stride(1) == 1:
             out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
             gemm_f32_batched(x.unsqueeze(1), w.unsqueeze(0), out.unsqueeze(1))

@@ -73,7 +73,7 @@ class GQAAttention(Mixer):
         s = self.spec
         T = x.shape[0]
         with span("qkv proj"):
-            qkv = ops.linear(x, self.w_qkv)
+            qkv = ops.linear(x, self.w_qkv, early=True)
         o = step.buffer("attn_o", (T, s.n_heads * s.head_dim), self.dtype)
         if step.all_decode and ops.decode_attention_takes_qkv(qkv.dtype, s.n_heads, s.n_kv_heads, s.head_dim):
             table = self.position.rotate_half_table()

@@ -157,7 +157,7 @@ class ProjectedMixer(Mixer):
 
     def forward(self, x, step, cache, state, writes_cache=True, sink=None):
         with span("mixer in proj"):
-            proj = ops.linear(x, self.w_in)
+            proj = ops.linear(x, self.w_in, early=True)
         heads = self.mix(proj, step, cache, state, writes_cache)
         with span("o proj"):
             return ops.linear(heads, self.w_o, sink=sink)

@@ -204,7 +204,7 @@ class BiasedAttention(Mixer):
         s = self.spec
         T = x.shape[0]
         with span("q|k|v|gate proj"):
-            proj = ops.linear(x, self.w_in)
+            proj = ops.linear(x, self.w_in, early=True)
         other = None
         if s.value_source:
             step.carry[self.CARRY_KEY] = proj[:, self.v_off:self.v_off + s.n_kv_heads * s.v_dim]

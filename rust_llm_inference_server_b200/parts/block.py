@@ -275,7 +275,7 @@ class ParallelBlock:
             if sink is not None:
                 sink.exact = True            # the two results were never rounded apart
                 return resid, ops.linear(heads, self.mixer.w_o, sink=sink, second=(act, ff.w_down))
-            return resid, (ops.linear(heads, self.mixer.w_o), ops.linear(act, ff.w_down))
+            return resid, (ops.linear(heads, self.mixer.w_o, early=True), ops.linear(act, ff.w_down, early=True))
 
 
 class _JointInput(Part):
@@ -346,7 +346,7 @@ class StreamJoin(Part):
             x = self._stream(resid, pending, step)
             base = step.carry.get(self.base_key)
             if base is None:
-                base = step.carry[self.base_key] = ops.linear(step.carry[self.EMBEDDED], self.w_0, out_dtype=torch.float32)
+                base = step.carry[self.base_key] = ops.linear(step.carry[self.EMBEDDED], self.w_0, out_dtype=torch.float32, early=True)
             sink = next_block.entry_sink(resid, step) if self.fuses_norms(step) and next_block is not None else None
             if isinstance(sink, ops.ResidualSink):
                 sink.base, sink.exact = base, True

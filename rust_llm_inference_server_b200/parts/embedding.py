@@ -74,7 +74,7 @@ class LMHead(LogitsHead):
 
     def forward(self, h, step):
         with span("lm head"):
-            logits = ops.linear(h, self.weight, out_dtype=torch.float32)
+            logits = ops.linear(h, self.weight, out_dtype=torch.float32, early=True)
             if self.logit_scale is not None or self.soft_cap is not None:
                 ops.logit_transform(logits, self.logit_scale, self.soft_cap)
             return logits

@@ -72,7 +72,7 @@ class SwiGLU(FeedForward):
             # prefill: the tcgen05 product with the gating in its epilogue (the gate|up activations never reach HBM)
             return ops.gemm_tcgen05(x, self.w_gate_up, "swiglu4") if silu \
                 else ops.gemm_tcgen05(x, self.w_gate_up, "glu4", glu=(self.slope, limit, shift, self.cubic), bias=self.b_gate_up)
-        gu = ops.linear(x, self.w_gate_up)
+        gu = ops.linear(x, self.w_gate_up, early=True)
         act = step.buffer("ffn_act", (T, s.intermediate), self.dtype)
         if silu:
             return ops.swiglu(gu, act, self.interleave)
@@ -85,7 +85,7 @@ class SwiGLU(FeedForward):
         with span("mlp down proj"):
             if sink is not None:
                 return ops.linear(act, self.w_down, sink=sink, bias=self.b_down)
-            y = ops.linear(act, self.w_down)
+            y = ops.linear(act, self.w_down, early=True)
             if self.b_down is not None and not defer_bias:
                 y = ops.bias_act(y, self.b_down, step.buffer("ffn_out", tuple(y.shape), self.dtype), "none")
             return y
@@ -123,11 +123,11 @@ class DenseFF(FeedForward):
     def forward(self, x, step, defer_bias: bool = False):
         """With `defer_bias` the caller adds `self.b_down` itself (in float32, while norming)."""
         with span("mlp up proj"):
-            u = ops.linear(x, self.w_up)
+            u = ops.linear(x, self.w_up, early=True)
         with span("bias + activation"):
             act = ops.bias_act(u, self.b_up, step.buffer("ffn_act", tuple(u.shape), self.dtype), self.spec.activation)
         with span("mlp down proj"):
-            y = ops.linear(act, self.w_down)
+            y = ops.linear(act, self.w_down, early=True)
         if self.b_down is not None and not defer_bias:
             y = ops.bias_act(y, self.b_down, step.buffer("ffn_out", tuple(y.shape), self.dtype), "none")
         return y

@@ -116,11 +116,11 @@ class GatedDeltaRule(Mixer):
         s = self.spec
         T = x.shape[0]
         with span("q|k|v|gate|beta|decay proj"):
-            proj = ops.linear(x, self.w_in)
+            proj = ops.linear(x, self.w_in, early=True)
         up = None
         if self.w_up is not None:
             with span("low-rank decay|gate proj"):
-                up = ops.linear(proj[:, :self.low_cols], self.w_up)
+                up = ops.linear(proj[:, :self.low_cols], self.w_up, early=True)
 
         def logits(at, width):
             return (up if at[0] else proj)[:, at[1]:at[1] + width]

@@ -162,7 +162,7 @@ class LatentAttention(ProjectedMixer):
                 ops.act_norm(q, self.q_norm, self.eps, cq)
         if self.q_latent:
             with span("q up proj"):
-                q = ops.linear(cq, self.w_q_up)
+                q = ops.linear(cq, self.w_q_up, early=True)
         return q
 
     def _queries(self, q, z, qa, step, cache, stores) -> None:

@@ -47,7 +47,7 @@ class LightningAttention(Mixer):
         T, H = x.shape[0], s.n_heads
         qk, hv = H * s.dim, H * s.v_dim
         with span("q|k|v|gate proj"):
-            proj = ops.linear(x, self.w_in)
+            proj = ops.linear(x, self.w_in, early=True)
         o = step.buffer("lightning_o", (T, hv), torch.float32)
         with span("decayed recurrence"):
             ops.lightning_scan(proj, 0, qk, 2 * qk, o, state, self.decay, step, H, s.dim, s.v_dim)
@@ -55,7 +55,7 @@ class LightningAttention(Mixer):
         with span("norm * gate"):
             ops.act_norm(o, self.out_norm, self.eps, y, gate=proj[:, 2 * qk + hv:])
         with span("o proj"):
-            return ops.linear(y, self.w_o)
+            return ops.linear(y, self.w_o, early=True)
 
 
 register_mixer("lightning_attention", LightningAttention)

@@ -101,7 +101,7 @@ class Retention(_Recurrence):
         s = self.spec
         T, hv = x.shape[0], s.n_heads * s.v_dim
         with span("q|k|v|gate proj"):
-            proj = ops.linear(x, self.w_in)
+            proj = ops.linear(x, self.w_in, early=True)
         o = self._walk(proj, step, state, self.decay, rotation=self.rotation, positions=step.positions,
                        k_scale=self.k_scale)
         y = step.buffer("recurrence_y", (T, hv), self.dtype)
@@ -153,7 +153,7 @@ class ForgetGateRecurrence(_Recurrence):
         s = self.spec
         T, hv = x.shape[0], s.n_heads * s.v_dim
         with span("q|f|v proj"):
-            proj = ops.linear(x, self.w_in)
+            proj = ops.linear(x, self.w_in, early=True)
         o = self._walk(proj, step, state, None, complement_key=True, q_silu=True, lower=self.lower, gate_bias=self.f_bias)
         y = step.buffer("recurrence_y", (T, hv), self.dtype)
         with span("head norm"):

@@ -66,7 +66,7 @@ class StateSpace(Mixer):
         s = self.spec
         T = x.shape[0]
         with span("z|x|B|C|dt proj"):
-            proj = ops.linear(x, self.w_in)
+            proj = ops.linear(x, self.w_in, early=True)
         o = step.buffer("state_space_o", (T, self.inner), torch.float32)
         with span("conv + state space"):
             ops.state_space(proj, self.inner, self.dt_off, self.conv_w, self.conv_b, self.a_log, self.dt_bias, self.skip, state,

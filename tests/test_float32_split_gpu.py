@@ -77,3 +77,21 @@ def test_the_rule_asks_for_the_matrix_and_the_alignment():
     assert not ops._gemm_f32_splits(odd, w)
     odd.copy_(a)
     assert torch.allclose(ops.gemm_f32(odd, w), ops.gemm_f32(a, w), rtol=0, atol=1e-3)
+
+
+def test_weights_are_read_early_only_where_a_caller_says_so(monkeypatch):
+    """A matrix that a kernel before may still be writing is safe in every product; the parts, whose weights are loaded, say that theirs may be read early."""
+    from rust_llm_inference_server_b200 import ops
+    asked = []
+    real = ops._gemm_f32_split
+    monkeypatch.setattr(ops, "_gemm_f32_split", lambda a, w, out, early=False: (asked.append(early), real(a, w, out, early))[1])
+    a, w = operands(8, 3000, 2048)
+    norm = torch.ones(2048, device="cuda")
+    for _ in range(20):             # rows that are normed just before: a kernel that lets the next one start before it stores
+        made = torch.zeros_like(w)
+        ops.rmsnorm(w, norm, 1e-6, made)
+        got = ops.linear(a, made)
+        torch.cuda.synchronize()
+        assert torch.equal(got, ops.gemm_f32(a, made))
+    assert not any(asked)
+    assert torch.equal(ops.linear(a, w, early=True), ops.gemm_f32(a, w)) and asked.count(True) == 1
