@@ -27,7 +27,7 @@ constexpr int SEG = 256;                    // k of a segment
 // k of a stage, and for it: stages of a segment, bytes of float32 weights, columns of tensor memory that their three planes take
 constexpr int KS = 32, SEG_STAGES = SEG / KS, RAW_BYTES = FT * KS * 4, A_COLS = 3 * KS / 2;             // few rows
 constexpr int KM = 64, SEG_STAGES_M = SEG / KM, RAW_BYTES_M = FT * KM * 4, A_COLS_M = 3 * KM / 2;       // many
-constexpr int MAX_RINGS = 12, MAX_A = 6;    // stages of a ring in shared memory, and of the planes of weights in tensor memory
+constexpr int MAX_RINGS = 4, MAX_A = 4;     // stages of a ring in shared memory, and of the planes of weights in tensor memory
 
 struct Ctrl {
     uint64_t raw_full[MAX_RINGS], raw_empty[MAX_RINGS], b_full[MAX_RINGS], b_empty[MAX_RINGS], a_full[MAX_A], a_empty[MAX_A], acc_full[2], acc_empty[2];
@@ -43,8 +43,8 @@ struct SplitArgs {
     int M, N, K;
     int bn;             // rows of A a tile
     int stages;         // of k in all
-    int raw_ring;       // stages of the ring of float32 weights (few rows: and of float32 rows)
-    int rings;          // stages of the ring of A's planes (many rows)
+    int raw_ring;       // stages of the ring of float32 weights, and of A's planes (many rows)
+    int rings;
     int m_tiles;
     int per;            // segments of a CTA of the cluster (few rows)
     int early;          // the weights may be read before the kernel before has finished
@@ -335,13 +335,13 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
 // N 32000 47 / 81 (5.6 TB/s); K 8192 N 2048 22 / 37.  A tile of 128 features a cluster, whose CTAs take whole segments of k and leave their
 // sums in shared memory; the cluster then adds them up in the order of k, each CTA for a share of the features.  The rows of A are split
 // where the weights are.  Fourteen warps: 0-3 read the accumulators, 4-11 split (two sets), 12 asks for weights and rows, 13 issues the products.
-constexpr int FEW_THREADS = 448, FEW_A = 4;
+constexpr int FEW_THREADS = 448, FEW_RING = 4, FEW_A = 4;     // (a ring of an even number of stages, as above)
 
 template <int BN> struct Few {
     static constexpr int ROWS_BYTES = BN * KS * 4, STAGE = RAW_BYTES + ROWS_BYTES, PLANES = 3 * BN * KS * 2, ROW = FT * 4;
     static constexpr int ACC = BN == 16 ? 2 : 1;                // accumulators: of two segments where there is room for them
     static_assert(ACC * 2 * BN + FEW_A * A_COLS <= 256, "two CTAs an SM share its tensor memory");
-    static constexpr int smem(int rings, int rows) { return 1024 + rings * STAGE + FEW_A * PLANES + rows * ROW + (int)sizeof(Ctrl); }
+    static constexpr int smem(int rows) { return 1024 + FEW_RING * STAGE + FEW_A * PLANES + rows * ROW + (int)sizeof(Ctrl); }
 };
 
 template <int BN>
@@ -351,7 +351,7 @@ __global__ __launch_bounds__(FEW_THREADS, 2) void f32_split_few_kernel(const __g
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* ring = base;                                             // weights, then rows
-    unsigned char* planes = base + p.raw_ring * F::STAGE;
+    unsigned char* planes = base + FEW_RING * F::STAGE;
     float* sums = reinterpret_cast<float*>(planes + FEW_A * F::PLANES);     // [segment of this CTA][row][feature]
     Ctrl* ctrl = reinterpret_cast<Ctrl*>(reinterpret_cast<unsigned char*>(sums) + (parts == 1 ? 1 : p.per) * p.M * F::ROW);
     const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -389,7 +389,7 @@ __global__ __launch_bounds__(FEW_THREADS, 2) void f32_split_few_kernel(const __g
         if (lane == 0) {
             // weights that no kernel of a step writes are asked for before the wait; the rows after it
             if (!p.early) pdl_wait();
-            const int early = min(stages, p.raw_ring);
+            const int early = min(stages, FEW_RING);
             for (int it = 0; it < early; ++it) {
                 bar_expect_tx(&ctrl->raw_full[it], F::STAGE);
                 tma_load_2d(ring + it * F::STAGE, &map_w, (st0 + it) * KS, f0, &ctrl->raw_full[it]);
@@ -402,7 +402,7 @@ __global__ __launch_bounds__(FEW_THREADS, 2) void f32_split_few_kernel(const __g
                 bar_expect_tx(&ctrl->raw_full[s], F::STAGE);
                 tma_load_2d(dst, &map_w, (st0 + it) * KS, f0, &ctrl->raw_full[s]);
                 tma_load_2d(dst + RAW_BYTES, &map_a, (st0 + it) * KS, 0, &ctrl->raw_full[s]);
-                if (++s == p.raw_ring) { s = 0; ++turn; }
+                if (++s == FEW_RING) { s = 0; ++turn; }
             }
             pdl_trigger();
         }
@@ -438,7 +438,7 @@ __global__ __launch_bounds__(FEW_THREADS, 2) void f32_split_few_kernel(const __g
                 bar_arrive(&ctrl->raw_empty[s]);
             }
             s += 2;
-            if (s >= p.raw_ring) { s -= p.raw_ring; ++turn; }
+            if (s >= FEW_RING) { s -= FEW_RING; ++turn; }
         }
     } else {
         // the rows' planes, stage by stage, and behind each segment its sums
@@ -496,7 +496,7 @@ __global__ __launch_bounds__(FEW_THREADS, 2) void f32_split_few_kernel(const __g
                 bar_arrive(&ctrl->a_full[a]);
                 bar_arrive(&ctrl->raw_empty[s]);
             }
-            if (++s == p.raw_ring) { s = 0; ++turn; }
+            if (++s == FEW_RING) { s = 0; ++turn; }
         }
         while (fine && taken < mine) fine = take(taken++);
     }
@@ -559,7 +559,7 @@ int sm_count() {
     return sms;
 }
 
-constexpr int FEW_ROWS = 32, MAX_PARTS = 12;
+constexpr int FEW_ROWS = 32, MAX_PARTS = 12, SMEM_MOST = 227 * 1024;
 int g_bn = 0, g_parts = 0;      // held fixed by a measurement (0: automatic)
 
 template <int BN> int launch_few(SplitArgs p, cudaStream_t stream) {
@@ -572,18 +572,16 @@ template <int BN> int launch_few(SplitArgs p, cudaStream_t stream) {
     long long best = -1;
     for (int c = 1; c <= MAX_PARTS && c <= segs; ++c) {
         const int per = (segs + c - 1) / c;
-        if (c > 1 && F::smem(4, per * p.M) > 227 * 1024) continue;
+        if (c > 1 && F::smem(per * p.M) > SMEM_MOST) continue;
         const long long ctas = (long long)tiles * c;
         const long long cost = (ctas <= sms ? 7400LL : 9600LL) * per + (c > 1 ? 5000 : 2500), total = (ctas + 2 * sms - 1) / (2 * sms) * cost;
         if (best < 0 || total < best) { best = total; parts = c; }
     }
-    if (g_parts > 0 && g_parts <= segs && F::smem(4, (segs + g_parts - 1) / g_parts * p.M) <= 227 * 1024) parts = g_parts;
+    if (g_parts > 0 && g_parts <= segs && F::smem((g_parts == 1 ? 1 : (segs + g_parts - 1) / g_parts) * p.M) <= SMEM_MOST) parts = g_parts;
     p.per = (segs + parts - 1) / parts;
-    const int rows = (parts == 1 ? 1 : p.per) * p.M;
-    p.raw_ring = F::smem(6, rows) <= 113 * 1024 ? 6 : 4;       // (even, see above; room for a second CTA on the SM, of this product or of the kernel after it)
     CUtensorMap map_w, map_a;
     if (!map_f32(&map_w, p.W, p.N, p.K, p.ldw, FT) || !map_f32(&map_a, p.A, p.M, p.K, p.lda, BN)) return RLIS_ERR_UNSUPPORTED;
-    const int smem = F::smem(p.raw_ring, rows);
+    const int smem = F::smem((parts == 1 ? 1 : p.per) * p.M);
     cudaError_t e = cudaFuncSetAttribute(f32_split_few_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess && parts > 8) e = cudaFuncSetAttribute(f32_split_few_kernel<BN>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return (int)e;

@@ -20,7 +20,7 @@ def product(a, w):
 
 
 # rows at the ends of the kernels of few rows (16, 32) and of many, whose tiles have 16 to 160 rows in halves that are multiples of 16; features that end inside a
-# tile of 128; k that ends with, inside and one float4 into a stage of 32 or 64 and a segment of 256; k cut over 1 to 8 CTAs
+# tile of 128; k that ends with, inside and one float4 into a stage of 32 or 64 and a segment of 256; k cut over 1 to 12 CTAs
 @pytest.mark.parametrize("M,N,K", [(1, 128, 2048), (3, 40, 2052), (8, 2048, 2048), (8, 20000, 2304), (16, 300, 8192), (17, 129, 2300), (31, 3000, 4096), (32, 16400, 2052),
                                    (33, 128, 2048), (50, 2048, 2084), (97, 300, 2560), (180, 2900, 2048), (193, 9500, 2052), (700, 2048, 2336), (800, 19000, 2048)])
 def test_products_of_long_rows(M, N, K):
@@ -95,3 +95,34 @@ def test_weights_are_read_early_only_where_a_caller_says_so(monkeypatch):
         assert torch.equal(got, ops.gemm_f32(a, made))
     assert not any(asked)
     assert torch.equal(ops.linear(a, w, early=True), ops.gemm_f32(a, w)) and asked.count(True) == 1
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 300, 4100), (16, 200, 8192), (17, 300, 2052), (32, 500, 3072)])
+def test_every_cut_of_k_has_the_same_bits(M, N, K):
+    """k over 1 to 12 CTAs, as many as there are segments and shared memory has room for."""
+    from rust_llm_inference_server_b200 import ops
+    from rust_llm_inference_server_b200.ops.library import debug_set
+    a, w = operands(M, N, K)
+    want = product(a, w)
+    try:
+        for parts in range(1, 13):
+            debug_set("f32_split_parts", parts)
+            assert torch.equal(product(a, w), want), parts
+    finally:
+        debug_set("f32_split_parts", 0)
+    ops.check_device_errors()
+
+
+@pytest.mark.parametrize("M,N,K", [(33, 300, 2048), (170, 200, 4100)])
+def test_every_height_of_a_tile_has_the_same_bits(M, N, K):
+    from rust_llm_inference_server_b200 import ops
+    from rust_llm_inference_server_b200.ops.library import debug_set
+    a, w = operands(M, N, K)
+    want = product(a, w)
+    try:
+        for rows in range(16, 161, 16):
+            debug_set("f32_split_rows", rows)
+            assert torch.equal(product(a, w), want), rows
+    finally:
+        debug_set("f32_split_rows", 0)
+    ops.check_device_errors()
