@@ -18,6 +18,8 @@
 // Role in the reference: `x.matmul(w.t())`, crates/model/src/layers.rs:82.
 #include "tcgen05_utils.cuh"
 #include <float.h>
+#include <math.h>
+#include <mutex>
 
 namespace {
 using namespace tc;
@@ -345,7 +347,8 @@ template <int BN> struct Few {
 };
 
 template <int BN>
-__global__ __launch_bounds__(FEW_THREADS, 2) void f32_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
+// (16 warps, to which 14 are rounded up, of two CTAs an SM have 64 registers a thread; 32 rows leave no room for a second one)
+__global__ __launch_bounds__(BN == 16 ? 512 : FEW_THREADS, BN == 16 ? 2 : 1) void f32_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                                                                        const SplitArgs p, int parts) {
     using F = Few<BN>;
     extern __shared__ unsigned char smem_raw[];
@@ -559,32 +562,74 @@ int sm_count() {
     return sms;
 }
 
-constexpr int FEW_ROWS = 32, MAX_PARTS = 12, SMEM_MOST = 227 * 1024;
+constexpr int FEW_ROWS = 32, MAX_PARTS = 12, SMEM_MOST = 227 * 1024, SMEM_HALF = 112 * 1024, MAX_DEVICES = 64;     // (with half, two CTAs an SM)
 int g_bn = 0, g_parts = 0;      // held fixed by a measurement (0: automatic)
+
+// What is set for the kernels of few rows once a device, and the clusters of 1 .. MAX_PARTS CTAs that are resident at a time with one CTA an SM and with two.
+// (The runtime counts one CTA an SM for a kernel that allocates tensor memory.  Of the places of two, clusters of three and more fill 95 %, of nine and more
+// 85 %: with 148 SMs 48 clusters of 6 take two rounds and 32 of 8 one, 24 of 11 two and 24 of 10 one.)
+struct FewPlan {
+    std::once_flag once;
+    cudaError_t error = cudaSuccess;
+    int clusters[2][MAX_PARTS + 1] = {};
+};
+template <int BN> const FewPlan* few_plan() {
+    static FewPlan plans[MAX_DEVICES];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= MAX_DEVICES) return nullptr;
+    FewPlan& plan = plans[dev];
+    std::call_once(plan.once, [&] {
+        plan.error = cudaFuncSetAttribute(f32_split_few_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST);
+        if (plan.error == cudaSuccess) plan.error = cudaFuncSetAttribute(f32_split_few_kernel<BN>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        for (int parts = 1; parts <= MAX_PARTS && plan.error == cudaSuccess; ++parts) {
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = parts;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(parts);
+            cfg.blockDim = dim3(FEW_THREADS);
+            cfg.dynamicSmemBytes = SMEM_MOST;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            plan.error = cudaOccupancyMaxActiveClusters(&plan.clusters[0][parts], f32_split_few_kernel<BN>, &cfg);
+            plan.clusters[1][parts] = 2 * sm_count() * (parts > 8 ? 85 : parts > 2 ? 95 : 100) / (100 * parts);
+        }
+    });
+    return &plan;
+}
+
+// CTAs a tile, from what one takes, in ns: a segment 2,850 and 45 a row alone on its SM (with 32 rows a tile 3,500 and 35), 4,200 and 85 beside another, both
+// more with the CTAs that share the memory, and 2,100 or, with others of its cluster, 3,200 beside its segments.  A cluster has to fit into a GPC, so fewer CTAs
+// than there are places may already be too many for one round.  us with 1, 2, 4, 6 and 8 CTAs a tile, 8 rows: N 16384 K 2048 34, 30, 35, 45, 41; N 32000 51, 58,
+// 65, 85, 77; N 3072 28, 17, 12, 14, 10; N 2048 K 8192 103, 56, 31, 27, 26, with 11 22; N 6144 K 4096 55, 34, 28, 35, 32.  32 rows: N 3072 K 3072 56, 34, 21, 33, 31.
+template <int BN> int choose_parts(const FewPlan& plan, int tiles, int segs, int M) {
+    int parts = 1;
+    double least = -1;
+    for (int c = 1; c <= MAX_PARTS && c <= segs; ++c) {
+        const int per = (segs + c - 1) / c, bytes = Few<BN>::smem((c == 1 ? 1 : per) * M);
+        if (bytes > SMEM_MOST || plan.clusters[0][c] <= 0) continue;
+        const bool two = bytes <= SMEM_HALF && tiles > plan.clusters[0][c];
+        const double rounds = (double)tiles / plan.clusters[two][c], ctas = (double)c * (rounds < 1 ? tiles : plan.clusters[two][c]);
+        const double segment = two ? 4200 + 85 * M + 8 * ctas : BN == 16 ? 2850 + 45 * M + 8.5 * ctas : 3500 + 35 * M + 5 * ctas;
+        const double t = (rounds <= 3 ? ceil(rounds) : rounds + (two ? 0.4 : 0.6)) * (per * segment + (c > 1 ? 3200 : 2100));
+        if (least < 0 || t < least) { least = t; parts = c; }
+    }
+    return parts;
+}
 
 template <int BN> int launch_few(SplitArgs p, cudaStream_t stream) {
     using F = Few<BN>;
-    const int sms = sm_count(), tiles = (p.N + FT - 1) / FT, segs = (p.stages + SEG_STAGES - 1) / SEG_STAGES;
-    // CTAs a tile: by what a segment takes a CTA alone on its SM (about 7,400 cycles) and beside another (9,600), and by what a CTA takes beside its segments.
-    // 8 rows, us with 1, 2, 4 and 8 CTAs a tile: N 16384 K 2048 33, 29, 32, 39; N 32000 48, 55, 61, 72; N 3072 27, 16, 11, 9.5; N 2048 K 8192 105, 57, 31, 25,
-    // with 12 22 and with 16, which half a GPC has to hold, 28.
-    int parts = 1;
-    long long best = -1;
-    for (int c = 1; c <= MAX_PARTS && c <= segs; ++c) {
-        const int per = (segs + c - 1) / c;
-        if (c > 1 && F::smem(per * p.M) > SMEM_MOST) continue;
-        const long long ctas = (long long)tiles * c;
-        const long long cost = (ctas <= sms ? 7400LL : 9600LL) * per + (c > 1 ? 5000 : 2500), total = (ctas + 2 * sms - 1) / (2 * sms) * cost;
-        if (best < 0 || total < best) { best = total; parts = c; }
-    }
+    const FewPlan* plan = few_plan<BN>();
+    if (plan == nullptr) return RLIS_ERR_UNSUPPORTED;
+    if (plan->error != cudaSuccess) return (int)plan->error;
+    const int tiles = (p.N + FT - 1) / FT, segs = (p.stages + SEG_STAGES - 1) / SEG_STAGES;
+    int parts = choose_parts<BN>(*plan, tiles, segs, p.M);
     if (g_parts > 0 && g_parts <= segs && F::smem((g_parts == 1 ? 1 : (segs + g_parts - 1) / g_parts) * p.M) <= SMEM_MOST) parts = g_parts;
     p.per = (segs + parts - 1) / parts;
     CUtensorMap map_w, map_a;
     if (!map_f32(&map_w, p.W, p.N, p.K, p.ldw, FT) || !map_f32(&map_a, p.A, p.M, p.K, p.lda, BN)) return RLIS_ERR_UNSUPPORTED;
     const int smem = F::smem((parts == 1 ? 1 : p.per) * p.M);
-    cudaError_t e = cudaFuncSetAttribute(f32_split_few_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess && parts > 8) e = cudaFuncSetAttribute(f32_split_few_kernel<BN>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return (int)e;
     rlis_launch_cluster(f32_split_few_kernel<BN>, dim3((unsigned)(tiles * parts)), dim3(FEW_THREADS), (size_t)smem, stream, dim3((unsigned)parts, 1, 1), map_w, map_a, p, parts);
     return RLIS_LAUNCH_CHECK();
 }
