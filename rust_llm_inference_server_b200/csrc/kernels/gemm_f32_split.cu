@@ -7,8 +7,10 @@
 //     C = ((s0 + s1) + s2) + ..,   s = (w1 x1) + (w3 x1 + w2 x2 + w1 x3 + w2 x1 + w1 x2)
 // Off float64 by 2.5e-7 of the result at K 2048 and 8192 (normal numbers), where one chain of K FMAs is 8e-7 and 1.6e-6.  The segments and the order in
 // them are the same in both kernels below and for any number of rows, so a row's result does not depend on what else is in the batch.
-// A result that is not finite is worked out again as a chain of FMAs from the float32 operands: infinities and NaN, and numbers that
-// round to infinity in 8 bits, come out as that chain gives them.
+// The sum of three is exact from 2^-110 up only (2^-102 where subnormal operands count as zeros): below that the third part has bits under the smallest
+// bf16.  So the largest magnitude of every row of A and of W is taken along, and an output that what is lost could reach, that is, one below
+// K (x_max + w_max + 8) 2^-100, is worked out again as a chain of FMAs from the float32 operands; so is one that is not finite (infinities and NaN, and
+// numbers that round to infinity in 8 bits, come out as that chain gives them).
 //
 // W is the M side of the instruction (128 features a tile), split on the way: TMA brings 128 x 32 floats, warps turn a row of 32 into three
 // planes of bf16 and put them into tensor memory as the A operand.  The rows of A are the N side, from shared memory in three planes.
@@ -18,6 +20,7 @@
 // Role in the reference: `x.matmul(w.t())`, crates/model/src/layers.rs:82.
 #include "tcgen05_utils.cuh"
 #include <float.h>
+#include <stddef.h>
 #include <math.h>
 #include <mutex>
 
@@ -35,7 +38,11 @@ struct Ctrl {
     uint64_t raw_full[MAX_RINGS], raw_empty[MAX_RINGS], b_full[MAX_RINGS], b_empty[MAX_RINGS], a_full[MAX_A], a_empty[MAX_A], acc_full[2], acc_empty[2];
     uint32_t tmem_base;
     int abort;
+    uint32_t most;                  // magnitudes, as bits of bf16: the largest of the CTA's operands (few rows: rows and weights; many: weights),
+    uint16_t w_most[2][FT];         // of each row of weights, by the two sets of splitting warps,
+    uint16_t x_most[32];            // and of each row of A (few rows)
 };
+static_assert(offsetof(Ctrl, w_most) % 4 == 0 && offsetof(Ctrl, x_most) % 4 == 0, "two magnitudes to a word");
 
 struct SplitArgs {
     const float* A;
@@ -50,6 +57,9 @@ struct SplitArgs {
     int m_tiles;
     int per;            // segments of a CTA of the cluster (few rows)
     int early;          // the weights may be read before the kernel before has finished
+    float lost;         // K 2^-100
+    const float* x_most;    // the largest magnitude of every row of A, by pieces of ROW_PIECE (many rows)
+    int pieces;
 };
 
 // Two floats as three pairs of bf16 whose sum they are, low half first.
@@ -62,6 +72,14 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& p1, uint32_t&
     b -= __uint_as_float(p2 & 0xffff0000u);
     p3 = pack_bf16(a, b);
 }
+// The larger magnitudes of two pairs of bf16, half by half, whatever their signs (a NaN counts as nothing); the larger one of a pair; its value.
+__device__ __forceinline__ uint32_t larger2(uint32_t most, uint32_t p) {
+    uint32_t d;
+    asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(most), "r"(p));
+    return d;
+}
+__device__ __forceinline__ uint32_t larger_half(uint32_t most) { return max(most & 0x7fffu, most >> 16 & 0x7fffu); }
+__device__ __forceinline__ float magnitude(uint32_t bits) { return __uint_as_float(bits << 16); }
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
                  "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
@@ -111,7 +129,8 @@ template <int KT> __device__ __forceinline__ void stage_products(uint32_t main, 
 }
 
 // One row of KT float32 weights (boxes of 32: 128 bytes, 128-byte swizzle) into its three planes in tensor memory.
-template <int KT> __device__ __forceinline__ void split_weights(const unsigned char* raw, int row, uint32_t taddr) {
+// (`most`: the largest magnitudes so far.)
+template <int KT> __device__ __forceinline__ void split_weights(const unsigned char* raw, int row, uint32_t taddr, uint32_t& most) {
 #pragma unroll
     for (int kk = 0; kk < KT / 16; ++kk) {
         const unsigned char* src = raw + kk / 2 * (FT * 32 * 4) + row * (32 * 4);
@@ -121,6 +140,7 @@ template <int KT> __device__ __forceinline__ void split_weights(const unsigned c
             const float4 v = *reinterpret_cast<const float4*>(src + (((kk % 2 * 4 + c) ^ (row & 7)) << 4));
             split2(v.x, v.y, p1[2 * c], p2[2 * c], p3[2 * c]);
             split2(v.z, v.w, p1[2 * c + 1], p2[2 * c + 1], p3[2 * c + 1]);
+            most = larger2(larger2(most, p1[2 * c]), p1[2 * c + 1]);
         }
         tmem_st8(taddr + kk * 8, p1);
         tmem_st8(taddr + KT / 2 + kk * 8, p2);
@@ -129,40 +149,70 @@ template <int KT> __device__ __forceinline__ void split_weights(const unsigned c
     tmem_st_wait();
 }
 
-// An output that did not come out finite, as a chain of FMAs.
-__device__ __noinline__ float chain(const float* __restrict__ a, const float* __restrict__ w, int K) {
+// The magnitude of a row whose numbers are all zeros as bf16: zero, or the smallest one if some of them are not zero.
+__device__ __noinline__ float magnitude_below(const float* __restrict__ row, int K) {
+    uint32_t bits = 0;
+    int k = 0;
+    for (; k + 3 < K; k += 4) {
+        const uint4 v = *reinterpret_cast<const uint4*>(row + k);
+        bits |= v.x | v.y | v.z | v.w;
+    }
+    for (; k < K; ++k) bits |= __float_as_uint(row[k]);
+    return bits << 1 ? magnitude(1) : 0.f;
+}
+// An output that is not finite, or so small that the parts' sums may have lost some of it, as a chain of FMAs (`x`, `w`: the largest magnitudes of
+// the two rows, whatever else the tile holds).
+__device__ __noinline__ float chain(const float* __restrict__ a, const float* __restrict__ b, int K, float v, float x, float w, float lost) {
+    if (fabsf(v) <= FLT_MAX && (x == 0.f || w == 0.f || fabsf(v) >= lost * (x + w + 8.f))) return v;
     float acc = 0.f;
-    for (int k = 0; k < K; ++k) acc = fmaf(a[k], w[k], acc);
+    for (int k = 0; k < K; ++k) acc = fmaf(a[k], b[k], acc);
     return acc;
 }
-__device__ __forceinline__ void store(const SplitArgs& p, int m, int n, float v) {
-    if (!(fabsf(v) <= FLT_MAX)) v = chain(p.A + (size_t)m * p.lda, p.W + (size_t)n * p.ldw, p.K);
-    p.C[(size_t)m * p.ldc + n] = v;
-}
+// Whether an output is one that `chain` has to look at; `least`: what its rows' magnitudes come to at the most.
+__device__ __forceinline__ bool doubtful(float v, float least) { return !(fabsf(v) <= FLT_MAX && fabsf(v) >= least); }
 
-// The rows of A in three planes: planes[p][m][0 .. pitch), zeros beyond K.
-__global__ __launch_bounds__(256) void split_rows_kernel(const float* __restrict__ A, long long lda, bf16* __restrict__ planes, int M, int K, int pitch) {
+// The rows of A in three planes, planes[p][m][0 .. pitch), zeros beyond K, and the largest magnitude of each piece of a row.  A piece a warp, eight
+// loads in flight a lane.
+constexpr int ROW_PIECE = 1024;
+__global__ __launch_bounds__(256) void split_rows_kernel(const float* __restrict__ A, long long lda, bf16* __restrict__ planes, float* __restrict__ most, int M, int K,
+                                                         int pitch, int pieces) {
     pdl_wait_and_trigger();
-    const int per_row = pitch / 4, vec = ((reinterpret_cast<uintptr_t>(A) & 15) == 0 && lda % 4 == 0);
-    const size_t plane = (size_t)M * pitch;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < (size_t)M * per_row; i += (size_t)gridDim.x * blockDim.x) {
-        const int m = (int)(i / per_row), k = (int)(i % per_row) * 4;
-        const float* src = A + (size_t)m * lda + k;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (vec && k + 3 < K) v = *reinterpret_cast<const float4*>(src);
-        else {
-            if (k < K) v.x = src[0];
-            if (k + 1 < K) v.y = src[1];
-            if (k + 2 < K) v.z = src[2];
-            if (k + 3 < K) v.w = src[3];
+    const size_t plane = (size_t)M * pitch, units = (size_t)M * pieces;
+    const int lane = threadIdx.x & 31;
+    for (size_t u = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); u < units; u += (size_t)gridDim.x * 8) {
+        const size_t m = u / pieces;
+        const int k0 = (int)(u % pieces) * ROW_PIECE + lane * 4;
+        const float* src = A + m * lda;
+        bf16* dst = planes + m * pitch;
+        float4 v[ROW_PIECE / 128];
+#pragma unroll
+        for (int i = 0; i < ROW_PIECE / 128; ++i) {
+            const int k = k0 + i * 128;
+            v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k + 3 < K) v[i] = *reinterpret_cast<const float4*>(src + k);
+            else {
+                if (k < K) v[i].x = src[k];
+                if (k + 1 < K) v[i].y = src[k + 1];
+                if (k + 2 < K) v[i].z = src[k + 2];
+            }
         }
-        uint2 p1, p2, p3;
-        split2(v.x, v.y, p1.x, p2.x, p3.x);
-        split2(v.z, v.w, p1.y, p2.y, p3.y);
-        bf16* dst = planes + (size_t)m * pitch + k;
-        *reinterpret_cast<uint2*>(dst) = p1;
-        *reinterpret_cast<uint2*>(dst + plane) = p2;
-        *reinterpret_cast<uint2*>(dst + 2 * plane) = p3;
+        uint32_t largest = 0, any = 0;
+#pragma unroll
+        for (int i = 0; i < ROW_PIECE / 128; ++i) {
+            const int k = k0 + i * 128;
+            uint2 p1, p2, p3;
+            split2(v[i].x, v[i].y, p1.x, p2.x, p3.x);
+            split2(v[i].z, v[i].w, p1.y, p2.y, p3.y);
+            largest = larger2(larger2(largest, p1.x), p1.y);
+            any |= __float_as_uint(v[i].x) | __float_as_uint(v[i].y) | __float_as_uint(v[i].z) | __float_as_uint(v[i].w);
+            if (k < pitch) {
+                *reinterpret_cast<uint2*>(dst + k) = p1;
+                *reinterpret_cast<uint2*>(dst + plane + k) = p2;
+                *reinterpret_cast<uint2*>(dst + 2 * plane + k) = p3;
+            }
+        }
+        largest = __reduce_max_sync(0xffffffffu, max(larger_half(largest), any << 1 ? 1u : 0u));
+        if (lane == 0) most[u] = magnitude(largest);
     }
 }
 
@@ -180,8 +230,14 @@ constexpr int MANY_RING_BYTES = 225 * 1024;         // both rings
 constexpr int MANY_SMEM = 1024 + MANY_RING_BYTES + (int)sizeof(Ctrl);
 static_assert(MANY_SMEM <= 227 * 1024, "shared memory");
 
+__device__ __noinline__ float settle_many(const SplitArgs& p, int m, int n, float v, float w) {
+    float x = 0.f;
+    for (int i = 0; i < p.pieces; ++i) x = fmaxf(x, p.x_most[(size_t)m * p.pieces + i]);
+    return chain(p.A + (size_t)m * p.lda, p.W + (size_t)n * p.ldw, p.K, v, x, w, p.lost);
+}
+
 __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
-                                                                         const SplitArgs p) {
+                                                                         const __grid_constant__ SplitArgs p) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* raw = base;
@@ -195,6 +251,7 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
 
     if (threadIdx.x == 0) {
         ctrl->abort = 0;
+        ctrl->most = 0;
         for (int i = 0; i < MAX_RINGS; ++i) {
             bar_init(&ctrl->raw_full[i], 1);
             bar_init(&ctrl->raw_empty[i], 4);
@@ -269,12 +326,12 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
         const int set = (warp - 8) / 4, row = (warp & 3) * 32 + lane;
         const uint32_t taddr = a_base + ((uint32_t)((warp & 3) * 32) << 16);
         int s = set, a = set, b = set % p.rings;
-        uint32_t turn = 0, a_turn = 0, b_turn = set / p.rings;
+        uint32_t turn = 0, a_turn = 0, b_turn = set / p.rings, most = 0;
         for (int it = set; it < p.stages; it += 2) {
             if (!bar_wait_warp(&ctrl->raw_full[s], turn & 1, &ctrl->abort)) break;
             if (a_turn > 0 && !bar_wait_warp(&ctrl->a_empty[a], (a_turn - 1) & 1, &ctrl->abort)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            split_weights<KM>(raw + s * RAW_BYTES_M, row, taddr + (uint32_t)(a * A_COLS_M));
+            split_weights<KM>(raw + s * RAW_BYTES_M, row, taddr + (uint32_t)(a * A_COLS_M), most);
             if (!bar_wait_warp(&ctrl->b_full[b], b_turn & 1, &ctrl->abort)) break;
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -289,13 +346,22 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
             b += 2;
             if (b >= p.rings) { b -= p.rings; ++b_turn; }
         }
+        most = larger_half(most);
+        ctrl->w_most[set][row] = (uint16_t)most;
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0) atomicMax(&ctrl->most, most);
+        asm volatile("bar.arrive 1, 512;" ::: "memory");
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
         const int h = warp >> 2, q = warp & 3, cols = h ? n1 : n0, segs = cols == 0 ? 0 : (p.stages + SEG_STAGES_M - 1) / SEG_STAGES_M;
         const uint32_t main = tmem + (uint32_t)(h * 2 * n0) + ((uint32_t)(q * 32) << 16);
-        float sum[HALF];
+        const int m1 = m0 + h * n0;
+        float sum[HALF], x = 0.f;
 #pragma unroll
         for (int c = 0; c < HALF; ++c) sum[c] = 0.f;
+        pdl_wait();         // (C may still be read by the kernel before, too)
+        for (int i = m1 * p.pieces + lane; i < min(m1 + cols, p.M) * p.pieces; i += 32) x = fmaxf(x, p.x_most[i]);
+        x = warp_max(x);
         for (int seg = 0; seg < segs; ++seg) {
             if (!bar_wait_warp(&ctrl->acc_full[h], seg & 1, &ctrl->abort)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -314,12 +380,18 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
             __syncwarp();
             if (lane == 0) bar_arrive(&ctrl->acc_empty[h]);
         }
-        const int n = f0 + q * 32 + lane, m1 = m0 + h * n0;
-        pdl_wait();         // (C may still be read by the kernel before, whose end the producers alone have waited for)
+        const int n = f0 + q * 32 + lane;
+        asm volatile("bar.sync 1, 512;" ::: "memory");        // the weights' magnitudes are there
+        const float least = p.lost * (x + magnitude(ctrl->most) + 8.f);
         if (n < p.N && !ctrl->abort) {
+            float w = magnitude(max(ctrl->w_most[0][q * 32 + lane], ctrl->w_most[1][q * 32 + lane]));
+            if (w == 0.f) w = magnitude_below(p.W + (size_t)n * p.ldw, p.K);
 #pragma unroll
             for (int c = 0; c < HALF; ++c)
-                if (c < cols && m1 + c < p.M) store(p, m1 + c, n, sum[c]);
+                if (c < cols && m1 + c < p.M) {
+                    const int m = m1 + c;
+                    p.C[(size_t)m * p.ldc + n] = doubtful(sum[c], least) ? settle_many(p, m, n, sum[c], w) : sum[c];
+                }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -346,10 +418,22 @@ template <int BN> struct Few {
     static constexpr int smem(int rows) { return 1024 + FEW_RING * STAGE + FEW_A * PLANES + rows * ROW + (int)sizeof(Ctrl); }
 };
 
+// (the rows' magnitudes in the cluster's CTAs, which have a part of k each)
+__device__ __noinline__ float settle_few(const SplitArgs& p, Ctrl* ctrl, int parts, int m, int f, int n, float v) {
+    uint32_t x = 0, w = 0;
+    auto take = [](uint16_t* at, int i, uint32_t part) { return __float_as_uint(ld_dsmem(reinterpret_cast<float*>(at + (i & ~1)), part)) >> (i & 1) * 16 & 0xffffu; };
+    for (int part = 0; part < parts; ++part) {
+        x = max(x, take(ctrl->x_most, m, (uint32_t)part));
+        w = max(w, max(take(ctrl->w_most[0], f, (uint32_t)part), take(ctrl->w_most[1], f, (uint32_t)part)));
+    }
+    const float *a = p.A + (size_t)m * p.lda, *b = p.W + (size_t)n * p.ldw;
+    return chain(a, b, p.K, v, x ? magnitude(x) : magnitude_below(a, p.K), w ? magnitude(w) : magnitude_below(b, p.K), p.lost);
+}
+
 template <int BN>
 // (16 warps, to which 14 are rounded up, of two CTAs an SM have 64 registers a thread; 32 rows leave no room for a second one)
 __global__ __launch_bounds__(BN == 16 ? 512 : FEW_THREADS, BN == 16 ? 2 : 1) void f32_split_few_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
-                                                                       const SplitArgs p, int parts) {
+                                                                       const __grid_constant__ SplitArgs p, int parts) {
     using F = Few<BN>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -365,6 +449,7 @@ __global__ __launch_bounds__(BN == 16 ? 512 : FEW_THREADS, BN == 16 ? 2 : 1) voi
 
     if (threadIdx.x == 0) {
         ctrl->abort = 0;
+        ctrl->most = 0;
         for (int i = 0; i < MAX_RINGS; ++i) {
             bar_init(&ctrl->raw_full[i], 1);
             bar_init(&ctrl->raw_empty[i], 8);
@@ -428,12 +513,13 @@ __global__ __launch_bounds__(BN == 16 ? 512 : FEW_THREADS, BN == 16 ? 2 : 1) voi
         const int set = (warp - 4) / 4, row = (warp & 3) * 32 + lane;
         const uint32_t taddr = a_base + ((uint32_t)((warp & 3) * 32) << 16);
         int s = set, turn = 0;
+        uint32_t most = 0;
         for (int it = set; it < stages; it += 2) {
             const int a = it % FEW_A;
             if (!bar_wait_warp(&ctrl->raw_full[s], turn & 1, &ctrl->abort)) break;
             if (it >= FEW_A && !bar_wait_warp(&ctrl->a_empty[a], (it / FEW_A - 1) & 1, &ctrl->abort)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            split_weights<KS>(ring + s * F::STAGE, row, taddr + (uint32_t)(a * A_COLS));
+            split_weights<KS>(ring + s * F::STAGE, row, taddr + (uint32_t)(a * A_COLS), most);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) {
@@ -443,6 +529,10 @@ __global__ __launch_bounds__(BN == 16 ? 512 : FEW_THREADS, BN == 16 ? 2 : 1) voi
             s += 2;
             if (s >= FEW_RING) { s -= FEW_RING; ++turn; }
         }
+        most = larger_half(most);
+        ctrl->w_most[set][row] = (uint16_t)most;
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0) atomicMax(&ctrl->most, most);
     } else {
         // the rows' planes, stage by stage, and behind each segment its sums
         const int f = threadIdx.x;
@@ -473,6 +563,7 @@ __global__ __launch_bounds__(BN == 16 ? 512 : FEW_THREADS, BN == 16 ? 2 : 1) voi
         };
         int s = 0, turn = 0, taken = 0;
         bool fine = true;
+        uint32_t most[BN / 16] = {};
         for (int it = 0; it < stages; ++it) {
             const int a = it % FEW_A;
             // a segment's sums are due before the products that wait for their accumulator, and not before its last products are on their way
@@ -488,6 +579,7 @@ __global__ __launch_bounds__(BN == 16 ? 512 : FEW_THREADS, BN == 16 ? 2 : 1) voi
                 uint2 p1, p2, p3;
                 split2(v.x, v.y, p1.x, p2.x, p3.x);
                 split2(v.z, v.w, p1.y, p2.y, p3.y);
+                most[i] = larger2(larger2(most[i], p1.x), p1.y);
                 unsigned char* d = dst + r * (KS * 2) + (((c >> 1) ^ ((r >> 1) & 3)) << 4) + (c & 1) * 8;
                 *reinterpret_cast<uint2*>(d) = p1;
                 *reinterpret_cast<uint2*>(d + BN * KS * 2) = p2;
@@ -501,6 +593,15 @@ __global__ __launch_bounds__(BN == 16 ? 512 : FEW_THREADS, BN == 16 ? 2 : 1) voi
             }
             if (++s == FEW_RING) { s = 0; ++turn; }
         }
+#pragma unroll
+        for (int i = 0; i < BN / 16; ++i) {             // (while the last products are on their way)
+            uint32_t x = larger_half(most[i]);
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) x = max(x, __shfl_xor_sync(0xffffffffu, x, o));
+            if ((f & 7) == 0) ctrl->x_most[i * 16 + (f >> 3)] = (uint16_t)x;
+            x = __reduce_max_sync(0xffffffffu, x);
+            if (lane == 0) atomicMax(&ctrl->most, x);
+        }
         while (fine && taken < mine) fine = take(taken++);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -511,13 +612,17 @@ __global__ __launch_bounds__(BN == 16 ? 512 : FEW_THREADS, BN == 16 ? 2 : 1) voi
     }
     pdl_wait();             // (C may still be read by the kernel before, whose end one thread alone has waited for)
     if (parts == 1) {
-        for (int i = threadIdx.x; i < p.M * FT; i += FEW_THREADS)
-            if (f0 + i % FT < p.N && !ctrl->abort) store(p, i / FT, f0 + i % FT, sums[i]);
+        const float least = p.lost * (2.f * magnitude(ctrl->most) + 8.f);
+        for (int i = threadIdx.x; i < p.M * FT; i += FEW_THREADS) {
+            const int m = i / FT, n = f0 + i % FT;
+            if (n < p.N && !ctrl->abort) p.C[(size_t)m * p.ldc + n] = doubtful(sums[i], least) ? settle_few(p, ctrl, 1, m, i % FT, n, sums[i]) : sums[i];
+        }
     } else {
         cluster_sync_all();
         const int share = (FT + parts - 1) / parts, lo = part * share, width = max(0, min(FT - lo, share));
-        for (int i = threadIdx.x; i < p.M * width; i += FEW_THREADS) {
-            const int m = i / width, f = lo + i % width;
+        uint32_t most = lane < parts ? __float_as_uint(ld_dsmem(reinterpret_cast<float*>(&ctrl->most), (uint32_t)lane)) : 0u;      // (beside the sums, not before them)
+        for (int i0 = warp * 32; i0 < p.M * width; i0 += FEW_THREADS) {
+            const int i = min(i0 + lane, p.M * width - 1), m = i / width, f = lo + i % width;
             float v = 0.f;
             for (int s0 = 0; s0 < segs; s0 += 8) {
                 float x[8];
@@ -530,7 +635,9 @@ __global__ __launch_bounds__(BN == 16 ? 512 : FEW_THREADS, BN == 16 ? 2 : 1) voi
                 for (int j = 0; j < 8; ++j)
                     if (s0 + j < segs) v += x[j];
             }
-            if (f0 + f < p.N && !ctrl->abort) store(p, m, f0 + f, v);
+            const float least = p.lost * (2.f * magnitude(__reduce_max_sync(0xffffffffu, most)) + 8.f);
+            if (i0 + lane < p.M * width && f0 + f < p.N && !ctrl->abort)
+                p.C[(size_t)m * p.ldc + f0 + f] = doubtful(v, least) ? settle_few(p, ctrl, parts, m, f, f0 + f, v) : v;
         }
         cluster_sync_all();         // nobody leaves while another CTA reads its sums
     }
@@ -654,23 +761,28 @@ extern "C" int rlis_gemm_f32_split_few_rows(void) { return FEW_ROWS; }
 extern "C" void rlis_gemm_f32_split_set_rows(int n) { g_bn = n >= 16 && n <= MAX_BN && n % 16 == 0 ? n : 0; }
 extern "C" void rlis_gemm_f32_split_set_parts(int n) { g_parts = n >= 0 && n <= MAX_PARTS ? n : 0; }
 
+// Bytes of scratch a row (0: too long a row): its three planes and the magnitudes of its pieces.
+extern "C" int rlis_gemm_f32_split_row_bytes(int K) { return K <= 0 || K > (1 << 28) ? 0 : 6 * ((K + 7) / 8 * 8) + 4 * ((K + ROW_PIECE - 1) / ROW_PIECE); }
+
 // C[M, N] = A[M, K] W[N, K]^T, rows lda, ldw, ldc floats apart; A, W, lda and ldw on 16-byte boundaries, K >= 1.  More than
-// rlis_gemm_f32_split_few_rows() rows: `planes` is scratch of 3 * M * (K rounded up to 8) bf16 on a 16-byte boundary.  `early`: no kernel
+// rlis_gemm_f32_split_few_rows() rows: `planes` is scratch of M times rlis_gemm_f32_split_row_bytes(K) bytes on a 16-byte boundary.  `early`: no kernel
 // that is still running writes W, so that its first tiles may be asked for before those before in the stream have finished.
 extern "C" int rlis_gemm_f32_split(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc, int M, int N, int K, void* planes,
                                    int early, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || lda % 4 || ldw % 4 || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15)) return RLIS_ERR_UNSUPPORTED;
-    SplitArgs p = {A, W, C, lda, ldw, ldc, M, N, K, 0, (K + KS - 1) / KS, 0, 0, 1, 0, early};
+    SplitArgs p = {A, W, C, lda, ldw, ldc, M, N, K, 0, (K + KS - 1) / KS, 0, 0, 1, 0, early, K * 0x1p-100f, nullptr, (K + ROW_PIECE - 1) / ROW_PIECE};
     if (M <= 16) return launch_few<16>(p, stream);
     if (M <= FEW_ROWS) return launch_few<32>(p, stream);
     if (planes == nullptr || (reinterpret_cast<uintptr_t>(planes) & 15)) return RLIS_ERR_UNSUPPORTED;
     const int sms = sm_count(), pitch = (K + 7) / 8 * 8;
-    const long long pieces = (long long)M * (pitch / 4);
-    rlis_launch(split_rows_kernel, dim3((unsigned)(pieces / 256 + 1 < 8LL * sms ? pieces / 256 + 1 : 8LL * sms)), dim3(256), 0, stream, A, lda,
-                reinterpret_cast<bf16*>(planes), M, K, pitch);
+    float* most = reinterpret_cast<float*>(reinterpret_cast<bf16*>(planes) + (size_t)3 * M * pitch);
+    const long long blocks = ((long long)M * p.pieces + 7) / 8;
+    rlis_launch(split_rows_kernel, dim3((unsigned)(blocks < 8LL * sms ? blocks : 8LL * sms)), dim3(256), 0, stream, A, lda, reinterpret_cast<bf16*>(planes), most, M, K,
+                pitch, p.pieces);
     int rc = RLIS_LAUNCH_CHECK();
     if (rc != 0) return rc;
+    p.x_most = most;
     p.bn = choose_bn(M, N, (K + KM - 1) / KM, sms);
     p.m_tiles = (M + p.bn - 1) / p.bn;
     const int b_bytes = 3 * p.bn * KM * 2;

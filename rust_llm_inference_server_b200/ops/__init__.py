@@ -203,8 +203,9 @@ def _gemm_f32_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, early: 
     before the kernels before have finished, as `stream_gemm` does."""
     (M, K), N = a.shape, w.shape[0]
     few = lib().rlis_gemm_f32_split_few_rows()
-    rows = M if M <= few else max(few + 1, _SPLIT_PLANES // (6 * K))
-    planes = torch.empty((3 * min(M, rows) * ((K + 7) // 8 * 8),), dtype=torch.bfloat16, device=a.device) if M > few else None
+    row_bytes = lib().rlis_gemm_f32_split_row_bytes(K)
+    rows = M if M <= few else max(few + 1, _SPLIT_PLANES // row_bytes)
+    planes = torch.empty((min(M, rows) * row_bytes,), dtype=torch.uint8, device=a.device) if M > few else None
     for m in range(0, M, max(1, rows)):
         n = min(rows, M - m)
         check(lib().rlis_gemm_f32_split(a[m:].data_ptr(), a.stride(0), w.data_ptr(), K, out[m:].data_ptr(), out.stride(0), n, N, K,

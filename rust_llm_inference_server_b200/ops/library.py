@@ -31,6 +31,7 @@ SIGNATURES = {
     "rlis_gemm_f32_nt": [P, P, P, I, I, I, P],
     "rlis_gemm_f32_split": [P, LL, P, LL, P, LL, I, I, I, P, I, P],
     "rlis_gemm_f32_split_few_rows": [],
+    "rlis_gemm_f32_split_row_bytes": [I],
     "rlis_gemm_f32_shape": [I, I, I, I, I],
     "rlis_gemm_f32_shapes": [],
     "rlis_gemm_f32_nt_batched": [P, P, P, I, I, I, LL, LL, LL, I, LL, LL, LL, P],

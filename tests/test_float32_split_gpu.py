@@ -126,3 +126,26 @@ def test_every_height_of_a_tile_has_the_same_bits(M, N, K):
     finally:
         debug_set("f32_split_rows", 0)
     ops.check_device_errors()
+
+
+# powers of two that take a row's third part, its second and third, and all of it under the smallest bfloat16
+@pytest.mark.parametrize("M,N,K", [(4, 200, 2048), (11, 300, 2304), (20, 300, 2304), (40, 200, 2048), (200, 3000, 2052), (8, 2048, 8192), (3, 20000, 2048)])
+def test_small_numbers_are_as_exact_as_others(M, N, K):
+    """Rows of tiny numbers against ordinary and against huge weights, tiny weights, rows of zeros: what a chain of K FMAs may be off by, and no more."""
+    from rust_llm_inference_server_b200 import ops
+    a, w = operands(M, N, K)
+    for i in range(M):
+        a[i] *= 2.0 ** (0, -90, -100, -110, -115, -120, -124, -126, -130)[i % 9]
+    a[8:9] = 0.0
+    w[5:60] *= 2.0 ** 100
+    w[60:100] = 0.0
+    w[100:130] *= 2.0 ** -110
+    got = product(a, w)
+    want, size = a.double() @ w.double().t(), a.abs().double() @ w.abs().double().t()
+    # a rounding of half a unit at every step of the chain, and one of 2^-150 where a step's result is subnormal
+    assert bool(((got.double() - want).abs() <= K * 2.0 ** -24 * size + K * 2.0 ** -150).all())
+    assert not bool(got[:, 60:100].any()) and not bool(got[8:9].any())
+    for m in sorted({0, 1, 4, 6, M - 1} & set(range(M))):               # whatever else is in the batch
+        assert torch.equal(product(a[m:m + 1].contiguous(), w), got[m:m + 1])
+    assert torch.equal(product(a[:17].contiguous(), w), got[:17])
+    ops.check_device_errors()
