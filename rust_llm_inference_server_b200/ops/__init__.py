@@ -194,8 +194,11 @@ _SPLIT_PLANES = 128 << 20       # bytes of scratch that a product's rows are cut
 
 
 def _gemm_f32_splits(a: torch.Tensor, w: torch.Tensor) -> bool:
-    """Whether a [M, K] @ w[N, K]^T in float32 is done as six products of bfloat16 parts on the tensor cores: long rows on 16-byte boundaries."""
-    return w.shape[1] >= SPLIT_MIN_K and w.shape[1] % 4 == 0 and a.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+    """Whether a [M, K] @ w[N, K]^T in float32 is done as six products of bfloat16 parts on the tensor cores: long rows on 16-byte boundaries that do not
+    overlap (copies by tensor maps take no others).  The stride of a single row says nothing."""
+    M, K = a.shape
+    apart = M <= 1 or (a.stride(0) >= K and a.stride(0) % 4 == 0)
+    return K >= SPLIT_MIN_K and K % 4 == 0 and apart and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
 
 
 def _gemm_f32_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, early: bool = False) -> torch.Tensor:
@@ -208,7 +211,7 @@ def _gemm_f32_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, early: 
     planes = torch.empty((min(M, rows) * row_bytes,), dtype=torch.uint8, device=a.device) if M > few else None
     for m in range(0, M, max(1, rows)):
         n = min(rows, M - m)
-        check(lib().rlis_gemm_f32_split(a[m:].data_ptr(), a.stride(0), w.data_ptr(), K, out[m:].data_ptr(), out.stride(0), n, N, K,
+        check(lib().rlis_gemm_f32_split(a[m:].data_ptr(), a.stride(0) if M > 1 else K, w.data_ptr(), K, out[m:].data_ptr(), out.stride(0), n, N, K,
                                         planes.data_ptr() if n > few else None, int(early), _stream()), "gemm_f32")
     _count("gemm_f32.split")
     return out

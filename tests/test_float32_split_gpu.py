@@ -149,3 +149,26 @@ def test_small_numbers_are_as_exact_as_others(M, N, K):
         assert torch.equal(product(a[m:m + 1].contiguous(), w), got[m:m + 1])
     assert torch.equal(product(a[:17].contiguous(), w), got[:17])
     ops.check_device_errors()
+
+
+def test_rows_that_overlap_and_rows_alone():
+    """Rows that are one and the same, or a few numbers apart, go to the chains of FMAs as before; the stride of a single row is never used."""
+    from rust_llm_inference_server_b200 import ops
+    a, w = operands(5, 200, 2052)
+    flat = torch.randn(2052 + 64, device="cuda")
+    for M in (5, 40):
+        same, near = a[:1].expand(M, 2052), flat.as_strided((M, 2052), (1 if M > 5 else 4, 1))
+        for x in (same, near):
+            assert not ops._gemm_f32_splits(x, w)
+            assert torch.equal(ops.linear(x, w), chains(x, w))
+    for stride in (0, 3, 2052, 5000):
+        one = a.as_strided((1, 2052), (stride, 1))
+        assert torch.equal(ops.linear(one, w), product(a[:1].contiguous(), w))
+
+
+def chains(x, w):
+    from rust_llm_inference_server_b200.ops.library import check, lib
+    from rust_llm_inference_server_b200 import ops
+    x, out = x.contiguous(), torch.empty(x.shape[0], w.shape[0], device="cuda")
+    check(lib().rlis_gemm_f32_nt(x.data_ptr(), w.data_ptr(), out.data_ptr(), x.shape[0], w.shape[0], x.shape[1], ops._stream()), "gemm_f32")
+    return out
