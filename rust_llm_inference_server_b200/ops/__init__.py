@@ -1399,7 +1399,11 @@ def linear(x, w: torch.Tensor, out_dtype=None, sink=None, bias: torch.Tensor | N
     if bias is not None:
         raise KernelError("linear: a bias is taken with a sink")
     if x.dtype == torch.float32:
-        if w.dtype == torch.float32 and x.is_cuda and x.dim() == 2 and x.is_contiguous() and w.is_contiguous() and x.shape[1] == w.shape[1] and _gemm_f32_splits(x, w):
+        if x.dim() == 2 and x.is_contiguous():
+            _req(x, "x", torch.float32)
+            _req(w, "w", torch.float32, (None, x.shape[1]))
+            if not _gemm_f32_splits(x, w):
+                return gemm_f32(x, w)
             return _gemm_f32_split(x, w, torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device), early)
         if not x.is_contiguous() and x.dim() == 2 and x.stride(1) == 1:
             out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)

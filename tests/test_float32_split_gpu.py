@@ -172,3 +172,14 @@ def chains(x, w):
     x, out = x.contiguous(), torch.empty(x.shape[0], w.shape[0], device="cuda")
     check(lib().rlis_gemm_f32_nt(x.data_ptr(), w.data_ptr(), out.data_ptr(), x.shape[0], w.shape[0], x.shape[1], ops._stream()), "gemm_f32")
     return out
+
+
+def test_what_a_product_refuses():
+    """Operands off the device, of other types and of other sizes are errors before anything is launched."""
+    from rust_llm_inference_server_b200 import ops
+    a, w = operands(4, 64, 2048)
+    for bad in (w.cpu(), w.bfloat16(), w[:, :2044], w.t().contiguous().t(), w[:, None]):
+        with pytest.raises(ops.KernelError):
+            ops.linear(a, bad)
+    with pytest.raises(ops.KernelError):
+        ops.linear(a.cpu(), w)
