@@ -20,6 +20,9 @@ namespace wide {
 using namespace chunkprod;
 constexpr int D = 128, LDR = D + 4, VT = 64, WC = 16;       // heads; rows of 128; columns of v a CTA of the outputs, and of the walk
 constexpr int PREPARE_THREADS = 256, WALK_THREADS = 256, OUTPUT_THREADS = 128;
+// The least ln g that is summed: its power is 0 like that of anything below, and the differences of the sums over tokens behind it keep their bits (they come
+// as low as -1e30, beside which two floats hold nothing of a sum of ordinary ones).
+constexpr float LEAST = -1024.f;
 
 // Scratch of a (chunk, head), in floats: decayed q . k [key][query], W turned [entry][token], u [token][dv], the state before the
 // chunk [entry][dv], e^{L_end - L} and e^L.
@@ -80,7 +83,7 @@ __global__ __launch_bounds__(PREPARE_THREADS, 2) void delta_chunk_prepare(const 
         const Unit out(scratch, (size_t)blockIdx.x * z.nh + h, dv);
         if (threadIdx.x < 32) {             // two tokens a lane
             const int a = 2 * threadIdx.x;
-            const float g0 = a < n ? x[a * AW + C + z.nh + h] : 0.f, g1 = a + 1 < n ? x[(a + 1) * AW + C + z.nh + h] : 0.f;
+            const float g0 = a < n ? fmaxf(x[a * AW + C + z.nh + h], LEAST) : 0.f, g1 = a + 1 < n ? fmaxf(x[(a + 1) * AW + C + z.nh + h], LEAST) : 0.f;
             const float b0 = a < n ? x[a * AW + C + h] : 0.f, b1 = a + 1 < n ? x[(a + 1) * AW + C + h] : 0.f;
             float2 L = two_sum(make_float2(g0, 0.f), make_float2(g1, 0.f));
 #pragma unroll

@@ -99,6 +99,21 @@ def test_a_token_sees_nothing_of_what_comes_after_it(monkeypatch, at, part):
     assert part == "a" or not bool(torch.isfinite(out[at, :128]).all())          # (a decay that is not a number counts as 0)
 
 
+@pytest.mark.parametrize("logit", [300.0, 1e6, 1e30, float("inf")])
+def test_tokens_behind_a_decay_of_nothing_keep_theirs(monkeypatch, logit):
+    """A token whose decay is 0 (ln g far below float32's range of powers) empties the state; what comes after it decays as ever."""
+    from rust_llm_inference_server_b200 import ops
+    monkeypatch.setattr(ops, "_gated_delta_wide_pays", lambda *a: True)
+    c = Case([130], [7], 2, 2, 128, torch.float32)
+    for at in (0, 5, 70, 71, 127):
+        c.proj[at, c.C + c.nh] = logit
+    out, state, slots, wide = c.run()
+    want, states = c.plain(slots)
+    assert wide == 1 and float((out.double() - want).norm() / want.norm()) <= 2.0 ** -24 * 8
+    S = states[slots[0]][0]
+    assert float((state[slots[0], :S.numel()].double() - S).norm() / S.norm()) <= 2.0 ** -24 * 8
+
+
 def test_long_portions_go_by_64(monkeypatch):
     from rust_llm_inference_server_b200 import ops
     pays = ops._gated_delta_wide_pays
