@@ -1022,11 +1022,9 @@ int launch_bias_tc(const CUtensorMap& map_q, const CUtensorMap& map_k, const CUt
                    int window, cudaStream_t stream) {
     using SH = PShape<HD, TN, true>;
     const size_t smem = ba.bias != nullptr ? SH::smem_bias(ba.n_dist) : SH::SMEM;
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaFuncSetAttribute(attn_prefill_tc_kernel<HD, TN, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SH::smem_bias(BIAS_MAX_DIST));
-        attr_done = true;
-    }
+    static std::atomic<unsigned long long> done{0};
+    const cudaError_t e = rlis_allow_smem(attn_prefill_tc_kernel<HD, TN, false, true>, (int)SH::smem_bias(BIAS_MAX_DIST), done);
+    if (e != cudaSuccess) return (int)e;
     rlis_launch_cluster(attn_prefill_tc_kernel<HD, TN, false, true>, dim3((unsigned)(nkv * ((nh / nkv + 1) / 2)), (unsigned)n_tiles), PT_THREADS, smem, stream,
                         dim3(1, 1, 1), map_q, map_k, map_v, out, tiles, cu_seqlens, ctx_lens, block_tables, max_blocks, nh, nkv, page_size, cache_rows, scale, window,
                         1, DiffArgs{}, ba);

@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 
 // Element type codes used by every exported launcher.
 #define RLIS_F32 0
@@ -132,6 +133,19 @@ static inline void rlis_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, 
     cfg.attrs = attr;
     cfg.numAttrs = g_rlis_pdl ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// Dynamic shared memory that a kernel may ask for, set once a device: `done` holds a bit for each on which it is (a static one beside the launch).
+template <typename... KArgs>
+static inline cudaError_t rlis_allow_smem(void (*kernel)(KArgs...), int bytes, std::atomic<unsigned long long>& done) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (bit & done.load(std::memory_order_acquire)) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
 }
 
 // The same for a grid of thread-block clusters of `cluster` CTAs.

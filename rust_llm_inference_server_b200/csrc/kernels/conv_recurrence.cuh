@@ -966,14 +966,11 @@ template <typename T> static int launch_wide(const Args& g, long long tail_off, 
     constexpr int prepare_smem = (2 * D * LDT + 2 * CHUNK * LDT + 3 * 16 * 17) * 4, walk_smem = (D * LDT + CHUNK * LDR + (D + CHUNK) * (WC + 4)) * 4,
                   output_smem = (2 * D * LDT + 2 * CHUNK * LDT) * 4;
     static_assert(CHUNK * LDR <= D * LDT, "rows take the place of turned ones");
-    static bool attr_done = false;
-    if (!attr_done) {
-        cudaError_t e = cudaFuncSetAttribute(delta_chunk_prepare<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, prepare_smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_walk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, walk_smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_outputs<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, output_smem);
-        if (e != cudaSuccess) return (int)e;
-        attr_done = true;
-    }
+    static std::atomic<unsigned long long> prepare_done{0}, walk_done{0}, output_done{0};
+    cudaError_t e = rlis_allow_smem(delta_chunk_prepare<0>, prepare_smem, prepare_done);
+    if (e == cudaSuccess) e = rlis_allow_smem(delta_chunk_walk<T>, walk_smem, walk_done);
+    if (e == cudaSuccess) e = rlis_allow_smem(delta_chunk_outputs<0>, output_smem, output_done);
+    if (e != cudaSuccess) return (int)e;
     rlis_launch(delta_chunk_prepare<0>, dim3(g.wide_chunks, z.nh), PREPARE_THREADS, prepare_smem, stream, (const float*)g.act, g.wide, g.sq, g.n_seqs, z);
     rlis_launch(delta_chunk_walk<T>, dim3(g.n_seqs, z.nh, z.dv / WC), WALK_THREADS, walk_smem, stream, (const float*)g.act, g.wide, g.state, g.state_stride, tail_off,
                 (const T*)g.x, g.stride, g.sq, z);

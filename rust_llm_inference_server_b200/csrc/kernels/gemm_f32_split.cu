@@ -791,7 +791,8 @@ extern "C" int rlis_gemm_f32_split(const float* A, long long lda, const float* W
     p.raw_ring = p.rings * b_bytes + 4 * RAW_BYTES_M <= MANY_RING_BYTES ? 4 : 2;
     CUtensorMap map_w, map_a;
     if (!map_f32(&map_w, W, N, K, ldw, FT) || !map_planes(&map_a, reinterpret_cast<const bf16*>(planes), M, pitch, p.bn)) return RLIS_ERR_UNSUPPORTED;
-    const cudaError_t e = cudaFuncSetAttribute(f32_split_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MANY_SMEM);
+    static std::atomic<unsigned long long> done{0};
+    const cudaError_t e = rlis_allow_smem(f32_split_many_kernel, MANY_SMEM, done);
     if (e != cudaSuccess) return (int)e;
     const long long tiles = (long long)((N + FT - 1) / FT) * p.m_tiles;
     rlis_launch(f32_split_many_kernel, dim3((unsigned)tiles), dim3(MANY_THREADS), (size_t)MANY_SMEM, stream, map_w, map_a, p);

@@ -66,3 +66,12 @@ def test_a_table_of_biases_reaches_every_distance_that_a_tile_reads():
                             continue            # a block beyond the table's reach takes its last entry
                         first, last = pos0 - key0 - (tn - 1), pos0 + tq - 1 - key0          # (rows past the portion's end read, too)
                         assert -front <= first and last < n_dist + back, (tn, n_dist, pos0, tokens, key0)
+
+
+@pytest.mark.parametrize("name,kernel", [("conv_recurrence.cuh", "delta_chunk_prepare"), ("conv_recurrence.cuh", "delta_chunk_walk"), ("conv_recurrence.cuh", "delta_chunk_outputs"),
+                                         ("attention_prefill_tcgen05.cu", "attn_prefill_tc_kernel<HD, TN, false, true>"), ("gemm_f32_split.cu", "f32_split_many_kernel")])
+def test_shared_memory_is_allowed_on_every_device(name, kernel):
+    """What a launch asks for is set for each device that it meets (a flag for the process leaves the second device without), and its failure is told."""
+    text = source(name)
+    assert not re.search(r"cudaFuncSetAttribute\(" + re.escape(kernel) + r"\b", text)
+    assert re.search(r"\be = rlis_allow_smem\(" + re.escape(kernel) + r"(?:<[^>]*>)?,", text)
