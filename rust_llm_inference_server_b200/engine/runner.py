@@ -106,6 +106,7 @@ class StepContext:
 
 class ModelRunner:
     GRAPH_AFTER_STEPS = 2       # eager steps of a decode shape before its graph is captured
+    WORKSPACE_SLACK = 64 << 20  # bytes that a scratch buffer which has to grow may have beyond what is asked of it
 
     def __init__(self, model, cache_manager, storage, max_seq_len: int):
         self.model = model
@@ -149,7 +150,9 @@ class ModelRunner:
                 # (graphs cannot be dropped while one is being recorded; the step runs eagerly instead,
                 # which sizes the buffer, and the shape is captured the next time it comes)
                 raise _CaptureAbort(name)
-            cap = max(n, 2 * buf.numel() if buf is not None and buf.dtype == dtype else n)
+            cap = n
+            if buf is not None and buf.dtype == dtype:      # room for the next larger step, but no more than WORKSPACE_SLACK beyond this one
+                cap = max(n, min(2 * buf.numel(), n + self.WORKSPACE_SLACK // buf.element_size()))
             if name in self._recorded:
                 self._drop_graphs()     # captured graphs point at the old buffer
             buf = torch.empty((cap,), dtype=dtype, device=self.device)

@@ -537,7 +537,7 @@ def _gated_delta_wide_pays(n_tokens: int, n_seqs: int, longest: int, columns: in
     return longest >= 64 and after < 0.95 * before
 
 
-GATED_DELTA_WIDE_BYTES = 512 << 20      # of scratch; steps that would take more go 16 tokens at a time
+GATED_DELTA_WIDE_BYTES = 512 << 20      # of scratch, 148 KB a chunk and head; steps that would take more go 16 tokens at a time (a runner keeps up to 64 MB more)
 
 
 def _gated_delta_wide(step, T: int, n_heads: int, n_qk_heads: int, d: int, dv: int, taps: int, state: torch.Tensor, act: torch.Tensor,

@@ -30,3 +30,21 @@ def test_only_a_buffer_that_a_graph_points_into_takes_the_graphs_along():
     r._graphs["step"] = "recorded anew"                             # what the dropped graphs pointed into is forgotten
     r.workspace("decode", (500, 8), torch.float32)
     assert r._graphs == {"step": "recorded anew"}
+
+
+def test_a_buffer_that_grows_stays_near_what_is_asked_of_it():
+    """Small ones double, so that few steps reallocate; large ones have at most the slack beyond the largest step."""
+    r = runner()
+    slack = r.WORKSPACE_SLACK // 4
+    r.workspace("small", (1000,), torch.float32)
+    r.workspace("small", (1001,), torch.float32)
+    assert r._ws["small"].numel() == 2000
+    r.workspace("large", (2 * slack,), torch.float32)
+    r.workspace("large", (2 * slack + 1,), torch.float32)
+    assert r._ws["large"].numel() == 3 * slack + 1
+    assert r.workspace("large", (3 * slack,), torch.float32).data_ptr() == r._ws["large"].data_ptr()
+    r.workspace("large", (8 * slack,), torch.float32)
+    assert r._ws["large"].numel() == 8 * slack
+    r.workspace("other", (5,), torch.bfloat16)
+    r.workspace("other", (6,), torch.float32)           # of another type: nothing to go by
+    assert r._ws["other"].numel() == 6
