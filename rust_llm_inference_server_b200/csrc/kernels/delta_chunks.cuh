@@ -4,7 +4,7 @@
 //
 //   u = T (beta v) - W S0,  W = T (beta e^L k);   o_t = e^{L_t} S0^T q_t + sum_{i <= t} e^{L_t - L_i} (q_t . k_i) u_i;   S = e^{L_end} S0 + sum_t e^{L_end - L_t} k_t u_t^T
 //
-// which is the recurrence written out.  Only u and S go from chunk to chunk, two products of 64 x 128 a column block; everything else is done for all
+// which is the recurrence written out (the compact WY form of products of Householder-like factors).  Only u and S go from chunk to chunk, two products of 64 x 128 a column block; everything else is done for all
 // chunks at once, before and after:
 //   delta_chunk_prepare: (chunk, head)  T, T (beta v), W, the decayed q . k, the powers of the decay
 //   delta_chunk_walk:    (request, head, 16 columns)  the chunks in order: u, and the state before every chunk
@@ -52,7 +52,7 @@ template <int THREADS> __device__ __forceinline__ void stage_turned(float* dst, 
     }
 }
 
-// The sum of two numbers kept as sums of two floats (what a float sum leaves out, exactly, beside it).
+// The sum of two numbers kept as sums of two floats (what a float sum leaves out, exactly, beside it: Knuth's two-sum).
 __device__ __forceinline__ float2 two_sum(float2 a, float2 b) {
     const float s = __fadd_rn(a.x, b.x), t = __fsub_rn(s, a.x);
     return make_float2(s, __fadd_rn(__fadd_rn(__fsub_rn(a.x, __fsub_rn(s, t)), __fsub_rn(b.x, t)), __fadd_rn(a.y, b.y)));

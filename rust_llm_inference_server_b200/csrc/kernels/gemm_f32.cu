@@ -1,5 +1,5 @@
 // True 32-bit matrix product for the float32 path: C[M, N] = A[M, K] * W[N, K]^T with FFMA on the
-// CUDA cores, for rows shorter than 2,048, rows off 16-byte boundaries and batches (others: gemm_f32_split.cu).  Every output element is accumulated over k = 0..K-1 in
+// CUDA cores, for rows shorter than 2,048, rows off 16-byte boundaries or less than their length apart, and batches (others: gemm_f32_split.cu).  Every output element is accumulated over k = 0..K-1 in
 // that order, one fused multiply-add after the other, whichever kernel below computes it and
 // whatever M, N or the tile it falls in, so a row's result does not depend on what else is in the
 // batch.  Role in the reference: `x.matmul(w.t())`, crates/model/src/layers.rs:82.

@@ -1,16 +1,17 @@
-// 32-bit matrix product on the fifth-generation tensor cores: C[M, N] = A[M, K] * W[N, K]^T for float32 matrices with k of 1,024 and more.
+// 32-bit matrix product on the fifth-generation tensor cores: C[M, N] = A[M, K] * W[N, K]^T for float32 matrices, sent here from k of 2,048 on.
 //
-// A float32 number is exactly the sum of three bf16 numbers (8 bits each of its 24): x = x1 + x2 + x3.  Six of the nine products of two such
-// sums carry everything above 2^-26 of x w; each is exact in the tensor core's float32 accumulator, and what an accumulator loses is its own
-// truncation (measured: 0.37 of 2^-24 of it for every 16 of k).  So w1 x1 has an accumulator of its own and the five small products share another;
-// both are read out and added in float32, rounded to nearest, every 256 of k (a segment):
+// A float32 number from 2^-110 up is the sum of three bf16 numbers (8 bits each of its 24): x = x1 + x2 + x3, |x2| <= 2^-8 |x|, |x3| <= 2^-17 |x|.  Six of the nine
+// products of two such sums are formed; the other three come to 2^-24 of x w at the most (both just above a power of two) and 0.39 x 2^-26 root mean square.
+// (So over one to four terms the result is 1.03 to 1.2 times as far off as a chain of FMAs, which rounds that seldom; from about eight on it is closer.)  Each
+// product is exact in the tensor core's float32 accumulator, and what an accumulator loses is its own truncation (measured: 0.37 of 2^-24 of it for every 16
+// of k).  So w1 x1 has an accumulator of its own and the five small products share another; both are read out and added in float32, rounded to nearest, every 256
+// of k (a segment):
 //     C = ((s0 + s1) + s2) + ..,   s = (w1 x1) + (w3 x1 + w2 x2 + w1 x3 + w2 x1 + w1 x2)
 // Off float64 by 2.5e-7 of the result at K 2048 and 8192 (normal numbers), where one chain of K FMAs is 8e-7 and 1.6e-6.  The segments and the order in
 // them are the same in both kernels below and for any number of rows, so a row's result does not depend on what else is in the batch.
-// The sum of three is exact from 2^-110 up only (2^-102 where subnormal operands count as zeros): below that the third part has bits under the smallest
-// bf16.  So the largest magnitude of every row of A and of W is taken along, and an output that what is lost could reach, that is, one below
-// K (x_max + w_max + 8) 2^-100, is worked out again as a chain of FMAs from the float32 operands; so is one that is not finite (infinities and NaN, and
-// numbers that round to infinity in 8 bits, come out as that chain gives them).
+// Below 2^-110 (2^-102 where subnormal operands count as zeros) the third part has bits under the smallest bf16.  So the largest magnitude of every row of A
+// and of W is taken along, and an output that what is lost could reach, that is, one below K (x_max + w_max + 8) 2^-100, is worked out again as a chain of FMAs
+// from the float32 operands; so is one that is not finite (infinities and NaN, and numbers that round to infinity in 8 bits, come out as that chain gives them).
 //
 // W is the M side of the instruction (128 features a tile), split on the way: TMA brings 128 x 32 floats, warps turn a row of 32 into three
 // planes of bf16 and put them into tensor memory as the A operand.  The rows of A are the N side, from shared memory in three planes.
@@ -217,8 +218,8 @@ __global__ __launch_bounds__(256) void split_rows_kernel(const float* __restrict
 }
 
 // ------------------------------------------------------------------------------------------------
-// Many rows.  700 rows, us here and in FFMA tiles: K 2048 N 16384 238 / 1139, N 3072 50 / 218, N 2048 39 / 218; K 8192 N 2048 127 / 858; 2,048 rows of K 2048 N 16384
-// 625 / 2648 (220 TFLOP/s, six times that on the tensor cores: 1.3 PFLOP/s).  A stage takes the products' time (12 cycles a row) and about 1,100 cycles
+// Many rows.  700 rows, us here and in FFMA tiles: K 2048 N 16384 243 / 1139, N 3072 50 / 218, N 2048 38 / 218; K 8192 N 2048 130 / 858; 2,048 rows of K 2048 N 16384
+// 646 / 2648 (213 TFLOP/s, six times that on the tensor cores: 1.3 PFLOP/s).  A stage takes the products' time (12 cycles a row) and about 1,100 cycles
 // beside it, whatever the depth of the rings, so stages of 64 k are better than stages of 32 for tiles of few rows (48 rows 27 / 33 us, 200 39 / 50).
 // A tile of 128 features x bn rows of A a CTA (bn up to 160), in two halves of the rows with accumulators, an issuing warp and four adding
 // warps of their own: one warp alone spends more cycles between the bursts of two stages than the pipe has instructions queued.
@@ -405,8 +406,8 @@ __global__ __launch_bounds__(MANY_THREADS, 1) void f32_split_many_kernel(const _
 
 // ------------------------------------------------------------------------------------------------
 // Few rows (a decode step): bound by the memory's rate over W, and below it by a stage's way through the roles (raw weights, planes, products: about
-// 900 cycles with one CTA on an SM, 600 a stage with two).  8 rows, us here and as chains of FMAs: K 2048 N 2048 8.9 / 11.3, N 3072 9.8 / 16, N 16384 28 / 42,
-// N 32000 47 / 81 (5.6 TB/s); K 8192 N 2048 22 / 37.  A tile of 128 features a cluster, whose CTAs take whole segments of k and leave their
+// 900 cycles with one CTA on an SM, 600 a stage with two).  8 rows, us here and as chains of FMAs: K 2048 N 2048 9.7 / 11.1, N 3072 11.3 / 16, N 16384 32 / 44,
+// N 32000 52 / 83 (5.0 TB/s); K 8192 N 2048 24 / 38.  A tile of 128 features a cluster, whose CTAs take whole segments of k and leave their
 // sums in shared memory; the cluster then adds them up in the order of k, each CTA for a share of the features.  The rows of A are split
 // where the weights are.  Fourteen warps: 0-3 read the accumulators, 4-11 split (two sets), 12 asks for weights and rows, 13 issues the products.
 constexpr int FEW_THREADS = 448, FEW_RING = 4, FEW_A = 4;     // (a ring of an even number of stages, as above)

@@ -218,8 +218,8 @@ def _gemm_f32_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, early: 
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-    """out[M, N] = a[M, K] @ w[N, K]^T in true float32: rows of `SPLIT_MIN_K` and more on the tensor cores, every operand as the exact sum of three
-    bfloat16 numbers (`csrc/kernels/gemm_f32_split.cu`), others as chains of FMAs in the order of k.  A row has the same bits whatever other
+    """out[M, N] = a[M, K] @ w[N, K]^T in true float32: rows of `SPLIT_MIN_K` and more on the tensor cores, every operand as the sum of three bfloat16
+    numbers (`csrc/kernels/gemm_f32_split.cu`: what is left out, and which results go back to a chain), others as chains of FMAs in the order of k.  A row has the same bits whatever other
     rows there are."""
     M, K = a.shape
     N = w.shape[0]
@@ -265,7 +265,7 @@ def _small_rows(a: torch.Tensor) -> bool:
 
 def per_head_linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     """out[t, h, :] = w[h] @ a[t, h, :]: one small product a head (a [T, H, K] and out [T, H, N] may be
-    slices of wider rows, w [H, N, K]).  float32: this package's FFMA kernel; bfloat16 operands: up to 16 rows
+    slices of wider rows, w [H, N, K]).  float32: `gemm_f32_batched`; bfloat16 operands: up to 16 rows
     on 16-byte boundaries this package's kernel that reads every weight once (`rlis_per_head_small`), else the
     library's batched GEMM with float32 accumulation, into `out`'s element type."""
     if a.dtype == torch.float32:
@@ -1427,8 +1427,8 @@ def linear(x, w: torch.Tensor, out_dtype=None, sink=None, bias: torch.Tensor | N
 
 
 def linear_add(x: torch.Tensor, w: torch.Tensor, base: torch.Tensor) -> torch.Tensor:
-    """base + x @ w^T in float32 (base float32 [T, N]; x and w float32, or bfloat16 with float32 sums): this package's FFMA
-    product and an addition, or the library's product that adds."""
+    """base + x @ w^T in float32 (base float32 [T, N]; x and w float32, or bfloat16 with float32 sums): `gemm_f32`
+    and an addition, or the library's product that adds."""
     T, N = x.shape[0], w.shape[0]
     _req(base, "base", torch.float32, (T, N))
     if x.dtype == torch.float32:

@@ -29,7 +29,7 @@ def test_products_of_long_rows(M, N, K):
     out = product(a, w)
     want, size = a.double() @ w.double().t(), a.abs().double() @ w.abs().double().t()
     # an accumulator truncates (a unit of 2^-23) 16 times a segment, the small products' 80 times at 2^-8 of it, the segments are added with
-    # half a unit each, and three products below 2^-26 are left out
+    # half a unit each, and three products of together 2^-24 at the most are left out
     assert bool(((out.double() - want).abs() <= (18 + K / 512) * 2.0 ** -23 * size).all())
     assert float((out.double() - want).norm() / want.norm()) <= 4e-7            # (a chain of 2,048 FMAs is 8e-7 off)
     for m in sorted({1, 8, 16, 17, 32, 33, 100, 200} & set(range(M))):          # whatever else is in the batch
