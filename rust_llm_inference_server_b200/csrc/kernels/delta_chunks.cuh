@@ -20,8 +20,8 @@ namespace wide {
 using namespace chunkprod;
 constexpr int D = 128, LDR = D + 4, VT = 64, WC = 16;       // heads; rows of 128; columns of v a CTA of the outputs, and of the walk
 constexpr int PREPARE_THREADS = 256, WALK_THREADS = 256, OUTPUT_THREADS = 128;
-// The least ln g that is summed: its power is 0 like that of anything below, and the differences of the sums over tokens behind it keep their bits (they come
-// as low as -1e30, beside which two floats hold nothing of a sum of ordinary ones).
+// The least ln g that is summed: its power is 0 like that of anything below, and the differences of the sums over tokens behind it keep their bits (ln g comes
+// as low as -1e30, and from about 1e16 on the rounding of a sum of two such, left in the second float, leaves nothing there of ordinary ones).
 constexpr float LEAST = -1024.f;
 
 // Scratch of a (chunk, head), in floats: decayed q . k [key][query], W turned [entry][token], u [token][dv], the state before the

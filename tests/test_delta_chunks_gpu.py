@@ -99,7 +99,7 @@ def test_a_token_sees_nothing_of_what_comes_after_it(monkeypatch, at, part):
     assert part == "a" or not bool(torch.isfinite(out[at, :128]).all())          # (a decay that is not a number counts as 0)
 
 
-@pytest.mark.parametrize("logit", [300.0, 1e6, 1e30, float("inf")])
+@pytest.mark.parametrize("logit", [300.0, 1e6, 1e12, 1e20, 1e30, float("inf")])
 def test_tokens_behind_a_decay_of_nothing_keep_theirs(monkeypatch, logit):
     """A token whose decay is 0 (ln g far below float32's range of powers) empties the state; what comes after it decays as ever."""
     from rust_llm_inference_server_b200 import ops
