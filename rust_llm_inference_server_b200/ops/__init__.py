@@ -1928,10 +1928,11 @@ def _biased_tc_sizes(n_heads: int, n_kv_heads: int, dim: int, v_dim: int, page_s
     return bool(lib().rlis_attention_bias_prefill_tc_takes(n_heads, n_kv_heads, dim, v_dim, page_size, n_dist))
 
 
-# The longest context of a portion (cached tokens and its own) up to which it stays on mma.sync, by head size: a short one is all latency, of which the tcgen05 kernel has more.
-# us on tcgen05 and mma.sync, 32 heads of 64: 64 tokens 6.5 and 5.3, 128 7.8 and 7.4, 256 (a window and sinks) 10.6 and 10.6, 320 12.1 and 13.3, 448 15.0 and 18.4;
-# 16 heads of 128: 64 7.6 and 7.5, 96 8.4 and 10.2, 128 8.5 and 11.0.
-BIASED_TC_AFTER = {64: 320, 128: 96}
+# The longest context of a portion (cached tokens and its own) up to which it stays on mma.sync, by head size: a short one is all latency, of which the tcgen05
+# kernel has more.  us on tcgen05 and mma.sync, 32 heads of 64, a table and gates / a window and sinks: 64 tokens 6.5 and 5.3 / 6.2 and 4.7, 128 7.8 and 7.4 / 7.5 and 6.6,
+# 192 8.7 and 9.6 / 9.0 and 8.9, 256 9.4 and 11.2 / 10.6 and 10.6, 448 13.0 and 17.7 / 15.0 and 18.4; 16 heads of 128: 64 7.6 and 7.5 / 7.1 and 6.9, 96 8.4 and 10.2 / 8.3 and
+# 9.5.  Portions on both sides in one step are a launch each, one after the other: 100 and 500 tokens 20 us, both on mma.sync 18, both on tcgen05 14 (16 heads of 64).
+BIASED_TC_AFTER = {64: 128, 128: 64}
 
 
 def _biased_prefill_tc(q, k_cache, v_cache, out, bias, gate, gate_cols: int, slopes, n_heads: int, n_kv_heads: int, dim: int, v_dim: int, page_size: int,

@@ -105,8 +105,8 @@ def test_tokens_behind_a_decay_of_nothing_keep_theirs(monkeypatch, logit):
     from rust_llm_inference_server_b200 import ops
     monkeypatch.setattr(ops, "_gated_delta_wide_pays", lambda *a: True)
     c = Case([130], [7], 2, 2, 128, torch.float32)
-    for at in (0, 5, 70, 71, 127):
-        c.proj[at, c.C + c.nh] = logit
+    for i, at in enumerate((0, 5, 9, 70, 71, 90)):          # (sums of them that have to be rounded)
+        c.proj[at, c.C + c.nh] = logit * (1 + 0.37 * i)
     out, state, slots, wide = c.run()
     want, states = c.plain(slots)
     assert wide == 1 and float((out.double() - want).norm() / want.norm()) <= 2.0 ** -24 * 8
