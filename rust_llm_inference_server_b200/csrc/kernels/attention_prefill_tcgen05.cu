@@ -102,11 +102,11 @@
 // A bias by distance, a gate a head, a sink (BIAS; the formulas are in attention_bias.cu): the same kernel with blocks of 64 keys for both head sizes and
 // both heads' biases by distance in shared memory (times log2(e); with more entries in front and behind, so that no index needs a bound).  A block that
 // lies wholly beyond the table's reach adds the last row's constant; one within it reads a number a score (neighbouring rows read neighbouring numbers).
-// The weights are the ones that attention_bias_mma.cu forms: references move to the maximum with every block of 64 keys, the sum is of the weights before
-// rounding, and the sink joins it at the end, so the results agree but for the last bit of one number in 50,000 or more and a step may use both kernels.
-// (With blocks of 128 and a reference that lags, the highest weights are not exactly 1: off 64 bits by up to 9 % more.)  2,048 tokens, 32 heads of 64, a table
-// of 129: 50 us, with mma.sync (which keeps slopes, gates a channel, other sizes and longer tables) 92; a window of 1,024 and sinks, 409 and 1,092 tokens 31 and
-// 50; 16 heads of 128, 2,048 tokens 55 and 132.
+// The results have the bits of attention_bias_mma.cu's: references move to the maximum with every block of 64 keys, the sum is of the weights before
+// rounding and in the order of that kernel's fragments, and the sink joins it at the end; so which of the two a step takes shows in its time only.  (With
+// blocks of 128 and a reference that lags, the highest weights are not exactly 1: off 64 bits by up to 9 % more.)  2,048 tokens, 32 heads of 64, a table of 129: 49
+// us, with mma.sync (which keeps slopes, gates a channel, other sizes and longer tables) 92; a window of 1,024 and sinks, 409 and 1,092 tokens 31 and 50;
+// 16 heads of 128, 2,048 tokens 54 and 133.
 //
 // Every mbarrier wait is bounded (a fifth of a second); a wait that runs out sets the error word
 // (rlis_attention_prefill_tc_error), every role runs to its end without further waits, and the
@@ -233,9 +233,7 @@ __device__ __forceinline__ float sum_of_pair(uint64_t acc) {
 // P = exp2(s * scale - m) of 32 keys, rounded to bf16, into the row's lane of tensor memory: two
 // consecutive keys to a column, the layout in which the tensor core reads its A operand from there.
 // `lsum2`: the running sums of the even and of the odd keys.
-// ROUNDED: the sum is of the rounded values, the ones the product with V uses: the rounding of a dominant key then cancels between numerator and
-// denominator.  Otherwise of the weights as they are.
-template <bool MASK, bool ROUNDED>
+template <bool MASK>
 __device__ __forceinline__ void exp_of_chunk(const uint32_t (&v)[32], int c, int kmin, int kmax, uint64_t scale2,
                                              uint64_t neg_m2, uint32_t tmem_p_row, uint64_t& lsum2) {
     uint32_t pk[16];
@@ -249,10 +247,41 @@ __device__ __forceinline__ void exp_of_chunk(const uint32_t (&v)[32], int c, int
             if (!(idx <= kmax && idx >= kmin)) p0 = 0.f;
             if (!(idx + 1 <= kmax && idx + 1 >= kmin)) p1 = 0.f;
         }
+        // the sum is of the rounded values, the ones the product with V uses: the rounding of a
+        // dominant key then cancels between numerator and denominator
         const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
         pk[i] = *reinterpret_cast<const uint32_t*>(&h);
-        if (ROUNDED) add2(lsum2, pk[i] << 16, pk[i] & 0xffff0000u);
-        else add2(lsum2, __float_as_uint(p0), __float_as_uint(p1));
+        add2(lsum2, pk[i] << 16, pk[i] & 0xffff0000u);
+    }
+    tmem_st16(tmem_p_row + (uint32_t)(c * 16), pk);
+}
+// The same for scores that are in powers of two, summed as they are and in the order of mma.sync's fragments (attention_bias_mma.cu): keys 8 n + 2 q and
+// 8 n + 2 q + 1 for all n in the q-th of four sums, which two pairs hold.
+template <bool MASK>
+__device__ __forceinline__ void exp_of_chunk_by_quads(const uint32_t (&v)[32], int c, int kmin, int kmax, uint64_t neg_m2, uint32_t tmem_p_row,
+                                                      uint64_t (&lsum2)[2]) {
+    const uint64_t one2 = pair_of(1.0f);
+    uint32_t pk[16];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+        float p[8];
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+            const int idx = c * 32 + n * 8 + i;
+            fma2(p[i], p[i + 1], __uint_as_float(v[n * 8 + i]), __uint_as_float(v[n * 8 + i + 1]), one2, neg_m2);
+            p[i] = ex2_approx(p[i]);
+            p[i + 1] = ex2_approx(p[i + 1]);
+            if (MASK) {
+                if (!(idx <= kmax && idx >= kmin)) p[i] = 0.f;
+                if (!(idx + 1 <= kmax && idx + 1 >= kmin)) p[i + 1] = 0.f;
+            }
+            const __nv_bfloat162 h = __floats2bfloat162_rn(p[i], p[i + 1]);
+            pk[n * 4 + i / 2] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) add2(lsum2[q], __float_as_uint(p[4 * q + e]), __float_as_uint(p[4 * q + 2 + e]));
     }
     tmem_st16(tmem_p_row + (uint32_t)(c * 16), pk);
 }
@@ -644,7 +673,7 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
             if (move) {
                 corr = ex2_approx(m_ref - m_new);                    // 0 when nothing was seen before
                 m_ref = m_new;
-                l_run *= corr;
+                if (!BIAS) l_run *= corr;
             }
             const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
             // the product P V of the block before: P may be overwritten and O rescaled once it is done
@@ -683,7 +712,7 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
             }
             // P goes to tensor memory in two halves of the block's keys, each handed to the product
             // as soon as it is complete (O, if it was rescaled, is back there before the first)
-            const uint64_t scale2 = pair_of(BIAS ? 1.0f : scale_log2), neg_m2 = pair_of(-m_use);
+            const uint64_t scale2 = pair_of(scale_log2), neg_m2 = pair_of(-m_use);
             uint64_t lsum2 = 0ull;
             auto hand_over = [&](int half) {
                 tmem_st_wait();
@@ -691,26 +720,38 @@ __global__ __launch_bounds__(PT_THREADS, 2) void attn_prefill_tc_kernel(
                 __syncwarp();
                 if (lane == 0) bar_arrive(&ctrl->p_full[half]);
             };
-            if (need_mask) {
-                exp_of_chunk<true, !BIAS>(s0, 0, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+            if constexpr (BIAS) {
+                uint64_t quads2[2] = {0ull, 0ull};
+                if (need_mask) {
+                    exp_of_chunk_by_quads<true>(s0, 0, kmin, kmax, neg_m2, tmem_p_row, quads2);
+                    hand_over(0);
+                    exp_of_chunk_by_quads<true>(s1, 1, kmin, kmax, neg_m2, tmem_p_row, quads2);
+                } else {
+                    exp_of_chunk_by_quads<false>(s0, 0, kmin, kmax, neg_m2, tmem_p_row, quads2);
+                    hand_over(0);
+                    exp_of_chunk_by_quads<false>(s1, 1, kmin, kmax, neg_m2, tmem_p_row, quads2);
+                }
+                l_run = fmaf(l_run, corr, sum_of_pair(quads2[0]) + sum_of_pair(quads2[1]));
+            } else if (need_mask) {
+                exp_of_chunk<true>(s0, 0, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 if constexpr (TN == 64) hand_over(0);
-                exp_of_chunk<true, !BIAS>(s1, 1, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                exp_of_chunk<true>(s1, 1, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 if constexpr (TN > 64) {
                     hand_over(0);
-                    exp_of_chunk<true, !BIAS>(s2, 2, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
-                    exp_of_chunk<true, !BIAS>(s3, 3, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                    exp_of_chunk<true>(s2, 2, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                    exp_of_chunk<true>(s3, 3, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 }
             } else {
-                exp_of_chunk<false, !BIAS>(s0, 0, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                exp_of_chunk<false>(s0, 0, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 if constexpr (TN == 64) hand_over(0);
-                exp_of_chunk<false, !BIAS>(s1, 1, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                exp_of_chunk<false>(s1, 1, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 if constexpr (TN > 64) {
                     hand_over(0);
-                    exp_of_chunk<false, !BIAS>(s2, 2, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
-                    exp_of_chunk<false, !BIAS>(s3, 3, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                    exp_of_chunk<false>(s2, 2, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
+                    exp_of_chunk<false>(s3, 3, kmin, kmax, scale2, neg_m2, tmem_p_row, lsum2);
                 }
             }
-            l_run += sum_of_pair(lsum2);
+            if (!BIAS) l_run += sum_of_pair(lsum2);
             hand_over(1);
         }
         if (n_blk > 0) {
