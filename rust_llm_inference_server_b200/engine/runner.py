@@ -10,7 +10,6 @@ of all index arrays per step.
 
 from __future__ import annotations
 
-import bisect
 import gc
 from dataclasses import dataclass, field
 
@@ -41,17 +40,6 @@ def _align4(n: int) -> int:
     return (n + 3) & ~3
 
 
-def tiles_of_portions(lens: list, starts: list, tile, splits=()) -> tuple:
-    """The tiles (batch entry, first token) of the portions of more than one token, and how many of them belong to portions whose context (cached tokens
-    and their own) is longer than each of `splits` (ascending): those come first, whatever else is in the batch."""
-    tiles = [(b, t0) for b, n in enumerate(lens) if n > 1 for t0 in range(0, n, tile)] if tile else []
-    passed = [bisect.bisect_left(splits, s + n) for s, n in zip(starts, lens)]
-    # of those on one side the tiles with the most keys to read first: the GPU hands out CTAs in this order, and the
-    # long ones must not be the last to start
-    tiles.sort(key=lambda bt: (-passed[bt[0]], -(starts[bt[0]] + bt[1])))
-    return tiles, {at: sum(passed[b] > i for b, _ in tiles) for i, at in enumerate(splits)}
-
-
 class StepContext:
     """Index arrays of one step on the device, and the step's scratch buffers."""
 
@@ -79,7 +67,7 @@ class StepContext:
         self.n_prefill_tokens = 0
         self.prefill_rows = None                  # int32: rows of the tokens of longer entries
         self.n_prefill_tiles = 0
-        self.tiles_beyond = {}                    # by context length: how many of the tiles, the first ones, are of portions with a longer context
+        self.max_prefill_ctx = 0                  # the longest context among those portions (host)
         self.prefill_tiles = None                 # int32 [tiles, 2]: (batch entry, first token of the tile)
         self.n_wanted = 0                         # rows whose logits are asked for
         self.wants_every_row = False              # ... and they are all the step's rows, in order
@@ -120,7 +108,6 @@ class ModelRunner:
         self._caches = [storage.layer_cache(c) for c in range(len(model.cache_slot_specs))]
         # tokens of a portion that one CTA of the mixers' prompt kernels takes (None: no tile list)
         self.prefill_tile = model.prefill_tile
-        self.prefill_splits = model.prefill_splits
         self._states = storage.states
         self._ws: dict[str, torch.Tensor] = {}
         self._meta_host = None
@@ -226,7 +213,11 @@ class ModelRunner:
                 pf_rows.extend(range(k, k + n))
             k += n
         Bd, Tp = len(dec_rows), len(pf_rows)
-        pf_tiles, tiles_beyond = tiles_of_portions(lens, starts, self.prefill_tile, self.prefill_splits)
+        pf_tiles = [(b, t0) for b, n in enumerate(lens) if n > 1 for t0 in range(0, n, self.prefill_tile)] \
+            if self.prefill_tile else []
+        # the tiles with the most keys to read first: the GPU hands out CTAs in this order, and the
+        # long ones must not be the last to start
+        pf_tiles.sort(key=lambda bt: -(starts[bt[0]] + bt[1]))
         Nt = len(pf_tiles)
         o_dr = o_rows + _align4(max(W, 1))
         o_ds = o_dr + _align4(max(Bd, 1))
@@ -282,7 +273,7 @@ class ModelRunner:
         st.n_decode = Bd
         st.n_prefill_tokens = Tp
         st.n_prefill_tiles = Nt
-        st.tiles_beyond = tiles_beyond
+        st.max_prefill_ctx = max((s + n for s, n in zip(starts, lens) if n > 1), default=0)
         if Bd:
             st.decode_ctxs = [starts[b] + 1 for b in dec_seqs]
             st.max_decode_ctx = max(st.decode_ctxs)

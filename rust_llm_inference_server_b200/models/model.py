@@ -13,7 +13,7 @@ from .. import ops
 from ..ops import ScaledRows
 from ..config.registry import lookup_architecture
 from ..parts.block import StreamJoin
-from ..parts.base import Part, build_block, build_embedding, build_lm_head, build_norm, prefill_splits
+from ..parts.base import Part, build_block, build_embedding, build_lm_head, build_norm
 from ..parts.spec import EmbeddingSpec, LMHeadSpec, ModelSpec
 from ..weights.loader import PlacedSource, check_checkpoint
 from ..weights.safetensors_io import Checkpoint, open_model_dir
@@ -75,11 +75,6 @@ class Model:
         if len(tiles) > 1:
             raise ValueError(f"the mixers ask for prompt tiles of different sizes: {sorted(tiles)}")
         return tiles.pop() if tiles else None
-
-    @property
-    def prefill_splits(self):
-        """The context lengths by which the mixers' kernels tell portions of prompts apart, ascending."""
-        return prefill_splits(blk.mixer for blk in self.blocks)
 
     def parts(self):
         """Every part of the model, ends included."""

@@ -1928,32 +1928,21 @@ def _biased_tc_sizes(n_heads: int, n_kv_heads: int, dim: int, v_dim: int, page_s
     return bool(lib().rlis_attention_bias_prefill_tc_takes(n_heads, n_kv_heads, dim, v_dim, page_size, n_dist))
 
 
-# The longest context of a portion (cached tokens and its own) up to which it stays on mma.sync, by head size: a short one is all latency, of which the tcgen05
-# kernel has more.  us on tcgen05 and mma.sync, 32 heads of 64, a table and gates / a window and sinks: 64 tokens 6.5 and 5.3 / 6.2 and 4.7, 128 7.8 and 7.4 / 7.5 and 6.6,
-# 192 8.7 and 9.6 / 9.0 and 8.9, 256 9.4 and 11.2 / 10.6 and 10.6, 448 13.0 and 17.7 / 15.0 and 18.4; 16 heads of 128: 64 7.6 and 7.5 / 7.1 and 6.9, 96 8.4 and 10.2 / 8.3 and
-# 9.5.  Portions on both sides in one step are a launch each, one after the other: 100 and 500 tokens 20 us, both on mma.sync 18, both on tcgen05 14 (16 heads of 64).
+# The longest context of a step's portions (cached tokens and their own; single tokens beside them have a kernel of their own) up to which they stay on mma.sync, by
+# head size: a short one is all latency, of which the tcgen05 kernel has more.  us on tcgen05 and mma.sync, 32 heads of 64, a table and gates / a window and
+# sinks: 64 tokens 6.5 and 5.3 / 6.2 and 4.7, 128 7.8 and 7.4 / 7.5 and 6.6, 192 8.7 and 9.6 / 9.0 and 8.9, 256 9.4 and 11.2 / 10.6 and 10.6, 448 13.0 and 17.7 / 15.0 and
+# 18.4; 16 heads of 128: 64 7.6 and 7.5 / 7.1 and 6.9, 96 8.4 and 10.2 / 8.3 and 9.5.  Prompts of 100 and 500 tokens: 14 on tcgen05, 18 on mma.sync, 20 with a launch of
+# each (16 heads of 64).
 BIASED_TC_AFTER = {64: 128, 128: 64}
 
 
 def _biased_prefill_tc(q, k_cache, v_cache, out, bias, gate, gate_cols: int, slopes, n_heads: int, n_kv_heads: int, dim: int, v_dim: int, page_size: int,
                        max_ctx: int = 1 << 30) -> bool:
-    """Whether portions of prompts with these operands, up to `max_ctx` tokens of context, go to the tcgen05 kernel
-    (csrc/kernels/attention_prefill_tcgen05.cu)."""
+    """Whether portions of prompts with these operands, the longest of `max_ctx` tokens with those cached before it, go to the tcgen05 kernel
+    (csrc/kernels/attention_prefill_tcgen05.cu).  The bits are the same on either."""
     return (max_ctx > BIASED_TC_AFTER.get(dim, 1 << 30) and slopes is None and (gate is None or gate_cols == 1) and k_cache.shape[0] * n_kv_heads * page_size < 1 << 31
             and (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr() | out.data_ptr()) % 16 == 0
             and _biased_tc_sizes(n_heads, n_kv_heads, dim, v_dim, page_size, 0 if bias is None else bias.shape[0]))
-
-
-def _biased_tc_tiles(step, n_tiles: int, dim: int) -> int:
-    """How many of a step's tiles, the first ones, are of portions whose contexts are long enough for the tcgen05 kernel.  Each portion is judged by itself: a
-    request gets the same kernel alone and beside others."""
-    after = BIASED_TC_AFTER.get(dim)
-    if after is None:
-        return 0
-    beyond = getattr(step, "tiles_beyond", {}).get(after)
-    if beyond is not None:
-        return beyond
-    return n_tiles if getattr(step, "max_ctx_len", 1 << 30) > after else 0          # (a step without counts: by its longest context)
 
 
 def attention_biased(q, k_cache, v_cache, out, bias, gate, step, group: int, n_heads: int, n_kv_heads: int,
@@ -2004,20 +1993,18 @@ def attention_biased(q, k_cache, v_cache, out, bias, gate, step, group: int, n_h
             step.dec_seqs.data_ptr(), step.ctx_lens.data_ptr(), tables.data_ptr(), tables.shape[1], n_dec, n_heads,
             n_kv_heads, dim, v_dim, page_size, float(scale), int(window), pieces, sp, lp, gc, _stream()), "attention_bias_decode")
         _count("attention_bias.decode.mma" + (".split" if pieces > 1 else ""))
-    n_long = _biased_tc_tiles(step, n_tiles, dim) if n_tiles else 0
-    if n_long and _biased_prefill_tc(q, k_cache, v_cache, out, bias, gate, gc, slopes, n_heads, n_kv_heads, dim, v_dim, page_size):
+    if n_tiles and _biased_prefill_tc(q, k_cache, v_cache, out, bias, gate, gc, slopes, n_heads, n_kv_heads, dim, v_dim, page_size,
+                                      getattr(step, "max_prefill_ctx", 1 << 30)):
         check(lib().rlis_attention_bias_prefill_tc(
-            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), bp, n_dist, gp, gs, step.prefill_tiles.data_ptr(), n_long,
+            q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), bp, n_dist, gp, gs, step.prefill_tiles.data_ptr(), n_tiles,
             step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(), tables.data_ptr(), tables.shape[1], T, k_cache.shape[0], n_heads, n_kv_heads, dim,
             page_size, float(scale), int(window), sp, _stream()), "attention_bias_prefill_tc")
         _count("attention_bias.prefill.mma")
         launches_by_kernel["attention_bias.prefill.mma.tcgen05"] = launches_by_kernel.get("attention_bias.prefill.mma.tcgen05", 0) + 1
-    else:
-        n_long = 0
-    if n_tiles > n_long:
+    elif n_tiles:
         check(lib().rlis_attention_bias_prefill(
             q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), bp, n_dist, gp, gs,
-            step.prefill_tiles[n_long:].data_ptr(), n_tiles - n_long, step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(),
+            step.prefill_tiles.data_ptr(), n_tiles, step.cu_seqlens.data_ptr(), step.ctx_lens.data_ptr(),
             tables.data_ptr(), tables.shape[1], n_heads, n_kv_heads, dim, v_dim, page_size, float(scale), int(window),
             sp, lp, gc, _stream()), "attention_bias_prefill")
         _count("attention_bias.prefill.mma")

@@ -104,16 +104,6 @@ class LogitsHead(Part):
         raise NotImplementedError
 
 
-def prefill_splits(mixers) -> tuple:
-    """What the mixers ask for by `prefill_split`, ascending, each length once."""
-    asked = set()
-    for m in mixers:
-        asked.update(getattr(m, "prefill_splits", ()))
-        if getattr(m, "prefill_split", None) is not None:
-            asked.add(m.prefill_split)
-    return tuple(sorted(asked))
-
-
 class Mixer(Part):
     """Token mixing over a request's earlier tokens.  `forward` gets the normed activations
     [T, hidden] of all tokens of the step and returns [T, hidden] in the same element type."""
@@ -122,9 +112,6 @@ class Mixer(Part):
     # function then lists every portion of the step in tiles of that many tokens
     # (`step.prefill_tiles`).  None: the mixer needs no such list.
     prefill_tile: Optional[int] = None
-    # The longest context (cached tokens and the portion's own) with which a portion goes to another kernel than longer ones do: the step function lists
-    # the tiles of the portions beyond it first and counts them (`step.tiles_beyond`).  None: one kernel takes them all.
-    prefill_split: Optional[int] = None
 
     def cache_spec(self) -> Optional[KVCacheSpec]:
         return None

@@ -185,11 +185,6 @@ class BiasedAttention(Mixer):
     def prefill_tile(self):
         return ops.prefill_tile() if self._fast() else None
 
-    @property
-    def prefill_split(self):
-        s = self.spec
-        return ops.BIASED_TC_AFTER.get(s.dim) if self._fast() and s.v_dim == s.dim else None
-
     def launch_variant(self, step):
         if not step.n_decode or not self._fast():
             return None

@@ -6,7 +6,7 @@ import numpy as np
 
 from .. import ops
 from ..ops.profile import span
-from .base import Mixer, Part, build_mixer, prefill_splits, register_mixer
+from .base import Mixer, Part, build_mixer, register_mixer
 
 
 class ParallelMixer(Mixer):
@@ -60,10 +60,6 @@ class ParallelMixer(Mixer):
         if len(tiles) > 1:
             raise ValueError(f"the branches ask for prompt tiles of different sizes: {sorted(tiles)}")
         return tiles.pop() if tiles else None
-
-    @property
-    def prefill_splits(self):
-        return prefill_splits(self.branches)
 
     def launch_variant(self, step):
         return tuple(b.launch_variant(step) if getattr(type(b), "launch_variant", Part.launch_variant)

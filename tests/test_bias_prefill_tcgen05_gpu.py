@@ -121,10 +121,10 @@ def test_edges_come_out_as_with_the_other_kernel(monkeypatch, d):
     ops.check_device_errors()
 
 
-def test_a_portion_takes_its_kernel_whatever_is_beside_it():
-    """A short portion beside a long one and beside a single token of a long context: each the kernel, and the bits, that it has alone."""
+def test_a_portion_has_its_bits_whatever_is_beside_it():
+    """A short portion beside a long one and beside a single token of a long context: the bits that it has alone, and one launch for all portions, which
+    the portions choose and not the single token."""
     from rust_llm_inference_server_b200 import ops
-    from rust_llm_inference_server_b200.engine.runner import tiles_of_portions
     rng = torch.Generator().manual_seed(3)
     rnd = lambda *s: torch.randn(*s, generator=rng)
     d, nkv, nh, page, keys = 64, 2, 8, 16, ("attention_bias.prefill.mma.tcgen05", "attention_bias.prefill.mma")
@@ -139,11 +139,12 @@ def test_a_portion_takes_its_kernel_whatever_is_beside_it():
         dev = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
         part.n_seqs, part.block_tables, part.ctx_lens = len(rows), [st.block_tables[0][rows].contiguous()], dev([x + y for x, y in zip(n, c)])
         part.cu_seqlens = dev([0] + torch.tensor(n).cumsum(0).tolist())
-        tiles, part.tiles_beyond = tiles_of_portions(n, c, 64, (ops.BIASED_TC_AFTER[d],))
+        tiles = [(b, t) for b, x in enumerate(n) if x > 1 for t in range(0, x, 64)]
         part.prefill_tiles, part.n_prefill_tiles = dev(tiles), len(tiles)
         dec = [b for b, x in enumerate(n) if x == 1]
         part.n_decode, part.dec_rows, part.dec_seqs = len(dec), dev([sum(n[:b]) for b in dec]), dev(dec)
         part.max_ctx_len, part.max_decode_ctx = max(x + y for x, y in zip(n, c)), 901
+        part.max_prefill_ctx = max(x + y for x, y in zip(n, c) if x > 1)
         part.buffer = lambda name, shape, dtype: torch.empty(shape, dtype=dtype, device="cuda")
         at = [sum(lens[:b]) for b in range(3)]
         x = torch.cat([q[at[b]:at[b] + lens[b]] for b in rows])
@@ -153,7 +154,7 @@ def test_a_portion_takes_its_kernel_whatever_is_beside_it():
         return out.split(n), (tc, all_ - tc)
 
     (short,), (long,) = (run([b])[0] for b in (0, 1))
-    assert run([0])[1] == (0, 1) and run([1])[1] == (1, 0) and run([0, 2])[1] == (0, 1) and run([0, 1, 2])[1] == (1, 1)
+    assert run([0])[1] == (0, 1) and run([1])[1] == (1, 0) and run([0, 2])[1] == (0, 1) and run([0, 1, 2])[1] == (1, 0)
     both = run([0, 1, 2])[0]
     assert torch.equal(both[0], short) and torch.equal(both[1], long) and torch.equal(run([0, 2])[0][0], short)
     ops.check_device_errors()

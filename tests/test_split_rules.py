@@ -109,19 +109,3 @@ def test_the_delta_rule_by_64_tokens_is_taken_where_it_is_faster(heads, lens, si
     before = sixteen if by_sixteen else single
     took = wide if ops._gated_delta_wide_pays(sum(lens), len(lens), max(lens), heads * 128, 148, by_sixteen) else before
     assert took <= before and took <= 1.05 * min(before, wide)
-
-
-def test_portions_are_told_apart_by_their_own_contexts():
-    """Tiles of portions beyond a context length come first and are counted, whatever single tokens or other portions the step holds."""
-    from rust_llm_inference_server_b200.engine.runner import tiles_of_portions
-    lens, starts = [1, 130, 500, 64, 70], [4000, 0, 0, 400, 250]
-    tiles, beyond = tiles_of_portions(lens, starts, 64, (96, 320))
-    assert sorted(tiles) == [(b, t) for b in (1, 2, 3, 4) for t in range(0, lens[b], 64)]
-    assert beyond == {96: len(tiles), 320: 9} and {b for b, _ in tiles[:9]} == {2, 3} and {b for b, _ in tiles[9:]} == {1, 4}
-    ends = [starts[b] + t for b, t in tiles]
-    assert ends[:9] == sorted(ends[:9], reverse=True) and ends[9:] == sorted(ends[9:], reverse=True)
-    alone = tiles_of_portions([130], [0], 64, (96, 320))
-    assert alone == ([(0, 128), (0, 64), (0, 0)], {96: 3, 320: 0})
-    plain, none = tiles_of_portions(lens, starts, 64)          # kernels that ask for nothing: the most keys first
-    assert none == {} and [starts[b] + t for b, t in plain] == sorted((starts[b] + t for b, t in plain), reverse=True)
-    assert tiles_of_portions(lens, starts, None, (96,)) == ([], {96: 0}) and tiles_of_portions([1, 1], [5, 900], 64, (320,)) == ([], {320: 0})
