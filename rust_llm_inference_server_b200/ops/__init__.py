@@ -201,12 +201,17 @@ def _gemm_f32_splits(a: torch.Tensor, w: torch.Tensor) -> bool:
     return K >= SPLIT_MIN_K and K % 4 == 0 and apart and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
 
 
+@functools.lru_cache(maxsize=None)
+def _gemm_f32_split_sizes(K: int) -> tuple:
+    """Rows up to which the kernel of few rows takes a product, and bytes of scratch a row of the other."""
+    return lib().rlis_gemm_f32_split_few_rows(), lib().rlis_gemm_f32_split_row_bytes(K)
+
+
 def _gemm_f32_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, early: bool = False) -> torch.Tensor:
     """The product of `gemm_f32` on the tensor cores; rows of a and out may lie in wider ones.  `early`: w is a weight, whose first tiles may be read
     before the kernels before have finished, as `stream_gemm` does."""
     (M, K), N = a.shape, w.shape[0]
-    few = lib().rlis_gemm_f32_split_few_rows()
-    row_bytes = lib().rlis_gemm_f32_split_row_bytes(K)
+    few, row_bytes = _gemm_f32_split_sizes(K)
     rows = M if M <= few else max(few + 1, _SPLIT_PLANES // row_bytes)
     planes = torch.empty((min(M, rows) * row_bytes,), dtype=torch.uint8, device=a.device) if M > few else None
     for m in range(0, M, max(1, rows)):
@@ -217,10 +222,10 @@ def _gemm_f32_split(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, early: 
     return out
 
 
-def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, *, early: bool = False) -> torch.Tensor:
     """out[M, N] = a[M, K] @ w[N, K]^T in true float32: rows of `SPLIT_MIN_K` and more on the tensor cores, every operand as the sum of three bfloat16
-    numbers (`csrc/kernels/gemm_f32_split.cu`: what is left out, and which results go back to a chain), others as chains of FMAs in the order of k.  A row has the same bits whatever other
-    rows there are."""
+    numbers (`csrc/kernels/gemm_f32_split.cu`: what is left out, and which results go back to a chain), others as chains of FMAs in the order of k.  A row has
+    the same bits whatever other rows there are.  `early`: see `linear`."""
     M, K = a.shape
     N = w.shape[0]
     _req(a, "a", torch.float32)
@@ -229,7 +234,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) 
         out = torch.empty((M, N), dtype=torch.float32, device=a.device)
     _req(out, "out", torch.float32, (M, N))
     if _gemm_f32_splits(a, w):
-        return _gemm_f32_split(a, w, out)
+        return _gemm_f32_split(a, w, out, early)
     check(lib().rlis_gemm_f32_nt(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, _stream()),
           "gemm_f32")
     _count("gemm_f32")
@@ -1399,17 +1404,11 @@ def linear(x, w: torch.Tensor, out_dtype=None, sink=None, bias: torch.Tensor | N
     if bias is not None:
         raise KernelError("linear: a bias is taken with a sink")
     if x.dtype == torch.float32:
-        if x.dim() == 2 and x.is_contiguous():
-            _req(x, "x", torch.float32)
-            _req(w, "w", torch.float32, (None, x.shape[1]))
-            if not _gemm_f32_splits(x, w):
-                return gemm_f32(x, w)
-            return _gemm_f32_split(x, w, torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device), early)
         if not x.is_contiguous() and x.dim() == 2 and x.stride(1) == 1:
             out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=x.device)
             gemm_f32_batched(x.unsqueeze(1), w.unsqueeze(0), out.unsqueeze(1))
             return out
-        return gemm_f32(x, w)
+        return gemm_f32(x, w, early=early)
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise KernelError(f"linear: expected matching float32 or bfloat16 operands, got {x.dtype}, {w.dtype}")
     if not x.is_cuda:
