@@ -10,8 +10,8 @@
 // Off float64 by 2.5e-7 of the result at K 2048 and 8192 (normal numbers), where one chain of K FMAs is 8e-7 and 1.6e-6.  The segments and the order in
 // them are the same in both kernels below and for any number of rows, so a row's result does not depend on what else is in the batch.
 // Below 2^-110 (2^-102 where subnormal operands count as zeros) the third part has bits under the smallest bf16.  So the largest magnitude of every row of A
-// and of W is taken along, and an output that what is lost could reach, that is, one below K (x_max + w_max + 8) 2^-100, is worked out again as a chain of FMAs
-// from the float32 operands; so is one that is not finite (infinities and NaN, and numbers that round to infinity in 8 bits, come out as that chain gives them).
+// and of W is taken along, and an output that what is lost could reach, that is, one whose terms' magnitudes come to less than K (x_max + w_max + 8) 2^-100, is
+// worked out again as a chain of FMAs from the float32 operands; so is one that is not finite (infinities and NaN, and numbers that round to infinity in 8 bits, come out as that chain gives them).
 //
 // W is the M side of the instruction (128 features a tile), split on the way: TMA brings 128 x 32 floats, warps turn a row of 32 into three
 // planes of bf16 and put them into tensor memory as the A operand.  The rows of A are the N side, from shared memory in three planes.
@@ -162,9 +162,25 @@ __device__ __noinline__ float magnitude_below(const float* __restrict__ row, int
     return bits << 1 ? magnitude(1) : 0.f;
 }
 // An output that is not finite, or so small that the parts' sums may have lost some of it, as a chain of FMAs (`x`, `w`: the largest magnitudes of
-// the two rows, whatever else the tile holds).
+// the two rows, whatever else the tile holds).  One that came out small because its terms cancel has lost nothing beside its rounding and stays (of
+// ordinary rows one in four million is exactly zero).
 __device__ __noinline__ float chain(const float* __restrict__ a, const float* __restrict__ b, int K, float v, float x, float w, float lost) {
-    if (fabsf(v) <= FLT_MAX && (x == 0.f || w == 0.f || fabsf(v) >= lost * (x + w + 8.f))) return v;
+    const float least = lost * (x + w + 8.f);
+    if (fabsf(v) <= FLT_MAX) {
+        if (x == 0.f || w == 0.f || fabsf(v) >= least) return v;
+        float terms[4] = {};
+        int k = 0;
+#pragma unroll 8
+        for (; k + 3 < K; k += 4) {
+            const float4 p = *reinterpret_cast<const float4*>(a + k), q = *reinterpret_cast<const float4*>(b + k);
+            terms[0] = fmaf(fabsf(p.x), fabsf(q.x), terms[0]);
+            terms[1] = fmaf(fabsf(p.y), fabsf(q.y), terms[1]);
+            terms[2] = fmaf(fabsf(p.z), fabsf(q.z), terms[2]);
+            terms[3] = fmaf(fabsf(p.w), fabsf(q.w), terms[3]);
+        }
+        for (; k < K; ++k) terms[0] = fmaf(fabsf(a[k]), fabsf(b[k]), terms[0]);
+        if ((terms[0] + terms[1]) + (terms[2] + terms[3]) >= least) return v;
+    }
     float acc = 0.f;
     for (int k = 0; k < K; ++k) acc = fmaf(a[k], b[k], acc);
     return acc;

@@ -183,3 +183,12 @@ def test_what_a_product_refuses():
             ops.linear(a, bad)
     with pytest.raises(ops.KernelError):
         ops.linear(a.cpu(), w)
+
+
+@pytest.mark.parametrize("M", [4, 40])
+def test_sums_that_cancel_are_not_small_numbers(M):
+    """Terms that cancel exactly leave the zero that the segments' sums have, not the rounding of a chain."""
+    a, w = operands(M, 200, 2048)
+    w[:, 256:512], a[:, 256:512] = w[:, :256], -a[:, :256]              # a segment and its negative, term by term
+    a[:, 512:] = 0.0
+    assert not bool(product(a, w).any())
